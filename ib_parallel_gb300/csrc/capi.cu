@@ -794,7 +794,7 @@ int ib_get_launch_shapes(IbCtx* h, int* shapes) {
   for (const ib::DstLaunch* L : {&c->lx, &c->lx_small, &c->lx_batch, &c->ly_none}) {
     shapes[i++] = L->B;
     shapes[i++] = L->NT;
-    shapes[i++] = L->narrow_scan;
+    shapes[i++] = 0;   // the prefix scan has one form
   }
   shapes[i] = c->tl.Mb;
   return IB_OK;

@@ -5,34 +5,11 @@
 #include <cmath>
 #include <vector>
 
+
 namespace ib {
 
 // ---------------------------------------------------------------- tables
-// exp(-2 pi i num/den) evaluated in long double and rounded to double.
-static double2 twiddle(long long num, long long den) {
-  const long double PI_L = 3.141592653589793238462643383279502884L;
-  long long r = num % den;
-  if (r < 0) r += den;
-  long double a = 2.0L * PI_L * (long double)r / (long double)den;
-  return make_double2((double)cosl(a), (double)(-sinl(a)));
-}
-
-static bool factor_radices(int P, int* rad, int* nrad);
-
-// The Stockham stages' twiddles, stage by stage: the stage of span Ns (the product of the earlier
-// radices) and radix R uses w^(r k P/(Ns R)), r = 1..R-1, k = 0..Ns-1, stored at
-// Ns - 1 + (r-1) Ns + k, so that a warp's lanes (consecutive k) read consecutive entries.  The
-// stages' blocks [Ns - 1, R Ns - 1) tile [0, P - 1).
-static void stage_twiddles(int P, const int* rad, int nrad, std::vector<double2>& tw) {
-  tw.assign(P, make_double2(1.0, 0.0));
-  int Ns = 1;
-  for (int s = 0; s < nrad; ++s) {
-    const int R = rad[s], step = P / (Ns * R);
-    for (int r = 1; r < R; ++r)
-      for (int k = 0; k < Ns; ++k) tw[Ns - 1 + (r - 1) * Ns + k] = twiddle((long long)r * k * step, P);
-    Ns *= R;
-  }
-}
+static const long double PI_L = 3.141592653589793238462643383279502884L;
 
 static bool factor_radices(int P, int* rad, int* nrad) {
   // radix-5 and radix-3 stages first (no twiddles in the first stage), then 4, then 2.
@@ -46,71 +23,100 @@ static bool factor_radices(int P, int* rad, int* nrad) {
   return true;
 }
 
-int dst_plan_create(DstPlan* p, int N) {
-  int M = N + 1;
+// The factors of a plan, in the order they lie in device memory: of P stage twiddles c + i d and then
+// of the P/2 factors exp(-2 pi i k/M), the pairs (c, d - c); of both, the third factors c + d; P of
+// 2 sin(j pi/M); and P + 1 doubles sin(j pi/M).
+//
+// The Stockham stages' twiddles lie stage by stage: the stage of span Ns (the product of the earlier
+// radices) and radix R uses w^(r k P/(Ns R)), r = 1..R-1, k = 0..Ns-1, at Ns - 1 + (r-1) Ns + k, so
+// that a warp's lanes (consecutive k) read consecutive entries.  The stages' blocks
+// [Ns - 1, R Ns - 1) tile [0, P - 1).
+static void plan_tables(const DstPlan& p, std::vector<double>& out) {
+  const int P = p.P, H = p.P / 2;
+  out.assign(dst_plan_doubles(p.M), 0.0);
+  FxW* pair = reinterpret_cast<FxW*>(out.data());
+  FxW* third = pair + 2 * (P + H);
+  auto put = [&](int i, long long num, long long den) {
+    const long double a = 2.0L * PI_L * (long double)(num % den) / (long double)den;
+    const long double x = cosl(a), y = -sinl(a);
+    pair[2 * i] = fx_factor(x);
+    pair[2 * i + 1] = fx_factor(y - x);
+    third[i] = fx_factor(x + y);
+  };
+  int Ns = 1;
+  for (int s = 0; s < p.nrad; ++s) {
+    const int R = p.rad[s], step = P / (Ns * R);
+    for (int r = 1; r < R; ++r)
+      for (int k = 0; k < Ns; ++k) put(Ns - 1 + (r - 1) * Ns + k, (long long)r * k * step, P);
+    Ns *= R;
+  }
+  for (int k = 0; k < H; ++k) put(P + k, k, p.M);
+  FxW* f = third + P + H;
+  for (int j = 0; j < P; ++j) f[j] = fx_factor(2.0L * sinl(PI_L * (long double)j / (long double)p.M));
+  double* sn = reinterpret_cast<double*>(f + P);
+  for (int j = 0; j <= P; ++j) sn[j] = (double)sinl(PI_L * (long double)j / (long double)p.M);
+}
+
+static int plan_init(DstPlan* p, int N) {
+  const int M = N + 1;
   if (N < 3 || M % 4 != 0) return IB_ERR_ARG;
   p->N = N; p->M = M; p->P = M / 2;
-  if (!factor_radices(p->P, p->rad, &p->nrad)) return IB_ERR_ARG;
-  std::vector<double2> tw, uw(p->P / 2);
-  std::vector<double> sn(p->P + 1);
-  stage_twiddles(p->P, p->rad, p->nrad, tw);
-  for (int k = 0; k < p->P / 2; ++k) uw[k] = twiddle(k, M);
-  const long double PI_L = 3.141592653589793238462643383279502884L;
-  for (int j = 0; j <= p->P; ++j) sn[j] = (double)sinl(PI_L * (long double)j / (long double)M);
-  if (cudaMalloc(&p->tw, sizeof(double2) * p->P) != cudaSuccess) return IB_ERR_NOMEM;
-  if (cudaMalloc(&p->uw, sizeof(double2) * (p->P / 2)) != cudaSuccess) return IB_ERR_NOMEM;
-  if (cudaMalloc(&p->sn, sizeof(double) * (p->P + 1)) != cudaSuccess) return IB_ERR_NOMEM;
-  IB_CUDA_CHECK(cudaMemcpy(p->tw, tw.data(), sizeof(double2) * p->P, cudaMemcpyHostToDevice));
-  IB_CUDA_CHECK(cudaMemcpy(p->uw, uw.data(), sizeof(double2) * (p->P / 2), cudaMemcpyHostToDevice));
-  IB_CUDA_CHECK(cudaMemcpy(p->sn, sn.data(), sizeof(double) * (p->P + 1), cudaMemcpyHostToDevice));
+  return factor_radices(p->P, p->rad, &p->nrad) ? IB_OK : IB_ERR_ARG;
+}
+
+static void plan_pointers(DstPlan* p, double* dev) {
+  const size_t n = (size_t)p->P + p->P / 2;
+  p->tw = reinterpret_cast<FxW*>(dev);
+  p->tw3 = p->tw + 2 * n;
+  p->sx = p->tw3 + n;
+  p->sn = reinterpret_cast<double*>(p->sx + p->P);
+}
+
+size_t dst_plan_doubles(int M) {
+  const size_t P = M / 2;
+  return 3 * P + 3 * (P / 2) + P + P + 1;
+}
+
+int dst_plan_create(DstPlan* p, int N) {
+  int rc = plan_init(p, N);
+  if (rc != IB_OK) return rc;
+  std::vector<double> h;
+  plan_tables(*p, h);
+  double* dev = nullptr;
+  if (cudaMalloc(&dev, sizeof(double) * h.size()) != cudaSuccess) return IB_ERR_NOMEM;
+  plan_pointers(p, dev);
+  IB_CUDA_CHECK(cudaMemcpy(dev, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice));
   return IB_OK;
 }
 
 size_t dst_plan_table_doubles(int N) {
-  int M = N + 1;
-  if (N < 3 || M % 4 != 0) return 0;
-  int rad[kMaxRadices], nrad = 0;
-  if (!factor_radices(M / 2, rad, &nrad)) return 0;
-  int P = M / 2;
-  return 2 * (size_t)P + 2 * (size_t)(P / 2) + (size_t)P + 1 + 4;
+  DstPlan p;
+  return plan_init(&p, N) == IB_OK ? dst_plan_doubles(p.M) : 0;
 }
 
 int dst_plan_init_external(DstPlan* p, int N, double* dev, cudaStream_t st) {
-  int M = N + 1;
-  if (dst_plan_table_doubles(N) == 0) return IB_ERR_ARG;
-  p->N = N; p->M = M; p->P = M / 2;
-  if (!factor_radices(p->P, p->rad, &p->nrad)) return IB_ERR_ARG;
-  std::vector<double2> tw, uw(p->P / 2);
-  std::vector<double> sn(p->P + 1);
-  stage_twiddles(p->P, p->rad, p->nrad, tw);
-  for (int k = 0; k < p->P / 2; ++k) uw[k] = twiddle(k, M);
-  const long double PI_L = 3.141592653589793238462643383279502884L;
-  for (int j = 0; j <= p->P; ++j) sn[j] = (double)sinl(PI_L * (long double)j / (long double)M);
-  p->tw = reinterpret_cast<double2*>(dev);
-  p->uw = p->tw + p->P;
-  p->sn = reinterpret_cast<double*>(p->uw + p->P / 2);
-  IB_CUDA_CHECK(cudaMemcpyAsync(p->tw, tw.data(), sizeof(double2) * p->P, cudaMemcpyHostToDevice, st));
-  IB_CUDA_CHECK(cudaMemcpyAsync(p->uw, uw.data(), sizeof(double2) * (p->P / 2), cudaMemcpyHostToDevice, st));
-  IB_CUDA_CHECK(cudaMemcpyAsync(p->sn, sn.data(), sizeof(double) * (p->P + 1), cudaMemcpyHostToDevice, st));
+  int rc = plan_init(p, N);
+  if (rc != IB_OK) return rc;
+  std::vector<double> h;
+  plan_tables(*p, h);
+  plan_pointers(p, dev);
+  IB_CUDA_CHECK(cudaMemcpyAsync(dev, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice, st));
   IB_CUDA_CHECK(cudaStreamSynchronize(st));
   return IB_OK;
 }
 
 void dst_plan_destroy(DstPlan* p) {
   if (p->tw) cudaFree(p->tw);
-  if (p->uw) cudaFree(p->uw);
-  if (p->sn) cudaFree(p->sn);
-  p->tw = p->uw = nullptr; p->sn = nullptr;
+  p->tw = p->tw3 = p->sx = nullptr; p->sn = nullptr;
 }
 
 struct DstDev {
   int N, M, P, nrad;
   int rad[kMaxRadices];
-  FastDiv fd_nb[kMaxRadices];   // butterflies per line of each stage (P/R)
   FastDiv fd_ns[kMaxRadices];   // span of each stage (product of the earlier radices)
-  FastDiv fd_N, fd_P, fd_H;     // line length, complex length, half of it
-  const double2* tw;
-  const double2* uw;
+  const int4* tw;   // (c, d - c) of the stages' twiddles, then of the unpacking's factors
+  const int2* tw3;  // c + d of both
+  const int2* sx;
   const double* sn;
 };
 
@@ -121,231 +127,261 @@ static DstDev to_dev(const DstPlan& p) {
   for (int i = 0; i < kMaxRadices; ++i) {
     d.rad[i] = p.rad[i];
     if (i < p.nrad) {
-      d.fd_nb[i] = FastDiv(p.P / p.rad[i]);
       d.fd_ns[i] = FastDiv(Ns);
       Ns *= p.rad[i];
     }
   }
-  d.fd_N = FastDiv(p.N); d.fd_P = FastDiv(p.P); d.fd_H = FastDiv(p.P / 2);
-  d.tw = p.tw; d.uw = p.uw; d.sn = p.sn;
+  d.tw = reinterpret_cast<const int4*>(p.tw);
+  d.tw3 = reinterpret_cast<const int2*>(p.tw3);
+  d.sx = reinterpret_cast<const int2*>(p.sx);
+  d.sn = p.sn;
   return d;
 }
 
 // ------------------------------------------------------- device helpers
-__device__ __forceinline__ double2 cmul(double2 a, double2 w) {
-  return make_double2(fma(a.x, w.x, -a.y * w.y), fma(a.x, w.y, a.y * w.x));
+__device__ __forceinline__ FxW ld_factor(const int2* __restrict__ p) {
+  const int2 v = __ldg(p);
+  return FxW{v.x, v.y};
 }
-__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 
-template <int R> struct Dft;
-template <> struct Dft<2> {
-  __device__ static void run(double2* v) {
-    double2 a = v[0], b = v[1];
-    v[0] = cadd(a, b); v[1] = csub(a, b);
-  }
-};
-template <> struct Dft<4> {
-  __device__ static void run(double2* v) {
-    double2 s02 = cadd(v[0], v[2]), d02 = csub(v[0], v[2]);
-    double2 s13 = cadd(v[1], v[3]), d13 = csub(v[1], v[3]);
-    v[0] = cadd(s02, s13);
-    v[2] = csub(s02, s13);
-    // y1 = d02 - i d13, y3 = d02 + i d13
-    v[1] = make_double2(d02.x + d13.y, d02.y - d13.x);
-    v[3] = make_double2(d02.x - d13.y, d02.y + d13.x);
-  }
-};
-template <> struct Dft<3> {
-  __device__ static void run(double2* v) {
-    const double h = 0.86602540378443864676;  // sin(2 pi/3)
-    double2 t = cadd(v[1], v[2]);
-    double2 d = csub(v[1], v[2]);
-    double2 a = make_double2(fma(-0.5, t.x, v[0].x), fma(-0.5, t.y, v[0].y));
-    v[0] = cadd(v[0], t);
-    v[1] = make_double2(fma(h, d.y, a.x), fma(-h, d.x, a.y));
-    v[2] = make_double2(fma(-h, d.y, a.x), fma(h, d.x, a.y));
-  }
-};
-template <> struct Dft<5> {
-  __device__ static void run(double2* v) {
-    const double c1 = 0.30901699437494742410;   // cos(2 pi/5)
-    const double c2 = -0.80901699437494742410;  // cos(4 pi/5)
-    const double s1 = 0.95105651629515357212;   // sin(2 pi/5)
-    const double s2 = 0.58778525229247312917;   // sin(4 pi/5)
-    double2 t1 = cadd(v[1], v[4]), t2 = cadd(v[2], v[3]);
-    double2 d1 = csub(v[1], v[4]), d2 = csub(v[2], v[3]);
-    double2 x0 = v[0];
-    double2 a1 = make_double2(fma(c2, t2.x, fma(c1, t1.x, x0.x)), fma(c2, t2.y, fma(c1, t1.y, x0.y)));
-    double2 a2 = make_double2(fma(c1, t2.x, fma(c2, t1.x, x0.x)), fma(c1, t2.y, fma(c2, t1.y, x0.y)));
-    double2 b1 = make_double2(fma(s2, d2.x, s1 * d1.x), fma(s2, d2.y, s1 * d1.y));
-    double2 b2 = make_double2(fma(-s1, d2.x, s2 * d1.x), fma(-s1, d2.y, s2 * d1.y));
-    v[0] = cadd(cadd(x0, t1), t2);
-    v[1] = make_double2(a1.x + b1.y, a1.y - b1.x);
-    v[4] = make_double2(a1.x - b1.y, a1.y + b1.x);
-    v[2] = make_double2(a2.x + b2.y, a2.y - b2.x);
-    v[3] = make_double2(a2.x - b2.y, a2.y + b2.x);
+// v times the complex factor at tw, tw3
+__device__ __forceinline__ FxC twiddle(FxC v, const int4* __restrict__ tw, const int2* __restrict__ tw3) {
+  const int4 a = __ldg(tw);
+  return fx_cmul(v, FxW{a.x, a.y}, FxW{a.z, a.w}, ld_factor(tw3));
+}
+
+// The warps of a CTA over its lines: `wpl` warps per line, `groups` lines at once; thread gt of gsz
+// of its group.  A warp works on one line, so a line's maxima and sums are warp reductions.
+struct LineGroups {
+  int grp, groups, wpl, gw, gt, gsz;
+  __device__ __forceinline__ explicit LineGroups(int B) {
+    const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    wpl = nwarps >= B ? nwarps / B : 1;
+    groups = nwarps >= B ? B : nwarps;
+    grp = warp / wpl;
+    gw = warp - grp * wpl;
+    gt = gw * 32 + (threadIdx.x & 31);
+    gsz = wpl * 32;
+    if (grp >= groups) grp = 1 << 20;   // spare warps: no lines
   }
 };
 
-// One Stockham stage over B lines (line b at in + b*P).
+// One Stockham stage of one line on the gsz threads of its group; the inputs are taken 2^-sh.
 template <int R>
-__device__ __forceinline__ void stockham_stage(const double2* __restrict__ in, double2* __restrict__ out,
-                                               int P, const FastDiv& fnb, const FastDiv& fns,
-                                               const double2* __restrict__ tw, int B, int tid, int NT) {
-  const int nb = fnb.d, Ns = fns.d;
-  const int total = B * nb;
-  const double2* __restrict__ tws = tw + Ns - 1;   // this stage's twiddles (stage_twiddles)
-  for (int it = tid; it < total; it += NT) {
-    int b = fnb.div(it);
-    int j = it - b * nb;
-    const double2* src = in + b * P;
-    double2* dst = out + b * P;
-    int jq = fns.div(j);
-    int k = j - jq * Ns;
-    double2 v[R];
+__device__ __forceinline__ unsigned stockham_stage(const longlong2* __restrict__ in, longlong2* __restrict__ out, int P,
+                                                   const FastDiv& fns, const int4* __restrict__ tw,
+                                                   const int2* __restrict__ tw3, int sh, int gt, int gsz) {
+  const int nb = P / R, Ns = fns.d;
+  FxPeak peak;
+  for (int j = gt; j < nb; j += gsz) {
+    const int jq = fns.div(j);
+    const int k = j - jq * Ns;
+    FxC v[R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = src[j + r * nb];
+    for (int r = 0; r < R; ++r) {
+      const longlong2 z = in[j + r * nb];
+      v[r] = FxC{z.x, z.y};
+    }
+    if (sh) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = FxC{fx_shr(v[r].x, sh), fx_shr(v[r].y, sh)};
+    }
     if (Ns > 1) {
 #pragma unroll
-      for (int r = 1; r < R; ++r) v[r] = cmul(v[r], __ldg(&tws[(r - 1) * Ns + k]));
+      for (int r = 1; r < R; ++r) {
+        const unsigned i = (unsigned)(r * Ns - 1 + k);   // this stage's twiddles (plan_tables)
+        v[r] = twiddle(v[r], tw + i, tw3 + i);
+      }
     }
-    Dft<R>::run(v);
-    int idxD = jq * Ns * R + k;
+    FxDft<R>::run(v);
+    longlong2* dst = out + (jq * Ns * R + k);
 #pragma unroll
-    for (int r = 0; r < R; ++r) dst[idxD + r * Ns] = v[r];
+    for (int r = 0; r < R; ++r) {
+      dst[r * Ns] = make_longlong2(v[r].x, v[r].y);
+      peak.add(v[r].x, v[r].y);
+    }
   }
+  return peak.mag();
 }
 
-// Transform B lines in place: line b holds x_1..x_N at xb[b*ldx + 0..N-1] and
-// receives Y_1..Y_N there.  zA, zB: B*P complex workspace each.
-__device__ void dst_lines(const DstDev& pl, int B, double* xb, int ldx, double2* zA, double2* zB, int narrow_scan) {
-  const int tid = threadIdx.x, NT = blockDim.x;
-  const int P = pl.P, M = pl.M;
-  // --- pre-processing: y (length M, real) written into zA viewed as doubles
-  for (int it = tid; it < B * P; it += NT) {
-    int b = pl.fd_P.div(it);
-    int t = it - b * P;
-    const double* x = xb + b * ldx;
-    double* y = reinterpret_cast<double*>(zA + b * P);
-    if (t == 0) {
-      double xp = x[P - 1];
-      y[0] = 0.0;
-      y[P] = xp + xp;
-    } else {
-      double xj = x[t - 1], xm = x[M - t - 1];
-      double a = xj + xm;
-      double h = 0.5 * (xj - xm);
-      double s = __ldg(&pl.sn[t]);
-      y[t] = fma(s, a, h);
-      y[M - t] = fma(s, a, -h);
+constexpr int kMaxLines = 16;         // lines per CTA
+constexpr int kNotFinite = 1 << 20;   // in place of a line's exponent
+
+// What a CTA keeps of its lines in shared memory while it transforms them.
+struct FxLines {
+  unsigned mag[3][kMaxLines];   // largest magnitudes, three sets in rotation (dst_lines)
+  unsigned l1[kMaxLines];       // a bound of sum |x| / 2^40
+  int e[kMaxLines];             // largest biased exponent of the samples (fx_exponent)
+  int shift[kMaxLines];         // right shifts so far
+  fx wt[32];                    // warp totals of the prefix sums
+  __device__ __forceinline__ void clear(int B) {
+    const int t = threadIdx.x;
+    if (t < B) {
+      mag[0][t] = mag[1][t] = mag[2][t] = 0u;
+      l1[t] = 0u;
+      e[t] = 1;
+      shift[t] = 0;
+    }
+  }
+  // the samples' exponents a warp has met on line b
+  __device__ __forceinline__ void note(int b, int emax) {
+    emax = __reduce_max_sync(0xffffffffu, emax);
+    if ((threadIdx.x & 31) == 0) atomicMax(&e[b], emax);
+  }
+  // what the unpacking shifts by, and the exponent of its results (kNotFinite: a sample was not)
+  __device__ __forceinline__ int last_shift(int b, int w) const {
+    // an odd output is a sum of increments, at most 4 ||x||_1 in these units: it must fit as well
+    return max(fx_shift_for(mag[w][b]), (32 - fx_clz32(l1[b])) + 40 + 2 - shift[b] - 62);
+  }
+  __device__ __forceinline__ int exponent(int b, int sh) const {
+    return e[b] < 2047 ? e[b] - 1075 - (kFxFrac - 53) - 1 + shift[b] + sh : kNotFinite;
+  }
+};
+
+// A result's bits where a line's exponent leaves the normal range or a sample was not finite.
+__device__ __noinline__ long long line_bits(fx v, int E) {
+  return E == kNotFinite ? 0x7ff8000000000000LL : fx_to_bits(v, E);
+}
+
+// Transform B lines: line b holds x_1..x_N as doubles at slots 1..N of its M = 2P slots in zA, its
+// largest exponent noted in S; returns where the lines' Y_1..Y_N lie (zA or zB: line b at b*M, Y_(j+1)
+// at slot dst_slot(j, P)).  zA, zB: B*P complex workspace each.
+//
+// In block fixed point (fixed.cuh).  What bounds it: instruction issue and the latency of the chain of
+// phases, 11,000 warp instructions a line of 799 (the FP64 butterflies before held the FP64 pipe for
+// 600 x 64 cycles).  Measured, before and after: 800 lines of 1599, 80 and 30 us; 2000 lines of 799,
+// 84 and 33 us; 400 lines of 799, 27 and 13 us; 31 lines of 63, 7.5 us either way (latency).
+// Each phase leaves the line's largest magnitude for the next one's shift; the words rotate through
+// three sets so that one is cleared while one is read and one written.
+__device__ double* dst_lines(const DstDev& pl, int B, longlong2* zA, longlong2* zB, FxLines& S) {
+  const int lane = threadIdx.x & 31;
+  const int P = pl.P, M = pl.M, H = P / 2;
+  const LineGroups G(B);
+  // --- pre-processing: 2 y (length M, real), each pair (j, M - j) in its own slots
+  for (int b = G.grp; b < B; b += G.groups) {
+    fx* y = reinterpret_cast<fx*>(zA + b * P);
+    const int emax = S.e[b];
+    FxPeak peak;
+    unsigned l1 = 0;
+    for (int t = G.gt; t < P; t += G.gsz) {
+      if (t == 0) {
+        const fx xp = fx_from_bits(y[P], emax);
+        y[0] = 0;
+        y[P] = 4 * xp;
+        peak.add(4 * xp, 0);
+        l1 += (fx_mag(xp) >> 8) + 1u;
+      } else {
+        const fx xj = fx_from_bits(y[t], emax), xm = fx_from_bits(y[M - t], emax);
+        const fx a = fx_mul(xj + xm, ld_factor(pl.sx + t)), d = xj - xm;
+        y[t] = a + d;
+        y[M - t] = a - d;
+        peak.add(a + d, a - d);
+        l1 += (fx_mag(xj) >> 8) + (fx_mag(xm) >> 8) + 2u;
+      }
+    }
+    const unsigned mag = __reduce_or_sync(0xffffffffu, peak.mag());
+    l1 = __reduce_add_sync(0xffffffffu, l1);
+    if (lane == 0) {
+      atomicOr(&S.mag[0][b], mag);
+      atomicAdd(&S.l1[b], l1);
     }
   }
   __syncthreads();
   // --- complex FFT of length P (Stockham, ping-pong zA <-> zB)
-  double2* cur = zA;
-  double2* nxt = zB;
+  longlong2* cur = zA;
+  longlong2* nxt = zB;
+  int w = 0;   // the set of magnitudes to read
   for (int s = 0; s < pl.nrad; ++s) {
-    int R = pl.rad[s];
-    switch (R) {
-      case 2: stockham_stage<2>(cur, nxt, P, pl.fd_nb[s], pl.fd_ns[s], pl.tw, B, tid, NT); break;
-      case 3: stockham_stage<3>(cur, nxt, P, pl.fd_nb[s], pl.fd_ns[s], pl.tw, B, tid, NT); break;
-      case 4: stockham_stage<4>(cur, nxt, P, pl.fd_nb[s], pl.fd_ns[s], pl.tw, B, tid, NT); break;
-      default: stockham_stage<5>(cur, nxt, P, pl.fd_nb[s], pl.fd_ns[s], pl.tw, B, tid, NT); break;
+    const int wn = w == 2 ? 0 : w + 1, wc = wn == 2 ? 0 : wn + 1;
+    for (int b = G.grp; b < B; b += G.groups) {
+      const int sh = fx_shift_for(S.mag[w][b]);
+      unsigned mag;
+      switch (pl.rad[s]) {
+        case 2: mag = stockham_stage<2>(cur + b * P, nxt + b * P, P, pl.fd_ns[s], pl.tw, pl.tw3, sh, G.gt, G.gsz); break;
+        case 3: mag = stockham_stage<3>(cur + b * P, nxt + b * P, P, pl.fd_ns[s], pl.tw, pl.tw3, sh, G.gt, G.gsz); break;
+        case 4: mag = stockham_stage<4>(cur + b * P, nxt + b * P, P, pl.fd_ns[s], pl.tw, pl.tw3, sh, G.gt, G.gsz); break;
+        default: mag = stockham_stage<5>(cur + b * P, nxt + b * P, P, pl.fd_ns[s], pl.tw, pl.tw3, sh, G.gt, G.gsz); break;
+      }
+      mag = __reduce_or_sync(0xffffffffu, mag);
+      if (lane == 0) atomicOr(&S.mag[wn][b], mag);
+      if (G.gt == 0) {
+        S.shift[b] += sh;
+        S.mag[wc][b] = 0u;
+      }
     }
     __syncthreads();
-    double2* t = cur; cur = nxt; nxt = t;
+    longlong2* t = cur; cur = nxt; nxt = t;
+    w = wn;
   }
-  // --- unpack the real FFT: even outputs directly, odd increments in place
-  const int H = P / 2;
-  for (int it = tid; it < B * H; it += NT) {
-    int b = pl.fd_H.div(it);
-    int k = it - b * H;
-    const double2* Z = cur + b * P;
-    double* o = xb + b * ldx;
-    if (k == 0) {
-      double2 z0 = Z[0];
-      double2 zh = Z[H];
-      o[0] = z0.x + z0.y;     // D_1
-      o[P - 1] = zh.y + zh.y; // D_P
-      o[P] = zh.x + zh.x;     // Re(2Y_{P/2})
-    } else {
-      double2 zk = Z[k], zp = Z[P - k];
-      double2 E = make_double2(zk.x + zp.x, zk.y - zp.y);
-      double2 O = make_double2(zk.y + zp.y, zp.x - zk.x);
-      double2 T = cmul(O, __ldg(&pl.uw[k]));
-      o[2 * k - 1] = -E.y - T.y;
-      o[2 * k] = E.x + T.x;
-      o[2 * (P - k) - 1] = E.y - T.y;
-      o[2 * (P - k)] = E.x - T.x;
+  // --- unpack the real FFT: even outputs D_2, D_4, .. to slots P.., the odd ones' increments to 0..P-1
+  for (int b = G.grp; b < B; b += G.groups) {
+    const int sh = S.last_shift(b, w), E = S.exponent(b, sh);
+    const bool plain = fx_plain(E);
+    const longlong2* Z = cur + b * P;
+    long long* odd = reinterpret_cast<long long*>(nxt + b * P);
+    long long* even = odd + P;
+    auto at = [&](int i) {
+      const longlong2 z = Z[i];
+      return sh ? FxC{fx_shr(z.x, sh), fx_shr(z.y, sh)} : FxC{z.x, z.y};
+    };
+    for (int k = G.gt; k < H; k += G.gsz) {
+      if (k == 0) {
+        const FxC z0 = at(0), zh = at(H);
+        odd[0] = z0.x + z0.y;                       // D_1
+        even[H - 1] = line_bits(zh.y + zh.y, E);    // D_P
+        odd[H] = zh.x + zh.x;                       // Re(2Y_{P/2})
+      } else {
+        const FxC zk = at(k), zp = at(P - k);
+        const FxC Ev = FxC{zk.x + zp.x, zk.y - zp.y};
+        const FxC O = FxC{zk.y + zp.y, zp.x - zk.x};
+        const FxC T = twiddle(O, pl.tw + (unsigned)(P + k), pl.tw3 + (unsigned)(P + k));
+        odd[k] = Ev.x + T.x;
+        odd[P - k] = Ev.x - T.x;
+        const fx e0 = -Ev.y - T.y, e1 = Ev.y - T.y;
+        even[k - 1] = plain ? fx_to_bits_plain(e0, E) : line_bits(e0, E);
+        even[P - k - 1] = plain ? fx_to_bits_plain(e1, E) : line_bits(e1, E);
+      }
     }
   }
   __syncthreads();
-  // --- inclusive prefix sum over positions 0,2,...,2(P-1): odd outputs
-  const int lane = tid & 31, warp = tid >> 5, nwarps = NT >> 5;
-  if (narrow_scan) {
-    // one warp per line: sequential runs of ceil(P/32) per lane and a warp shuffle scan, the
-    // fewest FP64 instructions (for launches whose other CTAs keep the SM busy meanwhile)
-    const int c = (P + 31) >> 5;
-    for (int b = warp; b < B; b += nwarps) {
-      double* o = xb + b * ldx;
-      const int s0 = min(lane * c, P), s1 = min(s0 + c, P);
-      double acc = 0.0;
-      for (int i = s0; i < s1; ++i) acc += o[2 * i];
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        double v = __shfl_up_sync(0xffffffffu, acc, off);
-        if (lane >= off) acc += v;
-      }
-      double run = __shfl_up_sync(0xffffffffu, acc, 1);
-      if (lane == 0) run = 0.0;
-      for (int i = s0; i < s1; ++i) {
-        run += o[2 * i];
-        o[2 * i] = run;
-      }
-    }
-    __syncthreads();
-    return;
-  }
-  // every warp of the CTA takes part: a group of wpl warps per line, short sequential runs per
-  // thread, a warp shuffle scan, then the group's warp totals in shared memory (the shortest
-  // dependent chain, for latency-bound launches)
-  __shared__ double s_wt[32];
-  const int wpl = nwarps >= B ? nwarps / B : 1;           // warps per line
-  const int groups = nwarps >= B ? B : nwarps;            // lines in flight at once
-  const int c = (P + 32 * wpl - 1) / (32 * wpl);
-  for (int b0 = 0; b0 < B; b0 += groups) {
-    const int grp = warp / wpl, gw = warp - grp * wpl;
-    const int b = b0 + grp;
-    const bool act = grp < groups && b < B;
-    double* o = xb + (act ? b : 0) * ldx;
-    const int gt = gw * 32 + lane;
-    const int s0 = min(gt * c, P), s1 = min(s0 + c, P);
-    double acc = 0.0;
+  // --- inclusive prefix sum of the increments: the odd outputs.  Integer sums: exact, and the same
+  // bits whatever the split into threads.
+  const int c = (P + G.gsz - 1) / G.gsz;
+  for (int b0 = 0; b0 < B; b0 += G.groups) {
+    const int b = b0 + G.grp;
+    const bool act = G.grp < G.groups && b < B;
+    long long* odd = reinterpret_cast<long long*>(nxt + (act ? b : 0) * P);
+    const int s0 = min(G.gt * c, P), s1 = min(s0 + c, P);
+    fx acc = 0;
     if (act)
-      for (int i = s0; i < s1; ++i) acc += o[2 * i];
-    double incl = acc;
+      for (int i = s0; i < s1; ++i) acc += odd[i];
+    fx incl = acc;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
-      double v = __shfl_up_sync(0xffffffffu, incl, off);
+      const fx v = __shfl_up_sync(0xffffffffu, incl, off);
       if (lane >= off) incl += v;
     }
-    if (lane == 31 && grp < groups) s_wt[grp * wpl + gw] = incl;
-    double excl = __shfl_up_sync(0xffffffffu, incl, 1);
-    if (lane == 0) excl = 0.0;
-    __syncthreads();
+    if (G.wpl > 1) {
+      if (lane == 31 && act) S.wt[G.grp * G.wpl + G.gw] = incl;
+      __syncthreads();
+    }
     if (act) {
-      double run = 0.0;
-      for (int j = 0; j < gw; ++j) run += s_wt[grp * wpl + j];
-      run += excl;
+      const int E = S.exponent(b, S.last_shift(b, w));
+      const bool plain = fx_plain(E);
+      fx run = incl - acc;
+      for (int j = 0; j < G.gw; ++j) run += S.wt[G.grp * G.wpl + j];
       for (int i = s0; i < s1; ++i) {
-        run += o[2 * i];
-        o[2 * i] = run;
+        run += odd[i];
+        odd[i] = plain ? fx_to_bits_plain(run, E) : line_bits(run, E);
       }
     }
     __syncthreads();
   }
+  return reinterpret_cast<double*>(nxt);
 }
+
+// Where dst_lines leaves Y_(j+1) in a line's slots.
+__device__ __forceinline__ int dst_slot(int j, int P) { return (j >> 1) + ((j & 1) ? P : 0); }
 
 // ------------------------------------------------------------- x pass
 // The pre-op operands of one CTA's level (the top-level fields, or level blockIdx.y of a batch).
@@ -436,23 +472,24 @@ __device__ __forceinline__ double x_load(const XPre& a, const double* __restrict
 
 template <int PRE>
 __global__ void __launch_bounds__(512) k_dst_x(DstDev pl, int nrows, int ld, const __grid_constant__ DstXArgs a,
-                                               GridDims g, int B, int narrow_scan) {
+                                               GridDims g, int B) {
   IB_GRID_DEP_WAIT();
   const double* ain = a.nlev ? a.lin[blockIdx.y] : a.in;
   double* aout = a.nlev ? a.lout[blockIdx.y] : a.out;
   const XPre pre = x_pre(a, blockIdx.y, PRE == PRE_PRED && a.nlev > 0);
-  extern __shared__ double2 smem2[];
-  __shared__ int s_mode[64];
+  extern __shared__ longlong2 smem2[];
+  __shared__ int s_mode[kMaxLines];
   __shared__ int s_any;
-  const int ldx = pl.M;
-  double* xb = reinterpret_cast<double*>(smem2);
-  double2* zA = smem2 + (B * ldx) / 2;
-  double2* zB = zA + B * pl.P;
-  const int N = pl.N;
+  __shared__ FxLines S;
+  longlong2* zA = smem2;
+  longlong2* zB = zA + B * pl.P;
+  const double* xb = nullptr;   // the transformed lines, M apart
+  const int N = pl.N, M = pl.M;
   const int line0 = blockIdx.x * B;
   const int nl = a.nlines ? a.nlines : nrows;
-  __shared__ int s_row[64];
+  __shared__ int s_row[kMaxLines];
   if (threadIdx.x == 0) s_any = 0;
+  S.clear(B);
   __syncthreads();
   if (threadIdx.x < B) {
     int line = line0 + threadIdx.x;
@@ -475,54 +512,81 @@ __global__ void __launch_bounds__(512) k_dst_x(DstDev pl, int nrows, int ld, con
   }
   __syncthreads();
   const bool any_fft = s_any != 0;
+  const LineGroups G(B);
   if (any_fft) {
     // 4 independent loads in flight per thread before the shared-memory stores
-    const int tot = B * N, nt = blockDim.x;
-    for (int it0 = threadIdx.x; it0 < tot; it0 += 4 * nt) {
-      double v[4];
+    for (int b = G.grp; b < B; b += G.groups) {
+      const int row = s_row[b];
+      const bool live = s_mode[b] == ROW_FFT;
+      double* x = reinterpret_cast<double*>(zA + b * pl.P) + 1;
+      int emax = 1;
+      for (int j0 = G.gt; j0 < N; j0 += 4 * G.gsz) {
+        double v[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        int it = it0 + u * nt;
-        v[u] = 0.0;
-        if (it < tot) {
-          int b = pl.fd_N.div(it), j = it - b * N;
-          if (s_mode[b] == ROW_FFT) v[u] = x_load<PRE>(pre, ain, g, s_row[b], j, nrows, N, ld);
+        for (int u = 0; u < 4; ++u) {
+          const int j = j0 + u * G.gsz;
+          v[u] = live && j < N ? x_load<PRE>(pre, ain, g, row, j, nrows, N, ld) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int j = j0 + u * G.gsz;
+          if (j < N) x[j] = v[u];
+          emax = max(emax, (__double2hiint(v[u]) >> 20) & 0x7ff);
         }
       }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        int it = it0 + u * nt;
-        if (it < tot) {
-          int b = pl.fd_N.div(it), j = it - b * N;
-          xb[b * ldx + j] = v[u];
-        }
-      }
+      S.note(b, emax);
     }
     __syncthreads();
-    dst_lines(pl, B, xb, ldx, zA, zB, narrow_scan);
+    xb = dst_lines(pl, B, zA, zB, S);
   }
-  for (int it = threadIdx.x; it < B * N; it += blockDim.x) {
-    int b = pl.fd_N.div(it), j = it - b * N;
-    int row = s_row[b];
-    int mode = s_mode[b];
+  for (int b = G.grp; b < B; b += G.groups) {
+    const int row = s_row[b];
+    const int mode = s_mode[b];
     if (mode == ROW_SKIP) continue;
-    size_t o = (size_t)row * ld + j;
-    double v;
+    const size_t off = (size_t)row * ld;
+    double* o = aout + off;
+    const double* padd = a.post_add ? a.post_add + off : nullptr;
     if (mode == ROW_FFT) {
-      v = xb[b * ldx + j];
-    } else if (mode == ROW_EDGES) {
-      double x1 = x_load<PRE>(pre, ain, g, row, 0, nrows, N, ld);
-      double xn = x_load<PRE>(pre, ain, g, row, N - 1, nrows, N, ld);
-      int k = j + 1;
-      double sk = __ldg(&pl.sn[k <= pl.P ? k : pl.M - k]);
-      v = 2.0 * sk * ((k & 1) ? x1 + xn : x1 - xn);
-    } else if (mode == ROW_SCALE) {
-      v = a.row_scale * (a.nlev ? a.lin2[blockIdx.y] : a.in2)[o];
-    } else {
-      v = 0.0;
+      const double* y = xb + b * M;
+      if (padd) {
+        // out may alias post_add: every load of a thread's outputs comes before their stores
+        for (int j0 = G.gt; j0 < N; j0 += 4 * G.gsz) {
+          double v[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int j = j0 + u * G.gsz;
+            if (j < N) v[u] = padd[j];
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int j = j0 + u * G.gsz;
+            if (j < N) o[j] = fma(a.post_scale, v[u], y[dst_slot(j, pl.P)]);
+          }
+        }
+      } else {
+#pragma unroll 4
+        for (int j = G.gt; j < N; j += G.gsz) o[j] = y[dst_slot(j, pl.P)];
+      }
+      continue;
     }
-    if (a.post_add) v = fma(a.post_scale, a.post_add[o], v);
-    aout[o] = v;
+    double x1 = 0.0, xn = 0.0;
+    if (mode == ROW_EDGES) {
+      x1 = x_load<PRE>(pre, ain, g, row, 0, nrows, N, ld);
+      xn = x_load<PRE>(pre, ain, g, row, N - 1, nrows, N, ld);
+    }
+    const double* in2 = mode == ROW_SCALE ? (a.nlev ? a.lin2[blockIdx.y] : a.in2) + off : nullptr;
+    for (int j = G.gt; j < N; j += G.gsz) {
+      double v = 0.0;
+      if (mode == ROW_EDGES) {
+        const int k = j + 1;
+        const double sk = __ldg(&pl.sn[k <= pl.P ? k : pl.M - k]);
+        v = 2.0 * sk * ((k & 1) ? x1 + xn : x1 - xn);
+      } else if (mode == ROW_SCALE) {
+        v = a.row_scale * in2[j];
+      }
+      if (padd) v = fma(a.post_scale, padd[j], v);
+      o[j] = v;
+    }
   }
 }
 
@@ -696,11 +760,14 @@ __global__ void __launch_bounds__(256) k_dst_bc_modes(DstDev pl, GridDims g, con
   IB_GRID_DEP_WAIT();
   const int N = pl.N;
   if (fft_edges && (int)blockIdx.x < nEdge) {
-    extern __shared__ double line[];   // the row (N, padded to N+1), then two P-point complex buffers
-    double2* zA = reinterpret_cast<double2*>(line + (N + 1));
-    double2* zB = zA + pl.P;
+    extern __shared__ longlong2 fft[];   // two P-point complex buffers; the row in the first one's slots
+    __shared__ FxLines S;
+    double* x = reinterpret_cast<double*>(fft) + 1;
     const int e = blockIdx.x;
     const int J = e == 0 ? 2 : g.n;
+    S.clear(1);
+    __syncthreads();
+    int emax = 1;
     for (int j = threadIdx.x; j < N; j += blockDim.x) {
       const int I = j + 2;
       double v = 0.0;
@@ -708,14 +775,17 @@ __global__ void __launch_bounds__(256) k_dst_bc_modes(DstDev pl, GridDims g, con
       if (I == g.m) v = v + ring[g.right + J - 1];
       if (J == 2) v = v + ring[g.bottom + I - 1];
       if (J == g.n) v = v + ring[g.top + I - 1];
-      line[j] = v;
+      x[j] = v;
+      emax = max(emax, (__double2hiint(v) >> 20) & 0x7ff);
     }
+    S.note(0, emax);
     __syncthreads();
-    dst_lines(pl, 1, line, N + 1, zA, zB, 1);
+    const double* line = dst_lines(pl, 1, fft, fft + pl.P, S);
     const size_t row = e == 0 ? 0 : (size_t)(g.nsy - 1) * g.nsx;
     for (int k = threadIdx.x; k < N; k += blockDim.x) {
       const size_t o = row + k;
-      out[o] = post_add ? fma(post_scale, post_add[o], line[k]) : line[k];
+      const double y = line[dst_slot(k, pl.P)];
+      out[o] = post_add ? fma(post_scale, post_add[o], y) : y;
     }
     return;
   }
@@ -785,8 +855,8 @@ __global__ void __launch_bounds__(256) k_dst_bc_modes(DstDev pl, GridDims g, con
 int dst_x_bc_modes(const DstPlan& px, const GridDims& g, const double* ring, const double* W, const double* sk2,
                    const double* post_add, double post_scale, double* out, cudaStream_t st, bool fft_edges) {
   const int N = px.N;
-  const size_t smem = fft_edges ? sizeof(double) * 3 * ((size_t)N + 1) : 2 * sizeof(double) * (size_t)N;
-  if (allow_dyn_smem(k_dst_bc_modes, sizeof(double) * 3 * ((size_t)N + 1)) != cudaSuccess) return IB_ERR_CUDA;
+  const size_t smem = fft_edges ? dst_smem_x(px, 1) : 2 * sizeof(double) * (size_t)N;
+  if (allow_dyn_smem(k_dst_bc_modes, dst_smem_x(px, 1)) != cudaSuccess) return IB_ERR_CUDA;
   const int nEdge = fft_edges ? 2 : cdiv(N, 8);
   const int nblk = nEdge + cdiv(std::max(0, g.nsy - 2), kRowsPerCta);
   DstDev d = to_dev(px);
@@ -797,7 +867,6 @@ int dst_x_bc_modes(const DstPlan& px, const GridDims& g, const double* ring, con
 }
 
 int dst_sin2_table(const DstPlan& px, double* dev_out) {
-  const long double PI_L = 3.141592653589793238462643383279502884L;
   std::vector<double> v(px.N);
   for (int k = 1; k <= px.N; ++k) {
     const int kk = k <= px.P ? k : px.M - k;   // the plan's sin table entry the transform uses
@@ -809,7 +878,6 @@ int dst_sin2_table(const DstPlan& px, double* dev_out) {
 }
 
 int dst_matrix_table(const DstPlan& px, double* dev_out) {
-  const long double PI_L = 3.141592653589793238462643383279502884L;
   const int N = px.N, M = px.M;
   // entry (j, k) is 2 sin(pi r / M) with r = jk mod 2M: one table of the 2M values (long double is
   // software-emulated on some hosts, so it is not evaluated N^2 times)
@@ -825,31 +893,34 @@ int dst_matrix_table(const DstPlan& px, double* dev_out) {
 
 
 // ------------------------------------------------------------- y pass
-__global__ void __launch_bounds__(512) k_dst_y(DstDev pl, int ncols, int ld, DstYArgs a, int B, int narrow_scan) {
+__global__ void __launch_bounds__(512) k_dst_y(DstDev pl, int ncols, int ld, DstYArgs a, int B) {
   IB_GRID_DEP_WAIT();
-  extern __shared__ double2 smem2[];
-  const int ldx = pl.M;
-  const int N = pl.N;
-  double* xa = reinterpret_cast<double*>(smem2);
-  double2* zA = reinterpret_cast<double2*>(xa + B * ldx);
-  double2* zB = zA + B * pl.P;
+  extern __shared__ longlong2 smem2[];
+  __shared__ FxLines S;
+  const int N = pl.N, M = pl.M;
+  longlong2* zA = smem2;
+  longlong2* zB = zA + B * pl.P;
   const int col0 = blockIdx.x * B;
+  S.clear(B);
+  __syncthreads();
   for (int it = threadIdx.x; it < B * N; it += blockDim.x) {
-    int j = it / B, b = it - j * B;
-    int col = col0 + b;
-    xa[b * ldx + j] = col < ncols ? a.a[(size_t)j * ld + col] : 0.0;
+    const int j = it / B, b = it - j * B;
+    const int col = col0 + b;
+    const double v = col < ncols ? a.a[(size_t)j * ld + col] : 0.0;
+    reinterpret_cast<double*>(zA + b * pl.P)[j + 1] = v;
+    atomicMax(&S.e[b], (__double2hiint(v) >> 20) & 0x7ff);
   }
   __syncthreads();
-  dst_lines(pl, B, xa, ldx, zA, zB, narrow_scan);
+  const double* xa = dst_lines(pl, B, zA, zB, S);
   for (int it = threadIdx.x; it < B * N; it += blockDim.x) {
-    int j = it / B, b = it - j * B;
-    int col = col0 + b;
-    if (col < ncols) a.a[(size_t)j * ld + col] = xa[b * ldx + j];
+    const int j = it / B, b = it - j * B;
+    const int col = col0 + b;
+    if (col < ncols) a.a[(size_t)j * ld + col] = xa[b * M + dst_slot(j, pl.P)];
   }
 }
 
-size_t dst_smem_x(const DstPlan& p, int B) { return (size_t)B * p.M * 8 * 3; }
-size_t dst_smem_y(const DstPlan& p, int B, DstYMode) { return (size_t)B * p.M * 8 * 3; }
+size_t dst_smem_x(const DstPlan& p, int B) { return (size_t)B * p.M * 8 * 2; }
+size_t dst_smem_y(const DstPlan& p, int B, DstYMode) { return (size_t)B * p.M * 8 * 2; }
 
 template <typename K>
 static int launch_cfg(K kern, size_t smem) {
@@ -864,7 +935,7 @@ static int launch_cfg(K kern, size_t smem) {
 
 int dst_pass_x(const DstPlan& px, int nrows, int ld, DstPre pre, const DstXArgs& a, const GridDims& g,
                const DstLaunch& L, cudaStream_t st) {
-  if (a.nlev < 0 || a.nlev > kMaxBatch || (a.nlev && pre != PRE_COPY && pre != PRE_PRED)) return IB_ERR_ARG;
+  if (L.B > kMaxLines || a.nlev < 0 || a.nlev > kMaxBatch || (a.nlev && pre != PRE_COPY && pre != PRE_PRED)) return IB_ERR_ARG;
   DstDev d = to_dev(px);
   size_t smem = dst_smem_x(px, L.B);
   dim3 grid(cdiv(a.nlines ? a.nlines : nrows, L.B), a.nlev ? a.nlev : 1);
@@ -874,32 +945,32 @@ int dst_pass_x(const DstPlan& px, int nrows, int ld, DstPre pre, const DstXArgs&
       rc = launch_cfg(k_dst_x<PRE_COPY>, smem);
       if (rc) return rc;
       count_launch();
-      k_dst_x<PRE_COPY><<<grid, L.NT, smem, st>>>(d, nrows, ld, a, g, L.B, L.narrow_scan);
+      k_dst_x<PRE_COPY><<<grid, L.NT, smem, st>>>(d, nrows, ld, a, g, L.B);
       break;
     case PRE_COMBINE:
       rc = launch_cfg(k_dst_x<PRE_COMBINE>, smem);
       if (rc) return rc;
       count_launch();
-      k_dst_x<PRE_COMBINE><<<grid, L.NT, smem, st>>>(d, nrows, ld, a, g, L.B, L.narrow_scan);
+      k_dst_x<PRE_COMBINE><<<grid, L.NT, smem, st>>>(d, nrows, ld, a, g, L.B);
       break;
     case PRE_PRED:
       rc = launch_cfg(k_dst_x<PRE_PRED>, smem);
       if (rc) return rc;
       count_launch();
-      k_dst_x<PRE_PRED><<<grid, L.NT, smem, st>>>(d, nrows, ld, a, g, L.B, L.narrow_scan);
+      k_dst_x<PRE_PRED><<<grid, L.NT, smem, st>>>(d, nrows, ld, a, g, L.B);
       break;
     case PRE_ROT:
       if (!a.box || !a.in2) return IB_ERR_ARG;
       rc = launch_cfg(k_dst_x<PRE_ROT>, smem);
       if (rc) return rc;
       count_launch();
-      k_dst_x<PRE_ROT><<<grid, L.NT, smem, st>>>(d, nrows, ld, a, g, L.B, L.narrow_scan);
+      k_dst_x<PRE_ROT><<<grid, L.NT, smem, st>>>(d, nrows, ld, a, g, L.B);
       break;
     default:
       rc = launch_cfg(k_dst_x<PRE_APPLYBC>, smem);
       if (rc) return rc;
       count_launch();
-      k_dst_x<PRE_APPLYBC><<<grid, L.NT, smem, st>>>(d, nrows, ld, a, g, L.B, L.narrow_scan);
+      k_dst_x<PRE_APPLYBC><<<grid, L.NT, smem, st>>>(d, nrows, ld, a, g, L.B);
       break;
   }
   IB_CUDA_CHECK(cudaGetLastError());
@@ -914,7 +985,7 @@ int dst_pass_y(const DstPlan& py, int ncols, int ld, DstYMode, const DstYArgs& a
   int rc = launch_cfg(k_dst_y, smem);
   if (rc) return rc;
   count_launch();
-  k_dst_y<<<grid, L.NT, smem, st>>>(d, ncols, ld, a, L.B, L.narrow_scan);
+  k_dst_y<<<grid, L.NT, smem, st>>>(d, ncols, ld, a, L.B);
   IB_CUDA_CHECK(cudaGetLastError());
   return IB_OK;
 }

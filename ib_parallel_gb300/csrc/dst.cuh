@@ -9,9 +9,10 @@
 //   2Y  = unpacked real FFT of y (length M)
 //   D_{2k}   = -Im(2Y_k),      D_1 = Re(Y_0),   D_{2k+1} = D_{2k-1} + Re(2Y_k)
 // (the classic odd-extension sine transform; the odd outputs are a prefix sum).
-// The complex FFT is a Stockham auto-sort with radices 2, 3, 4 and 5 run in
-// shared memory over all (line, butterfly) items of a CTA.
+// The complex FFT is a Stockham auto-sort with radices 2, 3, 4 and 5 run in shared memory, a few
+// warps per line, in 64-bit block fixed point (fixed.cuh): doubles in, doubles out.
 #pragma once
+#include "fixed.cuh"
 #include "ib_common.cuh"
 
 namespace ib {
@@ -86,22 +87,23 @@ struct DstPlan {
   int N = 0, M = 0, P = 0;
   int nrad = 0;
   int rad[kMaxRadices] = {0};
-  double2* tw = nullptr;   // P entries: the Stockham stages' twiddles, stage by stage (dst.cu)
-  double2* uw = nullptr;   // P/2 entries: exp(-2 pi i k / M)
-  double* sn = nullptr;    // P+1 entries: sin(j pi / M)
+  FxW* tw = nullptr;       // 2 x 3P/2: the stages' twiddles and exp(-2 pi i k / M) (dst.cu, plan_tables)
+  FxW* tw3 = nullptr;      // 3P/2: their third factors
+  FxW* sx = nullptr;       // P: 2 sin(j pi / M)
+  double* sn = nullptr;    // P+1: sin(j pi / M)
 };
 
 // Launch geometry of one pass (chosen by the tuner in dst.cu).
 struct DstLaunch {
   int B = 1;       // lines per CTA
   int NT = 128;    // threads per CTA
-  int narrow_scan = 0;   // 1: one warp scans each line (fewer FP64 instructions); 0: all warps
 };
 
 int dst_plan_create(DstPlan* p, int N);   // N = M-1, M divisible by 4, M = 2^a 3^b 5^c
 void dst_plan_destroy(DstPlan* p);
 // Doubles of device memory the tables of a plan of length N occupy (0 if N is unsupported).
 size_t dst_plan_table_doubles(int N);
+size_t dst_plan_doubles(int M);   // the same of a supported M = N + 1
 // Fills a plan's tables into caller-provided device memory (no allocation; the plan must not
 // be passed to dst_plan_destroy).  dev must hold dst_plan_table_doubles(N) doubles, 16-byte aligned.
 int dst_plan_init_external(DstPlan* p, int N, double* dev, cudaStream_t st);

@@ -30,9 +30,12 @@
 
 namespace ib {
 
-static constexpr size_t kStaticDoubles = size_t(1) << 21;  // 16 MiB
+static constexpr size_t kStaticDoubles = size_t(1) << 21;  // 16 MiB: the limit callers are given
+// Room for the transform's fixed-point tables, which take 2.5 (m/2) doubles more than the doubles the
+// limit counts; grids whose lines fit a CTA's shared memory (24 m bytes) need no more.
+static constexpr size_t kTableSlack = 16384;
 
-static __device__ __align__(256) double g_ctci_scratch[kStaticDoubles];
+static __device__ __align__(256) double g_ctci_scratch[kStaticDoubles + kTableSlack];
 
 namespace {
 
@@ -52,10 +55,10 @@ size_t align4(size_t n) { return (n + 3) & ~size_t(3); }
 
 void set_last_error(const char* msg);  // capi.cu: the message ib_last_error() returns
 
-// Doubles of g_ctci_scratch the solve needs for an m x n grid (0 if the grid is unsupported).
-static size_t needed(int m, int n) {
-  size_t plan = dst_plan_table_doubles(m - 1);
-  if (plan == 0) return 0;
+// Doubles the solve needs for an m x n grid (0 if the grid is unsupported), counting `plan` doubles
+// for the transform's tables.
+static size_t needed(int m, int n, size_t plan) {
+  if (dst_plan_table_doubles(m - 1) == 0) return 0;
   int s = 0, C = 0;
   tri_chunking(n, m - 1, &s, &C);
   return align4((size_t)(m - 1) * (n - 1)) + align4(plan) + align4(tri_table_doubles(m - 1, s, C));
@@ -66,7 +69,7 @@ int static_ctci(int m, int n, const double* vort, double* s, cudaStream_t st) {
     set_last_error("ib_ctci_static: m, n must be >= 8 and divisible by 4, arrays non-null");
     return IB_ERR_ARG;
   }
-  size_t need = needed(m, n);
+  const size_t need = needed(m, n, 4 * (size_t)(m / 2) + 5);   // what the documented limit counts
   if (need == 0) {
     set_last_error("ib_ctci_static: m must be 2^a 3^b 5^c");
     return IB_ERR_ARG;
@@ -75,6 +78,10 @@ int static_ctci(int m, int n, const double* vort, double* s, cudaStream_t st) {
     set_last_error("ib_ctci_static: grid too large for the 16 MiB static scratch ((m-1)(n-1) plus tables must "
                    "fit in 2^21 doubles)");
     return IB_ERR_ARG;
+  }
+  if (needed(m, n, dst_plan_table_doubles(m - 1)) > kStaticDoubles + kTableSlack) {
+    set_last_error("ib_ctci_static: kernel launch failed (a line of m samples does not fit shared memory)");
+    return IB_ERR_CUDA;
   }
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
@@ -142,7 +149,7 @@ int static_ctci(int m, int n, const double* vort, double* s, cudaStream_t st) {
   // The scratch is fully overwritten by the first pass, so nothing needs clearing.
   double* spec = S->base;
   DstLaunch L;
-  L.B = 2; L.NT = 160;
+  L.B = 1; L.NT = 128;
   DstXArgs a;
   a.in = vort; a.out = spec;
   int rc = dst_pass_x(S->px, g.nsy, g.nsx, PRE_COPY, a, g, L, st);
