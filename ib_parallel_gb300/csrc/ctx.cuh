@@ -364,7 +364,9 @@ struct Ctx {
   long long fsi_post_launches = 0;
   int* fsi_cnt = nullptr;
   FusedPlan fused_plan;
-  double* cholM = nullptr;         // nf x nf (num_stat)
+  double* cholM = nullptr;         // nf x nf (num_stat): the Schur matrix, then its Cholesky factor
+  double* cholZ = nullptr;         // nf x nf: the factor's inverse in both triangles
+  double* chol_y = nullptr;        // nf: between the solve's two products
   bool chol_ready = false;
 
   // host-visible status

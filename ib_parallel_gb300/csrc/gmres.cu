@@ -378,65 +378,56 @@ __global__ void k_cholesky(int n, double* A, int* err) {
   }
 }
 
-// L L^T x = b with the Cholesky factor L (row-major, lower): forward then backward substitution
-// in blocks of 32 unknowns.  Each block first subtracts what the solved unknowns contribute (one
-// warp per unknown, lanes across the solved ones, a fixed shuffle tree), then warp 0 solves the
-// block's 32 x 32 triangle, staged in shared memory, with shuffles; no block-wide barrier inside
-// the triangles.
-__global__ void k_chol_solve(int n, const double* __restrict__ L, const double* __restrict__ b, double* x) {
+// Z = L^-1 for the Cholesky factor L (row-major, lower), one warp per column by forward substitution:
+// Z[r][c] = Z[c][r] = (L^-1)[r][c] for r >= c, so that both products of the solve read rows.  Run once
+// per factorisation.  L and Z are different arrays.
+__global__ void __launch_bounds__(32) k_tri_inverse(int n, const double* __restrict__ L, double* __restrict__ Z) {
   IB_GRID_DEP_WAIT();
-  extern __shared__ double y[];   // n unknowns, then the diagonal block (32 x 33)
-  double* dg = y + n;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) y[i] = b[i];
-  __syncthreads();
-  auto warp_sum = [](double v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-  };
-  for (int b0 = 0; b0 < n; b0 += 32) {   // L y = b
-    const int nb = min(32, n - b0);
-    for (int r = b0 + warp; r < b0 + nb; r += nw) {
-      double acc = 0.0;
-      for (int c = lane; c < b0; c += 32) acc = fma(L[(size_t)r * n + c], y[c], acc);
-      acc = warp_sum(acc);
-      if (lane == 0) y[r] -= acc;
+  extern __shared__ double col[];   // n entries of the column
+  const int j = blockIdx.x, lane = threadIdx.x;
+  for (int i = j; i < n; ++i) {
+    const double* row = L + (size_t)i * n;
+    double a0 = 0.0, a1 = 0.0;
+    int k = j + lane;
+    for (; k + 32 < i; k += 64) {
+      a0 = fma(row[k], col[k], a0);
+      a1 = fma(row[k + 32], col[k + 32], a1);
     }
-    for (int t = threadIdx.x; t < nb * nb; t += blockDim.x) dg[(t / nb) * 33 + t % nb] = L[(size_t)(b0 + t / nb) * n + b0 + t % nb];
-    __syncthreads();
-    if (warp == 0) {
-      double yr = lane < nb ? y[b0 + lane] : 0.0;
-      for (int i = 0; i < nb; ++i) {
-        if (lane == i) yr = yr / dg[i * 33 + i];
-        const double yi = __shfl_sync(0xffffffffu, yr, i);
-        if (lane > i && lane < nb) yr -= dg[lane * 33 + i] * yi;
-      }
-      if (lane < nb) y[b0 + lane] = yr;
-    }
-    __syncthreads();
+    if (k < i) a0 = fma(row[k], col[k], a0);
+    double s = a0 + a1;
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) col[i] = ((i == j ? 1.0 : 0.0) - s) / row[i];
+    __syncwarp();
   }
-  for (int b1 = n; b1 > 0; b1 -= 32) {   // L^T x = y
-    const int b0 = max(0, b1 - 32), nb = b1 - b0;
-    for (int c = b0 + warp; c < b1; c += nw) {
-      double acc = 0.0;
-      for (int r = b1 + lane; r < n; r += 32) acc = fma(L[(size_t)r * n + c], y[r], acc);
-      acc = warp_sum(acc);
-      if (lane == 0) y[c] -= acc;
-    }
-    for (int t = threadIdx.x; t < nb * nb; t += blockDim.x) dg[(t / nb) * 33 + t % nb] = L[(size_t)(b0 + t / nb) * n + b0 + t % nb];
-    __syncthreads();
-    if (warp == 0) {
-      double yr = lane < nb ? y[b0 + lane] : 0.0;
-      for (int i = nb - 1; i >= 0; --i) {
-        if (lane == i) yr = yr / dg[i * 33 + i];
-        const double xi = __shfl_sync(0xffffffffu, yr, i);
-        if (lane < i) yr -= dg[i * 33 + lane] * xi;
-      }
-      if (lane < nb) y[b0 + lane] = yr;
-    }
-    __syncthreads();
+  for (int i = j + lane; i < n; i += 32) {
+    Z[(size_t)j * n + i] = col[i];
+    Z[(size_t)i * n + j] = col[i];
   }
-  for (int i = threadIdx.x; i < n; i += blockDim.x) x[i] = y[i];
+}
+
+// y = L^-1 b (upper = 0) or y = L^-T b (upper = 1) from Z, a warp per row, four chains a lane.  The
+// stationary bodies' solve is the two products in turn (launch_chol_solve).  What bounds it: latency,
+// a few dependent FP64 operations of 64 cycles and the row's loads from L2.  The substitutions by
+// blocks of 32 it replaced ran on one CTA, 2 n / 32 dependent triangles: 304 us for the 314 unknowns
+// of the 157-point cylinder, against 7 us for the two products.
+constexpr int kTriRows = 4;   // rows (warps) per CTA
+__global__ void __launch_bounds__(32 * kTriRows) k_tri_product(int n, const double* __restrict__ Z,
+                                                               const double* __restrict__ b, double* __restrict__ y,
+                                                               int upper) {
+  IB_GRID_DEP_WAIT();
+  const int r = blockIdx.x * kTriRows + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= n) return;
+  const int c0 = upper ? r : 0, c1 = upper ? n : r + 1;
+  const double* row = Z + (size_t)r * n;
+  double a[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int c = c0 + lane; c < c1; c += 128) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (c + 32 * u < c1) a[u] = fma(row[c + 32 * u], b[c + 32 * u], a[u]);
+  }
+  double s = (a[0] + a[1]) + (a[2] + a[3]);
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) y[r] = s;
 }
 
 __global__ void k_copy_col(int n, const double* __restrict__ src, double* M, int col) {
@@ -456,11 +447,18 @@ int launch_cholesky(int n, double* A, int* d_err, cudaStream_t st) {
   IB_CUDA_CHECK(cudaGetLastError());
   return IB_OK;
 }
-int launch_chol_solve(int n, const double* Lf, const double* b, double* x, cudaStream_t st) {
-  size_t smem = sizeof(double) * ((size_t)n + 32 * 33);
-  IB_CUDA_CHECK(allow_dyn_smem(k_chol_solve, smem));
+int launch_tri_inverse(int n, const double* L, double* Z, cudaStream_t st) {
+  const size_t smem = sizeof(double) * (size_t)n;
+  IB_CUDA_CHECK(allow_dyn_smem(k_tri_inverse, smem));
   count_launch();
-  k_chol_solve<<<1, 1024, smem, st>>>(n, Lf, b, x);
+  k_tri_inverse<<<n, 32, smem, st>>>(n, L, Z);
+  IB_CUDA_CHECK(cudaGetLastError());
+  return IB_OK;
+}
+int launch_chol_solve(int n, const double* Z, const double* b, double* y, double* x, cudaStream_t st) {
+  count_launches(2);
+  k_tri_product<<<cdiv(n, kTriRows), 32 * kTriRows, 0, st>>>(n, Z, b, y, 0);
+  k_tri_product<<<cdiv(n, kTriRows), 32 * kTriRows, 0, st>>>(n, Z, y, x, 1);
   IB_CUDA_CHECK(cudaGetLastError());
   return IB_OK;
 }

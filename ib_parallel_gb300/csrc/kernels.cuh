@@ -283,9 +283,11 @@ struct FusedPlan {
 int launch_gmres_fused(const GmresDev& G, FusedPlan* plan, const double* At, const double* b, double* x, double rtol,
                        double atol, int max_it, cudaStream_t st);
 
-// dense symmetric positive definite solve (stationary-body path)
+// dense symmetric positive definite solve (stationary-body path): A = L L^T, Z = L^-1 (stored in both
+// triangles), then x = L^-T (y = L^-1 b)
 int launch_cholesky(int n, double* A, int* d_err, cudaStream_t st);
-int launch_chol_solve(int n, const double* Lf, const double* b, double* x, cudaStream_t st);
+int launch_tri_inverse(int n, const double* L, double* Z, cudaStream_t st);
+int launch_chol_solve(int n, const double* Z, const double* b, double* y, double* x, cudaStream_t st);
 int launch_copy_col(int n, const double* src, double* M, int col, cudaStream_t st);
 int launch_unit(int n, int i, double* e, cudaStream_t st);
 

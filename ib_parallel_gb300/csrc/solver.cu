@@ -225,7 +225,7 @@ int ctx_create(const IbParams* pin, const IbBody* bodies, int nbody, Ctx** out, 
   dbl += 3 * ((size_t)nt + 1) + 1;                       // fused FSI update: theta, sin, cos; ticket
   dbl += 8 * (size_t)nt + nt + 3;
   dbl += (size_t)(R + 1) * nf + (size_t)(R + 1) * R + 3 * (R + 1) + 4 + 4 * (size_t)nf + 2;
-  if (p.num_stat) dbl += (size_t)nf * nf;
+  if (p.num_stat) dbl += 2 * (size_t)nf * nf + nf;
   dbl += 8 * stage_n;
   size_t ints = 2 * (size_t)nf + 2 * (size_t)nf + 16 + 2 * (size_t)max_faces + 2 * 49 * (size_t)nf + 4 + 2 + 8;
   size_t bytes = dbl * 8 + ints * 4 + (size_t)nt * sizeof(TorsBody) + 256 * 400;
@@ -290,7 +290,11 @@ int ctx_create(const IbParams* pin, const IbBody* bodies, int nbody, Ctx** out, 
   c->G.scal = P.take<double>(4); c->G.ist = P.take<int>(8);
   c->gm_b = P.take<double>(nf + 1); c->gm_x = P.take<double>(nf + 1);
   c->G.xin = P.take<double>(nf); c->G.Av = P.take<double>(nf);
-  if (p.num_stat) c->cholM = P.take<double>((size_t)nf * nf);
+  if (p.num_stat) {
+    c->cholM = P.take<double>((size_t)nf * nf);
+    c->cholZ = P.take<double>((size_t)nf * nf);
+    c->chol_y = P.take<double>(nf);
+  }
   c->d_err = P.take<int>(1);
   c->stage_n = stage_n;
   for (int i = 0; i < 8; ++i) c->stage[i] = P.take<double>(stage_n);
@@ -1095,6 +1099,7 @@ static int preprocess_chol(Ctx* c) {
   RC(launch_cholesky(nf, c->cholM, c->d_err, c->st));
   int e = check_err(c);
   if (e) return IB_ERR_ARG;
+  RC(launch_tri_inverse(nf, c->cholM, c->cholZ, c->st));
   c->chol_ready = true;
   return IB_OK;
 }
@@ -1509,7 +1514,7 @@ static int op_direct_solve(Ctx* c) {
   } else {
     RC(launch_regT(g, c->nf, c->qx[0], c->q0x[0], c->qy[0], c->q0y[0], c->reg, nullptr, c->rhsf, st));
   }
-  RC(launch_chol_solve(c->nf, c->cholM, c->rhsf, c->f, st));
+  RC(launch_chol_solve(c->nf, c->cholZ, c->rhsf, c->chol_y, c->f, st));
   return op_redistribute(c, c->f, c->f_rdst);
 }
 
