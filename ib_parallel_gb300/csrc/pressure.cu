@@ -281,9 +281,8 @@ static int pressure_setup(Ctx* c) {
   const GridDims& g = c->g;
   const int m = g.m, n = g.n, L = c->L;
   const size_t cells = (size_t)m * n;
-  int s = 0, C = 0;
-  tri_chunking(n + 1, m, &s, &C);
-  const size_t tri_n = tri_table_doubles(m, s, C);
+  const TriShape tri_t = tri_chunking(n, m);
+  const size_t tri_n = tri_table_doubles(m, tri_t);
   const size_t dbl = (size_t)m * m + tri_n + 2 * (size_t)L * cells + 2 * cells + 2 * (size_t)L * g.ns +
                      (size_t)L * (g.nu + g.nv) + g.nu + g.nv + (size_t)std::max(c->nf, 1) + 2 * (size_t)g.nbc +
                      2 * (size_t)(m + n) + 64;
@@ -323,7 +322,7 @@ static int pressure_setup(Ctx* c) {
       const double sn = std::sin(pi * (double)k / (2.0 * (m + 1)));
       lx[k - 1] = 4.0 * sn * sn;
     }
-    RC(tri_build(&P.tri, m, n, lx.data(), -1.0 / (2.0 * (m + 1)), tri_mem));
+    RC(tri_build(&P.tri, m, n, tri_t, lx.data(), -1.0 / (2.0 * (m + 1)), tri_mem));
   }
   IB_CUDA_CHECK(cudaDeviceSynchronize());   // the tables' pageable copies have landed
   P.ready = true;

@@ -209,9 +209,8 @@ int ctx_create(const IbParams* pin, const IbBody* bodies, int nbody, Ctx** out, 
   dbl += (size_t)L * (3 * ns + 2 * nu + 2 * nv);         // state
   dbl += (size_t)L * ns;                                 // per-level predictor right-hand sides
   dbl += (size_t)L * (2 * ns + nu + nv);                 // Schur scratch
-  int tri_s = 0, tri_C = 0;
-  tri_chunking(g.n, g.nsx, &tri_s, &tri_C);
-  size_t tri_n = tri_table_doubles(g.nsx, tri_s, tri_C);
+  const TriShape tri_t = tri_chunking(g.nsy, g.nsx);
+  const size_t tri_n = tri_table_doubles(g.nsx, tri_t);
   dbl += (size_t)(2 + L) * tri_n;                        // tridiagonal tables
   dbl += 6 * ns + 2 * nu + 2 * nv;                       // work (+ ainv mode-space copy)
   dbl += (size_t)g.nsx * g.nsx + (size_t)g.nsy;          // DST matrix, row treatments
@@ -327,15 +326,15 @@ int ctx_create(const IbParams* pin, const IbBody* bodies, int nbody, Ctx** out, 
       c->con2.push_back(-0.5 * p.dt / del22 / c->normalize);
       c->cvis.push_back(0.5 * p.dt / del22 / p.Re);
     }
-    int rc2 = tri_build(&c->tri_ctci, g.nsx, g.nsy, lamx.data(), 1.0 / (2.0 * g.m), tri_mem);
+    int rc2 = tri_build(&c->tri_ctci, g.nsx, g.nsy, tri_t, lamx.data(), 1.0 / (2.0 * g.m), tri_mem);
     double c1 = c->cvis[0];
     for (int k = 0; k < g.nsx; ++k) shift[k] = lamx[k] + 1.0 / c1;
-    if (rc2 == IB_OK) rc2 = tri_build(&c->tri_ainv, g.nsx, g.nsy, shift.data(), 1.0 / (2.0 * g.m * c1), tri_mem + tri_n);
+    if (rc2 == IB_OK) rc2 = tri_build(&c->tri_ainv, g.nsx, g.nsy, tri_t, shift.data(), 1.0 / (2.0 * g.m * c1), tri_mem + tri_n);
     c->tri_pred.resize(L);
     for (int k = 0; k < L && rc2 == IB_OK; ++k) {
       double ck = c->cvis[k];
       for (int q = 0; q < g.nsx; ++q) shift[q] = lamx[q] + 1.0 / ck;
-      rc2 = tri_build(&c->tri_pred[k], g.nsx, g.nsy, shift.data(), 2.0 * g.n / ck, tri_mem + (2 + k) * tri_n);
+      rc2 = tri_build(&c->tri_pred[k], g.nsx, g.nsy, tri_t, shift.data(), 2.0 * g.n / ck, tri_mem + (2 + k) * tri_n);
     }
     if (rc2 != IB_OK) { *msg = "tridiagonal table upload failed"; ctx_destroy(c); return rc2; }
   }

@@ -59,9 +59,8 @@ void set_last_error(const char* msg);  // capi.cu: the message ib_last_error() r
 // for the transform's tables.
 static size_t needed(int m, int n, size_t plan) {
   if (dst_plan_table_doubles(m - 1) == 0) return 0;
-  int s = 0, C = 0;
-  tri_chunking(n, m - 1, &s, &C);
-  return align4((size_t)(m - 1) * (n - 1)) + align4(plan) + align4(tri_table_doubles(m - 1, s, C));
+  return align4((size_t)(m - 1) * (n - 1)) + align4(plan) +
+         align4(tri_table_doubles(m - 1, tri_chunking_even(n, m - 1)));
 }
 
 int static_ctci(int m, int n, const double* vort, double* s, cudaStream_t st) {
@@ -133,7 +132,9 @@ int static_ctci(int m, int n, const double* vort, double* s, cudaStream_t st) {
         double sn = std::sin(pi * (double)k / (2.0 * m));
         lamx[k - 1] = 4.0 * sn * sn;
       }
-      rc = tri_build(&S->tri, g.nsx, g.nsy, lamx.data(), 1.0 / (2.0 * m), tri_mem);
+      // chunks whose tables fit where the limit counts the equal chunks'
+      const TriShape shape = tri_chunking(g.nsy, g.nsx, tri_table_doubles(g.nsx, tri_chunking_even(n, g.nsx)));
+      rc = tri_build(&S->tri, g.nsx, g.nsy, shape, lamx.data(), 1.0 / (2.0 * m), tri_mem);
       if (rc != IB_OK) { set_last_error("ib_ctci_static: table upload failed"); return rc; }
       // tri_build copies from pageable host memory, and such a copy may return before its DMA
       // has reached the device; the solve kernels run on the caller's stream, which nothing

@@ -8,45 +8,84 @@
 
 namespace ib {
 
-void tri_chunking(int n, int nx, int* s, int* C) {
-  // The chunk period d = s+1 divides n, at most 32 chunks.  Every FP64 warp instruction holds
-  // its SM sub-partition's FP64 pipe for the same time whatever its active lanes, so the cost
-  // of one solve is the FP64 instructions of one chunk thread (about 5 per chunk row and one
-  // per interface) times the warps a sub-partition runs, minimised over the launch shapes
-  // (Mb modes x C chunks per CTA, Mb a power of two) the tuner can pick.
+// The chunk lengths with a register-resident kernel (k_tri_reg), and those of them that also take a
+// shorter last chunk.
+#define IB_TRI_EVEN(X) X(1) X(2) X(4) X(5) X(6) X(8) X(9) X(12) X(14) X(24) X(29)
+#define IB_TRI_BOTH(X) X(3) X(7) X(11) X(15) X(19) X(23) X(31) X(39) X(63)
+constexpr int kTriMaxM = 31;   // interfaces (C-1) the register prefetch holds
+
+static bool tri_reg_length(int s, bool tail) {
+  switch (s) {
+#define IB_CASE(SS) case SS:
+    IB_TRI_BOTH(IB_CASE) return true;
+    IB_TRI_EVEN(IB_CASE) return !tail;
+#undef IB_CASE
+    default: return false;
+  }
+}
+
+// Every FP64 warp instruction holds its SM sub-partition's FP64 pipe for the same time whatever its
+// active lanes, so the cost of one solve is the FP64 instructions of one chunk thread (about 5 per
+// chunk row and one per interface) times the warps a sub-partition runs, minimised over the launch
+// shapes (Mb modes x C chunks per CTA, Mb a power of two) the tuner can pick.
+static long long tri_cost(int s, int C, int nx) {
   constexpr int kSMs = 152;   // GB300: 4 sub-partitions each
+  const long long per = 5LL * s + C;
+  long long best = -1;
+  for (int Mb = 1; Mb <= 32; Mb *= 2) {
+    if (Mb * C > 1024) break;
+    const long long wpc = (Mb * C + 31) / 32;                 // warps per CTA
+    const long long ncta = (nx + Mb - 1) / Mb;
+    const long long mult = ((ncta + kSMs - 1) / kSMs * wpc + 3) / 4;   // warps per sub-partition
+    if (best < 0 || per * mult < best) best = per * mult;
+  }
+  return best;
+}
+
+TriShape tri_chunking_even(int n, int nx) {
+  // the chunk period d = s+1 divides n, at most 32 chunks
   long long best = -1;
   int bestd = n;
   for (int d = 2; d <= n; ++d) {
-    if (n % d) continue;
-    const int c = n / d;
-    if (c > 32) continue;
-    const long long per = 5LL * (d - 1) + c;
-    for (int Mb = 1; Mb <= 32; Mb *= 2) {
-      if (Mb * c > 1024) break;
-      const long long wpc = (Mb * c + 31) / 32;                 // warps per CTA
-      const long long ncta = (nx + Mb - 1) / Mb;
-      const long long mult = ((ncta + kSMs - 1) / kSMs * wpc + 3) / 4;   // warps per sub-partition
-      const long long cost = per * mult;
-      if (best < 0 || cost < best || (cost == best && d > bestd)) { best = cost; bestd = d; }
-    }
+    if (n % d || n / d > 32) continue;
+    const long long cost = tri_cost(d - 1, n / d, nx);
+    if (best < 0 || cost < best || (cost == best && d > bestd)) { best = cost; bestd = d; }
   }
-  *s = bestd - 1;
-  *C = n / bestd;
+  return TriShape{bestd - 1, n / bestd, bestd - 1};
 }
 
-size_t tri_table_doubles(int nx, int s, int C) {
-  const size_t m = C > 1 ? (size_t)(C - 1) : 1;
-  return (size_t)nx * (3 * (size_t)s + m * m);
+// Of the lengths with a register kernel, the cheapest; a shorter last chunk counts a tenth more (its
+// rows are predicated), and 63 rows, which spill, are taken only where no shorter chunk will do.  The shared-memory kernel took 37 us for 999 modes of 539 rows in its cheapest
+// equal chunks (15 of 35) and 160 us for 800 modes of 400 rows, whose period 401 is prime (one chunk);
+// in 14 chunks of 39 the first takes 22 us, and the second in 13 of 31 12 us.  It remains for more than
+// 32 x 64 rows.
+TriShape tri_chunking(int ny, int nx, size_t max_doubles) {
+  TriShape best;
+  double bestc = -1.0;
+  for (int s = 1; s <= 63; ++s) {
+    const int C = (ny + 1 + s) / (s + 1), r = ny - (C - 1) * (s + 1);
+    if (C - 1 > kTriMaxM || r < 1 || r > s || !tri_reg_length(s, r < s) || (s == 63 && bestc >= 0)) continue;
+    const TriShape t{s, C, r};
+    if (max_doubles && tri_table_doubles(nx, t) > max_doubles) continue;
+    const double cost = (double)tri_cost(s, C, nx) * (r < s ? 1.1 : 1.0);
+    if (bestc < 0 || cost <= bestc) { bestc = cost; best = t; }
+  }
+  return bestc < 0 ? tri_chunking_even(ny + 1, nx) : best;
 }
 
-int tri_build(TriOp* op, int nx, int ny, const double* shift, double sigma, double* dev) {
-  int s = 0, C = 0;
-  tri_chunking(ny + 1, nx, &s, &C);
-  op->nx = nx; op->ny = ny; op->s = s; op->C = C; op->sigma = sigma;
+size_t tri_table_doubles(int nx, const TriShape& t) {
+  const size_t m = t.C > 1 ? (size_t)(t.C - 1) : 1;
+  return (size_t)nx * ((t.r < t.s ? 4 : 3) * (size_t)t.s + m * m);
+}
+
+int tri_build(TriOp* op, int nx, int ny, const TriShape& t, const double* shift, double sigma, double* dev) {
+  const int s = t.s, C = t.C, r = t.r;
+  if ((C - 1) * (s + 1) + r != ny) return IB_ERR_ARG;
+  op->nx = nx; op->ny = ny; op->s = s; op->C = C; op->r = r; op->sigma = sigma;
   const int m = C > 1 ? C - 1 : 1;
   const size_t S = (size_t)s * nx, R = (size_t)m * m * nx;
-  std::vector<double> tab(3 * S + R, 0.0);
+  std::vector<double> tab((r < s ? 4 : 3) * S + R, 0.0);
+  double* gT = tab.data() + 3 * S + R;
   double* inv = tab.data();
   double* sinv = inv + S;
   double* gL = inv + 2 * S;
@@ -54,7 +93,7 @@ int tri_build(TriOp* op, int nx, int ny, const double* shift, double sigma, doub
   // the modes are independent: they are split over host threads (long double arithmetic is
   // software-emulated on some hosts and costs milliseconds per operator otherwise)
   auto modes = [&](int k0, int k1) {
-  std::vector<long double> beta(s), d(s), g(s), bp(m), z(m), x(m);
+  std::vector<long double> beta(s), d(s), g(s), gt(r), bp(m), z(m), x(m);
   for (int k = k0; k < k1; ++k) {
     long double a = 2.0L + (long double)shift[k];
     beta[0] = a;
@@ -69,12 +108,17 @@ int tri_build(TriOp* op, int nx, int ny, const double* shift, double sigma, doub
     g[s - 1] = d[s - 1];
     for (int j = s - 2; j >= 0; --j) g[j] = d[j] + g[j + 1] / beta[j];
     for (int j = 0; j < s; ++j) gL[(size_t)j * nx + k] = (double)g[j];
+    gt[r - 1] = d[r - 1];
+    for (int j = r - 2; j >= 0; --j) gt[j] = d[j] + gt[j + 1] / beta[j];
+    if (r < s)
+      for (int j = 0; j < r; ++j) gT[(size_t)j * nx + k] = (double)gt[j];
     if (C < 2) continue;
-    // interface system tridiag(-B, A, -B) of size m = C-1, tabulated as its dense inverse
-    // (one Thomas solve per unit vector, in extended precision)
-    long double A = a - 2.0L * g[0], B = g[s - 1];
-    bp[0] = A;
-    for (int c = 1; c < m; ++c) bp[c] = A - B * B / bp[c - 1];
+    // interface system tridiag(-B, A, -B) of size m = C-1 (the last diagonal entry with the last
+    // chunk's response), tabulated as its dense inverse (one Thomas solve per unit vector, in
+    // extended precision)
+    const long double A = a - 2.0L * g[0], B = g[s - 1], AT = a - g[0] - gt[0];
+    bp[0] = m == 1 ? AT : A;
+    for (int c = 1; c < m; ++c) bp[c] = (c == m - 1 ? AT : A) - B * B / bp[c - 1];
     for (int j = 0; j < m; ++j) {
       for (int c = 0; c < m; ++c) z[c] = ((c == j ? 1.0L : 0.0L) + (c > 0 ? B * z[c - 1] : 0.0L)) / bp[c];
       x[m - 1] = z[m - 1];
@@ -95,6 +139,7 @@ int tri_build(TriOp* op, int nx, int ny, const double* shift, double sigma, doub
   op->sinv = dev + S;
   op->gL = dev + 2 * S;
   op->rinv = dev + 3 * S;
+  op->gT = r < s ? dev + 3 * S + R : nullptr;
   IB_CUDA_CHECK(cudaMemcpy(dev, tab.data(), 8 * tab.size(), cudaMemcpyHostToDevice));
   return IB_OK;
 }
@@ -238,8 +283,8 @@ __global__ void k_tri(TriOp op, const double* __restrict__ F, double* U, int ld,
 // pivot and response tables (shared by a mode's chunks) are staged in shared memory, and the
 // result is stored straight to U.  Same arithmetic as k_tri.  In place allowed: a thread
 // writes only the rows it read, after the CTA's barriers.
-constexpr int kTriMaxM = 31;   // interfaces (C-1) the register prefetch holds
-template <int S>
+// TAIL: the last chunk has op.r < S rows.
+template <int S, bool TAIL>
 __device__ __forceinline__ void tri_reg_body(const TriOp& op, const double* __restrict__ F, double* U, int ld, int Mb,
                                              const TriBc& bc, double* sm) {
   const int C = op.C, d = S + 1, nx = op.nx;
@@ -251,9 +296,11 @@ __device__ __forceinline__ void tri_reg_body(const TriOp& op, const double* __re
   double* plast = pfirst + C * Mb;
   double* hv = plast + C * Mb;             // (C+1) x Mb
   double* yv = hv + (C + 1) * Mb;          // (C+1) x Mb
+  double* t_gT = yv + (C + 1) * Mb;        // S x Mb (TAIL)
   const int k0 = blockIdx.x * Mb, nthr = blockDim.x;
   const int t = threadIdx.x, kl = t % Mb, c = t / Mb;
   const int k = min(k0 + kl, nx - 1);
+  const int len = TAIL && c == C - 1 ? op.r : S;
   const bool chunk = c < C, store = chunk && k0 + kl < nx;
   const int r0 = c * d;
   // the tables are constant (built at creation): fetched before the wait for the previous
@@ -265,15 +312,17 @@ __device__ __forceinline__ void tri_reg_body(const TriOp& op, const double* __re
   for (int q = t; q < 3 * S * Mb; q += nthr) {
     const int row = q / Mb, kk = q - row * Mb;
     t_inv[q] = __ldg(op.inv + (size_t)row * nx + min(k0 + kk, nx - 1));
+    if (TAIL && row < S) t_gT[q] = __ldg(op.gT + (size_t)row * nx + min(k0 + kk, nx - 1));
   }
   IB_GRID_DEP_WAIT();
   double f[S];
 #pragma unroll
-  for (int j = 0; j < S; ++j) f[j] = chunk ? F[(size_t)(r0 + j) * ld + k] : 0.0;
+  for (int j = 0; j < S; ++j) f[j] = chunk && (!TAIL || j < len) ? F[(size_t)(r0 + j) * ld + k] : 0.0;
   double fi = (chunk && c >= 1) ? F[(size_t)(r0 - 1) * ld + k] : 0.0;
   if (chunk && bc.add2) {
 #pragma unroll
-    for (int j = 0; j < S; ++j) f[j] = f[j] + bc.add2[(size_t)(r0 + j) * ld + k];
+    for (int j = 0; j < S; ++j)
+      if (!TAIL || j < len) f[j] = f[j] + bc.add2[(size_t)(r0 + j) * ld + k];
     if (c >= 1) fi = fi + bc.add2[(size_t)(r0 - 1) * ld + k];
   }
   if (chunk && (bc.sd || bc.post_scale != 1.0)) {
@@ -284,10 +333,15 @@ __device__ __forceinline__ void tri_reg_body(const TriOp& op, const double* __re
       const double a = __ldg(bc.sk2 + k);
       const double* sdk = bc.sd + (k & 1) * op.ny;
 #pragma unroll
-      for (int j = 0; j < S; ++j) f[j] = fma(a, sdk[r0 + j], ps == 1.0 ? f[j] : ps * f[j]);
+      for (int j = 0; j < S; ++j)
+        if (!TAIL || j < len) f[j] = fma(a, sdk[r0 + j], ps == 1.0 ? f[j] : ps * f[j]);
       if (c >= 1) fi = fma(a, sdk[r0 - 1], ps == 1.0 ? fi : ps * fi);
       if (c == 0) f[0] += bc.edge[k];
-      if (c == C - 1) f[S - 1] += bc.edge[nx + k];
+      if (c == C - 1) {
+#pragma unroll
+        for (int j = 0; j < S; ++j)
+          if (j == len - 1) f[j] += bc.edge[nx + k];
+      }
     } else {
 #pragma unroll
       for (int j = 0; j < S; ++j) f[j] *= ps;
@@ -308,7 +362,7 @@ __device__ __forceinline__ void tri_reg_body(const TriOp& op, const double* __re
     double u = dp;
 #pragma unroll
     for (int j = S - 2; j >= 0; --j) {
-      u = fma(t_inv[j * Mb + kl], u, f[j]);
+      u = !TAIL || j < len - 1 ? fma(t_inv[j * Mb + kl], u, f[j]) : f[j];
       f[j] = u;
     }
     pfirst[c * Mb + kl] = u;
@@ -343,44 +397,45 @@ __device__ __forceinline__ void tri_reg_body(const TriOp& op, const double* __re
   if (store) {
     const double yl = yv[c * Mb + kl], yr = yv[(c + 1) * Mb + kl];
     double* dst = U + k;
+    const double* tg = TAIL && c == C - 1 ? t_gT : t_gL;
 #pragma unroll
     for (int j = 0; j < S; ++j) {
       double u = f[j];
-      u = fma(yl, t_gL[j * Mb + kl], u);
-      u = fma(yr, t_gL[(S - 1 - j) * Mb + kl], u);
-      dst[(size_t)(r0 + j) * ld] = u;
+      u = fma(yl, tg[j * Mb + kl], u);
+      u = fma(yr, t_gL[(S - 1 - j) * Mb + kl], u);   // the last chunk's right end value is 0
+      if (!TAIL || j < len) dst[(size_t)(r0 + j) * ld] = u;
     }
     if (c >= 1) dst[(size_t)(r0 - 1) * ld] = yl;
   }
 }
 
-template <int S>
+template <int S, bool TAIL>
 __global__ void __launch_bounds__(256) k_tri_reg(TriOp op, const double* __restrict__ F, double* U, int ld, int Mb,
                                                  TriBc bc) {
   extern __shared__ double sm[];
-  tri_reg_body<S>(op, F, U, ld, Mb, bc, sm);   // waits for the previous kernel after its tables
+  tri_reg_body<S, TAIL>(op, F, U, ld, Mb, bc, sm);   // waits for the previous kernel after its tables
 }
 
 // The same solve for every item of a batch, blockIdx.y picking the item (its tables, input,
 // output and boundary terms); the items share the chunking.
-template <int S>
+template <int S, bool TAIL>
 __global__ void __launch_bounds__(256) k_tri_reg_batch(const __grid_constant__ TriBatch b, int ld, int Mb) {
   extern __shared__ double sm[];
   const int y = blockIdx.y;
-  tri_reg_body<S>(b.op[y], b.F[y], b.U[y], ld, Mb, b.bc[y], sm);
+  tri_reg_body<S, TAIL>(b.op[y], b.F[y], b.U[y], ld, Mb, b.bc[y], sm);
 }
 
 static size_t tri_reg_smem(const TriOp& op, int Mb) {
-  return sizeof(double) * (size_t)Mb * (3 * (size_t)op.s + 2 * (size_t)op.C + 2 * ((size_t)op.C + 1));
+  return sizeof(double) * (size_t)Mb * ((op.r < op.s ? 4 : 3) * (size_t)op.s + 2 * (size_t)op.C + 2 * ((size_t)op.C + 1));
 }
 
-template <int S>
+template <int S, bool TAIL>
 static int launch_tri_reg(const TriOp& op, const double* F, double* U, int ld, int Mb, int threads, const TriBc& bc,
                           cudaStream_t st) {
   const size_t smem = tri_reg_smem(op, Mb);
-  if (allow_dyn_smem(k_tri_reg<S>, smem) != cudaSuccess) return IB_ERR_CUDA;
+  if (allow_dyn_smem(k_tri_reg<S, TAIL>, smem) != cudaSuccess) return IB_ERR_CUDA;
   count_launch();
-  k_tri_reg<S><<<cdiv(op.nx, Mb), threads, smem, st>>>(op, F, U, ld, Mb, bc);
+  k_tri_reg<S, TAIL><<<cdiv(op.nx, Mb), threads, smem, st>>>(op, F, U, ld, Mb, bc);
   IB_CUDA_CHECK(cudaGetLastError());
   return IB_OK;
 }
@@ -400,16 +455,21 @@ int tri_solve(const TriOp& op, const double* F, double* U, int ld, const TriLaun
     // at most 256 threads (the register-resident chunk needs the registers)
     const int Mr = std::max(1, std::min(Mb, 256 / op.C));
     const int tr = ((Mr * op.C + 31) / 32) * 32;
+    const bool tail = op.r < op.s;
     switch (op.s) {
 #define IB_TRI_REG(SS) \
-      case SS: return launch_tri_reg<SS>(op, F, U, ld, Mr, tr, bc, st);
-      IB_TRI_REG(1) IB_TRI_REG(2) IB_TRI_REG(3) IB_TRI_REG(4) IB_TRI_REG(5) IB_TRI_REG(6) IB_TRI_REG(7)
-      IB_TRI_REG(8) IB_TRI_REG(9) IB_TRI_REG(11) IB_TRI_REG(12) IB_TRI_REG(14) IB_TRI_REG(15) IB_TRI_REG(19)
-      IB_TRI_REG(23) IB_TRI_REG(24) IB_TRI_REG(29) IB_TRI_REG(31) IB_TRI_REG(39)
+      case SS: if (!tail) return launch_tri_reg<SS, false>(op, F, U, ld, Mr, tr, bc, st); break;
+      IB_TRI_EVEN(IB_TRI_REG)
+#undef IB_TRI_REG
+#define IB_TRI_REG(SS) \
+      case SS: return tail ? launch_tri_reg<SS, true>(op, F, U, ld, Mr, tr, bc, st) \
+                           : launch_tri_reg<SS, false>(op, F, U, ld, Mr, tr, bc, st);
+      IB_TRI_BOTH(IB_TRI_REG)
 #undef IB_TRI_REG
       default: break;
     }
   }
+  if (op.r < op.s) return IB_ERR_ARG;   // tri_chunking gives the shared-memory kernel equal chunks
   size_t smem = tri_smem(op, Mb);
   if (allow_dyn_smem(k_tri, smem) != cudaSuccess) return IB_ERR_CUDA;
   count_launch();
@@ -418,23 +478,18 @@ int tri_solve(const TriOp& op, const double* F, double* U, int ld, const TriLaun
   return IB_OK;
 }
 
-template <int S>
+template <int S, bool TAIL>
 static int launch_tri_reg_batch(const TriBatch& b, int ld, int Mb, int threads, cudaStream_t st) {
   const size_t smem = tri_reg_smem(b.op[0], Mb);
-  if (allow_dyn_smem(k_tri_reg_batch<S>, smem) != cudaSuccess) return IB_ERR_CUDA;
+  if (allow_dyn_smem(k_tri_reg_batch<S, TAIL>, smem) != cudaSuccess) return IB_ERR_CUDA;
   count_launch();
-  k_tri_reg_batch<S><<<dim3(cdiv(b.op[0].nx, Mb), b.n), threads, smem, st>>>(b, ld, Mb);
+  k_tri_reg_batch<S, TAIL><<<dim3(cdiv(b.op[0].nx, Mb), b.n), threads, smem, st>>>(b, ld, Mb);
   IB_CUDA_CHECK(cudaGetLastError());
   return IB_OK;
 }
 
 bool tri_batch_supported(const TriOp& op) {
-  if (op.C - 1 > kTriMaxM || op.C > 256) return false;
-  switch (op.s) {
-    case 1: case 2: case 3: case 4: case 5: case 6: case 7: case 8: case 9: case 11: case 12: case 14:
-    case 15: case 19: case 23: case 24: case 29: case 31: case 39: return true;
-    default: return false;
-  }
+  return op.C - 1 <= kTriMaxM && op.C <= 256 && tri_reg_length(op.s, op.r < op.s);
 }
 
 int tri_solve_batch(const TriBatch& b, int ld, const TriLaunch& L, cudaStream_t st) {
@@ -445,12 +500,16 @@ int tri_solve_batch(const TriBatch& b, int ld, const TriLaunch& L, cudaStream_t 
     if (b.op[i].nx != o.nx || b.op[i].ny != o.ny || b.op[i].s != o.s || b.op[i].C != o.C) return IB_ERR_ARG;
   const int Mr = std::max(1, std::min(L.Mb, 256 / o.C));
   const int tr = ((Mr * o.C + 31) / 32) * 32;
+  const bool tail = o.r < o.s;
   switch (o.s) {
 #define IB_TRI_REG(SS) \
-    case SS: return launch_tri_reg_batch<SS>(b, ld, Mr, tr, st);
-    IB_TRI_REG(1) IB_TRI_REG(2) IB_TRI_REG(3) IB_TRI_REG(4) IB_TRI_REG(5) IB_TRI_REG(6) IB_TRI_REG(7)
-    IB_TRI_REG(8) IB_TRI_REG(9) IB_TRI_REG(11) IB_TRI_REG(12) IB_TRI_REG(14) IB_TRI_REG(15) IB_TRI_REG(19)
-    IB_TRI_REG(23) IB_TRI_REG(24) IB_TRI_REG(29) IB_TRI_REG(31) IB_TRI_REG(39)
+    case SS: return tail ? IB_ERR_ARG : launch_tri_reg_batch<SS, false>(b, ld, Mr, tr, st);
+    IB_TRI_EVEN(IB_TRI_REG)
+#undef IB_TRI_REG
+#define IB_TRI_REG(SS) \
+    case SS: return tail ? launch_tri_reg_batch<SS, true>(b, ld, Mr, tr, st) \
+                         : launch_tri_reg_batch<SS, false>(b, ld, Mr, tr, st);
+    IB_TRI_BOTH(IB_TRI_REG)
 #undef IB_TRI_REG
     default: return IB_ERR_ARG;
   }

@@ -14,7 +14,7 @@
 // where c = dt/(2 Delta_k^2 Re) and L the 5-point Laplacian with zero boundary.
 //
 // Every system is tridiag(-1, a_k, -1) of size n-1.  For parallelism it is cut
-// into C chunks of s = n/C - 1 rows separated by C-1 interface rows: each chunk is
+// into C chunks of s rows (the last one of r <= s) separated by C-1 interface rows: each chunk is
 // solved with zero ends (Thomas with tabulated pivots), the interface values then
 // satisfy a constant-coefficient tridiagonal system of size C-1 (solved with its
 // tabulated inverse), and each chunk adds the interface responses (tabulated).
@@ -26,24 +26,32 @@ namespace ib {
 
 struct TriOp {
   int nx = 0, ny = 0;     // modes (m-1), rows (n-1)
-  int s = 0, C = 0;       // chunk rows, chunks: (s+1)*C = ny+1
+  int s = 0, C = 0;       // chunk rows, chunks
+  int r = 0;              // rows of the last chunk: (s+1)(C-1) + r = ny
   double sigma = 1.0;     // right-hand-side scale
   double* inv = nullptr;  // s x nx: 1/pivot
   double* sinv = nullptr; // s x nx: sigma/pivot
   double* gL = nullptr;   // s x nx: chunk response to a unit left end value
   double* rinv = nullptr; // (C-1)^2 x nx: inverse of the interface system, row-major per mode
+  double* gT = nullptr;   // s x nx, r < s only: the last chunk's response to a unit left end value
 };
 
 struct TriLaunch {
   int Mb = 8;             // modes per CTA
 };
 
-// Chunking for ny = n-1 rows (n divisible by 4) and nx modes: C*(s+1) = n.
-void tri_chunking(int n, int nx, int* s, int* C);
+struct TriShape {
+  int s = 0, C = 0, r = 0;
+};
+// Chunking of ny rows and nx modes.  max_doubles > 0: with tables of at most that many doubles.
+TriShape tri_chunking(int ny, int nx, size_t max_doubles = 0);
+// The chunking into equal chunks alone (n = ny + 1 divisible), whose tables size the static solve's
+// limit (static_ctci.cu).
+TriShape tri_chunking_even(int n, int nx);
 // Tables for shifts a_k = 2 + shift_k (k = 0..nx-1), uploaded into caller-provided
 // device memory of tri_table_doubles() doubles.
-size_t tri_table_doubles(int nx, int s, int C);
-int tri_build(TriOp* op, int nx, int ny, const double* shift, double sigma, double* dev_mem);
+size_t tri_table_doubles(int nx, const TriShape& t);
+int tri_build(TriOp* op, int nx, int ny, const TriShape& t, const double* shift, double sigma, double* dev_mem);
 // Boundary terms a solve adds to its right-hand side as it loads it (a finer level of the
 // coarse-to-fine recursions, dst_ring_edge_from_modes): row r of mode k is
 //     post_scale (F[r][k] + add2[r][k]) + sk2[k] sd[(k & 1) ny + r]
