@@ -48,6 +48,8 @@ struct PressureOp {
   std::vector<double*> rhs, p, oqx, oqy, nlx, nly;   // per level
   double *y = nullptr, *tmp = nullptr, *hx = nullptr, *hy = nullptr, *fdt = nullptr;
   double *ubc = nullptr, *vbc = nullptr, *ring = nullptr;
+  double *Wd = nullptr, *fold = nullptr;   // the x transform's bf16 digits of sin and of a level's rows
+  int* ex = nullptr;                       // the rows' exponents
 };
 
 // The buffers and the stream one application of the Schur operator's fluid part works in

@@ -7,15 +7,17 @@
 // (coarsify_pressure).  The solve on one level, ddti (myfft.F90:192-203), is the 2-D DST-I of
 // the m x n cell grid with the eigenvalues of D D^T: as for ctci, the y direction is a per-mode
 // tridiagonal solve, and the x direction -- length m, whose m + 1 (801 at 800 cells) the FFT's
-// radices 2, 3, 5 do not divide -- is a product with the DST-I matrix W (m x m), with FP64 FMAs:
-// the same product on the FP64 tensor cores (mma.sync m8n8k4, kept as the measured alternative)
-// ran 686 us against 623 us at 800 x 400 on GB300, whose FP64 tensor path is no faster than its
-// FP64 pipe.  Arithmetic follows the reference's expressions: products
+// radices 2, 3, 5 do not divide -- is a product with the DST-I matrix, its factors split into bf16 digits
+// for the tensor cores (k_pfold, k_pprod).  The same product in FP64 is kept as the measured alternative: with FMAs
+// 623 us at 800 x 400, on the FP64 tensor cores (mma.sync m8n8k4) 686 us, GB300's FP64 tensor path
+// being no faster than its FP64 pipe.  Arithmetic follows the reference's expressions: products
 // that the reference rounds before a sum are rounded separately here (no contraction).
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "ctx.cuh"
+#include "fixed.cuh"
 
 namespace ib {
 
@@ -114,6 +116,203 @@ static int launch_pgemm(bool mma, int R, int N, int K, const double* A, int lda,
   return cudaGetLastError() == cudaSuccess ? IB_OK : IB_ERR_CUDA;
 }
 
+// ------------------------------------------------------------------ x transform on the tensor cores
+// Y_k = 2 sum_j x_j sin(pi j k / M), M = m + 1 odd.  sin(pi (M - j) k / M) = -(-1)^k sin(pi j k / M),
+// so odd k take u_j = x_j + x_(M-j) and even k take v_j = x_j - x_(M-j), j = 1..m/2: two products with
+// m/2 x m/2 matrices, half the multiply-adds.  Both factors are 53-bit integers (of the row's exponent,
+// and of 1) cut into eight balanced digits of 7 bits, which bf16 holds exactly; the products of digits
+// i and j with i + j = p <= 7 sum in one FP32 accumulator, exactly (8 products x 64^2 x 512 terms =
+// 2^24), and the eight accumulators of an output combine in 64-bit integers.  What is left out (p > 7)
+// is below a unit of the 53rd bit, so the result is nearer the exact product than the FP64 sum was.
+// 36 bf16 products take the place of one in FP64, at a rate over 300 times higher (the splitting is
+// the error-free one of Ozaki, Ogita, Oishi and Rump, 2012).
+// What bounds it: the latency of its dependent steps (tensor pipe 41% busy).  Measured at 800 x 400: 55 us
+// and 5 us for the folding, against 621 us with FP64 FMAs and 99 us with 32 x 32-bit integer
+// multiply-adds; in steps of 32 terms (82 KB a CTA, a second wave of 34 CTAs) 68 us.
+constexpr int kDigits = 8;
+// The CTA's tile (two warps of 16 x 32) and step: 338 CTAs at 800 x 400, all resident at once (49 KB each).
+constexpr int kQM = 32, kQN = 32, kQK = 16;
+constexpr int kQPitch = kQK + 8;              // bf16 a staged row: 48 bytes, no bank conflicts for ldmatrix
+constexpr int kQChunk = 512;                  // terms the accumulators hold exactly
+
+// v (|v| <= 2^53) in digits of 7 bits, the last one least
+__host__ __device__ __forceinline__ void p_digits(fx v, int* d) {
+#pragma unroll
+  for (int i = kDigits - 1; i > 0; --i) {
+    d[i] = (int)(((v + 64) & 127) - 64);
+    v = (v - d[i]) >> 7;
+  }
+  d[0] = (int)v;
+}
+// the bf16 of a small integer
+__host__ __device__ __forceinline__ unsigned short p_bf16(int d) {
+  const float f = (float)d;
+#if defined(__CUDA_ARCH__)
+  return (unsigned short)(__float_as_uint(f) >> 16);
+#else
+  unsigned u;
+  memcpy(&u, &f, 4);
+  return (unsigned short)(u >> 16);
+#endif
+}
+
+// Row blockIdx.x of an R x m field: its exponent, and the digits of u_j and v_j: [u, v][digit][row][j],
+// rows and terms padded (Rp, Kp) with zeros that nothing writes.
+__global__ void __launch_bounds__(256) k_pfold(int m, int Rp, int Kp, const double* __restrict__ A,
+                                               unsigned short* __restrict__ fold, int* __restrict__ ex) {
+  IB_GRID_DEP_WAIT();
+  __shared__ int s_e;
+  const int r = blockIdx.x, H = m / 2;
+  const long long* x = reinterpret_cast<const long long*>(A) + (size_t)r * m;
+  if (threadIdx.x == 0) s_e = 1;
+  __syncthreads();
+  int e = 1;
+  for (int j = threadIdx.x; j < m; j += blockDim.x) e = max(e, fx_exponent((unsigned)((unsigned long long)x[j] >> 32)));
+  e = __reduce_max_sync(0xffffffffu, e);
+  if ((threadIdx.x & 31) == 0) atomicMax(&s_e, e);
+  __syncthreads();
+  e = s_e;
+  if (threadIdx.x == 0) ex[r] = e;
+  const size_t plane = (size_t)Rp * Kp;
+  for (int j = threadIdx.x; j < H; j += blockDim.x) {
+    const fx a = fx_from_bits(x[j], e), b = fx_from_bits(x[m - 1 - j], e);   // below 2^56
+    int du[kDigits], dv[kDigits];
+    p_digits(fx_shr(a + b, kFxFrac - 52), du);
+    p_digits(fx_shr(a - b, kFxFrac - 52), dv);
+    unsigned short* u = fold + (size_t)r * Kp + j;
+#pragma unroll
+    for (int i = 0; i < kDigits; ++i) {
+      u[i * plane] = p_bf16(du[i]);
+      u[(kDigits + i) * plane] = p_bf16(dv[i]);
+    }
+  }
+}
+
+__device__ __forceinline__ unsigned p_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void p_ldmatrix(unsigned* r, unsigned addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+__device__ __forceinline__ void p_mma(float* c, const unsigned* a, const unsigned* b) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+               "{%0, %1, %2, %3};\n"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
+// C = the folded rows times the digits of sin, of parity blockIdx.z ([digit][output c][term j], padded
+// to Np x Kp): outputs k = 2c+1 (z = 0) or 2c+2.  LONG: more than kQChunk terms, combined chunk by chunk
+// with `shift` bits dropped.
+template <bool LONG>
+__global__ void __launch_bounds__(64) k_pprod(int R, int m, int Rp, int Np, int Kp,
+                                              const unsigned short* __restrict__ fold,
+                                              const unsigned short* __restrict__ Wd, const int* __restrict__ ex,
+                                              double* __restrict__ C, int shift) {
+  IB_GRID_DEP_WAIT();
+  extern __shared__ __align__(16) unsigned short stage[];   // two stages of A and B: [digit][row][kQPitch]
+  constexpr int kPart = kDigits * kQM * kQPitch;            // one operand of one stage
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int H = m / 2, r0 = blockIdx.y * kQM, c0 = blockIdx.x * kQN;
+  const unsigned short* A = fold + (size_t)blockIdx.z * kDigits * Rp * Kp + (size_t)r0 * Kp;
+  const unsigned short* B = Wd + (size_t)blockIdx.z * kDigits * Np * Kp + (size_t)c0 * Kp;
+  auto load = [&](int k0, int s) {
+    unsigned short* sa = stage + s * 2 * kPart;
+    unsigned short* sb = sa + kPart;
+    for (int t = tid; t < kDigits * kQM * (kQK / 8); t += 64) {   // 16 bytes each
+      const int q = t % (kQK / 8), row = t / (kQK / 8) % kQM, d = t / (kQK / 8 * kQM);
+      const unsigned off = (unsigned)((d * kQM + row) * kQPitch + q * 8);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(p_smem(sa + off)),
+                   "l"(A + ((size_t)d * Rp + row) * Kp + k0 + q * 8));
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(p_smem(sb + off)),
+                   "l"(B + ((size_t)d * Np + row) * Kp + k0 + q * 8));
+    }
+    asm volatile("cp.async.commit_group;\n");
+  };
+  float acc[kDigits][4][4];
+  fx tot[4][4];
+#pragma unroll
+  for (int p = 0; p < kDigits; ++p)
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[p][n][q] = 0.0f;
+  // sum_p acc_p 2^(7 (7 - p)) in units 2^3 (of the products' 2^49), which the 53 x 53-bit terms need
+  auto combine = [&](int n, int q) {
+    fx v = 0;
+#pragma unroll
+    for (int p = 0; p < kDigits - 1; ++p) v += (fx)__float2int_rn(acc[p][n][q]) << (7 * (kDigits - 1 - p) - 3);
+    return v + fx_shr((fx)__float2int_rn(acc[kDigits - 1][n][q]), 3);
+  };
+  if (LONG) {
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) tot[n][q] = 0;
+  }
+  load(0, 0);
+  const int steps = Kp / kQK;
+  for (int s = 0; s < steps; ++s) {
+    if (s + 1 < steps) {
+      load((s + 1) * kQK, (s + 1) & 1);
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    }
+    __syncthreads();
+    const unsigned short* sa = stage + (s & 1) * 2 * kPart + warp * 16 * kQPitch;
+    const unsigned short* sb = stage + (s & 1) * 2 * kPart + kPart;
+#pragma unroll
+    for (int kk = 0; kk < kQK; kk += 16) {
+      unsigned a[kDigits][4];
+#pragma unroll
+      for (int d = 0; d < kDigits; ++d)   // rows 0-7, 8-15 at kk, then at kk + 8
+        p_ldmatrix(a[d], p_smem(sa + (d * kQM + (lane & 15)) * kQPitch + kk + (lane >> 4) * 8));
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        unsigned b[kDigits][4];
+#pragma unroll
+        for (int d = 0; d < kDigits; ++d)   // outputs 0-7 at kk, kk + 8, then outputs 8-15
+          p_ldmatrix(b[d], p_smem(sb + (d * kQN + h * 16 + (lane >> 4) * 8 + (lane & 7)) * kQPitch + kk +
+                                  ((lane >> 3) & 1) * 8));
+#pragma unroll
+        for (int i = 0; i < kDigits; ++i)
+#pragma unroll
+          for (int j = 0; j < kDigits - i; ++j) {
+            p_mma(acc[i + j][2 * h], a[i], b[j]);
+            p_mma(acc[i + j][2 * h + 1], a[i], b[j] + 2);
+          }
+      }
+    }
+    if (LONG && ((s + 1) * kQK % kQChunk == 0 || s + 1 == steps)) {
+#pragma unroll
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          tot[n][q] += fx_shr(combine(n, q), shift);
+#pragma unroll
+          for (int p = 0; p < kDigits; ++p) acc[p][n][q] = 0.0f;
+        }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int n = 0; n < 4; ++n)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int r = r0 + warp * 16 + (lane >> 2) + (q >> 1) * 8, c = c0 + n * 8 + 2 * (lane & 3) + (q & 1);
+      if (r >= R || c >= H) continue;
+      // terms are (53-bit value) (53-bit sine) 2^(e - 1075 + (kFxFrac - 52) - (kFxFrac - 53)) 2^-53, twice
+      const fx v = LONG ? tot[n][q] : combine(n, q);
+      const long long y = ex[r] < 2047 ? fx_to_bits(v, ex[r] - 1074 + shift) : 0x7ff8000000000000LL;
+      reinterpret_cast<long long*>(C)[(size_t)r * m + 2 * c + blockIdx.z] = y;
+    }
+}
+constexpr size_t kQSmem = sizeof(unsigned short) * 4 * kDigits * kQM * kQPitch;
+
+// padded sizes of an n x m field's folded rows and of the sine digits
+static int p_pad(int v) { return (v + 31) / 32 * 32; }
+
 // ------------------------------------------------------------------ stencils
 // velocity-squared term fac ((qx(i+1,j)+qx(i,j))^2 + (qy(i,j+1)+qy(i,j))^2) of cell (i, j)
 // (1-based), q = q + q0 (get_bc_phi1 :731-767, static_plus_dynamic :842-853); every product
@@ -150,19 +349,30 @@ __device__ __forceinline__ double ghosted(const GridDims& g, const double* f, co
   return f[(J - 2) * g.nsx + (I - 2)];
 }
 
-// nonlinear_corner2edge (:459-501) divided by del^2: u-faces then v-faces
+// x / d for a constant d, r = 1/d to nearest: one step q + (x - q d) r on q = x r rounds as the
+// quotient does where q is within a unit of it (Markstein, IBM J. Res. Dev. 34, 1990, theorem 8.1),
+// and within a unit of it otherwise (none of 1.6e8 random quotients by grid spacings differed).  Three
+// FP64 operations; away from the middle of the exponent range, the division.
+__device__ __forceinline__ double p_div_const(double x, double d, double r) {
+  const double q = x * r;
+  const unsigned e = ((unsigned)__double2hiint(q) >> 20) & 0x7ffu;
+  return e - 100u < 1847u ? fma(fma(-q, d, x), r, q) : x / d;
+}
+
+// nonlinear_corner2edge (:459-501) divided by del^2: u-faces then v-faces; d2 = 2 del^2 takes the mean's
+// half with it, exactly
 __global__ void k_p_corner2edge(GridDims g, const double* __restrict__ oqx, const double* __restrict__ oqy,
-                                const double* __restrict__ ubc, const double* __restrict__ vbc, double d2,
+                                const double* __restrict__ ubc, const double* __restrict__ vbc, double d2, double r2,
                                 double* __restrict__ nlx, double* __restrict__ nly) {
   IB_GRID_DEP_WAIT();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < g.nu) {
     const int i = t % g.nux + 1, j = t / g.nux + 1;
-    nlx[t] = 0.5 * (ghosted(g, oqx, ubc, i, j + 1) + ghosted(g, oqx, ubc, i, j)) / d2;
+    nlx[t] = p_div_const(ghosted(g, oqx, ubc, i, j + 1) + ghosted(g, oqx, ubc, i, j), d2, r2);
   } else if (t < g.nu + g.nv) {
     const int s = t - g.nu;
     const int i = s % g.nvx + 1, j = s / g.nvx + 1;
-    nly[s] = 0.5 * (ghosted(g, oqy, vbc, i + 1, j) + ghosted(g, oqy, vbc, i, j)) / d2;
+    nly[s] = p_div_const(ghosted(g, oqy, vbc, i + 1, j) + ghosted(g, oqy, vbc, i, j), d2, r2);
   }
 }
 
@@ -285,7 +495,8 @@ static int pressure_setup(Ctx* c) {
   const size_t tri_n = tri_table_doubles(m, tri_t);
   const size_t dbl = (size_t)m * m + tri_n + 2 * (size_t)L * cells + 2 * cells + 2 * (size_t)L * g.ns +
                      (size_t)L * (g.nu + g.nv) + g.nu + g.nv + (size_t)std::max(c->nf, 1) + 2 * (size_t)g.nbc +
-                     2 * (size_t)(m + n) + 64;
+                     2 * (size_t)(m + n) + 64 + 4 * (size_t)p_pad(m / 2) * p_pad(m / 2) +
+                     4 * (size_t)p_pad(n) * p_pad(m / 2) + (size_t)n + 16;
   IB_CUDA_CHECK(cudaMalloc(&P.mem, 8 * dbl));
   IB_CUDA_CHECK(cudaMemset(P.mem, 0, 8 * dbl));
   double* q = P.mem;
@@ -301,6 +512,9 @@ static int pressure_setup(Ctx* c) {
   P.fdt = take(std::max(c->nf, 1));
   P.ubc = take(g.nbc); P.vbc = take(g.nbc);
   P.ring = take(2 * (size_t)(m + n));
+  P.Wd = take(4 * (size_t)p_pad(m / 2) * p_pad(m / 2));   // 2 parities x 8 digits x 2 bytes
+  P.fold = take(4 * (size_t)p_pad(n) * p_pad(m / 2));
+  P.ex = reinterpret_cast<int*>(take(n));
   // W[j][k] = 2 sin(pi (j+1)(k+1) / (m+1)), the DST-I matrix of length m (symmetric)
   {
     std::vector<double> W((size_t)m * m), tab(2 * (size_t)(m + 1));
@@ -311,6 +525,21 @@ static int pressure_setup(Ctx* c) {
       for (int k = 0; k < m; ++k)   // sin(pi r / M) is 2M-periodic in r
         W[(size_t)j * m + k] = tab[((long long)(j + 1) * (k + 1)) % (2 * M)];
     IB_CUDA_CHECK(cudaMemcpy(P.W, W.data(), 8 * W.size(), cudaMemcpyHostToDevice));
+    // the digits of sin(pi (j+1) k / M) 2^53 by parity (k_pprod)
+    const int H = m / 2, Hp = p_pad(H);
+    std::vector<int> digit(2 * (size_t)M * kDigits);
+    for (long long r = 0; r < 2 * M; ++r) {
+      const long double s = sinl(PI_L * (long double)r / (long double)M) * 9007199254740992.0L;
+      p_digits((fx)(s < 0 ? s - 0.5L : s + 0.5L), digit.data() + r * kDigits);
+    }
+    std::vector<unsigned short> wd(2 * (size_t)kDigits * Hp * Hp, 0);
+    for (int z = 0; z < 2; ++z)
+      for (int q = 0; q < H; ++q)
+        for (int j = 0; j < H; ++j) {
+          const int* d = digit.data() + ((long long)(j + 1) * (2 * q + 1 + z)) % (2 * M) * kDigits;
+          for (int i = 0; i < kDigits; ++i) wd[(((size_t)z * kDigits + i) * Hp + q) * Hp + j] = p_bf16(d[i]);
+        }
+    IB_CUDA_CHECK(cudaMemcpy(P.Wd, wd.data(), sizeof(unsigned short) * wd.size(), cudaMemcpyHostToDevice));
   }
   // ddti = S_x S_y [1 / (lam N)] S_y S_x with lam = -(lx + ly), N = 4 (m+1)(n+1); with
   // S_y diag(1/(lx + ly)) S_y = 2 (n+1) (lx + T_y)^-1, T_y = tridiag(-1, 2, -1) of n rows:
@@ -334,14 +563,35 @@ void pressure_free(Ctx* c) {
   c->pres = PressureOp{};
 }
 
-static int ddti(Ctx* c, const double* rhs, double* out, bool mma) {
+// out = the DST-I along x of the n rows of in
+static int p_transform(Ctx* c, const double* in, double* out) {
   PressureOp& P = c->pres;
-  const int m = c->g.m, n = c->g.n;
-  RC(launch_pgemm(mma, n, m, m, rhs, m, P.W, m, P.y, m, c->st));
+  const int m = c->g.m, n = c->g.n, H = m / 2, Hp = p_pad(H), Rp = p_pad(n);
+  unsigned short* fold = reinterpret_cast<unsigned short*>(P.fold);
+  const unsigned short* Wd = reinterpret_cast<const unsigned short*>(P.Wd);
+  int shift = 0;   // bits by which a sum of H terms may pass one of kQChunk
+  while ((kQChunk << shift) < H) ++shift;
+  const dim3 grid(Hp / kQN, Rp / kQM, 2);
+  count_launches(2);
+  k_pfold<<<n, 256, 0, c->st>>>(m, Rp, Hp, in, fold, P.ex);
+  if (H > kQChunk) {
+    if (allow_dyn_smem(k_pprod<true>, kQSmem) != cudaSuccess) return IB_ERR_CUDA;
+    k_pprod<true><<<grid, 64, kQSmem, c->st>>>(n, m, Rp, Hp, Hp, fold, Wd, P.ex, out, shift);
+  } else {
+    if (allow_dyn_smem(k_pprod<false>, kQSmem) != cudaSuccess) return IB_ERR_CUDA;
+    k_pprod<false><<<grid, 64, kQSmem, c->st>>>(n, m, Rp, Hp, Hp, fold, Wd, P.ex, out, shift);
+  }
+  return cudaGetLastError() == cudaSuccess ? IB_OK : IB_ERR_CUDA;
+}
+
+static int ddti(Ctx* c, const double* rhs, double* out) {
+  PressureOp& P = c->pres;
+  const int m = c->g.m;
+  RC(p_transform(c, rhs, P.y));
   TriLaunch T;
   T.Mb = 8;
   RC(tri_solve(P.tri, P.y, P.y, m, T, c->st));
-  return launch_pgemm(mma, n, m, m, P.y, m, P.W, m, out, m, c->st);
+  return p_transform(c, P.y, out);
 }
 
 int op_pressure(Ctx* c) {
@@ -367,8 +617,8 @@ int op_pressure(Ctx* c) {
     }
     const double d = c->delta * (double)(1 << k);
     count_launch();
-    k_p_corner2edge<<<cdiv(g.nu + g.nv, B), B, 0, st>>>(g, P.oqx[k], P.oqy[k], P.ubc, P.vbc, d * d, P.nlx[k],
-                                                        P.nly[k]);
+    k_p_corner2edge<<<cdiv(g.nu + g.nv, B), B, 0, st>>>(g, P.oqx[k], P.oqy[k], P.ubc, P.vbc, 2.0 * (d * d), 0.5 / (d * d),
+                                                        P.nlx[k], P.nly[k]);
   }
   // -D E^T f / dt on the finest level, restricted onto the coarser ones, then D N(q) added
   IB_CUDA_CHECK(cudaMemsetAsync(P.rhs[0], 0, 8 * cells, st));
@@ -402,7 +652,7 @@ int op_pressure(Ctx* c) {
     }
     count_launch();
     k_p_apply_bc<<<cdiv(cells, B), B, 0, st>>>(g, P.rhs[k], P.ring);
-    RC(ddti(c, P.rhs[k], P.p[k], false));
+    RC(ddti(c, P.rhs[k], P.p[k]));
   }
   for (int k = 0; k < L; ++k) {
     const double d = c->delta * std::pow(2.0, k);
