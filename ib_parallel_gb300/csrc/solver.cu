@@ -600,6 +600,7 @@ int op_vort2flux(Ctx* c, double* const* w, double* const* s, double* const* qx, 
       TriBc bc;
       if (k < L - 1) bc = level_bc(c, k, k == 0 && skip0 ? 2.0 * g.m : 1.0);
       if (k == 0 && skip0) bc.add2 = hat0_add;
+      bc.early = k < L - 1;   // the modes are the batched transform's (or the predictor's), before level k+1's ring
       {
         ProfScope ps(c, 1, pass_bytes(c, 1, 1));
         RC(tri_solve(c->tri_ctci, modes(k), F, g.nsx, c->tl, st, bc));
@@ -1434,6 +1435,7 @@ static int op_predict_levels(Ctx* c, bool seed_rhs_old) {
       // its boundary terms, added by the solve
       TriBc bc;
       if (k < L - 1) bc = level_bc(c, k, 1.0);
+      bc.early = k < L - 1;   // the transform's modes, before level k+1's ring
       {
         ProfScope ps(c, 1, pass_bytes(c, 1, 1));
         RC(tri_solve(c->tri_pred[k], F, F, g.nsx, c->tl, st, bc));

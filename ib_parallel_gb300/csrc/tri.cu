@@ -12,7 +12,7 @@ namespace ib {
 // shorter last chunk.
 #define IB_TRI_EVEN(X) X(1) X(2) X(4) X(5) X(6) X(8) X(9) X(12) X(14) X(24) X(29)
 #define IB_TRI_BOTH(X) X(3) X(7) X(11) X(15) X(19) X(23) X(31) X(39) X(63)
-constexpr int kTriMaxM = 31;   // interfaces (C-1) the register prefetch holds
+constexpr int kTriMaxM = 31;   // most interfaces (C-1) of the register-resident kernel
 
 static bool tri_reg_length(int s, bool tail) {
   switch (s) {
@@ -57,7 +57,7 @@ TriShape tri_chunking_even(int n, int nx) {
 // Of the lengths with a register kernel, the cheapest; a shorter last chunk counts a tenth more (its
 // rows are predicated), and 63 rows, which spill, are taken only where no shorter chunk will do.  The shared-memory kernel took 37 us for 999 modes of 539 rows in its cheapest
 // equal chunks (15 of 35) and 160 us for 800 modes of 400 rows, whose period 401 is prime (one chunk);
-// in 14 chunks of 39 the first takes 22 us, and the second in 13 of 31 12 us.  It remains for more than
+// in 14 chunks of 39 the first takes 19 us, and the second in 13 of 31 12 us.  It remains for more than
 // 32 x 64 rows.
 TriShape tri_chunking(int ny, int nx, size_t max_doubles) {
   TriShape best;
@@ -279,11 +279,20 @@ __global__ void k_tri(TriOp op, const double* __restrict__ F, double* U, int ld,
 
 // The same solve with each thread's chunk in registers (S = op.s known at compile time): the
 // chunk rows and the interface row above are loaded straight from F (all loads in flight at
-// once), the thread's row of the interface inverse is prefetched into registers, only the
-// pivot and response tables (shared by a mode's chunks) are staged in shared memory, and the
-// result is stored straight to U.  Same arithmetic as k_tri.  In place allowed: a thread
-// writes only the rows it read, after the CTA's barriers.
+// once), the tables (pivots and responses, shared by a mode's chunks, and each thread's row of the
+// interface inverse) arrive in shared memory by asynchronous copies meanwhile, and the result is
+// stored straight to U.  Same arithmetic as k_tri.  In place allowed: a thread writes only the
+// rows it read, after the CTA's barriers.
+// What bounds it: the FP64 pipe, 5 S + C - 1 instructions of 64 cycles a warp, and the latency of
+// the loads.  128 registers a thread let every CTA be resident (1535 modes in 32 chunks: 384 CTAs of
+// four warps in one wave; with the inverse's rows in registers, 246 a thread, they took two).
+// Measured, before and after: 1535 modes of 1023 rows 37.2 and 31.5 us; 1599 of 799, 29.2 and 21.5; 999 of
+// 539 (TAIL), 21.9 and 18.5; 799 of 399, 11.0 and 10.4.
 // TAIL: the last chunk has op.r < S rows.
+__device__ __forceinline__ void tri_copy8(double* dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+}
+
 template <int S, bool TAIL>
 __device__ __forceinline__ void tri_reg_body(const TriOp& op, const double* __restrict__ F, double* U, int ld, int Mb,
                                              const TriBc& bc, double* sm) {
@@ -296,7 +305,8 @@ __device__ __forceinline__ void tri_reg_body(const TriOp& op, const double* __re
   double* plast = pfirst + C * Mb;
   double* hv = plast + C * Mb;             // (C+1) x Mb
   double* yv = hv + (C + 1) * Mb;          // (C+1) x Mb
-  double* t_gT = yv + (C + 1) * Mb;        // S x Mb (TAIL)
+  double* t_r = yv + (C + 1) * Mb;         // m x C Mb: row c-1 of a mode's interface inverse, per thread
+  double* t_gT = t_r + m * C * Mb;         // S x Mb (TAIL)
   const int k0 = blockIdx.x * Mb, nthr = blockDim.x;
   const int t = threadIdx.x, kl = t % Mb, c = t / Mb;
   const int k = min(k0 + kl, nx - 1);
@@ -305,16 +315,17 @@ __device__ __forceinline__ void tri_reg_body(const TriOp& op, const double* __re
   const int r0 = c * d;
   // the tables are constant (built at creation): fetched before the wait for the previous
   // kernel, so that under a programmatic edge they arrive while it finishes
-  double rr[kTriMaxM];
-#pragma unroll
-  for (int j = 0; j < kTriMaxM; ++j)
-    rr[j] = (chunk && c >= 1 && j < m) ? __ldg(op.rinv + ((size_t)(c - 1) * m + j) * nx + k) : 0.0;
   for (int q = t; q < 3 * S * Mb; q += nthr) {
-    const int row = q / Mb, kk = q - row * Mb;
-    t_inv[q] = __ldg(op.inv + (size_t)row * nx + min(k0 + kk, nx - 1));
-    if (TAIL && row < S) t_gT[q] = __ldg(op.gT + (size_t)row * nx + min(k0 + kk, nx - 1));
+    const int row = q / Mb, kk = min(k0 + q - row * Mb, nx - 1);
+    tri_copy8(t_inv + q, op.inv + (size_t)row * nx + kk);
+    if (TAIL && row < S) tri_copy8(t_gT + q, op.gT + (size_t)row * nx + kk);
   }
-  IB_GRID_DEP_WAIT();
+  if (chunk && c >= 1) {
+    const double* src = op.rinv + (size_t)(c - 1) * m * nx + k;
+    for (int j = 0; j < m; ++j) tri_copy8(t_r + j * C * Mb + t, src + (size_t)j * nx);
+  }
+  asm volatile("cp.async.commit_group;\n");
+  if (!bc.early) IB_GRID_DEP_WAIT();
   double f[S];
 #pragma unroll
   for (int j = 0; j < S; ++j) f[j] = chunk && (!TAIL || j < len) ? F[(size_t)(r0 + j) * ld + k] : 0.0;
@@ -325,6 +336,7 @@ __device__ __forceinline__ void tri_reg_body(const TriOp& op, const double* __re
       if (!TAIL || j < len) f[j] = f[j] + bc.add2[(size_t)(r0 + j) * ld + k];
     if (c >= 1) fi = fi + bc.add2[(size_t)(r0 - 1) * ld + k];
   }
+  if (bc.early) IB_GRID_DEP_WAIT();
   if (chunk && (bc.sd || bc.post_scale != 1.0)) {
     // boundary terms (tri_rhs) on the chunk rows and the interface row above; row 0 is chunk
     // 0's first row and row ny-1 chunk C-1's last
@@ -337,10 +349,15 @@ __device__ __forceinline__ void tri_reg_body(const TriOp& op, const double* __re
         if (!TAIL || j < len) f[j] = fma(a, sdk[r0 + j], ps == 1.0 ? f[j] : ps * f[j]);
       if (c >= 1) fi = fma(a, sdk[r0 - 1], ps == 1.0 ? fi : ps * fi);
       if (c == 0) f[0] += bc.edge[k];
-      if (c == C - 1) {
+      if (!TAIL && c == C - 1) f[S - 1] += bc.edge[nx + k];
+      if (TAIL && c == C - 1) {
+        const double e = bc.edge[nx + k];
 #pragma unroll
         for (int j = 0; j < S; ++j)
-          if (j == len - 1) f[j] += bc.edge[nx + k];
+          if (j == len - 1) {
+            f[j] += e;
+            asm volatile("" : "+d"(f[j]));   // keeps the rows in registers (not one indexed store)
+          }
       }
     } else {
 #pragma unroll
@@ -348,6 +365,7 @@ __device__ __forceinline__ void tri_reg_body(const TriOp& op, const double* __re
       fi *= ps;
     }
   }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   __syncthreads();
   // phase 1: chunk solve with zero ends (the products sigma/pivot * f are off the forward
   // recurrence, which takes one FMA per row)
@@ -375,17 +393,15 @@ __device__ __forceinline__ void tri_reg_body(const TriOp& op, const double* __re
   if (chunk) {
     if (c >= 1) {
       const double* hh = hv + Mb + kl;
+      const double* rr = t_r + t;
       double y0 = 0.0, y1 = 0.0;
-#pragma unroll
-      for (int j = 0; j + 1 < kTriMaxM; j += 2) {
-        if (j + 1 < m) {
-          y0 = fma(rr[j], hh[j * Mb], y0);
-          y1 = fma(rr[j + 1], hh[(j + 1) * Mb], y1);
-        } else if (j < m) {
-          y0 = fma(rr[j], hh[j * Mb], y0);
-        }
+      int j = 0;
+#pragma unroll 4
+      for (; j + 1 < m; j += 2) {
+        y0 = fma(rr[j * C * Mb], hh[j * Mb], y0);
+        y1 = fma(rr[(j + 1) * C * Mb], hh[(j + 1) * Mb], y1);
       }
-      if ((kTriMaxM & 1) && m == kTriMaxM) y0 = fma(rr[kTriMaxM - 1], hh[(kTriMaxM - 1) * Mb], y0);
+      if (j < m) y0 = fma(rr[j * C * Mb], hh[j * Mb], y0);
       yv[c * Mb + kl] = y0 + y1;
     } else {
       yv[kl] = 0.0;
@@ -410,7 +426,7 @@ __device__ __forceinline__ void tri_reg_body(const TriOp& op, const double* __re
 }
 
 template <int S, bool TAIL>
-__global__ void __launch_bounds__(256) k_tri_reg(TriOp op, const double* __restrict__ F, double* U, int ld, int Mb,
+__global__ void __launch_bounds__(256, 2) k_tri_reg(TriOp op, const double* __restrict__ F, double* U, int ld, int Mb,
                                                  TriBc bc) {
   extern __shared__ double sm[];
   tri_reg_body<S, TAIL>(op, F, U, ld, Mb, bc, sm);   // waits for the previous kernel after its tables
@@ -419,14 +435,15 @@ __global__ void __launch_bounds__(256) k_tri_reg(TriOp op, const double* __restr
 // The same solve for every item of a batch, blockIdx.y picking the item (its tables, input,
 // output and boundary terms); the items share the chunking.
 template <int S, bool TAIL>
-__global__ void __launch_bounds__(256) k_tri_reg_batch(const __grid_constant__ TriBatch b, int ld, int Mb) {
+__global__ void __launch_bounds__(256, 2) k_tri_reg_batch(const __grid_constant__ TriBatch b, int ld, int Mb) {
   extern __shared__ double sm[];
   const int y = blockIdx.y;
   tri_reg_body<S, TAIL>(b.op[y], b.F[y], b.U[y], ld, Mb, b.bc[y], sm);
 }
 
 static size_t tri_reg_smem(const TriOp& op, int Mb) {
-  return sizeof(double) * (size_t)Mb * ((op.r < op.s ? 4 : 3) * (size_t)op.s + 2 * (size_t)op.C + 2 * ((size_t)op.C + 1));
+  return sizeof(double) * (size_t)Mb * ((op.r < op.s ? 4 : 3) * (size_t)op.s + 2 * (size_t)op.C + 2 * ((size_t)op.C + 1) +
+                                             (size_t)op.C * std::max(op.C - 1, 1));
 }
 
 template <int S, bool TAIL>

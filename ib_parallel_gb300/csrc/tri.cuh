@@ -63,6 +63,9 @@ struct TriBc {
   const double* edge = nullptr;
   const double* add2 = nullptr;
   double post_scale = 1.0;
+  // F and add2 were complete before the kernel launched just ahead began (that kernel waits for its
+  // predecessors before it reads or writes anything): they may be read before the wait for it
+  bool early = false;
 };
 
 // In place (F may equal U): U = sigma * A^-1 (F with the boundary terms bc) for every mode column.
