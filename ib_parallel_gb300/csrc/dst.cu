@@ -452,12 +452,9 @@ __device__ __forceinline__ double x_load(const XPre& a, const double* __restrict
       }
     }
     const double* w = a.in4;
-    double nb = 0.0;
-    if (j > 0) nb += w[idx - 1];
-    if (j < N - 1) nb += w[idx + 1];
-    if (row > 0) nb += w[idx - ld];
-    if (row < nrows - 1) nb += w[idx + ld];
-    v = fma(a.beta, nb, fma(a.alpha, w[idx], base));
+    const double wl = j > 0 ? w[idx - 1] : 0.0, wr = j < N - 1 ? w[idx + 1] : 0.0;
+    const double wd = row > 0 ? w[idx - ld] : 0.0, wu = row < nrows - 1 ? w[idx + ld] : 0.0;
+    v = fma(a.beta, (wl + wr) + (wd + wu), fma(a.alpha, w[idx], base));
   } else {
     // apply_bc (operators_fluid.F90:539-549): left, right, bottom, top; a null input is zero
     v = in ? in[idx] : 0.0;
@@ -606,7 +603,9 @@ __global__ void __launch_bounds__(512) k_dst_x(DstDev pl, int nrows, int ld, con
 // [nlr, nlr + 2 nbt) kReSeg entries of the left half of the bottom or top side and their
 // mirrors; then one warp per mode k for the two edge dot products (dst_ring_from_modes launches
 // the first two groups alone, sd and edge null).
-constexpr int kReWarps = 8;
+// 4 against 8 warps: 401 CTAs against 187 at 800 x 400, so no SM has twice its share; 7.6 against 7.9 us
+// (8.2 before the two edge sums of a mode shared one reduction, warp_sum2)
+constexpr int kReWarps = 4;
 constexpr int kReSeg = 2 * (kReWarps - 1);   // entries a CTA writes on a side (kReWarps vertices)
 __global__ void __launch_bounds__(32 * kReWarps) k_ring_edge(int N, GridDims g, const double* __restrict__ spec,
                                                              int ld, const double* __restrict__ W,

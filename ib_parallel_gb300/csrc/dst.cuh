@@ -44,6 +44,16 @@ __device__ __forceinline__ double warp_sum(double acc) {
   return acc;
 }
 
+// The sums over the lanes of two values: the halves of the warp first take one value each, so both
+// cost the five additions of one.  Valid on every lane.
+__device__ __forceinline__ double2 warp_sum2(double a, double b) {
+  const bool up = threadIdx.x & 16;
+  double v = (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  const double w = __shfl_xor_sync(0xffffffffu, v, 16);
+  return up ? make_double2(w, v) : make_double2(v, w);
+}
+
 // A mode row's inverse x transform at a point and at its mirror image.  W's row N-1-r is
 // (-1)^k times row r in mode k, so the two values are e + o and e - o, with e and o the row's
 // sums over even and odd modes.  A lane of warp_dot_part meets only modes of its own parity,
@@ -80,7 +90,7 @@ __device__ __forceinline__ double2 warp_edge_dot(const double* __restrict__ Ec, 
     a0 = fma(ek[t], s0[2 * t], a0);
     b0 = fma(ek[t], s1[2 * t], b0);
   }
-  return make_double2(warp_sum(a0 + a1), warp_sum(b0 + b1));
+  return warp_sum2(a0 + a1, b0 + b1);
 }
 
 struct DstPlan {
