@@ -362,42 +362,48 @@ int launch_redistribute_field(const GridDims& g, int nf, const double* f, const 
   return IB_OK;
 }
 
-// write_force2: out[b] = 2 delta sum_x f/dt, out[nbody+b] = 2 delta sum_y f/dt, each sum in the
-// order of the unknowns.  One warp per body: the lanes divide (f/dt, about ten FP64 instructions
-// each) a chunk of the unknowns at a time into shared memory, then lane 0 adds the x terms and
-// lane 1 the y terms in order.  With mirror set the coefficients, and the nt hinge angles after
-// them, are also written there (pinned host memory the device maps).
-constexpr int kForceChunk = 1024;
-__global__ void k_force_coeffs(int nf, int nbody, const int* __restrict__ comp, const int* __restrict__ bid,
-                               const double* __restrict__ f, double dt, double delta, double* out, double* mirror,
-                               const double* __restrict__ theta, int nt) {
+// write_force2: out[b] = 2 delta (sum_x f) / dt, out[nbody+b] = 2 delta (sum_y f) / dt, one CTA per
+// body: lane-strided sums, a shuffle tree per warp and the warps' sums.  With mirror set the
+// coefficients, and the nt hinge angles after them, are also written there (pinned host memory the
+// device maps).  What bounds it: a chain of about 25 dependent FP64 additions.  Summed in the unknowns'
+// order by one lane per component it took 30 us for 314 unknowns and 12 us for 102; 3 us so.
+constexpr int kForceWarps = 4;
+__global__ void __launch_bounds__(32 * kForceWarps) k_force_coeffs(int nf, int nbody, const int* __restrict__ comp,
+                                                                   const int* __restrict__ bid,
+                                                                   const double* __restrict__ f, double dt,
+                                                                   double delta, double* out, double* mirror,
+                                                                   const double* __restrict__ theta, int nt) {
   IB_GRID_DEP_WAIT();
-  __shared__ double q[kForceChunk];
-  const int b = blockIdx.x, lane = threadIdx.x;
-  double acc = 0.0;   // lane 0: x terms, lane 1: y terms
-  for (int k0 = 0; k0 < nf; k0 += kForceChunk) {
-    const int n = min(kForceChunk, nf - k0);
-    for (int i = lane; i < n; i += 32) q[i] = bid[k0 + i] == b ? f[k0 + i] / dt : 0.0;
-    __syncwarp();
-    if (lane < 2)
-      for (int i = 0; i < n; ++i)
-        if (bid[k0 + i] == b && (comp[k0 + i] == 1) == (lane == 0)) acc = acc + q[i];
-    __syncwarp();
+  __shared__ double part[2][kForceWarps];
+  const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double ax = 0.0, ay = 0.0;
+  for (int k = tid; k < nf; k += 32 * kForceWarps) {
+    const double v = bid[k] == b ? f[k] : 0.0;
+    const bool isx = comp[k] == 1;
+    ax += isx ? v : 0.0;
+    ay += isx ? 0.0 : v;
   }
-  if (lane < 2) {
-    const double v = 2.0 * delta * acc;
-    out[lane * nbody + b] = v;
-    if (mirror) mirror[lane * nbody + b] = v;
+  // the halves of the warp take one sum each
+  const bool up = lane & 16;
+  double s = (up ? ay : ax) + __shfl_xor_sync(0xffffffffu, up ? ax : ay, 16);
+  for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((lane & 15) == 0) part[lane >> 4][warp] = s;
+  __syncthreads();
+  if (tid < 2) {
+    const double acc = (part[tid][0] + part[tid][1]) + (part[tid][2] + part[tid][3]);
+    const double v = 2.0 * delta * (acc / dt);
+    out[tid * nbody + b] = v;
+    if (mirror) mirror[tid * nbody + b] = v;
   }
   if (mirror && b == 0)
-    for (int t = lane; t < nt; t += 32) mirror[2 * nbody + t] = theta[t];
+    for (int t = tid; t < nt; t += 32 * kForceWarps) mirror[2 * nbody + t] = theta[t];
 }
 
 int launch_force_coeffs(int nf, int nbody, const int* comp, const int* bid, const double* f, double dt,
                         double delta, double* out, cudaStream_t st, double* mirror, const double* theta, int nt) {
   if (nbody == 0) return IB_OK;
   count_launch();
-  k_force_coeffs<<<nbody, 32, 0, st>>>(nf, nbody, comp, bid, f, dt, delta, out, mirror, theta, nt);
+  k_force_coeffs<<<nbody, 32 * kForceWarps, 0, st>>>(nf, nbody, comp, bid, f, dt, delta, out, mirror, theta, nt);
   IB_CUDA_CHECK(cudaGetLastError());
   return IB_OK;
 }
