@@ -6,41 +6,28 @@
 
 namespace ib {
 
-// Smoothed 6-point delta function.  Literals without a d exponent in the Fortran
-// source are default REAL, i.e. single precision: they appear as float literals.
-__device__ inline double deltafnc_dev(double x1, double x2, double dr) {
-  double r = fabs(x1 - x2);
-  double r1 = r / dr;
-  double r2 = r1 * r1;
-  double r3 = r2 * r1;
-  double r4 = r3 * r1;
-  const double s3 = sqrt(3.0);
-  double v;
-  if (r1 <= 1.0) {
-    double a5 = asin((1.0 / 2.0) * s3 * (2.0 * r1 - 1.0));
-    double a8 = sqrt(1.0 - 12.0 * r2 + 12.0 * r1);
-    v = 0.4166666667e-1 * r4 + ((double)(-.1388888889f) + 0.3472222222e-1 * a8) * r3 +
-        (-0.7121664902e-1 - 0.5208333333e-1 * a8 + (double)(0.2405626122f) * a5) * r2 +
-        (-(double)(.2405626122f) * a5 - (double)(.3792313933f) + (double)(.1012731481f) * a8) * r1 +
-        0.8018753741e-1 * a5 - 0.4195601852e-1 * a8 + (double)(.6485698427f);
-  } else if (r1 <= 2.0) {
-    double a6 = asin((1.0 / 2.0) * s3 * (-3.0 + 2.0 * r1));
-    double a9 = sqrt(-23.0 + 36.0 * r1 - 12.0 * r2);
-    v = -0.6250000000e-1 * r4 + ((double)(.4861111111f) - 0.1736111111e-1 * a9) * r3 +
-        ((double)(-1.143175026f) + 0.7812500000e-1 * a9 - (double)(.1202813061f) * a6) * r2 +
-        ((double)(.8751991178f) + (double)(.3608439183f) * a6 - (double)(.1548032407f) * a9) * r1 -
-        (double)(.2806563809f) * a6 + 0.822848104e-2 + (double)(.1150173611f) * a9;
-  } else if (r1 <= 3.0) {
-    double a1 = asin((1.0 / 2.0 * (2.0 * r1 - 5.0)) * s3);
-    double a7 = sqrt(-71.0 - 12.0 * r2 + 60.0 * r1);
-    v = 0.2083333333e-1 * r4 + (0.3472222222e-2 * a7 - (double)(.2638888889f)) * r3 +
-        ((double)(1.214391675f) - 0.2604166667e-1 * a7 + 0.2405626122e-1 * a1) * r2 +
-        (-(double)(.1202813061f) * a1 - (double)(2.449273192f) + 0.7262731481e-1 * a7) * r1 +
-        (double)(.1523563211f) * a1 + (double)(1.843201677f) - 0.7306134259e-1 * a7;
-  } else {
-    v = 0.0;
-  }
-  return v / dr;
+// The smoothed 6-point delta function (grid.F90:955-1003) over dr, from its table (delta_table,
+// ibm.cu): on each of its three pieces (r1 = |x1 - x2| / dr up to 1, 2 and 3) kDeltaSub polynomials of
+// degree kDeltaDeg.  The pieces do not meet exactly (single-precision literals), so which one a point
+// falls on follows from r1 rounded as the reference rounds it.
+// What bounds it: a chain of FP64 operations of 64 cycles.  The closed form (an arcsine, a square root,
+// two divisions) takes about 218 on one lane, the division for r1 and the polynomial about 30.  The
+// weights of 78 unknowns (k_reg_weights) took 17.4 us with it and take 4.5, the end of an FSI iteration
+// of 102 (k_fsi_update) 25.5 and 15.0.
+constexpr int kDeltaSub = 32, kDeltaDeg = 16;
+constexpr int kDeltaTable = 3 * kDeltaSub * (kDeltaDeg + 1);
+__device__ __forceinline__ double deltafnc_dev(double x1, double x2, double dr, const double* __restrict__ tab) {
+  const double r1 = fabs(x1 - x2) / dr;
+  if (!(r1 <= 3.0)) return 0.0;
+  const int piece = r1 <= 1.0 ? 0 : (r1 <= 2.0 ? 1 : 2);
+  const double s = (double)kDeltaSub * (r1 - (double)piece);
+  const int sub = min((int)s, kDeltaSub - 1);
+  const double x = fma(2.0, s, -(double)(2 * sub + 1));
+  const double* c = tab + (piece * kDeltaSub + sub) * (kDeltaDeg + 1);
+  double v = __ldg(c + kDeltaDeg);
+#pragma unroll
+  for (int i = kDeltaDeg - 1; i >= 0; --i) v = fma(v, x, __ldg(c + i));
+  return v;
 }
 
 // compute_dx + update_xb (operators_struct.F90:402-505, 600-620) of torsional body t, the
@@ -85,72 +72,47 @@ __device__ __forceinline__ double2 tors_point(const TorsBody& b, int idx, double
 }
 
 // Stencil origins and the 49 weights (l outer, p inner) of the 8 unknowns k0..k0+7 on one CTA
-// of 4 warps, from their positions pos[u] = (x, y).  With phi the fractional position of a
-// point in its cell, the 7 stencil offsets q sit at distances |q - 3 - phi| (in cells), so
-// offsets {3,4}, {2,5} and {1,6} fall in the first, second and third piece of the delta
-// function and offset 0 at its edge.  Warp w evaluates one offset pair for the x and y factors
-// of all 8 unknowns, so its lanes take one branch of the FP64-latency-bound evaluation instead
-// of all three; the factors meet in shared memory for the products.  Writes the weights to w
-// (and wsm[u][.] when given), the origins to ix, iy (and org[u][.]); stale |= 1 when an origin
+// of 4 warps, from their positions pos[u] = (x, y): a thread per unknown, axis and offset q (the
+// eighth of each axis idle); the factors meet in shared memory for the products.  Writes the weights
+// to w (and wsm[u][.] when given), the origins to ix, iy and org[u][.]; stale |= 1 when an origin
 // moved; err = IB_ERR_DOMAIN when a stencil leaves the grid.  Ends with a CTA barrier.
 __device__ __forceinline__ void reg_weights_cta(const GridDims& g, int nf, int k0, const double (*pos)[2], double d,
-                                                double ox, double oy, const int* __restrict__ comp, int* ix, int* iy,
-                                                double* w, int* stale, int* err, double (*fac)[7],
-                                                double (*wsm)[49], int (*org)[2]) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const double d2 = 0.5 * d;
-  int pi, q;
-  if (warp < 3) {
-    pi = lane >> 1;
-    const int lo = 3 - warp, hi = 4 + warp;   // {3,4}, {2,5}, {1,6}
-    q = (lane & 1) ? hi : lo;
-  } else {
-    pi = lane;
-    q = 0;
-  }
-  const int u = pi >> 1, k = k0 + u, axis = pi & 1;
-  if (pi < 16 && k < nf) {
-    const double xk = pos[u][0], yk = pos[u][1];
-    const int cx = (int)((xk + ox) / d) + 1;   // Fortran INT truncates toward zero
-    const int cy = (int)((yk + oy) / d) + 1;
-    const bool isx = comp[k] == 1;
-    const int off = q - 3;
-    double fv;
+                                                double ox, double oy, const double* __restrict__ tab,
+                                                const int* __restrict__ comp, int* ix, int* iy, double* w, int* stale,
+                                                int* err, double (*fac)[7], double (*wsm)[49], int (*org)[2]) {
+  const int tid = threadIdx.x;
+  const int u = tid >> 4, axis = (tid >> 3) & 1, q = tid & 7, k = k0 + u;
+  if (k < nf && q < 7) {
+    const double z = pos[u][axis], o = axis ? oy : ox;
+    const int c = (int)((z + o) / d) + 1;   // Fortran INT truncates toward zero
     // The grid coordinate is rounded after the product and again after the sum, as the
     // reference's expression delta*(indexx-1+p)-offsetx is (grid.F90:459-528): the delta
     // function is discontinuous at 3 cells (its single-precision constants leave about 1e-8
     // there), so a point on a grid line (e.g. x = 0 with offsetx = 1, delta = 0.02) must see
     // the same side of that edge, which a fused multiply-add could change by one rounding.
-    if (axis == 0) {
-      double x = __dsub_rn(__dmul_rn(d, (double)(cx - 1 + off)), ox);
-      if (!isx) x = __dadd_rn(x, d2);
-      fv = deltafnc_dev(x, xk, d);
-    } else {
-      double y = __dsub_rn(__dmul_rn(d, (double)(cy - 1 + off)), oy);
-      if (isx) y = __dadd_rn(y, d2);
-      fv = deltafnc_dev(y, yk, d);
-    }
-    fac[pi][q] = fv;
-    if (warp == 3 && axis == 0) {
-      // the contribution lists depend on the stencil origins only: rebuild them when one moved
-      if (ix[k] != cx || iy[k] != cy) atomicOr(stale, 1);
-      ix[k] = cx;
-      iy[k] = cy;
-      if (org) {
-        org[u][0] = cx;
-        org[u][1] = cy;
-      }
-      // faces touched: u-face i in [1,m+1], j in [1,n]; v-face i in [1,m], j in [1,n+1]
-      const int imax = isx ? g.m + 1 : g.m, jmax = isx ? g.n : g.n + 1;
-      if (cx - 3 < 1 || cx + 3 > imax || cy - 3 < 1 || cy + 3 > jmax) atomicExch(err, IB_ERR_DOMAIN);
-    }
+    double x = __dsub_rn(__dmul_rn(d, (double)(c - 1 + q - 3)), o);
+    if ((comp[k] == 1) == (axis == 1)) x = __dadd_rn(x, 0.5 * d);   // faces lie half a cell off across
+    const double fv = deltafnc_dev(x, z, d, tab);
+    fac[2 * u + axis][q] = axis == 0 ? d * d * fv : fv;
+    if (q == 0) org[u][axis] = c;
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < 8 * 49; t += blockDim.x) {
+  if (tid < 8 && k0 + tid < nf) {
+    const int kk = k0 + tid, cx = org[tid][0], cy = org[tid][1];
+    const bool isx = comp[kk] == 1;
+    // the contribution lists depend on the stencil origins only: rebuild them when one moved
+    if (ix[kk] != cx || iy[kk] != cy) atomicOr(stale, 1);
+    ix[kk] = cx;
+    iy[kk] = cy;
+    // faces touched: u-face i in [1,m+1], j in [1,n]; v-face i in [1,m], j in [1,n+1]
+    const int imax = isx ? g.m + 1 : g.m, jmax = isx ? g.n : g.n + 1;
+    if (cx - 3 < 1 || cx + 3 > imax || cy - 3 < 1 || cy + 3 > jmax) atomicExch(err, IB_ERR_DOMAIN);
+  }
+  for (int t = tid; t < 8 * 49; t += blockDim.x) {
     const int uu = t / 49, sl = t - uu * 49;
     if (k0 + uu >= nf) break;
     const int l = sl / 7, p = sl - l * 7;
-    const double wv = d * d * fac[2 * uu][p] * fac[2 * uu + 1][l];
+    const double wv = fac[2 * uu][p] * fac[2 * uu + 1][l];
     w[(size_t)(k0 + uu) * 49 + sl] = wv;
     if (wsm) wsm[uu][sl] = wv;
   }

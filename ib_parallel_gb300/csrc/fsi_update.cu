@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(128) k_fsi_update(FsiUpdateArgs a) {
     pos[tid][1] = a.yb[k0 + tid];
   }
   __syncthreads();
-  reg_weights_cta(a.g, a.nf, k0, pos, a.delta, a.ox, a.oy, a.comp, a.ix, a.iy, a.w, a.stale, a.d_err, fac, wsm,
+  reg_weights_cta(a.g, a.nf, k0, pos, a.delta, a.ox, a.oy, a.dtab, a.comp, a.ix, a.iy, a.w, a.stale, a.d_err, fac, wsm,
                   org);
   if (a.rows && tid < 8 && k0 + tid < kend) {
     // E(curl s) at this stencil reads the streamfunction on vertex rows cy-5 .. cy+2

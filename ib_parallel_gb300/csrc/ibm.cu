@@ -7,25 +7,89 @@
 // reg is a face-major gather: for every face of the stencil bounding box the
 // contributing unknowns are listed in ascending order, so each face sums its
 // contributions in the same order as the reference's sequential scatter-add.
+#include <cmath>
+
 #include "fsi_dev.cuh"
 
 namespace ib {
 
+// The smoothed 6-point delta function (grid.F90:955-1003) on piece 0, 1 or 2.  Literals without a d
+// exponent in the Fortran source are default REAL, i.e. single precision: they appear as float
+// literals.
+static long double delta_piece(int piece, long double r1) {
+  typedef long double L;
+  const L s3 = (L)std::sqrt(3.0), r2 = r1 * r1, r3 = r2 * r1, r4 = r3 * r1;
+  if (piece == 0) {
+    const L a5 = asinl(0.5L * s3 * (2.0L * r1 - 1.0L)), a8 = sqrtl(1.0L - 12.0L * r2 + 12.0L * r1);
+    return (L)0.4166666667e-1 * r4 + ((L)(-.1388888889f) + (L)0.3472222222e-1 * a8) * r3 +
+           ((L)-0.7121664902e-1 - (L)0.5208333333e-1 * a8 + (L)(0.2405626122f) * a5) * r2 +
+           (-(L)(.2405626122f) * a5 - (L)(.3792313933f) + (L)(.1012731481f) * a8) * r1 + (L)0.8018753741e-1 * a5 -
+           (L)0.4195601852e-1 * a8 + (L)(.6485698427f);
+  }
+  if (piece == 1) {
+    const L a6 = asinl(0.5L * s3 * (-3.0L + 2.0L * r1)), a9 = sqrtl(-23.0L + 36.0L * r1 - 12.0L * r2);
+    return (L)-0.6250000000e-1 * r4 + ((L)(.4861111111f) - (L)0.1736111111e-1 * a9) * r3 +
+           ((L)(-1.143175026f) + (L)0.7812500000e-1 * a9 - (L)(.1202813061f) * a6) * r2 +
+           ((L)(.8751991178f) + (L)(.3608439183f) * a6 - (L)(.1548032407f) * a9) * r1 - (L)(.2806563809f) * a6 +
+           (L)0.822848104e-2 + (L)(.1150173611f) * a9;
+  }
+  const L a1 = asinl((0.5L * (2.0L * r1 - 5.0L)) * s3), a7 = sqrtl(-71.0L - 12.0L * r2 + 60.0L * r1);
+  return (L)0.2083333333e-1 * r4 + ((L)0.3472222222e-2 * a7 - (L)(.2638888889f)) * r3 +
+         ((L)(1.214391675f) - (L)0.2604166667e-1 * a7 + (L)0.2405626122e-1 * a1) * r2 +
+         (-(L)(.1202813061f) * a1 - (L)(2.449273192f) + (L)0.7262731481e-1 * a7) * r1 + (L)(.1523563211f) * a1 +
+         (L)(1.843201677f) - (L)0.7306134259e-1 * a7;
+}
+
+// Its polynomials over `delta`: on each of kDeltaSub parts of a piece the Chebyshev interpolant in
+// x in [-1, 1], as powers of x.  The nearest branch points (1/2 +- 1/sqrt(3) from a piece's start) lie
+// 5.95 half widths from the centre of the nearest part, so its coefficients fall as 11.8^-i: what
+// degree 16 leaves out is below 1e-17.
+size_t delta_table_doubles() { return kDeltaTable; }
+void delta_table(double delta, double* out) {
+  const long double PI_L = 3.141592653589793238462643383279502884L;
+  constexpr int n = kDeltaDeg + 1;
+  for (int piece = 0; piece < 3; ++piece)
+    for (int sub = 0; sub < kDeltaSub; ++sub) {
+      long double f[n], c[n], mono[n] = {}, t0[n] = {}, t1[n] = {};
+      for (int i = 0; i < n; ++i) {
+        const long double x = cosl(PI_L * (i + 0.5L) / n);
+        f[i] = delta_piece(piece, piece + (sub + 0.5L + 0.5L * x) / kDeltaSub);
+      }
+      for (int j = 0; j < n; ++j) {
+        c[j] = 0.0L;
+        for (int i = 0; i < n; ++i) c[j] += f[i] * cosl(PI_L * j * (i + 0.5L) / n);
+        c[j] *= (j == 0 ? 1.0L : 2.0L) / n;
+      }
+      t0[0] = 1.0L;   // T_0 and T_1, then T_(j+1) = 2 x T_j - T_(j-1)
+      t1[1] = 1.0L;
+      for (int j = 0; j < n; ++j) {
+        for (int i = 0; i < n; ++i) mono[i] += c[j] * t0[i];
+        long double t2[n];
+        for (int i = 0; i < n; ++i) t2[i] = (i > 0 ? 2.0L * t1[i - 1] : 0.0L) - t0[i];
+        for (int i = 0; i < n; ++i) { t0[i] = t1[i]; t1[i] = t2[i]; }
+      }
+      for (int i = 0; i < n; ++i)
+        out[(piece * kDeltaSub + sub) * n + i] = (double)(mono[i] / (long double)delta);
+    }
+}
+
 // Stencil origins and weights of 8 unknowns per CTA (reg_weights_cta).
 __global__ void __launch_bounds__(128) k_reg_weights(GridDims g, int nf, const double* __restrict__ xb,
                                                      const double* __restrict__ yb, double d, double ox,
-                                                     double oy, const int* __restrict__ comp, int* ix, int* iy,
-                                                     double* w, int* stale, int* err) {
+                                                     double oy, const double* __restrict__ tab,
+                                                     const int* __restrict__ comp, int* ix, int* iy, double* w,
+                                                     int* stale, int* err) {
   IB_GRID_DEP_WAIT();
   __shared__ double fac[16][7];    // [2*unknown + axis][offset], axis 0: x factor, 1: y factor
   __shared__ double pos[8][2];
+  __shared__ int org[8][2];
   const int k0 = blockIdx.x * 8;
   if ((int)threadIdx.x < 8 && k0 + (int)threadIdx.x < nf) {
     pos[threadIdx.x][0] = xb[k0 + threadIdx.x];
     pos[threadIdx.x][1] = yb[k0 + threadIdx.x];
   }
   __syncthreads();
-  reg_weights_cta(g, nf, k0, pos, d, ox, oy, comp, ix, iy, w, stale, err, fac, nullptr, nullptr);
+  reg_weights_cta(g, nf, k0, pos, d, ox, oy, tab, comp, ix, iy, w, stale, err, fac, nullptr, org);
 }
 
 // Bounding box of all stencils (one CTA).  bbox[0..3] = i0, j0, ni, nj of the face box;
@@ -142,8 +206,8 @@ int launch_reg_weights(const GridDims& g, int nf, const double* xb, const double
   // launch_reg_lists skips its work (each kernel returns at once) unless a stencil origin moved
   IB_CUDA_CHECK(cudaMemsetAsync(r.stale, 0, sizeof(int), st));
   count_launch();
-  k_reg_weights<<<cdiv(nf, 8), 128, 0, st>>>(g, nf, xb, yb, delta, offx, offy, r.comp, r.ix, r.iy, r.w, r.stale,
-                                              d_err);
+  k_reg_weights<<<cdiv(nf, 8), 128, 0, st>>>(g, nf, xb, yb, delta, offx, offy, r.tab, r.comp, r.ix, r.iy, r.w,
+                                              r.stale, d_err);
   IB_CUDA_CHECK(cudaGetLastError());
   return IB_OK;
 }

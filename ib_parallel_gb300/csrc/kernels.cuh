@@ -74,7 +74,12 @@ struct RegDev {
   int max_faces;    // capacity of cnt_* (faces)
   int max_list;     // capacity of lst_*
   int* stale;       // set by the weights kernel when a stencil origin moved: lists to rebuild
+  const double* tab;   // the delta function's polynomials (delta_table)
 };
+
+// The delta function's table for a grid spacing, delta_table_doubles() doubles of host memory.
+size_t delta_table_doubles();
+void delta_table(double delta, double* out);
 
 int launch_reg_build(const GridDims& g, int nf, const double* xb, const double* yb, double delta, double offx,
                      double offy, RegDev& r, int* d_err, cudaStream_t st);
@@ -162,6 +167,7 @@ struct FsiUpdateArgs {
   GridDims g;
   int nf;
   double ox, oy;
+  const double* dtab;
   const int* comp;
   int *ix, *iy;
   double* w;

@@ -220,6 +220,7 @@ int ctx_create(const IbParams* pin, const IbBody* bodies, int nbody, Ctx** out, 
   dbl += (size_t)g.nsx * g.nsx + (size_t)L * (2 * (size_t)g.nsy + 2 * (size_t)g.nsx);   // edge matrix, terms
   dbl += (size_t)(L - 1) * ns + (size_t)g.nsy;           // vort2flux's coarse-level modes, row modes
   dbl += 8 * (size_t)nf + 2 * (size_t)nbody + 49 * (size_t)nf;
+  dbl += delta_table_doubles();
   dbl += 49 * (size_t)nf + (size_t)nf + 1;               // weights snapshot (+ its origins, as doubles)
   dbl += 3 * ((size_t)nt + 1) + 1;                       // fused FSI update: theta, sin, cos; ticket
   dbl += 8 * (size_t)nt + nt + 3;
@@ -266,6 +267,8 @@ int ctx_create(const IbParams* pin, const IbBody* bodies, int nbody, Ctx** out, 
   c->tmpf2 = P.take<double>(nf); c->forces = P.take<double>(2 * nbody + 1); c->ub = P.take<double>(nf);
   c->comp = P.take<int>(nf); c->bid = P.take<int>(nf);
   c->reg.comp = c->comp; c->reg.ix = P.take<int>(nf); c->reg.iy = P.take<int>(nf);
+  double* dtab = P.take<double>(delta_table_doubles());
+  c->reg.tab = dtab;
   c->reg.w = P.take<double>(49 * (size_t)nf); c->reg.bbox = P.take<int>(16);
   c->reg.cnt_x = P.take<int>(max_faces); c->reg.cnt_y = P.take<int>(max_faces);
   c->reg.lst_x = P.take<int>(49 * (size_t)nf + 1); c->reg.lst_y = P.take<int>(49 * (size_t)nf + 1);
@@ -380,6 +383,9 @@ int ctx_create(const IbParams* pin, const IbBody* bodies, int nbody, Ctx** out, 
     }
   }
   if (nf > 0) {
+    std::vector<double> tab(delta_table_doubles());
+    delta_table(c->delta, tab.data());
+    IB_CUDA_CHECK(cudaMemcpy(dtab, tab.data(), 8 * tab.size(), cudaMemcpyHostToDevice));
     IB_CUDA_CHECK(cudaMemcpy(c->xb, xb_h.data(), 8 * (size_t)nf, cudaMemcpyHostToDevice));
     IB_CUDA_CHECK(cudaMemcpy(c->yb, yb_h.data(), 8 * (size_t)nf, cudaMemcpyHostToDevice));
     IB_CUDA_CHECK(cudaMemcpy(c->comp, c->comp_h.data(), 4 * (size_t)nf, cudaMemcpyHostToDevice));
@@ -1321,7 +1327,7 @@ static int capture_fsi_loop(Ctx* c, cudaStream_t st) {
         u.tb = c->tb; u.ts = c->ts; u.nt = c->nt; u.dt = p.dt; u.delta = c->delta; u.f = c->f;
         u.xb = c->xb; u.yb = c->yb; u.err = c->err_fsi;
         u.th_next = c->tors_next; u.sin_next = c->tors_next + (c->nt + 1); u.cos_next = c->tors_next + 2 * (c->nt + 1);
-        u.g = g; u.nf = c->nf; u.ox = p.offsetx; u.oy = p.offsety; u.comp = c->reg.comp;
+        u.g = g; u.nf = c->nf; u.ox = p.offsetx; u.oy = p.offsety; u.dtab = c->reg.tab; u.comp = c->reg.comp;
         u.ix = c->reg.ix; u.iy = c->reg.iy; u.w = c->reg.w; u.stale = c->reg.stale; u.d_err = c->d_err;
         u.tile_of = I.tile_of; u.ntx = I.ntx; u.tile = Influence::kTile;
         u.pval = c->sd.on ? nullptr : I.pval; u.pidx = I.pidx; u.used = I.used; u.flag = I.flag;

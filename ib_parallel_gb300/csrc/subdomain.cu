@@ -598,6 +598,7 @@ int sd_setup(Ctx* c, int full_rectangular, double sdxi, double sdxe, double sdyi
     }
   }
   S.reg.comp = S.ucomp;
+  S.reg.tab = c->reg.tab;
   S.reg.max_faces = max_faces;
   S.reg.max_list = 49 * nfs;
   std::vector<double> ux(nfs), uy(nfs);
