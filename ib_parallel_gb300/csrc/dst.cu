@@ -11,18 +11,6 @@ namespace ib {
 // ---------------------------------------------------------------- tables
 static const long double PI_L = 3.141592653589793238462643383279502884L;
 
-static bool factor_radices(int P, int* rad, int* nrad) {
-  // radix-5 and radix-3 stages first (no twiddles in the first stage), then 4, then 2.
-  int n = 0, q = P;
-  while (q % 5 == 0) { rad[n++] = 5; q /= 5; }
-  while (q % 3 == 0) { rad[n++] = 3; q /= 3; }
-  while (q % 4 == 0) { rad[n++] = 4; q /= 4; }
-  while (q % 2 == 0) { rad[n++] = 2; q /= 2; }
-  if (q != 1 || n > kMaxRadices) return false;
-  *nrad = n;
-  return true;
-}
-
 // The factors of a plan, in the order they lie in device memory: of P stage twiddles c + i d and then
 // of the P/2 factors exp(-2 pi i k/M), the pairs (c, d - c); of both, the third factors c + d; P of
 // 2 sin(j pi/M); and P + 1 doubles sin(j pi/M).
@@ -61,7 +49,8 @@ static int plan_init(DstPlan* p, int N) {
   const int M = N + 1;
   if (N < 3 || M % 4 != 0) return IB_ERR_ARG;
   p->N = N; p->M = M; p->P = M / 2;
-  return factor_radices(p->P, p->rad, &p->nrad) ? IB_OK : IB_ERR_ARG;
+  p->nrad = fx_radices(p->P, p->rad, kMaxRadices);
+  return p->nrad > 0 ? IB_OK : IB_ERR_ARG;
 }
 
 static void plan_pointers(DstPlan* p, double* dev) {
@@ -150,21 +139,70 @@ __device__ __forceinline__ FxC twiddle(FxC v, const int4* __restrict__ tw, const
   return fx_cmul(v, FxW{a.x, a.y}, FxW{a.z, a.w}, ld_factor(tw3));
 }
 
-// The warps of a CTA over its lines: `wpl` warps per line, `groups` lines at once; thread gt of gsz
-// of its group.  A warp works on one line, so a line's maxima and sums are warp reductions.
-struct LineGroups {
-  int grp, groups, wpl, gw, gt, gsz;
-  __device__ __forceinline__ explicit LineGroups(int B) {
-    const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+constexpr int kMaxLines = 16;         // lines per CTA
+constexpr int kMaxWarps = 16;         // warps per CTA
+constexpr int kNotFinite = 1 << 20;   // in place of a line's exponent
+
+// The warps of a CTA over its B lines: wpl warps per line, `groups` lines at once (computed on the
+// host: the divisions cost every warp of a short kernel).  A warp works on one line at a time, so a
+// line's maxima and sums are warp reductions.
+struct LineShape {
+  int B, wpl, groups, inv;
+  LineShape(int B_, int NT) : B(B_) {
+    const int nwarps = NT / 32;
     wpl = nwarps >= B ? nwarps / B : 1;
     groups = nwarps >= B ? B : nwarps;
-    grp = warp / wpl;
+    inv = (65536 + wpl - 1) / wpl;   // (warp inv) >> 16 = warp / wpl for the few warps there are
+  }
+};
+struct LineGroups {
+  int B, wpl, groups, grp, gw, gt, gsz;
+  __device__ __forceinline__ explicit LineGroups(const LineShape& s) : B(s.B), wpl(s.wpl), groups(s.groups) {
+    const int warp = threadIdx.x >> 5;
+    grp = (warp * s.inv) >> 16;
     gw = warp - grp * wpl;
     gt = gw * 32 + (threadIdx.x & 31);
     gsz = wpl * 32;
     if (grp >= groups) grp = 1 << 20;   // spare warps: no lines
   }
 };
+
+// What a CTA keeps of its lines beside their samples: a word per line and warp, so that nothing has
+// to be cleared or added atomically.
+struct FxLines {
+  unsigned mag[2][kMaxWarps];   // largest magnitudes, of the phase before and of this one
+  unsigned l1[kMaxWarps];       // a bound of sum |x| / 2^40
+  int e[kMaxWarps];             // largest biased exponent of the samples (fx_exponent)
+  int shift[kMaxLines];         // right shifts so far
+  fx wt[kMaxWarps];             // warp totals of the prefix sums
+};
+
+// Dynamic shared memory of the transforms: the FxLines, then two buffers of B P complex values.
+extern __shared__ longlong2 fx_smem[];
+constexpr int kLinesWords = (sizeof(FxLines) + sizeof(longlong2) - 1) / sizeof(longlong2);
+__device__ __forceinline__ FxLines& fx_lines() { return *reinterpret_cast<FxLines*>(fx_smem); }
+__device__ __forceinline__ double* fx_line(int b, int P) {   // line b's 2P slots in the first buffer
+  return reinterpret_cast<double*>(fx_smem + kLinesWords + b * P);
+}
+// the samples' largest exponent that this warp has met on line b
+__device__ __forceinline__ void fx_note(const LineGroups& G, int b, int emax) {
+  emax = __reduce_max_sync(0xffffffffu, emax);
+  if ((threadIdx.x & 31) == 0) fx_lines().e[b * G.wpl + G.gw] = emax;
+}
+// line b's words of its warps, one per lane (`none` on the others)
+template <typename T>
+__device__ __forceinline__ T fx_words(const LineGroups& G, const T* words, int b, T none) {
+  const int lane = threadIdx.x & 31;
+  return lane < G.wpl ? words[b * G.wpl + lane] : none;
+}
+__device__ __forceinline__ unsigned fx_or(const LineGroups& G, const unsigned* words, int b) {
+  return __reduce_or_sync(0xffffffffu, fx_words(G, words, b, 0u));
+}
+
+// A result's bits where a line's exponent leaves the normal range or a sample was not finite.
+__device__ __noinline__ long long line_bits(fx v, int E) {
+  return E == kNotFinite ? 0x7ff8000000000000LL : fx_to_bits(v, E);
+}
 
 // One Stockham stage of one line on the gsz threads of its group; the inputs are taken 2^-sh.
 template <int R>
@@ -174,8 +212,6 @@ __device__ __forceinline__ unsigned stockham_stage(const longlong2* __restrict__
   const int nb = P / R, Ns = fns.d;
   FxPeak peak;
   for (int j = gt; j < nb; j += gsz) {
-    const int jq = fns.div(j);
-    const int k = j - jq * Ns;
     FxC v[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -186,7 +222,9 @@ __device__ __forceinline__ unsigned stockham_stage(const longlong2* __restrict__
 #pragma unroll
       for (int r = 0; r < R; ++r) v[r] = FxC{fx_shr(v[r].x, sh), fx_shr(v[r].y, sh)};
     }
+    int k = 0;
     if (Ns > 1) {
+      k = fns.mod(j);
 #pragma unroll
       for (int r = 1; r < R; ++r) {
         const unsigned i = (unsigned)(r * Ns - 1 + k);   // this stage's twiddles (plan_tables)
@@ -194,7 +232,7 @@ __device__ __forceinline__ unsigned stockham_stage(const longlong2* __restrict__
       }
     }
     FxDft<R>::run(v);
-    longlong2* dst = out + (jq * Ns * R + k);
+    longlong2* dst = out + ((j - k) * R + k);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       dst[r * Ns] = make_longlong2(v[r].x, v[r].y);
@@ -204,63 +242,27 @@ __device__ __forceinline__ unsigned stockham_stage(const longlong2* __restrict__
   return peak.mag();
 }
 
-constexpr int kMaxLines = 16;         // lines per CTA
-constexpr int kNotFinite = 1 << 20;   // in place of a line's exponent
-
-// What a CTA keeps of its lines in shared memory while it transforms them.
-struct FxLines {
-  unsigned mag[3][kMaxLines];   // largest magnitudes, three sets in rotation (dst_lines)
-  unsigned l1[kMaxLines];       // a bound of sum |x| / 2^40
-  int e[kMaxLines];             // largest biased exponent of the samples (fx_exponent)
-  int shift[kMaxLines];         // right shifts so far
-  fx wt[32];                    // warp totals of the prefix sums
-  __device__ __forceinline__ void clear(int B) {
-    const int t = threadIdx.x;
-    if (t < B) {
-      mag[0][t] = mag[1][t] = mag[2][t] = 0u;
-      l1[t] = 0u;
-      e[t] = 1;
-      shift[t] = 0;
-    }
-  }
-  // the samples' exponents a warp has met on line b
-  __device__ __forceinline__ void note(int b, int emax) {
-    emax = __reduce_max_sync(0xffffffffu, emax);
-    if ((threadIdx.x & 31) == 0) atomicMax(&e[b], emax);
-  }
-  // what the unpacking shifts by, and the exponent of its results (kNotFinite: a sample was not)
-  __device__ __forceinline__ int last_shift(int b, int w) const {
-    // an odd output is a sum of increments, at most 4 ||x||_1 in these units: it must fit as well
-    return max(fx_shift_for(mag[w][b]), (32 - fx_clz32(l1[b])) + 40 + 2 - shift[b] - 62);
-  }
-  __device__ __forceinline__ int exponent(int b, int sh) const {
-    return e[b] < 2047 ? e[b] - 1075 - (kFxFrac - 53) - 1 + shift[b] + sh : kNotFinite;
-  }
-};
-
-// A result's bits where a line's exponent leaves the normal range or a sample was not finite.
-__device__ __noinline__ long long line_bits(fx v, int E) {
-  return E == kNotFinite ? 0x7ff8000000000000LL : fx_to_bits(v, E);
-}
-
-// Transform B lines: line b holds x_1..x_N as doubles at slots 1..N of its M = 2P slots in zA, its
-// largest exponent noted in S; returns where the lines' Y_1..Y_N lie (zA or zB: line b at b*M, Y_(j+1)
-// at slot dst_slot(j, P)).  zA, zB: B*P complex workspace each.
+// Transform the CTA's lines: line b holds x_1..x_N as doubles at slots 1..N of fx_line(b), its largest
+// exponents noted (fx_note); every thread calls it after a barrier.  Returns where the lines'
+// Y_1..Y_N lie (line b at b*M, Y_(j+1) at slot dst_slot(j, P)).
 //
 // In block fixed point (fixed.cuh).  What bounds it: instruction issue and the latency of the chain of
-// phases, 11,000 warp instructions a line of 799 (the FP64 butterflies before held the FP64 pipe for
-// 600 x 64 cycles).  Measured, before and after: 800 lines of 1599, 80 and 30 us; 2000 lines of 799,
-// 84 and 33 us; 400 lines of 799, 27 and 13 us; 31 lines of 63, 7.5 us either way (latency).
-// Each phase leaves the line's largest magnitude for the next one's shift; the words rotate through
-// three sets so that one is cleared while one is read and one written.
-__device__ double* dst_lines(const DstDev& pl, int B, longlong2* zA, longlong2* zB, FxLines& S) {
+// phases (the FP64 butterflies before held the FP64 pipe for 600 x 64 cycles a line of 799); at 2000
+// lines the ALU and multiply pipes are half busy, 0.6 instructions a cycle and sub-partition.  The
+// twiddles loaded ahead of each barrier took 128 registers and 15% more time.
+// Measured with FP64 butterflies, and so: 800 lines of 1599, 80 and 28 us; 2000 of 799, 84 and 31; 399
+// of 799, 27 and 11.5; 199 of 399, 16 and 9.2; 31 of 63, 7.5 and 6.4.
+__device__ __forceinline__ const double* dst_lines(const DstDev& pl, const LineGroups& G) {
+  FxLines& S = fx_lines();
   const int lane = threadIdx.x & 31;
-  const int P = pl.P, M = pl.M, H = P / 2;
-  const LineGroups G(B);
+  const int P = pl.P, M = pl.M, H = P / 2, B = G.B;
+  longlong2* cur = fx_smem + kLinesWords;
+  longlong2* nxt = cur + B * P;
+  int w = 0;   // the set of magnitudes written
   // --- pre-processing: 2 y (length M, real), each pair (j, M - j) in its own slots
   for (int b = G.grp; b < B; b += G.groups) {
-    fx* y = reinterpret_cast<fx*>(zA + b * P);
-    const int emax = S.e[b];
+    fx* y = reinterpret_cast<fx*>(cur + b * P);
+    const int emax = __reduce_max_sync(0xffffffffu, fx_words(G, S.e, b, 1));
     FxPeak peak;
     unsigned l1 = 0;
     for (int t = G.gt; t < P; t += G.gsz) {
@@ -282,40 +284,50 @@ __device__ double* dst_lines(const DstDev& pl, int B, longlong2* zA, longlong2* 
     const unsigned mag = __reduce_or_sync(0xffffffffu, peak.mag());
     l1 = __reduce_add_sync(0xffffffffu, l1);
     if (lane == 0) {
-      atomicOr(&S.mag[0][b], mag);
-      atomicAdd(&S.l1[b], l1);
+      S.mag[0][b * G.wpl + G.gw] = mag;
+      S.l1[b * G.wpl + G.gw] = l1;
+      if (G.gw == 0) S.shift[b] = 0;
     }
   }
   __syncthreads();
-  // --- complex FFT of length P (Stockham, ping-pong zA <-> zB)
-  longlong2* cur = zA;
-  longlong2* nxt = zB;
-  int w = 0;   // the set of magnitudes to read
+  // --- complex FFT of length P (Stockham, between the two buffers)
   for (int s = 0; s < pl.nrad; ++s) {
-    const int wn = w == 2 ? 0 : w + 1, wc = wn == 2 ? 0 : wn + 1;
     for (int b = G.grp; b < B; b += G.groups) {
-      const int sh = fx_shift_for(S.mag[w][b]);
+      const int sh = fx_shift_for(fx_or(G, S.mag[w], b));
+      const longlong2* in = cur + b * P;
+      longlong2* out = nxt + b * P;
       unsigned mag;
       switch (pl.rad[s]) {
-        case 2: mag = stockham_stage<2>(cur + b * P, nxt + b * P, P, pl.fd_ns[s], pl.tw, pl.tw3, sh, G.gt, G.gsz); break;
-        case 3: mag = stockham_stage<3>(cur + b * P, nxt + b * P, P, pl.fd_ns[s], pl.tw, pl.tw3, sh, G.gt, G.gsz); break;
-        case 4: mag = stockham_stage<4>(cur + b * P, nxt + b * P, P, pl.fd_ns[s], pl.tw, pl.tw3, sh, G.gt, G.gsz); break;
-        default: mag = stockham_stage<5>(cur + b * P, nxt + b * P, P, pl.fd_ns[s], pl.tw, pl.tw3, sh, G.gt, G.gsz); break;
+#define IB_STAGE(R) \
+        case R: mag = stockham_stage<R>(in, out, P, pl.fd_ns[s], pl.tw, pl.tw3, sh, G.gt, G.gsz); break;
+        IB_STAGE(2) IB_STAGE(3) IB_STAGE(4)
+#undef IB_STAGE
+        default: mag = stockham_stage<5>(in, out, P, pl.fd_ns[s], pl.tw, pl.tw3, sh, G.gt, G.gsz); break;
       }
       mag = __reduce_or_sync(0xffffffffu, mag);
-      if (lane == 0) atomicOr(&S.mag[wn][b], mag);
-      if (G.gt == 0) {
-        S.shift[b] += sh;
-        S.mag[wc][b] = 0u;
+      if (lane == 0) {
+        S.mag[w ^ 1][b * G.wpl + G.gw] = mag;
+        if (G.gw == 0) S.shift[b] += sh;
       }
     }
     __syncthreads();
     longlong2* t = cur; cur = nxt; nxt = t;
-    w = wn;
+    w ^= 1;
   }
+  // what the unpacking shifts by (an odd output is a sum of increments, at most 4 ||x||_1 in these
+  // units: it must fit as well), and the exponent of its results
+  auto last = [&](int b, int* E) {
+    const unsigned l1 = __reduce_add_sync(0xffffffffu, fx_words(G, S.l1, b, 0u));
+    const int e = __reduce_max_sync(0xffffffffu, fx_words(G, S.e, b, 1));
+    const int done = S.shift[b];
+    const int sh = max(fx_shift_for(fx_or(G, S.mag[w], b)), (32 - fx_clz32(l1)) + 40 + 2 - done - 62);
+    *E = e < 2047 ? e - 1075 - (kFxFrac - 53) - 1 + done + sh : kNotFinite;
+    return sh;
+  };
   // --- unpack the real FFT: even outputs D_2, D_4, .. to slots P.., the odd ones' increments to 0..P-1
   for (int b = G.grp; b < B; b += G.groups) {
-    const int sh = S.last_shift(b, w), E = S.exponent(b, sh);
+    int E;
+    const int sh = last(b, &E);
     const bool plain = fx_plain(E);
     const longlong2* Z = cur + b * P;
     long long* odd = reinterpret_cast<long long*>(nxt + b * P);
@@ -366,7 +378,8 @@ __device__ double* dst_lines(const DstDev& pl, int B, longlong2* zA, longlong2* 
       __syncthreads();
     }
     if (act) {
-      const int E = S.exponent(b, S.last_shift(b, w));
+      int E;
+      last(b, &E);
       const bool plain = fx_plain(E);
       fx run = incl - acc;
       for (int j = 0; j < G.gw; ++j) run += S.wt[G.grp * G.wpl + j];
@@ -377,7 +390,7 @@ __device__ double* dst_lines(const DstDev& pl, int B, longlong2* zA, longlong2* 
     }
     __syncthreads();
   }
-  return reinterpret_cast<double*>(nxt);
+  return reinterpret_cast<const double*>(nxt);
 }
 
 // Where dst_lines leaves Y_(j+1) in a line's slots.
@@ -467,55 +480,48 @@ __device__ __forceinline__ double x_load(const XPre& a, const double* __restrict
   return v;
 }
 
+// 64 registers a thread for every pre-operation: the predictor's FP64 stencil then overlaps other CTAs'
+// integer phases (at 86 registers 236 us for 5119 lines of 1535, at 64 199 us; plain passes need 60 to 64).
 template <int PRE>
-__global__ void __launch_bounds__(512) k_dst_x(DstDev pl, int nrows, int ld, const __grid_constant__ DstXArgs a,
-                                               GridDims g, int B) {
+__global__ void __launch_bounds__(512, 2) k_dst_x(DstDev pl, int nrows, int ld, const __grid_constant__ DstXArgs a,
+                                               GridDims g, LineShape shape) {
   IB_GRID_DEP_WAIT();
   const double* ain = a.nlev ? a.lin[blockIdx.y] : a.in;
   double* aout = a.nlev ? a.lout[blockIdx.y] : a.out;
   const XPre pre = x_pre(a, blockIdx.y, PRE == PRE_PRED && a.nlev > 0);
-  extern __shared__ longlong2 smem2[];
-  __shared__ int s_mode[kMaxLines];
-  __shared__ int s_any;
-  __shared__ FxLines S;
-  longlong2* zA = smem2;
-  longlong2* zB = zA + B * pl.P;
-  const double* xb = nullptr;   // the transformed lines, M apart
-  const int N = pl.N, M = pl.M;
-  const int line0 = blockIdx.x * B;
-  const int nl = a.nlines ? a.nlines : nrows;
-  __shared__ int s_row[kMaxLines];
-  if (threadIdx.x == 0) s_any = 0;
-  S.clear(B);
-  __syncthreads();
-  if (threadIdx.x < B) {
-    int line = line0 + threadIdx.x;
-    int row = a.nlines ? a.row0 + line * a.row_step : line;
-    s_row[threadIdx.x] = row;
-    int mode = ROW_FFT;
-    if (line >= nl || row >= nrows) mode = ROW_SKIP;
-    else if (a.rowrange) {
+  const LineGroups G(shape);
+  const int B = G.B, N = pl.N, M = pl.M;
+  // the row and treatment of the CTA's line b
+  auto line_of = [&](int b, int* row) -> int {
+    const int line = blockIdx.x * B + b;
+    const int r = a.nlines ? a.row0 + line * a.row_step : line;
+    *row = r;
+    if (line >= (a.nlines ? a.nlines : nrows) || r >= nrows) return ROW_SKIP;
+    if (a.rowrange) {
       const int lo = max(0, a.rowrange[0] - a.row_margin), hi = min(nrows, a.rowrange[1] + a.row_margin);
-      mode = (row >= lo && row < hi) ? ROW_FFT : a.rowrange[2];
-      if (a.fft_edge_rows && (row == 0 || row == nrows - 1)) mode = ROW_FFT;
       if (a.rows_used && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
         a.rows_used[0] = lo;
         a.rows_used[1] = hi;
       }
+      if ((r >= lo && r < hi) || (a.fft_edge_rows && (r == 0 || r == nrows - 1))) return ROW_FFT;
+      return a.rowrange[2];
     }
-    else if (a.rowmode && (int)blockIdx.y >= a.rowmode_level0) mode = a.rowmode[row];
-    s_mode[threadIdx.x] = mode;
-    if (mode == ROW_FFT) atomicOr(&s_any, 1);
+    if (a.rowmode && (int)blockIdx.y >= a.rowmode_level0) return a.rowmode[r];
+    return ROW_FFT;
+  };
+  int any_fft = 0;
+  for (int b = G.grp; b < B; b += G.groups) {
+    int row;
+    any_fft |= line_of(b, &row) == ROW_FFT;
   }
-  __syncthreads();
-  const bool any_fft = s_any != 0;
-  const LineGroups G(B);
+  if (B > 1) any_fft = __syncthreads_or(any_fft);   // of one line every warp knows
+  const double* xb = nullptr;   // the transformed lines, M apart
   if (any_fft) {
     // 4 independent loads in flight per thread before the shared-memory stores
     for (int b = G.grp; b < B; b += G.groups) {
-      const int row = s_row[b];
-      const bool live = s_mode[b] == ROW_FFT;
-      double* x = reinterpret_cast<double*>(zA + b * pl.P) + 1;
+      int row;
+      const bool live = line_of(b, &row) == ROW_FFT;
+      double* x = fx_line(b, pl.P) + 1;
       int emax = 1;
       for (int j0 = G.gt; j0 < N; j0 += 4 * G.gsz) {
         double v[4];
@@ -531,14 +537,14 @@ __global__ void __launch_bounds__(512) k_dst_x(DstDev pl, int nrows, int ld, con
           emax = max(emax, (__double2hiint(v[u]) >> 20) & 0x7ff);
         }
       }
-      S.note(b, emax);
+      fx_note(G, b, emax);
     }
     __syncthreads();
-    xb = dst_lines(pl, B, zA, zB, S);
+    xb = dst_lines(pl, G);
   }
   for (int b = G.grp; b < B; b += G.groups) {
-    const int row = s_row[b];
-    const int mode = s_mode[b];
+    int row;
+    const int mode = line_of(b, &row);
     if (mode == ROW_SKIP) continue;
     const size_t off = (size_t)row * ld;
     double* o = aout + off;
@@ -755,17 +761,15 @@ constexpr int kRowsPerCta = 8;
 __global__ void __launch_bounds__(256) k_dst_bc_modes(DstDev pl, GridDims g, const double* __restrict__ ring,
                                                       const double* __restrict__ W, const double* __restrict__ sk2,
                                                       const double* __restrict__ post_add, double post_scale,
-                                                      double* __restrict__ out, int nEdge, int fft_edges) {
+                                                      double* __restrict__ out, int nEdge, int fft_edges,
+                                                      LineShape shape) {
   IB_GRID_DEP_WAIT();
   const int N = pl.N;
   if (fft_edges && (int)blockIdx.x < nEdge) {
-    extern __shared__ longlong2 fft[];   // two P-point complex buffers; the row in the first one's slots
-    __shared__ FxLines S;
-    double* x = reinterpret_cast<double*>(fft) + 1;
+    const LineGroups G(shape);   // one line, the row
+    double* x = fx_line(0, pl.P) + 1;
     const int e = blockIdx.x;
     const int J = e == 0 ? 2 : g.n;
-    S.clear(1);
-    __syncthreads();
     int emax = 1;
     for (int j = threadIdx.x; j < N; j += blockDim.x) {
       const int I = j + 2;
@@ -777,9 +781,9 @@ __global__ void __launch_bounds__(256) k_dst_bc_modes(DstDev pl, GridDims g, con
       x[j] = v;
       emax = max(emax, (__double2hiint(v) >> 20) & 0x7ff);
     }
-    S.note(0, emax);
+    fx_note(G, 0, emax);
     __syncthreads();
-    const double* line = dst_lines(pl, 1, fft, fft + pl.P, S);
+    const double* line = dst_lines(pl, G);
     const size_t row = e == 0 ? 0 : (size_t)(g.nsy - 1) * g.nsx;
     for (int k = threadIdx.x; k < N; k += blockDim.x) {
       const size_t o = row + k;
@@ -860,7 +864,7 @@ int dst_x_bc_modes(const DstPlan& px, const GridDims& g, const double* ring, con
   const int nblk = nEdge + cdiv(std::max(0, g.nsy - 2), kRowsPerCta);
   DstDev d = to_dev(px);
   count_launch();
-  k_dst_bc_modes<<<nblk, 256, smem, st>>>(d, g, ring, W, sk2, post_add, post_scale, out, nEdge, fft_edges ? 1 : 0);
+  k_dst_bc_modes<<<nblk, 256, smem, st>>>(d, g, ring, W, sk2, post_add, post_scale, out, nEdge, fft_edges ? 1 : 0, LineShape(1, 256));
   IB_CUDA_CHECK(cudaGetLastError());
   return IB_OK;
 }
@@ -892,25 +896,25 @@ int dst_matrix_table(const DstPlan& px, double* dev_out) {
 
 
 // ------------------------------------------------------------- y pass
-__global__ void __launch_bounds__(512) k_dst_y(DstDev pl, int ncols, int ld, DstYArgs a, int B) {
+__global__ void __launch_bounds__(512) k_dst_y(DstDev pl, int ncols, int ld, DstYArgs a, LineShape shape) {
   IB_GRID_DEP_WAIT();
-  extern __shared__ longlong2 smem2[];
-  __shared__ FxLines S;
-  const int N = pl.N, M = pl.M;
-  longlong2* zA = smem2;
-  longlong2* zB = zA + B * pl.P;
+  const LineGroups G(shape);
+  const int B = G.B, N = pl.N, M = pl.M;
   const int col0 = blockIdx.x * B;
-  S.clear(B);
-  __syncthreads();
-  for (int it = threadIdx.x; it < B * N; it += blockDim.x) {
+  for (int it = threadIdx.x; it < B * N; it += blockDim.x) {   // a row's B columns side by side
     const int j = it / B, b = it - j * B;
     const int col = col0 + b;
-    const double v = col < ncols ? a.a[(size_t)j * ld + col] : 0.0;
-    reinterpret_cast<double*>(zA + b * pl.P)[j + 1] = v;
-    atomicMax(&S.e[b], (__double2hiint(v) >> 20) & 0x7ff);
+    fx_line(b, pl.P)[j + 1] = col < ncols ? a.a[(size_t)j * ld + col] : 0.0;
   }
   __syncthreads();
-  const double* xa = dst_lines(pl, B, zA, zB, S);
+  for (int b = G.grp; b < B; b += G.groups) {
+    const double* x = fx_line(b, pl.P) + 1;
+    int emax = 1;
+    for (int j = G.gt; j < N; j += G.gsz) emax = max(emax, (__double2hiint(x[j]) >> 20) & 0x7ff);
+    fx_note(G, b, emax);
+  }
+  __syncthreads();
+  const double* xa = dst_lines(pl, G);
   for (int it = threadIdx.x; it < B * N; it += blockDim.x) {
     const int j = it / B, b = it - j * B;
     const int col = col0 + b;
@@ -918,8 +922,8 @@ __global__ void __launch_bounds__(512) k_dst_y(DstDev pl, int ncols, int ld, Dst
   }
 }
 
-size_t dst_smem_x(const DstPlan& p, int B) { return (size_t)B * p.M * 8 * 2; }
-size_t dst_smem_y(const DstPlan& p, int B, DstYMode) { return (size_t)B * p.M * 8 * 2; }
+size_t dst_smem_x(const DstPlan& p, int B) { return sizeof(longlong2) * ((size_t)kLinesWords + (size_t)B * p.M); }
+size_t dst_smem_y(const DstPlan& p, int B, DstYMode) { return dst_smem_x(p, B); }
 
 template <typename K>
 static int launch_cfg(K kern, size_t smem) {
@@ -934,7 +938,7 @@ static int launch_cfg(K kern, size_t smem) {
 
 int dst_pass_x(const DstPlan& px, int nrows, int ld, DstPre pre, const DstXArgs& a, const GridDims& g,
                const DstLaunch& L, cudaStream_t st) {
-  if (L.B > kMaxLines || a.nlev < 0 || a.nlev > kMaxBatch || (a.nlev && pre != PRE_COPY && pre != PRE_PRED)) return IB_ERR_ARG;
+  if (L.B > kMaxLines || L.NT > 32 * kMaxWarps || a.nlev < 0 || a.nlev > kMaxBatch || (a.nlev && pre != PRE_COPY && pre != PRE_PRED)) return IB_ERR_ARG;
   DstDev d = to_dev(px);
   size_t smem = dst_smem_x(px, L.B);
   dim3 grid(cdiv(a.nlines ? a.nlines : nrows, L.B), a.nlev ? a.nlev : 1);
@@ -944,32 +948,32 @@ int dst_pass_x(const DstPlan& px, int nrows, int ld, DstPre pre, const DstXArgs&
       rc = launch_cfg(k_dst_x<PRE_COPY>, smem);
       if (rc) return rc;
       count_launch();
-      k_dst_x<PRE_COPY><<<grid, L.NT, smem, st>>>(d, nrows, ld, a, g, L.B);
+      k_dst_x<PRE_COPY><<<grid, L.NT, smem, st>>>(d, nrows, ld, a, g, LineShape(L.B, L.NT));
       break;
     case PRE_COMBINE:
       rc = launch_cfg(k_dst_x<PRE_COMBINE>, smem);
       if (rc) return rc;
       count_launch();
-      k_dst_x<PRE_COMBINE><<<grid, L.NT, smem, st>>>(d, nrows, ld, a, g, L.B);
+      k_dst_x<PRE_COMBINE><<<grid, L.NT, smem, st>>>(d, nrows, ld, a, g, LineShape(L.B, L.NT));
       break;
     case PRE_PRED:
       rc = launch_cfg(k_dst_x<PRE_PRED>, smem);
       if (rc) return rc;
       count_launch();
-      k_dst_x<PRE_PRED><<<grid, L.NT, smem, st>>>(d, nrows, ld, a, g, L.B);
+      k_dst_x<PRE_PRED><<<grid, L.NT, smem, st>>>(d, nrows, ld, a, g, LineShape(L.B, L.NT));
       break;
     case PRE_ROT:
       if (!a.box || !a.in2) return IB_ERR_ARG;
       rc = launch_cfg(k_dst_x<PRE_ROT>, smem);
       if (rc) return rc;
       count_launch();
-      k_dst_x<PRE_ROT><<<grid, L.NT, smem, st>>>(d, nrows, ld, a, g, L.B);
+      k_dst_x<PRE_ROT><<<grid, L.NT, smem, st>>>(d, nrows, ld, a, g, LineShape(L.B, L.NT));
       break;
     default:
       rc = launch_cfg(k_dst_x<PRE_APPLYBC>, smem);
       if (rc) return rc;
       count_launch();
-      k_dst_x<PRE_APPLYBC><<<grid, L.NT, smem, st>>>(d, nrows, ld, a, g, L.B);
+      k_dst_x<PRE_APPLYBC><<<grid, L.NT, smem, st>>>(d, nrows, ld, a, g, LineShape(L.B, L.NT));
       break;
   }
   IB_CUDA_CHECK(cudaGetLastError());
@@ -984,7 +988,7 @@ int dst_pass_y(const DstPlan& py, int ncols, int ld, DstYMode, const DstYArgs& a
   int rc = launch_cfg(k_dst_y, smem);
   if (rc) return rc;
   count_launch();
-  k_dst_y<<<grid, L.NT, smem, st>>>(d, ncols, ld, a, L.B);
+  k_dst_y<<<grid, L.NT, smem, st>>>(d, ncols, ld, a, LineShape(L.B, L.NT));
   IB_CUDA_CHECK(cudaGetLastError());
   return IB_OK;
 }

@@ -1430,7 +1430,11 @@ static int op_predict_levels(Ctx* c, bool seed_rhs_old) {
       a.lout[k] = c->hat[k];
     }
     ProfScope ps(c, 0, pass_bytes(c, 4 * L, L));
-    RC(dst_pass_x(c->px, g.nsy, g.nsx, PRE_PRED, a, g, c->lx_batch, st));
+    // a line a CTA whatever the plain passes take: the most CTAs, so that some are in the FP64 stencil
+    // while others transform (five levels of 800 x 400: 52 us, in the plain passes' tuned shape 58)
+    DstLaunch lp;
+    lp.B = 1; lp.NT = 128;
+    RC(dst_pass_x(c->px, g.nsy, g.nsx, PRE_PRED, a, g, lp, st));
   }
   if (c->rmap.on) {
     RC(rm_predict(c));   // the same recursion with the chain of level solves collapsed
