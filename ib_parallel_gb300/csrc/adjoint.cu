@@ -34,13 +34,53 @@ namespace {
 
 constexpr int kT = 256;
 
-// out = ((c0 B0) + (c1 B1)) + (c2 B2), rounded step by step
-__global__ void k_adj_combine(int n, const double* __restrict__ b0, const double* __restrict__ b1,
-                              const double* __restrict__ b2, double c0, double c1, double c2, double* __restrict__ out) {
+// The frame flux of every level, ((c0 B0) + (c1 B1)) + (c2 B2) rounded step by step: level
+// blockIdx.y's u-faces to ox, its v-faces to oy.  Memory traffic bounds it; one launch for all levels
+// (it was one or two a level, 4.2 us each at 600 x 300).
+struct FrameArgs {
+  const double* bases;   // [basis][level][u-faces, v-faces]
+  double c0, c1, c2;
+  int L, nu, nv;
+  double* ox[kMaxLevels];
+  double* oy[kMaxLevels];
+};
+__global__ void __launch_bounds__(kT) k_adj_frame(FrameArgs a) {
   IB_GRID_DEP_WAIT();
+  const int k = blockIdx.y, per = a.nu + a.nv;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  out[i] = __dadd_rn(__dadd_rn(__dmul_rn(c0, b0[i]), __dmul_rn(c1, b1[i])), __dmul_rn(c2, b2[i]));
+  if (i >= per) return;
+  const size_t all = (size_t)a.L * per;
+  const double* b = a.bases + (size_t)k * per + i;
+  const double v = __dadd_rn(__dadd_rn(__dmul_rn(a.c0, b[0]), __dmul_rn(a.c1, b[all])), __dmul_rn(a.c2, b[2 * all]));
+  if (i < a.nu) a.ox[k][i] = v;
+  else a.oy[k][i - a.nu] = v;
+}
+
+// Copies up to kMaxCopies arrays (blockIdx.y).  What bounds it is memory traffic: a copy each took
+// 5.5 us for 1.4 MB, all 21 of a 600 x 300 state 115 us.
+constexpr int kMaxCopies = 5 * kMaxLevels + 1;
+struct CopyArgs {
+  const double* src[kMaxCopies];
+  double* dst[kMaxCopies];
+  int n[kMaxCopies];
+};
+constexpr int kCopyUnroll = 4;
+__global__ void __launch_bounds__(kT) k_adj_copies(CopyArgs a) {
+  IB_GRID_DEP_WAIT();
+  const int e = blockIdx.y, n = a.n[e], i0 = blockIdx.x * (kT * kCopyUnroll) + threadIdx.x;
+  const double* __restrict__ src = a.src[e];
+  double* __restrict__ dst = a.dst[e];
+  double v[kCopyUnroll];
+#pragma unroll
+  for (int u = 0; u < kCopyUnroll; ++u) {
+    const int i = i0 + u * kT;
+    v[u] = i < n ? src[i] : 0.0;
+  }
+#pragma unroll
+  for (int u = 0; u < kCopyUnroll; ++u) {
+    const int i = i0 + u * kT;
+    if (i < n) dst[i] = v[u];
+  }
 }
 
 // T[i][j] = M[j][i] (n x n)
@@ -52,14 +92,32 @@ __global__ void k_adj_transpose(int n, const double* __restrict__ M, double* __r
   T[t] = M[(size_t)j * n + i];
 }
 
-// out = a x + b y (y may be null)
-__global__ void k_adj_axpby(int n, double a, const double* __restrict__ x, double b, const double* __restrict__ y,
-                            double* __restrict__ out) {
+// out = x + y
+__global__ void k_adj_add(int n, const double* __restrict__ x, const double* y, double* out) {
   IB_GRID_DEP_WAIT();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const double v = a * x[i];
-  out[i] = y ? v + b * y[i] : v;
+  out[i] = x[i] + y[i];
+}
+
+// The predictor's transpose at a vertex, from t = K x (x its output's adjoint, K = normalize
+// (I - cL)^-1):
+//  - omega's adjoint (I - cL)^-1 (I + cL) x = 2 (I - cL)^-1 x - x = two_over_norm t - x, added to lom;
+//  - rhs's, con1 t + lro (with con2 t at the first step, where rhs_old is rhs), and rhs_old's, con2 t.
+// Memory traffic bounds it.  The identity takes the place of a second predictor solve (two x passes,
+// one with the predictor's stencil, and a tridiagonal solve: 40 us a level at 600 x 300).
+__global__ void k_adj_pred(int n, const double* __restrict__ t, const double* __restrict__ x, double two_over_norm,
+                           double con1, double con2, bool first, const double* __restrict__ lro,
+                           double* __restrict__ lom, double* __restrict__ lrhs, double* __restrict__ lro_n) {
+  IB_GRID_DEP_WAIT();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double ti = t[i];
+  lom[i] = fma(two_over_norm, ti, -x[i]) + lom[i];
+  double r = fma(con1, ti, lro[i]);
+  if (first) r = fma(con2, ti, r);
+  lrhs[i] = r;
+  lro_n[i] = first ? 0.0 : con2 * ti;
 }
 
 // the ghosted vertex (r, c) (0-based rows and columns of the (n+1) x (m+1) frame) of which the
@@ -83,18 +141,10 @@ __device__ __forceinline__ double curl_T_at(const GridDims& g, const double* __r
   return v;
 }
 
-// ring += the ring's part of curl^T (the edges of the ghosted frame)
-__global__ void k_adj_ring_curl(GridDims g, const double* __restrict__ lx, const double* __restrict__ ly,
-                                double* __restrict__ ring) {
-  IB_GRID_DEP_WAIT();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= g.nbc) return;
-  int r, c;
-  if (ring_vertex(g, t, &r, &c)) ring[t] += curl_T_at(g, lx, ly, r, c);
-}
-
-// ring = fac * the boundary rows and columns of v (apply_bc^T; the ring's end entries zero)
-__global__ void k_adj_apply_bc(GridDims g, const double* __restrict__ v, double fac, double* __restrict__ ring) {
+// ring = fac * the boundary rows and columns of v (apply_bc^T; the ring's end entries zero), and with
+// lx set the ring's part of curl^T (the edges of the ghosted frame) added
+__global__ void k_adj_apply_bc(GridDims g, const double* __restrict__ v, double fac, const double* __restrict__ lx,
+                               const double* __restrict__ ly, double* __restrict__ ring) {
   IB_GRID_DEP_WAIT();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= g.nbc) return;
@@ -112,12 +162,17 @@ __global__ void k_adj_apply_bc(GridDims g, const double* __restrict__ v, double 
     const int i = t - g.top - 1;
     if (i >= 0 && i <= g.m - 2) out = fac * v[(g.n - 2) * g.nsx + i];
   }
+  if (lx) {
+    int r, c;
+    if (ring_vertex(g, t, &r, &c)) out += curl_T_at(g, lx, ly, r, c);
+  }
   ring[t] = out;
 }
 
-// s += get_bc^T(fac ring): every point of the coarse centre's perimeter gathers the ring
-// entries it was copied to and half of each midpoint beside it
-__global__ void k_adj_get_bc(GridDims g, const double* __restrict__ ring, double fac, double* __restrict__ s) {
+// s += get_bc^T(fac (ring + ring2)), ring2 null for none: every point of the coarse centre's perimeter
+// gathers the ring entries it was copied to and half of each midpoint beside it
+__global__ void k_adj_get_bc(GridDims g, const double* __restrict__ ring, const double* __restrict__ ring2, double fac,
+                             double* __restrict__ s) {
   IB_GRID_DEP_WAIT();
   const int i0 = g.m / 4 + 1, i1 = 3 * g.m / 4 + 1, j0 = g.n / 4 + 1, j1 = 3 * g.n / 4 + 1;
   const int nrow = i1 - i0 + 1, ncol = j1 - j0 - 1;
@@ -130,9 +185,10 @@ __global__ void k_adj_get_bc(GridDims g, const double* __restrict__ ring, double
   else return;
   auto line = [&](int base, int p, int p0, int p1, int q0) -> double {   // p along the line, q0 its start offset
     const int e = base + 2 * (p - 1 - q0);
-    double v = fac * ring[e];
-    if (p < p1) v += 0.5 * (fac * ring[e + 1]);
-    if (p > p0) v += 0.5 * (fac * ring[e - 1]);
+    auto r = [&](int t) { return fac * (ring2 ? ring[t] + ring2[t] : ring[t]); };
+    double v = r(e);
+    if (p < p1) v += 0.5 * r(e + 1);
+    if (p > p0) v += 0.5 * r(e - 1);
     return v;
   };
   double v = 0.0;
@@ -193,7 +249,7 @@ __device__ __forceinline__ double v_at(const GridDims& g, const double* qy, cons
 }
 
 // nonlinear^T in its vorticity argument (interior vertices, added to lom) and its ghost ring
-// (written to lbc; the corner entries of the left and right columns stay zero)
+// (written to lbc; zero in the corner entries of the left and right columns)
 __global__ void k_adj_nl_vertex(GridDims g, const double* __restrict__ qx, const double* __restrict__ q0x,
                                 const double* __restrict__ qy, const double* __restrict__ q0y,
                                 const double* __restrict__ lx, const double* __restrict__ ly, double* __restrict__ lom,
@@ -213,8 +269,12 @@ __global__ void k_adj_nl_vertex(GridDims g, const double* __restrict__ qx, const
     lom[(r - 1) * g.nsx + (c - 1)] += w;
   } else if (r == 0) {
     lbc[g.bottom + c] = w;
+    if (c == 0) lbc[g.left] = 0.0;
+    if (c == g.m) lbc[g.right] = 0.0;
   } else if (r == g.n) {
     lbc[g.top + c] = w;
+    if (c == 0) lbc[g.left + g.n] = 0.0;
+    if (c == g.m) lbc[g.right + g.n] = 0.0;
   } else if (c == 0) {
     lbc[g.left + r] = w;
   } else {
@@ -270,38 +330,49 @@ struct DotArgs {
   int L, nu, nv;
   double* part;          // 3 x kDotBlocks partial sums
 };
-constexpr int kDotBlocks = 152;
+constexpr int kDotBlocks = 2 * 152;
 
-// part[b][blk] = the block's slice of sum over levels of <lq0, B_b> (fixed-order tree)
-__global__ void k_adj_dots(DotArgs a) {
+// part[b][blk] = the block's slice of sum over levels of <lq0, B_b>: each thread's strided terms, a
+// shuffle tree per warp, the warps' sums in order.  Memory traffic bounds it (the adjoint read once
+// for the three bases).
+__global__ void __launch_bounds__(kT) k_adj_dots(DotArgs a) {
   IB_GRID_DEP_WAIT();
-  __shared__ double red[256];
-  const int b = blockIdx.y, blk = blockIdx.x;
+  __shared__ double red[3][kT / 32];
   const int per = a.nu + a.nv;
-  const long long total = (long long)a.L * per;
-  double acc = 0.0;
-  for (long long t = (long long)blk * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    const int k = (int)(t / per), i = (int)(t % per);
-    double l = i < a.nu ? a.lx[k][i] : a.ly[k][i - a.nu];
-    if (k == 0) l += i < a.nu ? a.ax[i] : a.ay[i - a.nu];
-    acc = fma(l, a.bases[((size_t)b * a.L + k) * per + i], acc);
+  const size_t all = (size_t)a.L * per;
+  double acc[3] = {0.0, 0.0, 0.0};
+  for (int k = 0; k < a.L; ++k) {
+    const double* b = a.bases + (size_t)k * per;
+    const double* lx = a.lx[k];
+    const double* ly = a.ly[k];
+#pragma unroll 4
+    for (int i = blockIdx.x * kT + threadIdx.x; i < per; i += kDotBlocks * kT) {
+      double l = i < a.nu ? lx[i] : ly[i - a.nu];
+      if (k == 0) l += i < a.nu ? a.ax[i] : a.ay[i - a.nu];
+      for (int q = 0; q < 3; ++q) acc[q] = fma(l, b[q * all + i], acc[q]);
+    }
   }
-  red[threadIdx.x] = acc;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int q = 0; q < 3; ++q) {
+    for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+    if (lane == 0) red[q][warp] = acc[q];
+  }
   __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-    __syncthreads();
+  if (threadIdx.x < 3) {
+    double s = 0.0;
+    for (int w = 0; w < kT / 32; ++w) s += red[threadIdx.x][w];
+    a.part[threadIdx.x * kDotBlocks + blockIdx.x] = s;
   }
-  if (threadIdx.x == 0) a.part[b * gridDim.x + blk] = red[0];
 }
 
-__global__ void k_adj_dots_sum(const double* __restrict__ part, int nblk, double* __restrict__ out) {
+// out[b] = the sum of part[b], a warp per basis
+__global__ void k_adj_dots_sum(const double* __restrict__ part, double* __restrict__ out) {
   IB_GRID_DEP_WAIT();
-  const int b = threadIdx.x;
-  if (b >= 3) return;
+  const int b = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double s = 0.0;
-  for (int i = 0; i < nblk; ++i) s += part[b * nblk + i];
-  out[b] = s;
+  for (int i = lane; i < kDotBlocks; i += 32) s += part[b * kDotBlocks + i];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) out[b] = s;
 }
 
 int blocks(long long n) { return (int)cdiv(n, kT); }
@@ -319,24 +390,39 @@ struct Adj {
   cudaStream_t st;
 };
 
-int axpby(cudaStream_t st, int n, double a, const double* x, double b, const double* y, double* out) {
+int add(cudaStream_t st, int n, const double* x, const double* y, double* out) {
   count_launch();
-  k_adj_axpby<<<blocks(n), kT, 0, st>>>(n, a, x, b, y, out);
+  k_adj_add<<<blocks(n), kT, 0, st>>>(n, x, y, out);
   IB_CUDA_CHECK(cudaGetLastError());
   return IB_OK;
 }
 
-int get_bc_T(const GridDims& g, const double* ring, double fac, double* s, cudaStream_t st) {
+// the frame flux of the coefficients fr on every level
+int frame_flux(Ctx* c, const double* fr, double* const* ox, double* const* oy) {
+  const GridDims& g = c->g;
+  FrameArgs f;
+  f.bases = c->adj.bases;
+  f.c0 = fr[0]; f.c1 = fr[1]; f.c2 = fr[2];
+  f.L = c->L; f.nu = g.nu; f.nv = g.nv;
+  for (int k = 0; k < c->L; ++k) { f.ox[k] = ox[k]; f.oy[k] = oy[k]; }
+  count_launch();
+  k_adj_frame<<<dim3(blocks(g.nu + g.nv), c->L), kT, 0, c->st>>>(f);
+  IB_CUDA_CHECK(cudaGetLastError());
+  return IB_OK;
+}
+
+int get_bc_T(const GridDims& g, const double* ring, const double* ring2, double fac, double* s, cudaStream_t st) {
   const int n = 2 * (g.m / 2 + 1) + 2 * (g.n / 2 - 1);
   count_launch();
-  k_adj_get_bc<<<blocks(n), kT, 0, st>>>(g, ring, fac, s);
+  k_adj_get_bc<<<blocks(n), kT, 0, st>>>(g, ring, ring2, fac, s);
   IB_CUDA_CHECK(cudaGetLastError());
   return IB_OK;
 }
 
-int apply_bc_T(const GridDims& g, const double* v, double fac, double* ring, cudaStream_t st) {
+int apply_bc_T(const GridDims& g, const double* v, double fac, const double* lx, const double* ly, double* ring,
+               cudaStream_t st) {
   count_launch();
-  k_adj_apply_bc<<<blocks(g.nbc), kT, 0, st>>>(g, v, fac, ring);
+  k_adj_apply_bc<<<blocks(g.nbc), kT, 0, st>>>(g, v, fac, lx, ly, ring);
   IB_CUDA_CHECK(cudaGetLastError());
   return IB_OK;
 }
@@ -353,24 +439,18 @@ int coarsify_chain_T(Adj& a, double* const* lam) {
 }
 
 // vort2flux's solves transposed: flux adjoints (null: zero) of every level -> vorticity
-// adjoints added to lw
-int vsolve_T(Adj& a, double* const* lqx, double* const* lqy, double* const* lw) {
+// adjoints, lw = from + theirs
+int vsolve_T(Adj& a, double* const* lqx, double* const* lqy, double* const* from, double* const* lw) {
   AdjointState& A = a.A;
   const GridDims& g = a.g;
   for (int k = 0; k < a.L; ++k) {
     const bool has = lqx[k] != nullptr;
     if (has) RC(launch_rot(g, lqx[k], lqy[k], A.t1, a.st));
     else IB_CUDA_CHECK(cudaMemsetAsync(A.t1, 0, 8 * (size_t)g.ns, a.st));
-    if (k > 0) RC(get_bc_T(g, A.ring1, 1.0, A.t1, a.st));
+    if (k > 0) RC(get_bc_T(g, A.ring1, nullptr, 1.0, A.t1, a.st));
     RC(op_ctci(a.c, A.t1, A.t2, nullptr));
-    RC(axpby(a.st, g.ns, 1.0, A.t2, 1.0, lw[k], lw[k]));
-    if (k < a.L - 1) {
-      RC(apply_bc_T(g, A.t2, 1.0, A.ring1, a.st));
-      if (has) {
-        count_launch();
-        k_adj_ring_curl<<<blocks(g.nbc), kT, 0, a.st>>>(g, lqx[k], lqy[k], A.ring1);
-      }
-    }
+    RC(add(a.st, g.ns, A.t2, from[k], lw[k]));
+    if (k < a.L - 1) RC(apply_bc_T(g, A.t2, 1.0, lqx[k], lqy[k], A.ring1, a.st));
   }
   IB_CUDA_CHECK(cudaGetLastError());
   return IB_OK;
@@ -390,17 +470,18 @@ int step_T(Adj& a, int slot, int it, const double* frame, const double* dforce_h
   auto t_qx = [&](int k) { return tp + k * per + g.ns; };
   auto t_qy = [&](int k) { return tp + k * per + g.ns + g.nu; };
   // the step's frame flux (for nonlinear's transpose) and the force adjoint
-  for (int k = 0; k < L; ++k) {
-    const double* B[3];
-    for (int b = 0; b < 3; ++b) B[b] = A.bases + ((size_t)b * L + k) * (g.nu + g.nv);
-    count_launch();
-    k_adj_combine<<<blocks(g.nu + g.nv), kT, 0, st>>>(g.nu + g.nv, B[0], B[1], B[2], frame[0], frame[1], frame[2],
-                                                       A.q0 + k * (size_t)(g.nu + g.nv));
+  {
+    double* ox[kMaxLevels];
+    double* oy[kMaxLevels];
+    for (int k = 0; k < L; ++k) {
+      ox[k] = A.q0 + k * (size_t)(g.nu + g.nv);
+      oy[k] = ox[k] + g.nu;
+    }
+    RC(frame_flux(c, frame, ox, oy));
   }
   IB_CUDA_CHECK(cudaMemcpyAsync(A.dforce, dforce_h, 16 * (size_t)c->nbody, cudaMemcpyHostToDevice, st));
   // final vort2flux: its solves, then its coarsify
-  for (int k = 0; k < L; ++k) IB_CUDA_CHECK(cudaMemcpyAsync(A.lw[k], A.lom[k], 8 * (size_t)g.ns, cudaMemcpyDeviceToDevice, st));
-  RC(vsolve_T(a, A.lqx.data(), A.lqy.data(), A.lw.data()));
+  RC(vsolve_T(a, A.lqx.data(), A.lqy.data(), A.lom.data(), A.lw.data()));
   RC(coarsify_chain_T(a, A.lw.data()));
   // correction omega_0 - ainv(rot(reg f)), the direct solve, the force coefficients
   RC(op_ainv(c, A.lw[0], A.t1));
@@ -440,50 +521,40 @@ int step_T(Adj& a, int slot, int it, const double* frame, const double* dforce_h
   } else {
     RC(launch_reg(g, c->nf, A.lrhsf, c->reg, A.ax, A.ay, st));
   }
-  for (int k = 0; k < L; ++k) IB_CUDA_CHECK(cudaMemcpyAsync(A.lostar[k], A.lw[k], 8 * (size_t)g.ns, cudaMemcpyDeviceToDevice, st));
   {
     std::vector<double*> zx(L, nullptr), zy(L, nullptr);
     zx[0] = A.ax;
     zy[0] = A.ay;
-    RC(vsolve_T(a, zx.data(), zy.data(), A.lostar.data()));
+    RC(vsolve_T(a, zx.data(), zy.data(), A.lw.data(), A.lostar.data()));
   }
   RC(coarsify_chain_T(a, A.lostar.data()));
   // the predictor, level by level from the finest (each level reads its coarser neighbour)
-  for (int k = 0; k < L; ++k) IB_CUDA_CHECK(cudaMemsetAsync(A.lom_n[k], 0, 8 * (size_t)g.ns, st));
+  IB_CUDA_CHECK(cudaMemsetAsync(A.lom_n[0], 0, 8 * (size_t)L * g.ns, st));   // the levels lie one after the other
   for (int k = 0; k < L; ++k) {
-    // t = (I - cL)^-1 lostar_k (the boundary right-hand side's adjoint), om = (I + cL)(I - cL)^-1 lostar_k
-    IB_CUDA_CHECK(cudaMemsetAsync(A.t1, 0, 8 * (size_t)g.ns, st));
-    RC(op_predictor(c, k, A.t1, A.zero_v, A.zero_v, A.lostar[k]));
-    IB_CUDA_CHECK(cudaMemcpyAsync(A.t2, A.lostar[k], 8 * (size_t)g.ns, cudaMemcpyDeviceToDevice, st));
-    RC(op_predictor(c, k, A.t2, A.zero_v, A.zero_v, A.zero_v));
-    RC(axpby(st, g.ns, 1.0, A.t2, 1.0, A.lom_n[k], A.lom_n[k]));
-    // lrhs = con1 t + lro_k (+ con2 t at the first step, where rhs_old is rhs)
-    RC(axpby(st, g.ns, c->con1[k], A.t1, 1.0, A.lro[k], A.t3));
-    if (it == 1) {
-      RC(axpby(st, g.ns, c->con2[k], A.t1, 1.0, A.t3, A.t3));
-      IB_CUDA_CHECK(cudaMemsetAsync(A.lro_n[k], 0, 8 * (size_t)g.ns, st));
-    } else {
-      RC(axpby(st, g.ns, c->con2[k], A.t1, 0.0, nullptr, A.lro_n[k]));
-    }
+    // t = normalize (I - cL)^-1 lostar_k: the adjoint of the right-hand side; omega's and the
+    // right-hand sides' follow from it
+    RC(op_predictor_solve(c, k, A.lostar[k], A.t1));
+    count_launch();
+    k_adj_pred<<<blocks(g.ns), kT, 0, st>>>(g.ns, A.t1, A.lostar[k], 2.0 / c->normalize, c->con1[k], c->con2[k],
+                                            it == 1, A.lro[k], A.lom_n[k], A.t3, A.lro_n[k]);
+    IB_CUDA_CHECK(cudaGetLastError());
     // rhsbc = apply_bc(lastbc) + apply_bc(omegabc): both rings' adjoint
-    RC(apply_bc_T(g, A.t1, c->vfac[k], A.ring2, st));
-    if (k < L - 1) RC(get_bc_T(g, A.ring2, 0.25, A.lostar[k + 1], st));
+    if (k < L - 1) {
+      RC(apply_bc_T(g, A.t1, c->vfac[k], nullptr, nullptr, A.ring2, st));
+      RC(get_bc_T(g, A.ring2, nullptr, 0.25, A.lostar[k + 1], st));
+    }
     // rhs = rot(nonlinear(omega_k, q_k + q0_k, lastbc_k))
     RC(launch_curl(g, A.t3, c->zero_ring, A.hx, A.hy, st));
     if (k < L - 1) RC(launch_get_bc(g, t_om(k + 1), 0.25, A.ring3, st));
-    else IB_CUDA_CHECK(cudaMemsetAsync(A.ring3, 0, 8 * (size_t)g.nbc, st));
-    IB_CUDA_CHECK(cudaMemsetAsync(A.ring1, 0, 8 * (size_t)g.nbc, st));
     const double* q0x = A.q0 + k * (size_t)(g.nu + g.nv);
     const double* q0y = q0x + g.nu;
     count_launches(2);
     k_adj_nl_vertex<<<blocks((long long)(g.n + 1) * (g.m + 1)), kT, 0, st>>>(g, t_qx(k), q0x, t_qy(k), q0y, A.hx,
                                                                              A.hy, A.lom_n[k], A.ring1);
-    k_adj_nl_faces<<<blocks(g.nu + g.nv), kT, 0, st>>>(g, t_om(k), A.ring3, A.hx, A.hy, A.lqx_n[k], A.lqy_n[k]);
+    k_adj_nl_faces<<<blocks(g.nu + g.nv), kT, 0, st>>>(g, t_om(k), k < L - 1 ? A.ring3 : c->zero_ring, A.hx, A.hy,
+                                                            A.lqx_n[k], A.lqy_n[k]);
     IB_CUDA_CHECK(cudaGetLastError());
-    if (k < L - 1) {
-      RC(axpby(st, g.nbc, 1.0, A.ring2, 1.0, A.ring1, A.ring1));
-      RC(get_bc_T(g, A.ring1, 0.25, A.lom_n[k + 1], st));
-    }
+    if (k < L - 1) RC(get_bc_T(g, A.ring2, A.ring1, 0.25, A.lom_n[k + 1], st));
   }
   // dJ/d(u, v, W): the frame flux's adjoint (nonlinear's on every level, the Schur right-hand
   // side's on level 0) against each basis
@@ -491,8 +562,8 @@ int step_T(Adj& a, int slot, int it, const double* frame, const double* dforce_h
   for (int k = 0; k < L; ++k) { d.lx[k] = A.lqx_n[k]; d.ly[k] = A.lqy_n[k]; }
   d.ax = A.ax; d.ay = A.ay; d.bases = A.bases; d.L = L; d.nu = g.nu; d.nv = g.nv; d.part = A.dpart;
   count_launches(2);
-  k_adj_dots<<<dim3(kDotBlocks, 3), 256, 0, st>>>(d);
-  k_adj_dots_sum<<<1, 32, 0, st>>>(A.dpart, kDotBlocks, dframe_d);
+  k_adj_dots<<<kDotBlocks, kT, 0, st>>>(d);
+  k_adj_dots_sum<<<1, 96, 0, st>>>(A.dpart, dframe_d);
   IB_CUDA_CHECK(cudaGetLastError());
   std::swap(A.lom, A.lom_n);
   std::swap(A.lqx, A.lqx_n);
@@ -509,48 +580,58 @@ size_t state_doubles(const Ctx* c) {
   return (size_t)c->L * (3 * (size_t)g.ns + g.nu + g.nv) + (size_t)c->nf;
 }
 
-int save_state(Ctx* c, double* dst) {
-  const GridDims& g = c->g;
-  double* p = dst;
-  for (int k = 0; k < c->L; ++k) {
-    for (auto [src, n] : {std::pair<const double*, size_t>{c->omega[k], (size_t)g.ns}, {c->s[k], (size_t)g.ns},
-                          {c->qx[k], (size_t)g.nu}, {c->qy[k], (size_t)g.nv}, {c->rhs_old[k], (size_t)g.ns}}) {
-      IB_CUDA_CHECK(cudaMemcpyAsync(p, src, 8 * n, cudaMemcpyDeviceToDevice, c->st));
-      p += n;
-    }
-  }
-  IB_CUDA_CHECK(cudaMemcpyAsync(p, c->f, 8 * (size_t)c->nf, cudaMemcpyDeviceToDevice, c->st));
-  return IB_OK;
-}
-
-int load_state(Ctx* c, const double* src) {
-  const GridDims& g = c->g;
-  const double* p = src;
-  for (int k = 0; k < c->L; ++k) {
-    for (auto [dst, n] : {std::pair<double*, size_t>{c->omega[k], (size_t)g.ns}, {c->s[k], (size_t)g.ns},
-                          {c->qx[k], (size_t)g.nu}, {c->qy[k], (size_t)g.nv}, {c->rhs_old[k], (size_t)g.ns}}) {
-      IB_CUDA_CHECK(cudaMemcpyAsync(dst, p, 8 * n, cudaMemcpyDeviceToDevice, c->st));
-      p += n;
-    }
-  }
-  IB_CUDA_CHECK(cudaMemcpyAsync(c->f, p, 8 * (size_t)c->nf, cudaMemcpyDeviceToDevice, c->st));
-  return IB_OK;
-}
-
-int set_frame(Ctx* c, const double* fr) {
-  AdjointState& A = c->adj;
-  const GridDims& g = c->g;
-  for (int k = 0; k < c->L; ++k) {
-    const double* B[3];
-    for (int b = 0; b < 3; ++b) B[b] = A.bases + ((size_t)b * c->L + k) * (g.nu + g.nv);
-    count_launches(2);
-    k_adj_combine<<<blocks(g.nu), kT, 0, c->st>>>(g.nu, B[0], B[1], B[2], fr[0], fr[1], fr[2], c->q0x[k]);
-    k_adj_combine<<<blocks(g.nv), kT, 0, c->st>>>(g.nv, B[0] + g.nu, B[1] + g.nu, B[2] + g.nu, fr[0], fr[1], fr[2],
-                                                   c->q0y[k]);
-  }
+int launch_copies(const CopyArgs& a, int cnt, int nmax, cudaStream_t st) {
+  count_launch();
+  k_adj_copies<<<dim3(cdiv(nmax, kT * kCopyUnroll), cnt), kT, 0, st>>>(a);
   IB_CUDA_CHECK(cudaGetLastError());
   return IB_OK;
 }
+
+// The state's arrays to (store) or from p.
+int copy_state(Ctx* c, double* p, bool store) {
+  const GridDims& g = c->g;
+  CopyArgs a;
+  int cnt = 0, nmax = 0;
+  auto one = [&](double* v, int n) {
+    a.src[cnt] = store ? v : p;
+    a.dst[cnt] = store ? p : v;
+    a.n[cnt++] = n;
+    nmax = std::max(nmax, n);
+    p += n;
+  };
+  for (int k = 0; k < c->L; ++k) {
+    one(c->omega[k], g.ns);
+    one(c->s[k], g.ns);
+    one(c->qx[k], g.nu);
+    one(c->qy[k], g.nv);
+    one(c->rhs_old[k], g.ns);
+  }
+  one(c->f, c->nf);
+  return launch_copies(a, cnt, nmax, c->st);
+}
+int save_state(Ctx* c, double* dst) { return copy_state(c, dst, true); }
+int load_state(Ctx* c, double* src) { return copy_state(c, src, false); }
+
+// omega, qx and qy of every level to the tape at tp
+int tape_inputs(Ctx* c, double* tp) {
+  const GridDims& g = c->g;
+  CopyArgs a;
+  int cnt = 0;
+  auto one = [&](const double* v, int n) {
+    a.src[cnt] = v;
+    a.dst[cnt] = tp;
+    a.n[cnt++] = n;
+    tp += n;
+  };
+  for (int k = 0; k < c->L; ++k) {
+    one(c->omega[k], g.ns);
+    one(c->qx[k], g.nu);
+    one(c->qy[k], g.nv);
+  }
+  return launch_copies(a, cnt, std::max(g.nu, g.nv), c->st);
+}
+
+int set_frame(Ctx* c, const double* fr) { return frame_flux(c, fr, c->q0x.data(), c->q0y.data()); }
 
 }  // namespace
 
@@ -593,7 +674,7 @@ static int adjoint_alloc(Ctx* c) {
   const size_t per_basis = (size_t)L * (g.nu + g.nv);
   const size_t n = 3 * per_basis + per_basis /* q0 */ + 4 * (size_t)L * g.ns /* lom, lro (x2) */ +
                    2 * (size_t)L * (g.nu + g.nv) /* lq (x2) */ + 2 * (size_t)L * g.ns /* lw, lostar */ +
-                   4 * (size_t)g.ns /* t1-t3, zero */ + 3 * (size_t)(g.nu + g.nv) /* hx hy, ax ay */ +
+                   3 * (size_t)g.ns /* t1-t3 */ + 3 * (size_t)(g.nu + g.nv) /* hx hy, ax ay */ +
                    3 * (size_t)g.nbc + 2 * (size_t)std::max(c->nf, 1) + 2 * (size_t)std::max(c->nbody, 1) +
                    3 * 4096 + 3 * (size_t)kDotBlocks + (size_t)std::max(c->nf, 1) * std::max(c->nf, 1);
   IB_CUDA_CHECK(cudaMalloc(&A.mem, 8 * n));
@@ -606,7 +687,7 @@ static int adjoint_alloc(Ctx* c) {
   lv(A.lom, g.ns); lv(A.lom_n, g.ns); lv(A.lro, g.ns); lv(A.lro_n, g.ns);
   lv(A.lqx, g.nu); lv(A.lqy, g.nv); lv(A.lqx_n, g.nu); lv(A.lqy_n, g.nv);
   lv(A.lw, g.ns); lv(A.lostar, g.ns);
-  A.t1 = take(g.ns); A.t2 = take(g.ns); A.t3 = take(g.ns); A.zero_v = take(g.ns);
+  A.t1 = take(g.ns); A.t2 = take(g.ns); A.t3 = take(g.ns);
   A.hx = take(g.nu); A.hy = take(g.nv); A.ax = take(g.nu); A.ay = take(g.nv);
   take(g.nu + g.nv);
   A.ring1 = take(g.nbc); A.ring2 = take(g.nbc); A.ring3 = take(g.nbc);
@@ -640,21 +721,29 @@ int op_adjoint_forward(Ctx* c, int nsteps, int K, const double* frames, double* 
   RC(adjoint_alloc(c));
   const int nseg = (nsteps + K - 1) / K;
   const size_t sd = state_doubles(c);
-  if (A.ckpt) cudaFree(A.ckpt);
-  if (A.tape) cudaFree(A.tape);
-  A.ckpt = nullptr;
-  A.tape = nullptr;
-  {
+  // kept from the last forward where they have the size to within a factor of two (both are held
+  // after a forward anyway)
+  const size_t nck = sd * (nseg + 1) + 2 * (size_t)nsteps * c->nbody;
+  const size_t ntape = (size_t)K * c->L * (c->g.ns + c->g.nu + c->g.nv);
+  auto fits = [](size_t n, size_t cap) { return n <= cap && cap / 2 <= n; };
+  if (!fits(nck, A.ckpt_cap) || !fits(ntape, A.tape_cap)) {
+    if (A.ckpt) cudaFree(A.ckpt);
+    if (A.tape) cudaFree(A.tape);
+    A.ckpt = A.tape = nullptr;
+    A.ckpt_cap = A.tape_cap = 0;
+    A.ready = false;
     size_t freeb = 0, totalb = 0;
     IB_CUDA_CHECK(cudaMemGetInfo(&freeb, &totalb));
-    const size_t need = 8 * (sd * (nseg + 1) + (size_t)K * c->L * (c->g.ns + c->g.nu + c->g.nv));
-    if (need > freeb / 2) {
+    if (8 * (nck + ntape) > freeb / 2) {
       *msg = "checkpoints and tape do not fit in device memory (raise K?)";
       return IB_ERR_NOMEM;
     }
+    IB_CUDA_CHECK(cudaMalloc(&A.ckpt, 8 * nck));
+    A.ckpt_cap = nck;
+    IB_CUDA_CHECK(cudaMalloc(&A.tape, 8 * ntape));
+    A.tape_cap = ntape;
   }
-  IB_CUDA_CHECK(cudaMalloc(&A.ckpt, 8 * sd * (nseg + 1)));
-  IB_CUDA_CHECK(cudaMalloc(&A.tape, 8 * (size_t)K * c->L * (c->g.ns + c->g.nu + c->g.nv)));
+  double* fdev = A.ckpt + sd * (nseg + 1);   // each step's force coefficients, read at the end
   A.nsteps = nsteps;
   A.K = K;
   A.nseg = nseg;
@@ -668,18 +757,18 @@ int op_adjoint_forward(Ctx* c, int nsteps, int K, const double* frames, double* 
     }
     RC(set_frame(c, frames + 3 * (size_t)n));
     RC(op_advance(c));
-    RC(launch_force_coeffs(c->nf, c->nbody, c->comp, c->bid, c->f, c->p.dt, c->delta, c->forces, c->st));
-    std::vector<double> fc(2 * (size_t)c->nbody);
-    IB_CUDA_CHECK(cudaMemcpyAsync(fc.data(), c->forces, 16 * (size_t)c->nbody, cudaMemcpyDeviceToHost, c->st));
-    IB_CUDA_CHECK(cudaStreamSynchronize(c->st));
-    for (int b = 0; b < c->nbody; ++b) {
-      forces[((size_t)n * c->nbody + b) * 2] = fc[b];
-      forces[((size_t)n * c->nbody + b) * 2 + 1] = fc[c->nbody + b];
-    }
+    RC(launch_force_coeffs(c->nf, c->nbody, c->comp, c->bid, c->f, c->p.dt, c->delta, c->forces, c->st,
+                           fdev + 2 * (size_t)n * c->nbody, nullptr, 0));
   }
   RC(save_state(c, A.ckpt + sd * nseg));
   A.it_ckpt[nseg] = c->itime;
+  std::vector<double> fc(2 * (size_t)nsteps * c->nbody);
+  IB_CUDA_CHECK(cudaMemcpyAsync(fc.data(), fdev, 8 * fc.size(), cudaMemcpyDeviceToHost, c->st));
   IB_CUDA_CHECK(cudaStreamSynchronize(c->st));
+  for (int n = 0; n < nsteps; ++n)
+    for (int b = 0; b < c->nbody; ++b)
+      for (int q = 0; q < 2; ++q)
+        forces[((size_t)n * c->nbody + b) * 2 + q] = fc[(2 * (size_t)n + q) * c->nbody + b];
   A.ready = true;
   return IB_OK;
 }
@@ -696,12 +785,10 @@ int op_adjoint_backward(Ctx* c, const double* dforces, double* dframes, std::str
   const size_t per = (size_t)g.ns + g.nu + g.nv;
   Adj a{c, A, g, L, c->st};
   // the adjoint state after the last step: zero
-  for (int k = 0; k < L; ++k) {
-    IB_CUDA_CHECK(cudaMemsetAsync(A.lom[k], 0, 8 * (size_t)g.ns, c->st));
-    IB_CUDA_CHECK(cudaMemsetAsync(A.lro[k], 0, 8 * (size_t)g.ns, c->st));
-    IB_CUDA_CHECK(cudaMemsetAsync(A.lqx[k], 0, 8 * (size_t)g.nu, c->st));
-    IB_CUDA_CHECK(cudaMemsetAsync(A.lqy[k], 0, 8 * (size_t)g.nv, c->st));
-  }
+  IB_CUDA_CHECK(cudaMemsetAsync(A.lom[0], 0, 8 * (size_t)L * g.ns, c->st));
+  IB_CUDA_CHECK(cudaMemsetAsync(A.lro[0], 0, 8 * (size_t)L * g.ns, c->st));
+  IB_CUDA_CHECK(cudaMemsetAsync(A.lqx[0], 0, 8 * (size_t)L * g.nu, c->st));
+  IB_CUDA_CHECK(cudaMemsetAsync(A.lqy[0], 0, 8 * (size_t)L * g.nv, c->st));
   const bool graphs = c->use_whole_step;
   for (int seg = A.nseg - 1; seg >= 0; --seg) {
     const int n0 = seg * A.K, n1 = std::min(A.nsteps, n0 + A.K);
@@ -709,13 +796,7 @@ int op_adjoint_backward(Ctx* c, const double* dforces, double* dframes, std::str
     RC(load_state(c, A.ckpt + sd * seg));
     c->itime = A.it_ckpt[seg];
     for (int n = n0; n < n1; ++n) {
-      double* tp = A.tape + (size_t)(n - n0) * L * per;
-      for (int k = 0; k < L; ++k) {
-        IB_CUDA_CHECK(cudaMemcpyAsync(tp + k * per, c->omega[k], 8 * (size_t)g.ns, cudaMemcpyDeviceToDevice, c->st));
-        IB_CUDA_CHECK(cudaMemcpyAsync(tp + k * per + g.ns, c->qx[k], 8 * (size_t)g.nu, cudaMemcpyDeviceToDevice, c->st));
-        IB_CUDA_CHECK(cudaMemcpyAsync(tp + k * per + g.ns + g.nu, c->qy[k], 8 * (size_t)g.nv, cudaMemcpyDeviceToDevice,
-                                      c->st));
-      }
+      RC(tape_inputs(c, A.tape + (size_t)(n - n0) * L * per));
       RC(set_frame(c, A.frames.data() + 3 * (size_t)n));
       RC(op_advance(c));
     }

@@ -232,12 +232,13 @@ struct AdjointState {
   std::vector<double> frames;          // nsteps x (u, v, W)
   std::vector<long long> it_ckpt;      // itime at each checkpoint
   void* mem = nullptr;                 // the fixed-size buffers below
-  double* ckpt = nullptr;              // (nseg + 1) states
+  double* ckpt = nullptr;              // (nseg + 1) states, then every step's force coefficients
   double* tape = nullptr;              // K x levels x (omega, qx, qy)
+  size_t ckpt_cap = 0, tape_cap = 0;   // their lengths
   double* bases = nullptr;             // 3 x levels x (u-faces, v-faces)
   double* q0 = nullptr;                // one step's frame flux, levels x (u-faces, v-faces)
   std::vector<double*> lom, lro, lqx, lqy, lom_n, lro_n, lqx_n, lqy_n, lw, lostar;
-  double *t1 = nullptr, *t2 = nullptr, *t3 = nullptr, *zero_v = nullptr;
+  double *t1 = nullptr, *t2 = nullptr, *t3 = nullptr;
   double *hx = nullptr, *hy = nullptr, *ax = nullptr, *ay = nullptr;
   double *ring1 = nullptr, *ring2 = nullptr, *ring3 = nullptr;
   double *lf = nullptr, *lrhsf = nullptr, *dforce = nullptr, *dframe = nullptr, *dpart = nullptr;
@@ -441,6 +442,7 @@ int op_ctci(Ctx* c, const double* in, double* out, const double* ring);  // ring
 int op_ainv(Ctx* c, const double* in, double* out);
 int op_dst(Ctx* c, const double* in, double* out);
 int op_predictor(Ctx* c, int k, double* om, const double* rhs, const double* rhs_old, const double* rhsbc);
+int op_predictor_solve(Ctx* c, int k, const double* in, double* out);
 // coarse_modes_given: the coarser levels' vorticity outside the rows coarsify writes is the
 // inverse x transform of the predictor's modes still in hat[k] (within a time step only)
 // hat0_add (with hat0_given): the finest level's modes are hat[0] + hat0_add

@@ -529,6 +529,13 @@ int op_predictor(Ctx* c, int k, double* om, const double* rhs, const double* rhs
   return spectral_solve(c, PRE_PRED, a, c->tri_pred[k], om);
 }
 
+// The predictor's solve alone: out = normalize (I - cL)^-1 in.
+int op_predictor_solve(Ctx* c, int k, const double* in, double* out) {
+  DstXArgs a;
+  a.in = in;
+  return spectral_solve(c, PRE_COPY, a, c->tri_pred[k], out);
+}
+
 static int ring_from_modes(Ctx* c, const double* spec, double* s, double* ring, double fac = 1.0);
 
 // The boundary terms level k's solve adds: from its ring, left by level k+1.
