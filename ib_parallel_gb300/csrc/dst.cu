@@ -607,8 +607,10 @@ __global__ void __launch_bounds__(512, 2) k_dst_x(DstDev pl, int nrows, int ld, 
 // (warp_sum_mirror); E keeps only its entries of equal parity.  CTAs of kReWarps warps:
 // [0, nlr) take kReSeg entries of both the left and the right side (kReWarps vertex pairs);
 // [nlr, nlr + 2 nbt) kReSeg entries of the left half of the bottom or top side and their
-// mirrors; then one warp per mode k for the two edge dot products (dst_ring_from_modes launches
-// the first two groups alone, sd and edge null).
+// mirrors; then one warp per mode k for the two edge dot products.  dst_ring_from_modes launches
+// the first two groups alone (sd and edge null); a caller that reads sd and edge only launches the
+// second group empty (nbt 0, ring null).  What bounds it is FP64: the bottom and top vertices are a
+// quarter of its dot products at 800 x 400.
 // 4 against 8 warps: 401 CTAs against 187 at 800 x 400, so no SM has twice its share; 7.6 against 7.9 us
 // (8.2 before the two edge sums of a mode shared one reduction, warp_sum2)
 constexpr int kReWarps = 4;
@@ -641,8 +643,10 @@ __global__ void __launch_bounds__(32 * kReWarps) k_ring_edge(int N, GridDims g, 
         const double vl = (p & 1) ? 0.5 * (sp[qq] + sp[qq + 1]) : sp[qq];
         const double vr = (p & 1) ? 0.5 * (spm[qq] + spm[qq + 1]) : spm[qq];
         const double xl = vl * fac, xr = vr * fac;
-        ring[g.left + p] = xl;
-        ring[g.right + p] = xr;
+        if (ring) {
+          ring[g.left + p] = xl;
+          ring[g.right + p] = xr;
+        }
         const int r = p - 1;
         if (sd && r >= 0 && r < g.nsy) {
           sd[r] = xl + xr;
@@ -702,7 +706,7 @@ int dst_ring_from_modes(const DstPlan& px, const GridDims& g, const double* spec
 
 int dst_ring_edge_from_modes(const DstPlan& px, const GridDims& g, const double* spec, int ld, const double* W,
                              const double* E, double fac, double* ring, double* sd, double* edge, cudaStream_t st) {
-  const int nlr = cdiv(g.n + 1, kReSeg), nbt = cdiv(g.m / 2 + 1, kReSeg);
+  const int nlr = cdiv(g.n + 1, kReSeg), nbt = ring ? cdiv(g.m / 2 + 1, kReSeg) : 0;
   count_launch();
   k_ring_edge<<<nlr + 2 * nbt + cdiv(px.N, kReWarps), 32 * kReWarps, 0, st>>>(px.N, g, spec, ld, W, E, fac, ring, sd,
                                                                               edge, nlr, nbt);

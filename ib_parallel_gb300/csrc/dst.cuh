@@ -197,7 +197,7 @@ int dst_x_bc_modes(const DstPlan& px, const GridDims& g, const double* ring, con
 // evaluated at the points get_bc reads only (dot products with W).
 int dst_ring_from_modes(const DstPlan& px, const GridDims& g, const double* spec, int ld, const double* W, double fac,
                         double* ring, cudaStream_t st);
-// The same ring, plus the boundary terms the finer level's solve adds to its right-hand side
+// The same ring (null: not wanted), plus the boundary terms the finer level's solve adds to its right-hand side
 // modes (tri_solve's TriBc): sd (2 x nsy) the sums and differences of the ring's left and right
 // entries 1..n-1, edge (2 x N) the x transforms of its bottom and top entries 1..m-1, from the
 // edge matrix E (dst_edge_matrix) and the coarse modes of the two rows get_bc reads.

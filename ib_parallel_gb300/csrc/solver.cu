@@ -549,10 +549,11 @@ static TriBc level_bc(Ctx* c, int k, double post_scale) {
 }
 
 // Level k's ring (fac * get_bc of the coarser level's streamfunction or vorticity, from its
-// modes spec) and the boundary terms of its solve.
-static int ring_edge_from_modes(Ctx* c, const double* spec, int k, double fac) {
-  return dst_ring_edge_from_modes(c->px, c->g, spec, c->g.nsx, c->wmat, c->emat, fac, c->ringv[k], c->sdv[k],
-                                  c->edgev[k], c->st);
+// modes spec) and the boundary terms of its solve; the ring itself only where something reads it (a
+// curl of the level: the solves read the boundary terms).
+static int ring_edge_from_modes(Ctx* c, const double* spec, int k, double fac, bool want_ring) {
+  return dst_ring_edge_from_modes(c->px, c->g, spec, c->g.nsx, c->wmat, c->emat, fac, want_ring ? c->ringv[k] : nullptr,
+                                  c->sdv[k], c->edgev[k], c->st);
 }
 
 // vort2flux (operators_fluid.F90:237-377).  all_levels=false writes the streamfunction and the
@@ -618,7 +619,7 @@ int op_vort2flux(Ctx* c, double* const* w, double* const* s, double* const* qx, 
         ProfScope ps(c, 1, pass_bytes(c, 1, 1));
         RC(tri_solve(c->tri_ctci, modes(k), F, g.nsx, c->tl, st, bc));
       }
-      if (k > 0) RC(ring_edge_from_modes(c, F, k - 1, 1.0));
+      if (k > 0) RC(ring_edge_from_modes(c, F, k - 1, 1.0, all_levels || k == 1));
     }
   }
   if (!all_levels) {
@@ -1457,7 +1458,7 @@ static int op_predict_levels(Ctx* c, bool seed_rhs_old) {
         ProfScope ps(c, 1, pass_bytes(c, 1, 1));
         RC(tri_solve(c->tri_pred[k], F, F, g.nsx, c->tl, st, bc));
       }
-      if (k > 0) RC(ring_edge_from_modes(c, F, k - 1, 0.25 * c->vfac[k - 1]));
+      if (k > 0) RC(ring_edge_from_modes(c, F, k - 1, 0.25 * c->vfac[k - 1], false));
     }
   }
   // every row of every level back: coarsify rewrites only the centre columns of a coarser
