@@ -150,7 +150,8 @@ int beam_build(Ctx* c, const IbBody* bodies, int nbody, std::string* msg) {
   c->nbeam = (int)hdev.size();
   c->beams_h = hdev;
   if (c->nbeam > 0) {
-    if (cudaMalloc(&c->beams, sizeof(BeamDev) * c->nbeam) != cudaSuccess) { *msg = "beam allocation failed"; return IB_ERR_NOMEM; }
+    if (cudaMalloc(&c->beams, sizeof(BeamDev) * c->nbeam + sizeof(double)) != cudaSuccess) { *msg = "beam allocation failed"; return IB_ERR_NOMEM; }
+    c->beam_err = (double*)(c->beams + c->nbeam);
     if (cudaMemcpy(c->beams, hdev.data(), sizeof(BeamDev) * c->nbeam, cudaMemcpyHostToDevice) != cudaSuccess)
       return IB_ERR_CUDA;
     if (cudaDeviceSynchronize() != cudaSuccess) return IB_ERR_CUDA;
@@ -163,6 +164,7 @@ void beam_free(Ctx* c) {
   c->beam_mem.clear();
   if (c->beams) cudaFree(c->beams);
   c->beams = nullptr;
+  c->beam_err = nullptr;
   c->nbeam = 0;
 }
 
@@ -305,10 +307,10 @@ __global__ void __launch_bounds__(kBeamThreads) k_beam_rhs(const BeamDev* __rest
 
 __global__ void __launch_bounds__(kBeamThreads) k_beam_dx(const BeamDev* __restrict__ beams, int nbeam, BeamFac fc,
                                                           const double* __restrict__ f, double* xb, double* yb,
-                                                          double* err) {
+                                                          double* err, int fresh) {
   IB_GRID_DEP_WAIT();
   __shared__ double red[kBeamThreads / 32];
-  double emax = err[0];   // the torsional bodies' maximum (zero without them)
+  double emax = fresh ? 0.0 : err[0];   // the torsional bodies' maximum (zero without them)
   for (int i = 0; i < nbeam; ++i) {
     const BeamDev b = beams[i];
     const int nd = b.ndof;
@@ -414,10 +416,11 @@ int launch_beam_rhs(Ctx* c, double* y, cudaStream_t st) {
   k_beam_rhs<<<1, kBeamThreads, 0, st>>>(c->beams, c->nbeam, BeamFac(c->p.dt, c->delta), y);
   return after(IB_OK);
 }
-int launch_beam_dx(Ctx* c, const double* f, cudaStream_t st) {
+int launch_beam_dx(Ctx* c, const double* f, cudaStream_t st, bool own_err) {
   if (c->nbeam == 0) return IB_OK;
   count_launch();
-  k_beam_dx<<<1, kBeamThreads, 0, st>>>(c->beams, c->nbeam, BeamFac(c->p.dt, c->delta), f, c->xb, c->yb, c->err_fsi);
+  k_beam_dx<<<1, kBeamThreads, 0, st>>>(c->beams, c->nbeam, BeamFac(c->p.dt, c->delta), f, c->xb, c->yb,
+                                        own_err ? c->beam_err : c->err_fsi, own_err ? 1 : 0);
   return after(IB_OK);
 }
 int launch_beam_btimes(Ctx* c, const double* x, double* y, cudaStream_t st) {

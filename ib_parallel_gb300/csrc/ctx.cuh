@@ -315,6 +315,7 @@ struct Ctx {
   // family-3 beams (beam.cu)
   int nbeam = 0;
   BeamDev* beams = nullptr;
+  double* beam_err = nullptr;      // after the beams: their largest |dq| in a device FSI iteration
   std::vector<BeamDev> beams_h;
   std::vector<double*> beam_mem;
   int *comp = nullptr, *bid = nullptr;
@@ -461,7 +462,8 @@ int op_write_variables(Ctx* c, const char* path, std::string* msg);
 int beam_build(Ctx* c, const IbBody* bodies, int nbody, std::string* msg);
 void beam_free(Ctx* c);
 int launch_beam_rhs(Ctx* c, double* y, cudaStream_t st);
-int launch_beam_dx(Ctx* c, const double* f, cudaStream_t st);
+// own_err: the largest |dq| goes to beam_err alone, for the device FSI loop; else it joins err_fsi
+int launch_beam_dx(Ctx* c, const double* f, cudaStream_t st, bool own_err = false);
 int launch_beam_btimes(Ctx* c, const double* x, double* y, cudaStream_t st);
 int launch_beam_add_b(Ctx* c, double* St, cudaStream_t st);
 int launch_beam_initial_acc(Ctx* c, const double* f, cudaStream_t st);

@@ -1,6 +1,7 @@
 // The end of one device FSI iteration in one kernel: structure update, weights and influence
 // patches at the new positions (k_tors_dx, k_reg_weights and k_inf_patch of the host loop, on
-// the same device bodies), and the loop condition.
+// the same device bodies), and the loop condition.  Beams are updated by their own kernel just
+// before: their points are read as a rigid body's are, their error joins the condition.
 #include "fsi_dev.cuh"
 
 namespace ib {
@@ -112,6 +113,7 @@ __global__ void __launch_bounds__(128) k_fsi_update(FsiUpdateArgs a) {
   } else if (a.nt > 1) {
     for (int t = 0; t < a.nt; ++t) e = fmax(e, a.err[1 + t]);
   }
+  if (a.beam_err) e = fmax(e, *a.beam_err);
   a.err[0] = e;
   const int n = a.cnt[0] + 1;
   const int bf = *a.flag;

@@ -162,6 +162,7 @@ struct FsiUpdateArgs {
   double dt, delta;
   const double* f;
   double *xb, *yb, *err;
+  const double* beam_err = nullptr;   // the beams' largest |dq| (null without beams)
   double *th_next, *sin_next, *cos_next;   // nt each: written before they are committed
   // weights (RegDev's origins and weights, the stale flag, the domain error)
   GridDims g;

@@ -1241,7 +1241,9 @@ __global__ void k_fsi_loop_init(int* cnt, int* band_flag, unsigned* done) {
 // and the redistribution reads the copy, so neither is on the chain from one solve to the
 // next.  The band flag and the touched-vertex flags are cleared by the kernels that read
 // them (the condition, the compaction), so the patches need no memsets; the end of the
-// iteration is one kernel (k_fsi_update).  The body's launches are counted once
+// iteration is one kernel (k_fsi_update; beams are updated by k_beam_dx before it).  Run from the host
+// instead, an iteration ends with a wait for its residual: the four iterations of a 600 x 300 beam step
+// left the GPU idle a quarter of the time (1.10 ms a step, 0.85 so).  The body's launches are counted once
 // (fsi_body_launches), the lists after the loop in fsi_post_launches.
 // Adds the FSI iterations to the graph `st` is capturing (see build_fsi_loop).
 static int capture_fsi_loop(Ctx* c, cudaStream_t st) {
@@ -1288,6 +1290,7 @@ static int capture_fsi_loop(Ctx* c, cudaStream_t st) {
         IB_CUDA_CHECK(cudaEventRecord(ev_b, s2));
         if (c->nt < c->nbody) IB_CUDA_CHECK(cudaMemsetAsync(c->rhsf, 0, 8 * (size_t)c->nf, s2));
         RC(launch_tors_rhs(c->nt, c->tb, c->ts, p.dt, c->delta, c->rhsf, s2));
+        RC(launch_beam_rhs(c, c->rhsf, s2));
         if (c->ub_on) RC(launch_sub_scaled(c->nf, c->delta, c->ub, c->rhsf, s2));
         if (c->sd.on) {   // P E_o (q + q0), P from s1
           IB_CUDA_CHECK(cudaStreamWaitEvent(s2, ev_p, 0));
@@ -1310,6 +1313,7 @@ static int capture_fsi_loop(Ctx* c, cudaStream_t st) {
           RC(inf_assemble_kp(c, s1, true));
           IB_CUDA_CHECK(cudaStreamWaitEvent(s1, ev_rhs, 0));
           RC(inf_assemble_ptk(c, s1));
+          RC(launch_beam_add_b(c, I.St, s1));
         }
         RC(launch_gmres_fused(c->G, &c->fused_plan, I.St, c->rhsf, c->f, p.rtol, p.atol, p.gmres_max_it, s1));
         // s2: redistribution with the copy, beside the structure update and the weights and
@@ -1326,14 +1330,16 @@ static int capture_fsi_loop(Ctx* c, cudaStream_t st) {
         c->st = s1;
         RC(rrd);
         IB_CUDA_CHECK(cudaEventRecord(ev_rd, s2));
-        // structure update, weights and patches at the new positions, the condition (after the
-        // copy and the lists of the current weights are taken)
+        // structure update (the beams' first), weights and patches at the new positions, the
+        // condition (after the copy and the lists of the current weights are taken)
+        RC(launch_beam_dx(c, c->f, s1, true));
         IB_CUDA_CHECK(cudaStreamWaitEvent(s1, ev_lists, 0));
         I.patch_fresh = false;
         I.active = false;
         FsiUpdateArgs u;
         u.tb = c->tb; u.ts = c->ts; u.nt = c->nt; u.dt = p.dt; u.delta = c->delta; u.f = c->f;
         u.xb = c->xb; u.yb = c->yb; u.err = c->err_fsi;
+        u.beam_err = c->nbeam > 0 ? c->beam_err : nullptr;
         u.th_next = c->tors_next; u.sin_next = c->tors_next + (c->nt + 1); u.cos_next = c->tors_next + 2 * (c->nt + 1);
         u.g = g; u.nf = c->nf; u.ox = p.offsetx; u.oy = p.offsety; u.dtab = c->reg.tab; u.comp = c->reg.comp;
         u.ix = c->reg.ix; u.iy = c->reg.iy; u.w = c->reg.w; u.stale = c->reg.stale; u.d_err = c->d_err;
@@ -1560,7 +1566,7 @@ static int whole_step_mode(Ctx* c) {
   if (p.num_stat) return 0;
   const Influence& I = c->inf;
   const bool operator_ready = c->sd.on ? c->sd.ready : (I.built && I.patch_fresh && I.flag_h == 0);
-  const bool loop = (c->nt > 0) && c->nbeam == 0 && p.schur_mode != 1 && c->use_fused &&
+  const bool loop = (c->nt > 0 || c->nbeam > 0) && p.schur_mode != 1 && c->use_fused &&
                     !c->graph_fsi_loop.failed && c->fused_plan.state == 1 && operator_ready;
   return loop ? 1 : 0;
 }
@@ -1590,6 +1596,7 @@ static int build_step_graph(Ctx* c, int mode) {
     cudaGraphConditionalHandle h = 0;
     if (rc == IB_OK && mode == 1) {
       rc = launch_tors_save(c->nt, c->ts, st);
+      if (rc == IB_OK) rc = launch_beam_save(c, st);
       const long long b0 = launch_count();
       Influence& I = c->inf;
       const bool fresh = I.patch_fresh, active = I.active;
@@ -1733,7 +1740,7 @@ int op_advance_begin(Ctx* c) {
         Influence& I = c->inf;
         const bool operator_ready = c->sd.on ? c->sd.ready : (I.built && I.patch_fresh && I.flag_h == 0);
         const bool device_loop = moved && p.schur_mode != 1 && c->use_step_graphs && c->use_fused && !c->prof_on &&
-                                 !c->stage_on && (!c->step_prof || c->step_prof_dev) && c->nbeam == 0 &&
+                                 !c->stage_on && (!c->step_prof || c->step_prof_dev) &&
                                  !c->graph_fsi_loop.failed && c->fused_plan.state == 1 && operator_ready;
         if (device_loop && (c->graph_fsi_loop.exec || build_fsi_loop(c) == IB_OK)) {
           IB_CUDA_CHECK(cudaGraphLaunch(c->graph_fsi_loop.exec, st));

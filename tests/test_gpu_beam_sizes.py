@@ -1,10 +1,11 @@
-"""The beam kernels where their row groups can go wrong: fewer DOFs than a group of lanes, more than a
+"""The FSI iterations of beams on the device against the same iterations run from the host: the same
+kernels' arithmetic, so the same steps bit for bit.  And the beam kernels where their row groups can go wrong: fewer DOFs than a group of lanes, more than a
 pass of the CTA covers, elements longer than several points and shorter than one, two beams; the
 structure operators against the oracle's dense formulation."""
 import numpy as np
 import pytest
 
-from helpers import PLATE, pair, rel
+from helpers import PLATE, pair, rel, small_plate
 from ib_parallel_gb300 import geometry as GEO
 from ib_parallel_gb300 import ibgpu as G
 from dataclasses import replace
@@ -37,3 +38,30 @@ def test_beam_operators(sizes):
         scale = o.delta * 2.0 / PLATE["dt"] * np.abs(qo).max()
         assert np.abs(g.struct_rhs() - o.compute_rhs()).max() < tol * scale
     g.close()
+
+
+@pytest.mark.parametrize("beams,plate", [([(9, 0, 0.0)], False), ([(9, 3, -0.3), (7, 0, 0.3)], False), ([(9, 0, -0.3)], True)])
+@pytest.mark.parametrize("subdomain", [False, True])
+def test_device_iterations_match_the_host_loop(beams, plate, subdomain):
+    bodies = [_beam(*b) for b in beams]
+    if plate:   # a torsional body beside the beam: both errors join the loop's condition
+        t = small_plate()
+        bodies.append(replace(t, y=np.asarray(t.y) + 0.3))
+    kw = dict(PLATE, n=64, offsetx=1.5, offsety=2.0)   # room for the sub-domain's cloud
+    gd, gh = (G.Simulation(G.Params(**kw), bodies) for _ in range(2))
+    if subdomain:
+        for g in (gd, gh):
+            g.subdomain_setup(-0.4, 1.4, -0.7, 0.6, PLATE["len"] / PLATE["m"])
+    gh.step_profile(1)   # times the phases: the host runs the iterations
+    for step in range(6):
+        gd.advance()
+        gh.advance()
+        assert gd.counters() == gh.counters(), step
+        for a, b in zip(gd.beam_state(), gh.beam_state()):
+            assert np.array_equal(a, b), step
+        assert np.array_equal(gd.get_vector("f"), gh.get_vector("f"))
+        for k in range(PLATE["mgridlev"]):
+            assert np.array_equal(gd.get_field("omega", k), gh.get_field("omega", k)), (step, k)
+    assert gd.step_graph_stats()["graph"] >= 3 and gh.step_graph_stats()["graph"] == 0
+    gd.close()
+    gh.close()
