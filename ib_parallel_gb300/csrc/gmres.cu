@@ -98,9 +98,10 @@ __device__ __forceinline__ void norm_and_scale(double s, double* tt, double* inv
 
 // Givens update of Arnoldi step `it` (KSPGMRESUpdateHessenberg): the new Hessenberg column is
 // h[0..it], tt; the previous rotations are applied with the rotated value carried in a
-// register (one dependent FMA per rotation), then the new rotation (from rsqrt of c^2+tt^2),
-// the rotated residual g and the convergence reason.  Writes H column `it` (ld = restart+1).
-__device__ void givens_step(double* __restrict__ col, const double* __restrict__ h, double tt, int it,
+// register (one dependent FMA per rotation), then the new rotation (from rsqrt of c^2 + sq, sq the
+// squared norm that tt is the root of), the rotated residual g and the convergence reason.  Writes H
+// column `it` (ld = restart+1).  For restarts that a warp cannot hold; givens_finish_warp otherwise.
+__device__ void givens_step(double* __restrict__ col, const double* __restrict__ h, double tt, double sq, int it,
                             double* __restrict__ cs, double* __restrict__ sn, double* __restrict__ g, double prev_res,
                             double ttol, double* res_out, int* reason_out) {
   const bool hapend = happy_breakdown(tt, g[it]);
@@ -115,7 +116,7 @@ __device__ void givens_step(double* __restrict__ col, const double* __restrict__
   double res;
   int reason = 0;
   if (!hapend) {
-    const double r2 = fma(c, c, tt * tt);
+    const double r2 = fma(c, c, sq);
     if (r2 == 0.0) {
       reason = -9;  // KSP_DIVERGED_NULL
       res = prev_res;
@@ -140,6 +141,76 @@ __device__ void givens_step(double* __restrict__ col, const double* __restrict__
   }
   *res_out = res;
   *reason_out = reason;
+}
+
+// The previous rotations applied to the new Hessenberg column h[0..it], on one whole warp (it < 32).
+// Rotation j maps the carried value c to -sn_j c + cs_j h_{j+1}; lane j holds that affine map and the
+// maps are composed by a parallel prefix (5 levels at most; one dependent FMA per rotation took 64
+// cycles each, longer than the rest of the step once the cycle was ten vectors long).  Returns the
+// value after all of them; *colv is entry `lane` of the rotated column (lane < it).
+__device__ __forceinline__ double givens_chain_warp(const double* h, const double* cs, const double* sn, int it,
+                                                    double* colv) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const bool mine = lane < it;
+  const double csj = mine ? cs[lane] : 0.0, snj = mine ? sn[lane] : 0.0;
+  const double hj1 = mine ? h[lane + 1] : 0.0, h0 = h[0];
+  double A = -snj, B = csj * hj1;
+  if (lane == 0) {   // the first map at its argument: a constant
+    B = fma(A, h0, B);
+    A = 0.0;
+  }
+  for (int d = 1; d < it; d <<= 1) {
+    const double Ap = __shfl_up_sync(full, A, d), Bp = __shfl_up_sync(full, B, d);
+    if (lane >= d) {
+      B = fma(A, Bp, B);
+      A = A * Ap;
+    }
+  }
+  const double before = __shfl_up_sync(full, B, 1);   // the value before rotation `lane`
+  *colv = fma(snj, hj1, csj * (lane == 0 ? h0 : before));
+  return it > 0 ? __shfl_sync(full, B, it - 1) : h0;
+}
+
+// The rest of step `it` from the chain's value c, tt and rn = rsqrt(r2), r2 = c^2 + tt^2: givens_step's.
+__device__ __forceinline__ void givens_finish_warp(double* col, double c, double colv, double r2, double rn, double tt,
+                                                   int it, double* cs, double* sn, double* g, double prev_res,
+                                                   double ttol, double* res_out, int* reason_out) {
+  const int lane = threadIdx.x & 31;
+  const double gi = g[it];   // read by every lane before lane 0 rewrites it
+  if (lane < it) col[lane] = colv;
+  const bool hapend = happy_breakdown(tt, gi);
+  const double ci = c * rn, si = tt * rn;
+  __syncwarp();
+  if (lane == 0) {
+    col[it + 1] = tt;
+    double res;
+    int reason = 0;
+    if (!hapend) {
+      if (r2 == 0.0) {
+        reason = -9;  // KSP_DIVERGED_NULL
+        res = prev_res;
+        col[it] = c;
+      } else {
+        cs[it] = ci;
+        sn[it] = si;
+        g[it + 1] = -(si * gi);
+        g[it] = ci * gi;
+        col[it] = fma(si, tt, ci * c);
+        res = fabs(g[it + 1]);
+      }
+    } else {
+      col[it] = c;
+      res = 0.0;
+    }
+    if (reason == 0) {
+      if (res <= ttol) reason = 2;
+      else if (hapend) reason = -3;
+    }
+    *res_out = res;
+    *reason_out = reason;
+  }
+  __syncwarp();
 }
 
 // KSPGMRESBuildSoln back substitution y[0..k] = R^-1 g (R the rotated Hessenberg, ld = R+1), on
@@ -211,6 +282,7 @@ __global__ void k_gmres_start(GmresDev G, const double* __restrict__ b, const do
     G.scal[1] = rnorm;
     G.scal[2] = bnorm;
     G.scal[3] = rnorm;
+    G.scal[4] = 1.0;   // xin is V0 itself
     G.g[0] = rnorm;
     G.ist[2] = 0;
     int reason = 0;
@@ -224,13 +296,14 @@ __global__ void k_gmres_start(GmresDev G, const double* __restrict__ b, const do
   }
 }
 
-// One Arnoldi step on w = A V[it] (in G.Av): classical Gram-Schmidt (all projections
-// against the unmodified w), normalisation, Givens update.
+// One Arnoldi step on w = A V[it] (scal[4] G.Av: the operator is applied to the vector before its
+// normalisation, and its output scaled): classical Gram-Schmidt (all projections against the
+// unmodified w), normalisation, Givens update.
 __global__ void k_gmres_arnoldi(GmresDev G, int max_it, cudaGraphConditionalHandle h_inner, int use_cond) {
   IB_GRID_DEP_WAIT();
   __shared__ double part[64 * kSlices];
   __shared__ double h[64];
-  __shared__ double s_tt[2];
+  __shared__ double s_tt[3];
   if (G.ist[3] == 0) {
     if (use_cond && threadIdx.x == 0) cudaGraphSetConditional(h_inner, 0u);
     return;
@@ -238,7 +311,10 @@ __global__ void k_gmres_arnoldi(GmresDev G, int max_it, cudaGraphConditionalHand
   const int nf = G.nf, R = G.restart, tid = threadIdx.x;
   const int it = G.ist[2];
   double* w = G.V + (size_t)(it + 1) * nf;
-  const double* Av = G.Av;
+  double* Av = G.Av;
+  const double scale = G.scal[4];
+  for (int i = tid; i < nf; i += blockDim.x) Av[i] = Av[i] * scale;
+  __syncthreads();
   // projections: a partial per (j, slice), then the slices in order
   for (int q = tid; q < (it + 1) * kSlices; q += blockDim.x) {
     const int j = q / kSlices, c = q % kSlices;
@@ -257,25 +333,40 @@ __global__ void k_gmres_arnoldi(GmresDev G, int max_it, cudaGraphConditionalHand
     part[tid] = slice_dot_seq(w, w, lo, hi);
   }
   __syncthreads();
-  if (tid == 0) norm_and_scale(tree8_seq(part), &s_tt[0], &s_tt[1]);
+  if (tid == 0) {
+    s_tt[2] = tree8_seq(part);
+    norm_and_scale(s_tt[2], &s_tt[0], &s_tt[1]);
+  }
   __syncthreads();
   const double tt = s_tt[0];
   const double inv = s_tt[1];
+  const double sfac = tt != 0.0 ? inv : 1.0;
   for (int i = tid; i < nf; i += blockDim.x) {
-    double v = tt != 0.0 ? w[i] * inv : w[i];
-    w[i] = v;
+    const double v = w[i];
     G.xin[i] = v;
+    w[i] = v * sfac;
+  }
+  if (tid >= 32) return;
+  const double sq = s_tt[2], prev_res = G.scal[1], ttol = G.scal[0];
+  double* col = G.H + (size_t)it * (R + 1);
+  double res = 0.0;
+  int reason = 0;
+  if (R <= 32) {
+    double colv;
+    const double c = givens_chain_warp(h, G.cs, G.sn, it, &colv);
+    const double r2 = fma(c, c, sq);
+    givens_finish_warp(col, c, colv, r2, r2 != 0.0 ? rsqrt(r2) : 0.0, tt, it, G.cs, G.sn, G.g, prev_res, ttol, &res,
+                       &reason);
+  } else if (tid == 0) {
+    givens_step(col, h, tt, sq, it, G.cs, G.sn, G.g, prev_res, ttol, &res, &reason);
   }
   if (tid == 0) {
-    double* col = G.H + (size_t)it * (R + 1);
-    double res;
-    int reason;
-    givens_step(col, h, tt, it, G.cs, G.sn, G.g, G.scal[1], G.scal[0], &res, &reason);
     const int itn = it + 1;
     const int its = G.ist[0] + 1;
     G.ist[2] = itn;
     G.ist[0] = its;
     G.scal[1] = res;
+    G.scal[4] = sfac;
     G.ist[1] = reason;
     const int active = (reason == 0 && itn < R && its < max_it) ? 1 : 0;
     G.ist[3] = active;
@@ -495,77 +586,22 @@ struct ClusterSmem {
 constexpr int kClusterThreads = 128;
 constexpr int kProdThreads = 96;
 
-// givens_step's arithmetic on one whole warp (it < 32): lane j holds rotation j and the
-// product cs[j]*h[j+1] in registers, the chain of rotated values runs on every lane in step
-// (each step's operands by shuffle, so nothing waits on shared memory), lane j keeps the value
-// before rotation j and forms column entry j.
-__device__ void givens_step_warp(double* __restrict__ col, const double* __restrict__ h, double tt, int it,
-                                 double* __restrict__ cs, double* __restrict__ sn, double* __restrict__ g,
-                                 double prev_res, double ttol, double* res_out, int* reason_out) {
-  const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  const bool mine = lane < it;
-  const double csj = mine ? cs[lane] : 0.0, snj = mine ? sn[lane] : 0.0;
-  const double hj1 = mine ? h[lane + 1] : 0.0;
-  const double pj = csj * hj1;
-  const double gi = g[it];   // read by every lane before lane 0 rewrites it
-  double c = h[0], cmine = 0.0;
-#pragma unroll 8
-  for (int j = 0; j < it; ++j) {
-    const double sj = __shfl_sync(full, snj, j), pp = __shfl_sync(full, pj, j);
-    if (lane == j) cmine = c;
-    c = fma(-sj, c, pp);
-  }
-  if (mine) col[lane] = fma(snj, hj1, csj * cmine);
-  const bool hapend = happy_breakdown(tt, gi);
-  const double r2 = fma(c, c, tt * tt);
-  const double rn = r2 != 0.0 ? rsqrt(r2) : 0.0;
-  const double ci = c * rn, si = tt * rn;
-  if (lane == 0) {
-    col[it + 1] = tt;
-    double res;
-    int reason = 0;
-    if (!hapend) {
-      if (r2 == 0.0) {
-        reason = -9;  // KSP_DIVERGED_NULL
-        res = prev_res;
-        col[it] = c;
-      } else {
-        cs[it] = ci;
-        sn[it] = si;
-        g[it + 1] = -(si * gi);
-        g[it] = ci * gi;
-        col[it] = fma(si, tt, ci * c);
-        res = fabs(g[it + 1]);
-      }
-    } else {
-      col[it] = c;
-      res = 0.0;
-    }
-    if (reason == 0) {
-      if (res <= ttol) reason = 2;
-      else if (hapend) reason = -3;
-    }
-    *res_out = res;
-    *reason_out = reason;
-  }
-  __syncwarp();
-}
-
 // One restarted GMRES solve on the assembled operator A (column-major, At[j*nf + r] = A[r][j])
 // across a cluster of kSlices CTAs.  CTA c owns the rows and vector elements of slice c: its
 // rows of A, its slice of every Krylov vector, of x and of b.  Per Arnoldi step:
-//   A: warps 0-2 form the product of its rows with the full current vector (rows in groups of
-//      S lanes) and its partial projections; meanwhile warp 3 applies the Givens update of
-//      the previous step;                                                    cluster barrier
+//   A: warps 0-2 gather the new vector, not yet normalised, form the product of their rows with it
+//      (rows in groups of S lanes), scale it and their slice of the vector by 1/norm and form the
+//      partial projections; meanwhile warp 3 sums the norm, leaves the scale and applies the Givens
+//      update of the previous step;                                          cluster barrier
 //      the previous step's convergence decision is read from CTA 0 (every CTA branches
 //      alike), then the projections are summed over the slices (8 lanes per projection);
-//   B: w = A v - sum h_j v_j on the slice (8 lanes per row) and its partial norm, the
-//      unscaled slice kept for the others to read;                           cluster barrier
-//   C: every CTA gathers the unscaled slices while forming the norm, then scales its gathered
-//      copy and its own slice by 1/norm.
+//   B: w = A v - sum h_j v_j on the slice (8 lanes per row) and its partial norm; cluster barrier
+// What bounds it is latency: about 60 dependent FP64 instructions a step, 64 cycles each, and two
+// cluster barriers.  Scaling after the product keeps the norm's sum and square root beside the
+// product instead of before it.
 // No thread waits on a flag: the only waits are the cluster and CTA barriers, which every
-// thread of every CTA reaches the same number of times.
+// thread of every CTA reaches the same number of times (the scale's: warp 3 arrives once and warps
+// 0-2 wait once in each step with k > 0, k the same on all of them).
 __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(kClusterThreads)
     k_gmres_cluster(GmresDev G, const double* __restrict__ At, int a_in_smem, const double* __restrict__ b,
                     double* __restrict__ x, double rtol, double atol, int max_it) {
@@ -600,7 +636,10 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(kClusterThread
   double* As = nblk + 32;                           // nl x nf row-major when a_in_smem
   __shared__ int s_reason;                          // read remotely from CTA 0
   auto remote = [&](double* p, int c) -> const double* { return cl.map_shared_rank(p, c); };
-  auto bar_prod = [&]() { asm volatile("bar.sync 1, %0;" ::"r"(kProdThreads)); };
+  auto bar_prod = [&]() { asm volatile("bar.sync 1, %0;" ::"r"(kProdThreads) : "memory"); };
+  // the new vector's scale: warp 3 leaves it, warps 0-2 wait for it (each once a step after the first)
+  auto bar_scale_put = [&]() { asm volatile("bar.arrive 2, %0;" ::"r"(kClusterThreads) : "memory"); };
+  auto bar_scale_get = [&]() { asm volatile("bar.sync 2, %0;" ::"r"(kClusterThreads) : "memory"); };
   // slice partial of a.b in the fixed order: lane blk of an aligned group of LP lanes forms
   // block blk ((p0+p1)+(p2+p3) over rows 4blk..4blk+3), the group's xor tree the rest (valid
   // on every lane of the group); every lane of the warp calls it
@@ -752,11 +791,27 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(kClusterThread
     if (reason != 0) break;
     gather(Vs, 0);
     __syncthreads();
-    // ---- Arnoldi steps (k_gmres_arnoldi), the Givens update of step k-1 during step k
+    // ---- Arnoldi steps (k_gmres_arnoldi), the norm and the Givens update of step k-1 during step k
     k = 0;
     for (;;) {
       if (warp < 3) {
+        if (k > 0) {   // the new vector before its scaling, from every slice
+          for (int i = tid; i < nf; i += kProdThreads) {
+            const int c = i / ns;
+            vfull[i] = remote(wbuf, c)[i - c * ns];
+          }
+          bar_prod();
+        }
         matvec();
+        if (k > 0) {
+          bar_scale_get();   // scal[4]; and the raw product is complete
+          const double sfac = scal[4];
+          double* w = Vs + (size_t)k * ns;
+          for (int i = tid; i < nl; i += kProdThreads) {
+            avs[i] = avs[i] * sfac;
+            w[i] = wbuf[i] * sfac;
+          }
+        }
         bar_prod();
         for (int q0 = 0; q0 < LP * (k + 1); q0 += kProdThreads) {   // LP lanes per projection
           const int q = q0 + tid, j = q / LP, blk = q - j * LP;
@@ -765,9 +820,27 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(kClusterThread
           if (on && blk == 0) hp[j] = t;
         }
       } else if (k > 0) {
+        // one reciprocal square root serves the norm (lane 0) and the new rotation (lane 1)
+        const double pn = remote(scal, lane & 7)[0];
+        double colv;
+        const double c = givens_chain_warp(h, cs, sn, k - 1, &colv);
+        const double sq = tree8(pn);
+        const double r2 = fma(c, c, sq);
+        const double r = rsqrt(lane == 0 ? sq : r2);
+        double inv = __shfl_sync(full, r, 0);
+        const double r1 = __shfl_sync(full, r, 1), rn = r2 != 0.0 ? r1 : 0.0;
+        double tt = sq * inv;
+        if (!(sq > 0.0)) {
+          tt = sqrt(sq);
+          inv = 0.0;
+        }
+        if (lane == 0) scal[4] = tt != 0.0 ? inv : 1.0;
+        __syncwarp();
+        bar_scale_put();
         double res = 0.0;
         int rs = 0;
-        givens_step_warp(H + (size_t)(k - 1) * (R + 1), h, scal[2], k - 1, cs, sn, g, scal[3], ttol, &res, &rs);
+        givens_finish_warp(H + (size_t)(k - 1) * (R + 1), c, colv, r2, rn, tt, k - 1, cs, sn, g, scal[3], ttol, &res,
+                           &rs);
         if (lane == 0) {
           scal[3] = res;
           s_reason = rs;
@@ -815,33 +888,6 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(kClusterThread
         if (lane == 0) scal[0] = v;
       }
       cl.sync();                                  // partial norms and the unscaled slices
-      // the new vector: every CTA gathers the unscaled slices while warp 0 forms the norm,
-      // then scales its gathered copy and its own slice alike (the products of a normalise-
-      // then-gather, with one cluster barrier fewer)
-      {
-        const double pn = (warp == 0 && lane < 8) ? remote(scal, lane)[0] : 0.0;
-        for (int i = tid; i < nf; i += blockDim.x) {
-          const int c = i / ns;
-          vfull[i] = remote(wbuf, c)[i - c * ns];
-        }
-        if (warp == 0) {
-          const double sq = tree8(pn);
-          if (lane == 0) {
-            double tt, inv;
-            norm_and_scale(sq, &tt, &inv);
-            scal[2] = tt;
-            scal[4] = inv;
-          }
-        }
-      }
-      __syncthreads();
-      {
-        const double tt = scal[2], inv = scal[4];
-        double* w = Vs + (size_t)(k + 1) * ns;
-        for (int i = tid; i < nl; i += blockDim.x) w[i] = tt != 0.0 ? wbuf[i] * inv : wbuf[i];
-        for (int i = tid; i < nf; i += blockDim.x) vfull[i] = tt != 0.0 ? vfull[i] * inv : vfull[i];
-      }
-      __syncthreads();
       its += 1;
       k += 1;
     }

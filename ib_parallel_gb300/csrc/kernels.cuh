@@ -262,7 +262,7 @@ struct GmresDev {
   double* cs;
   double* sn;
   double* g;       // restart+1
-  double* scal;    // [0]=ttol [1]=res [2]=bnorm [3]=rnorm
+  double* scal;    // [0]=ttol [1]=res [2]=bnorm [3]=rnorm [4]=scale of the product of xin
   int* ist;        // [0]=its [1]=reason [2]=it (inner) [3]=active [4]=restart cycles
   double* xin;     // matvec input
   double* Av;      // matvec output

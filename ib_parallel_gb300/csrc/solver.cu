@@ -289,7 +289,7 @@ int ctx_create(const IbParams* pin, const IbBody* bodies, int nbody, Ctx** out, 
   c->G.nf = nf; c->G.restart = R;
   c->G.V = P.take<double>((size_t)(R + 1) * nf); c->G.H = P.take<double>((size_t)(R + 1) * R);
   c->G.cs = P.take<double>(R + 1); c->G.sn = P.take<double>(R + 1); c->G.g = P.take<double>(R + 1);
-  c->G.scal = P.take<double>(4); c->G.ist = P.take<int>(8);
+  c->G.scal = P.take<double>(5); c->G.ist = P.take<int>(8);
   c->gm_b = P.take<double>(nf + 1); c->gm_x = P.take<double>(nf + 1);
   c->G.xin = P.take<double>(nf); c->G.Av = P.take<double>(nf);
   if (p.num_stat) {
