@@ -385,9 +385,13 @@ __global__ void k_gmres_update(GmresDev G, double* __restrict__ x, int max_it, c
   __syncthreads();
   if (it > 0) {
     for (int i = threadIdx.x; i < nf; i += blockDim.x) {
-      double u = 0.0;
-      for (int j = 0; j < it; ++j) u = fma(y[j], G.V[(size_t)j * nf + i], u);
-      x[i] = x[i] + u;
+      double p[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        p[q] = 0.0;
+        for (int j = q; j < it; j += 8) p[q] = fma(y[j], G.V[(size_t)j * nf + i], p[q]);
+      }
+      x[i] = x[i] + tree8_seq(p);
     }
   }
   if (threadIdx.x == 0) {
@@ -572,36 +576,56 @@ namespace {
 struct ClusterSmem {
   int nf, R, ns;
   size_t base() const {
-    return (size_t)(R + 1) * ns + nf + 4 * (size_t)ns + 2 * (size_t)(R + 1) + (size_t)(R + 1) * R +
-           4 * (size_t)(R + 1) + 8 + 2 * (size_t)R + 32;
+    return (size_t)(R + 1) * ns + nf + 3 * (size_t)ns + (kSlices + 1) * (size_t)(R + 1) + (size_t)(R + 1) * R +
+           4 * (size_t)(R + 1) + 8 + kSlices + 32;
   }
   size_t with_a() const { return base() + (size_t)ns * nf; }
 };
 }  // namespace
 
-// Warps 0-2 run the dense product and the projections; warp 3 the Givens update meanwhile;
-// all four the rest.  Each warp sits on its own SM sub-partition, and an FP64 instruction
+// Warps 0-3 run the dense product, the projections and the vector updates; warp 4 the norm and the
+// Givens update meanwhile.  Warps 0-3 sit on an SM sub-partition each, and an FP64 instruction
 // holds its sub-partition's FP64 pipe for the same time whatever its active lanes, so every
 // sum below is spread over lanes (shuffle trees) rather than run down one thread.
-constexpr int kClusterThreads = 128;
-constexpr int kProdThreads = 96;
+constexpr int kClusterThreads = 160;
+constexpr int kProdThreads = 128;
+
+// back_substitute with a row per lane (k < 32): the same operations, r_l and R's entries in registers
+__device__ __forceinline__ void back_substitute_lanes(const double* H, int R, const double* g, int k, double* y) {
+  const int lane = threadIdx.x & 31;
+  double r = 0.0, rc = 0.0, out = 0.0;
+  if (lane <= k) {
+    r = g[lane];
+    rc = __drcp_rn(H[(size_t)lane * (R + 1) + lane]);
+  }
+#pragma unroll 4
+  for (int j = k; j >= 0; --j) {
+    const double hl = lane < j ? H[(size_t)j * (R + 1) + lane] : 0.0;
+    const double yj = __shfl_sync(0xffffffffu, r * rc, j);
+    if (lane == j) out = yj;
+    if (lane < j) r = fma(-hl, yj, r);
+  }
+  if (lane <= k) y[lane] = out;
+  __syncwarp();
+}
 
 // One restarted GMRES solve on the assembled operator A (column-major, At[j*nf + r] = A[r][j])
 // across a cluster of kSlices CTAs.  CTA c owns the rows and vector elements of slice c: its
 // rows of A, its slice of every Krylov vector, of x and of b.  Per Arnoldi step:
-//   A: warps 0-2 gather the new vector, not yet normalised, form the product of their rows with it
-//      (rows in groups of S lanes), scale it and their slice of the vector by 1/norm and form the
-//      partial projections; meanwhile warp 3 sums the norm, leaves the scale and applies the Givens
-//      update of the previous step;                                          cluster barrier
-//      the previous step's convergence decision is read from CTA 0 (every CTA branches
-//      alike), then the projections are summed over the slices (8 lanes per projection);
-//   B: w = A v - sum h_j v_j on the slice (8 lanes per row) and its partial norm; cluster barrier
-// What bounds it is latency: about 60 dependent FP64 instructions a step, 64 cycles each, and two
-// cluster barriers.  Scaling after the product keeps the norm's sum and square root beside the
-// product instead of before it.
+//   A: warps 0-3 form the product of their rows with the new vector, not yet normalised (rows in
+//      groups of S lanes), scale it and their slice of the vector by 1/norm and send every CTA
+//      their partial projections; meanwhile warp 4 sums the norm, leaves the scale and finishes
+//      the Givens update of the previous step, whose decision CTA 0 sends;   cluster barrier
+//   B: w = A v - sum h_j v_j on the slice (8 lanes per row, each lane sending the element to one
+//      CTA) and its partial norm, sent likewise; meanwhile warp 4 applies the earlier rotations to
+//      the new Hessenberg column;                                            cluster barrier
+// What bounds it is latency: about 45 dependent FP64 instructions a step, 64 cycles each, and two
+// cluster barriers of 500.  Scaling after the product keeps the norm's sum and square root beside the
+// product instead of before it; sending takes the place of reads of other CTAs' memory after the
+// barriers, 500 cycles each.
 // No thread waits on a flag: the only waits are the cluster and CTA barriers, which every
-// thread of every CTA reaches the same number of times (the scale's: warp 3 arrives once and warps
-// 0-2 wait once in each step with k > 0, k the same on all of them).
+// thread of every CTA reaches the same number of times (the scale's: warp 4 arrives once and warps
+// 0-3 wait once in each step with k > 0, k the same on all of them).
 __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(kClusterThreads)
     k_gmres_cluster(GmresDev G, const double* __restrict__ At, int a_in_smem, const double* __restrict__ b,
                     double* __restrict__ x, double rtol, double atol, int max_it) {
@@ -621,8 +645,8 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(kClusterThread
   double* avs = vfull + nf;                         // ns
   double* xsl = avs + ns;                           // ns
   double* bsl = xsl + ns;                           // ns
-  double* hp = bsl + ns;                            // R+1 partial projections (read remotely)
-  double* h = hp + (R + 1);                         // R+1
+  double* hp = bsl + ns;                            // kSlices x (R+1): every slice's partial projections
+  double* h = hp + kSlices * (size_t)(R + 1);       // R+1
   double* H = h + (R + 1);                          // (R+1) x R
   double* cs = H + (size_t)(R + 1) * R;
   double* sn = cs + (R + 1);
@@ -630,14 +654,13 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(kClusterThread
   double* yv = g + (R + 1);
   double* scal = yv + (R + 1);                      // [0],[1] partials (read remotely), [2] tt, [3] res,
                                                     // [4] 1/tt, [5] rnorm, [6] bnorm, [7] ttol
-  double* gbuf = scal + 8;                          // 2R: Givens scratch
-  double* wbuf = gbuf + 2 * (size_t)R;              // ns: the new vector before scaling (read remotely)
-  double* nblk = wbuf + ns;                         // 32: block partials of its norm
+  double* npart = scal + 8;                         // kSlices: every slice's partial norm
+  double* nblk = npart + kSlices;                   // 32: block partials of the slice's norm
   double* As = nblk + 32;                           // nl x nf row-major when a_in_smem
-  __shared__ int s_reason;                          // read remotely from CTA 0
-  auto remote = [&](double* p, int c) -> const double* { return cl.map_shared_rank(p, c); };
+  __shared__ int s_reason;                          // CTA 0's decision
+  auto remote = [&](double* p, int c) -> double* { return cl.map_shared_rank(p, c); };
   auto bar_prod = [&]() { asm volatile("bar.sync 1, %0;" ::"r"(kProdThreads) : "memory"); };
-  // the new vector's scale: warp 3 leaves it, warps 0-2 wait for it (each once a step after the first)
+  // the new vector's scale: warp 4 leaves it, warps 0-3 wait for it (each once a step after the first)
   auto bar_scale_put = [&]() { asm volatile("bar.arrive 2, %0;" ::"r"(kClusterThreads) : "memory"); };
   auto bar_scale_get = [&]() { asm volatile("bar.sync 2, %0;" ::"r"(kClusterThreads) : "memory"); };
   // slice partial of a.b in the fixed order: lane blk of an aligned group of LP lanes forms
@@ -664,29 +687,37 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(kClusterThread
     return p;
   };
 
-  if (a_in_smem)
-    for (int q = tid; q < nl * nf; q += blockDim.x) {
-      const int rl = q / nf, j = q - rl * nf;
-      As[q] = At[(size_t)j * nf + r0 + rl];
-    }
   for (int i = tid; i < nl; i += blockDim.x) {
     xsl[i] = x[r0 + i];
     bsl[i] = b[r0 + i];
   }
-  __syncthreads();
 
-  // avs = rows of A times vfull (warps 0-2): rows in groups of S lanes, one column segment
+  // avs = rows of A times vfull (warps 0-3): rows in groups of S lanes, one column segment
   // per lane, joined by seg_tree (k_dense_mv's layout and order)
   const int S = mv_segments(nf), gpw = 32 / S, cw = (nf + S - 1) / S;
   const int grp = lane / S, seg = lane - grp * S;
-  // When the slice's rows take one pass of the three warps and a segment fits, each lane keeps
+  // When the slice's rows take one pass of the four warps and a segment fits, each lane keeps
   // its segment of its row in registers for the whole solve (the same two chains, same order)
   constexpr int kRegSeg = 20;
-  const bool a_in_regs = nl <= 3 * gpw && cw <= kRegSeg;
+  constexpr int kProdWarps = kProdThreads / 32;
+  const bool a_in_regs = ns <= kProdWarps * gpw && cw <= kRegSeg;
   const int rl_r = warp * gpw + grp;
-  const bool live_r = warp < 3 && grp < gpw && rl_r < nl;
+  const bool live_r = warp < kProdWarps && grp < gpw && rl_r < nl;
   const int j0_r = min(nf, seg * cw), len_r = live_r ? min(nf, j0_r + cw) - j0_r : 0;
   double areg[kRegSeg];
+  if (a_in_regs) {
+#pragma unroll
+    for (int t = 0; t < kRegSeg; ++t) {
+      areg[t] = 0.0;
+      if (t < len_r) areg[t] = At[(size_t)(j0_r + t) * nf + r0 + rl_r];
+    }
+  } else if (a_in_smem) {
+    for (int q = tid; q < nl * nf; q += blockDim.x) {
+      const int rl = q / nf, j = q - rl * nf;
+      As[q] = At[(size_t)j * nf + r0 + rl];
+    }
+  }
+  __syncthreads();
   auto matvec = [&]() {
     if (a_in_regs) {
       double p = 0.0;
@@ -695,6 +726,7 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(kClusterThread
         const double* v = vfull + j0_r;
 #pragma unroll
         for (int t = 0; t < kRegSeg; t += 2) {
+          if (t >= cw) break;   // the same for every lane: no instructions for segments shorter than kRegSeg
           if (t + 1 < len_r) {
             e = fma(areg[t], v[t], e);
             o = fma(areg[t + 1], v[t + 1], o);
@@ -708,7 +740,7 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(kClusterThread
       if (live_r && seg == 0) avs[rl_r] = p;
       return;
     }
-    for (int rb = 0; rb < nl; rb += 3 * gpw) {
+    for (int rb = 0; rb < nl; rb += kProdWarps * gpw) {
       const int rl = rb + warp * gpw + grp;
       const bool live = grp < gpw && rl < nl;
       double p = 0.0;
@@ -732,14 +764,6 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(kClusterThread
     }
   };
 
-  if (a_in_regs) {
-#pragma unroll
-    for (int t = 0; t < kRegSeg; ++t) {
-      const int j = j0_r + t;
-      areg[t] = 0.0;
-      if (t < len_r) areg[t] = a_in_smem ? As[(size_t)rl_r * nf + j] : At[(size_t)j * nf + r0 + rl_r];
-    }
-  }
   int its = 0, cycles = 0, reason = 0, k = 0;
   double ttol = 0.0;
   for (;;) {
@@ -747,7 +771,7 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(kClusterThread
     cl.sync();                                    // every x slice is final
     gather(xsl, 0);
     __syncthreads();
-    if (warp < 3) matvec();
+    if (warp < kProdWarps) matvec();
     __syncthreads();
     for (int i = tid; i < nl; i += blockDim.x) Vs[i] = bsl[i] - avs[i];
     __syncthreads();
@@ -793,15 +817,9 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(kClusterThread
     __syncthreads();
     // ---- Arnoldi steps (k_gmres_arnoldi), the norm and the Givens update of step k-1 during step k
     k = 0;
+    double gc = 0.0, gcol = 0.0;   // warp 4: the last column's value after its earlier rotations, its entries
     for (;;) {
-      if (warp < 3) {
-        if (k > 0) {   // the new vector before its scaling, from every slice
-          for (int i = tid; i < nf; i += kProdThreads) {
-            const int c = i / ns;
-            vfull[i] = remote(wbuf, c)[i - c * ns];
-          }
-          bar_prod();
-        }
+      if (warp < kProdWarps) {
         matvec();
         if (k > 0) {
           bar_scale_get();   // scal[4]; and the raw product is complete
@@ -809,7 +827,7 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(kClusterThread
           double* w = Vs + (size_t)k * ns;
           for (int i = tid; i < nl; i += kProdThreads) {
             avs[i] = avs[i] * sfac;
-            w[i] = wbuf[i] * sfac;
+            w[i] = vfull[r0 + i] * sfac;
           }
         }
         bar_prod();
@@ -817,15 +835,13 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(kClusterThread
           const int q = q0 + tid, j = q / LP, blk = q - j * LP;
           const bool on = j <= k;
           const double t = slice_dot_lanes(avs, Vs + (size_t)(on ? j : 0) * ns, blk, on);
-          if (on && blk == 0) hp[j] = t;
+          if (on)
+            for (int c = blk; c < kSlices; c += LP) remote(hp, c)[rank * (R + 1) + j] = t;
         }
       } else if (k > 0) {
         // one reciprocal square root serves the norm (lane 0) and the new rotation (lane 1)
-        const double pn = remote(scal, lane & 7)[0];
-        double colv;
-        const double c = givens_chain_warp(h, cs, sn, k - 1, &colv);
-        const double sq = tree8(pn);
-        const double r2 = fma(c, c, sq);
+        const double sq = tree8(npart[lane & 7]);
+        const double r2 = fma(gc, gc, sq);
         const double r = rsqrt(lane == 0 ? sq : r2);
         double inv = __shfl_sync(full, r, 0);
         const double r1 = __shfl_sync(full, r, 1), rn = r2 != 0.0 ? r1 : 0.0;
@@ -839,66 +855,66 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(kClusterThread
         bar_scale_put();
         double res = 0.0;
         int rs = 0;
-        givens_finish_warp(H + (size_t)(k - 1) * (R + 1), c, colv, r2, rn, tt, k - 1, cs, sn, g, scal[3], ttol, &res,
+        givens_finish_warp(H + (size_t)(k - 1) * (R + 1), gc, gcol, r2, rn, tt, k - 1, cs, sn, g, scal[3], ttol, &res,
                            &rs);
-        if (lane == 0) {
-          scal[3] = res;
-          s_reason = rs;
-        }
+        if (lane == 0) scal[3] = res;
+        rs = __shfl_sync(full, rs, 0);
+        if (rank == 0 && lane < kSlices) *cl.map_shared_rank(&s_reason, lane) = rs;
       }
       cl.sync();                                  // partial projections; Givens of step k-1
-      {
-        // the first pass's slice partials are loaded together with CTA 0's decision
-        const int j = tid >> 3;
-        double p = j <= k ? remote(hp, tid & 7)[j] : 0.0;
-        if (k > 0) {
-          reason = *cl.map_shared_rank(&s_reason, 0);
-          if (reason != 0 || k >= R || its >= max_it) break;
-        }
-        p = tree8(p);
-        if (j <= k && (tid & 7) == 0) h[j] = p;
-        for (int q0 = kClusterThreads; q0 < 8 * (k + 1); q0 += kClusterThreads) {   // 8 lanes (slices) per j
-          const int q = q0 + tid, jj = q >> 3;
-          const double pp = tree8(jj <= k ? remote(hp, q & 7)[jj] : 0.0);
-          if (jj <= k && (q & 7) == 0) h[jj] = pp;
-        }
+      if (k > 0) {
+        reason = s_reason;
+        if (reason != 0 || k >= R || its >= max_it) break;
+      }
+      for (int q0 = 0; q0 < kSlices * (k + 1); q0 += kClusterThreads) {   // 8 lanes (slices) per projection
+        const int q = q0 + tid, j = q >> 3;
+        const double p = tree8(j <= k ? hp[(q & 7) * (R + 1) + j] : 0.0);
+        if (j <= k && (q & 7) == 0) h[j] = p;
       }
       __syncthreads();
-      // w = avs - sum_j h_j V_j on the slice (8 lanes, one chain each, per row) into wbuf; the
-      // lanes 0, 8, 16, 24 of a warp hold 4 consecutive rows: one block of the norm partial
-      const int npass = (8 * nl + kClusterThreads - 1) / kClusterThreads;
-      for (int q0 = 0; q0 < 8 * nl; q0 += kClusterThreads) {
-        const int q = q0 + tid, i = q >> 3, gq = q & 7;
-        double p = 0.0;
-        if (i < nl) {
-          p = gq == 0 ? avs[i] : 0.0;
-          for (int j = gq; j <= k; j += 8) p = fma(-h[j], Vs[(size_t)j * ns + i], p);
+      if (warp < kProdWarps) {
+        // w = avs - sum_j h_j V_j on the slice (8 lanes, one chain each, per row), lane c's copy to
+        // CTA c; the lanes 0, 8, 16, 24 of a warp hold 4 consecutive rows: one block of the norm partial
+        const int npass = (8 * nl + kProdThreads - 1) / kProdThreads;
+        for (int q0 = 0; q0 < 8 * nl; q0 += kProdThreads) {
+          const int q = q0 + tid, i = q >> 3, gq = q & 7;
+          double p = 0.0;
+          if (i < nl) {
+            p = gq == 0 ? avs[i] : 0.0;
+            for (int j = gq; j <= k; j += 8) p = fma(-h[j], Vs[(size_t)j * ns + i], p);
+          }
+          p = tree8(p);
+          if (i < nl) remote(vfull, gq)[r0 + i] = p;
+          double sq = i < nl ? p * p : 0.0;
+          sq += __shfl_xor_sync(full, sq, 8);
+          sq += __shfl_xor_sync(full, sq, 16);
+          if (lane == 0) nblk[q >> 5] = sq;
         }
-        p = tree8(p);
-        if (i < nl && gq == 0) wbuf[i] = p;
-        double sq = i < nl ? p * p : 0.0;
-        sq += __shfl_xor_sync(full, sq, 8);
-        sq += __shfl_xor_sync(full, sq, 16);
-        if (lane == 0) nblk[q >> 5] = sq;
+        bar_prod();
+        if (warp == 0) {
+          double v = lane < LP && lane < kProdWarps * npass ? nblk[lane] : 0.0;
+          for (int off = 1; off < LP; off <<= 1) v += __shfl_xor_sync(full, v, off);
+          v = __shfl_sync(full, v, 0);
+          if (lane < kSlices) remote(npart, lane)[rank] = v;
+        }
+      } else {
+        gc = givens_chain_warp(h, cs, sn, k, &gcol);
       }
-      __syncthreads();
-      if (warp == 0) {
-        double v = lane < LP && lane < 4 * npass ? nblk[lane] : 0.0;
-        for (int off = 1; off < LP; off <<= 1) v += __shfl_xor_sync(full, v, off);
-        if (lane == 0) scal[0] = v;
-      }
-      cl.sync();                                  // partial norms and the unscaled slices
+      cl.sync();                                  // the new vector and its partial norms
       its += 1;
       k += 1;
     }
     // ---- KSPGMRESBuildSoln (k_gmres_update): back substitution and x += V y on the slice
-    if (warp == 0 && k > 0) back_substitute(H, R, g, k - 1, yv, gbuf);
+    if (warp == 0 && k > 0) back_substitute_lanes(H, R, g, k - 1, yv);
     __syncthreads();
-    if (k > 0)
-      for (int i = tid; i < nl; i += blockDim.x) {
+    if (k > 0 && warp < kProdWarps)
+      for (int q0 = 0; q0 < 8 * nl; q0 += kProdThreads) {   // 8 lanes, one chain each, per row
+        const int q = q0 + tid, i = q >> 3, gq = q & 7;
         double u = 0.0;
-        for (int j = 0; j < k; ++j) u = fma(yv[j], Vs[(size_t)j * ns + i], u);
-        xsl[i] = xsl[i] + u;
+        if (i < nl)
+          for (int j = gq; j < k; j += 8) u = fma(yv[j], Vs[(size_t)j * ns + i], u);
+        u = tree8(u);
+        if (i < nl && gq == 0) xsl[i] = xsl[i] + u;
       }
     __syncthreads();
     if (reason != 0 || its >= max_it) break;

@@ -208,7 +208,7 @@ int launch_tors_trig(int nt, const TorsBody* tb, const TorsState& s, cudaStream_
 //   * the kSlices slice partials are combined by the pairwise tree
 //     ((p0+p1)+(p2+p3))+((p4+p5)+(p6+p7));
 //   * w = Av - sum_j h_j v_j runs eight chains (j = g, g+8, ...; chain 0 starts at Av) joined
-//     by the same pairwise tree;
+//     by the same pairwise tree, and so does the update V y (chains from zero);
 //   * a dense row product splits the row into mv_segments(nf) column segments of
 //     ceil(nf/S) columns, each summed as two chains (even and odd offsets) and e + o, the
 //     segments joined by a pairwise tree (seg_tree).
@@ -222,11 +222,11 @@ __host__ __device__ inline int slice_blocks_p2(int n) {
 }
 
 // Column segments per row of the dense product: the most (at most kSlices) for which the
-// rows of one slice, in groups of S lanes that stay within a warp, fit in three warps.
+// rows of one slice, in groups of S lanes that stay within a warp, fit in four warps.
 __host__ __device__ inline int mv_segments(int nf) {
   const int nl = (nf + kSlices - 1) / kSlices;
   for (int S = kSlices; S > 1; --S)
-    if (3 * (32 / S) >= nl) return S;
+    if (4 * (32 / S) >= nl) return S;
   return 1;
 }
 
