@@ -214,8 +214,9 @@ __device__ __forceinline__ void givens_finish_warp(double* col, double c, double
 }
 
 // KSPGMRESBuildSoln back substitution y[0..k] = R^-1 g (R the rotated Hessenberg, ld = R+1), on
-// one whole warp: the pivot reciprocals at once, then a column sweep (y_j = r_j / R_jj as
-// r_j * (1/R_jj); every r_l, l < j, loses R_lj y_j on its own lane).  rc: k+1 doubles.
+// one whole warp: the pivot reciprocals at once, then a column sweep on the unscaled r_j, from which
+// every r_l, l < j, loses (R_lj / R_jj) r_j on its own lane (the quotients stand beside the chain);
+// y_j = r_j / R_jj as r_j * (1/R_jj).  rc: k+1 doubles.
 __device__ void back_substitute(const double* __restrict__ H, int R, const double* __restrict__ g, int k,
                                 double* __restrict__ y, double* __restrict__ rc) {
   const int lane = threadIdx.x & 31;
@@ -226,10 +227,10 @@ __device__ void back_substitute(const double* __restrict__ H, int R, const doubl
   }
   __syncwarp();
   for (int j = k; j >= 0; --j) {
-    const double yj = y[j] * rc[j];
+    const double rj = y[j], rcj = rc[j];
     __syncwarp();
-    for (int l = lane; l < j; l += 32) y[l] = fma(-HH(l, j), yj, y[l]);
-    if (lane == 0) y[j] = yj;
+    for (int l = lane; l < j; l += 32) y[l] = fma(-(HH(l, j) * rcj), rj, y[l]);
+    if (lane == 0) y[j] = rj * rcj;
     __syncwarp();
   }
 }
@@ -593,19 +594,19 @@ constexpr int kProdThreads = 128;
 // back_substitute with a row per lane (k < 32): the same operations, r_l and R's entries in registers
 __device__ __forceinline__ void back_substitute_lanes(const double* H, int R, const double* g, int k, double* y) {
   const int lane = threadIdx.x & 31;
-  double r = 0.0, rc = 0.0, out = 0.0;
+  double r = 0.0, rc = 0.0;
   if (lane <= k) {
     r = g[lane];
     rc = __drcp_rn(H[(size_t)lane * (R + 1) + lane]);
   }
 #pragma unroll 4
-  for (int j = k; j >= 0; --j) {
+  for (int j = k; j > 0; --j) {
     const double hl = lane < j ? H[(size_t)j * (R + 1) + lane] : 0.0;
-    const double yj = __shfl_sync(0xffffffffu, r * rc, j);
-    if (lane == j) out = yj;
-    if (lane < j) r = fma(-hl, yj, r);
+    const double q = hl * __shfl_sync(0xffffffffu, rc, j);
+    const double rj = __shfl_sync(0xffffffffu, r, j);
+    if (lane < j) r = fma(-q, rj, r);
   }
-  if (lane <= k) y[lane] = out;
+  if (lane <= k) y[lane] = r * rc;
   __syncwarp();
 }
 
@@ -712,9 +713,10 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(kClusterThread
       if (t < len_r) areg[t] = At[(size_t)(j0_r + t) * nf + r0 + rl_r];
     }
   } else if (a_in_smem) {
-    for (int q = tid; q < nl * nf; q += blockDim.x) {
-      const int rl = q / nf, j = q - rl * nf;
-      As[q] = At[(size_t)j * nf + r0 + rl];
+#pragma unroll 8
+    for (int q = tid; q < nl * nf; q += kClusterThreads) {
+      const int j = q / nl, rl = q - j * nl;
+      As[rl * nf + j] = At[(size_t)j * nf + r0 + rl];
     }
   }
   __syncthreads();
@@ -727,12 +729,8 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(kClusterThread
 #pragma unroll
         for (int t = 0; t < kRegSeg; t += 2) {
           if (t >= cw) break;   // the same for every lane: no instructions for segments shorter than kRegSeg
-          if (t + 1 < len_r) {
-            e = fma(areg[t], v[t], e);
-            o = fma(areg[t + 1], v[t + 1], o);
-          } else if (t < len_r) {
-            e = fma(areg[t], v[t], e);
-          }
+          if (t < len_r) e = fma(areg[t], v[t], e);
+          if (t + 1 < len_r) o = fma(areg[t + 1], v[t + 1], o);
         }
         p = e + o;
       }
@@ -824,11 +822,10 @@ __global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(kClusterThread
         if (k > 0) {
           bar_scale_get();   // scal[4]; and the raw product is complete
           const double sfac = scal[4];
-          double* w = Vs + (size_t)k * ns;
-          for (int i = tid; i < nl; i += kProdThreads) {
-            avs[i] = avs[i] * sfac;
-            w[i] = vfull[r0 + i] * sfac;
-          }
+          if (warp < 2)
+            for (int i = tid; i < nl; i += 64) avs[i] = avs[i] * sfac;
+          else
+            for (int i = tid - 64; i < nl; i += 64) Vs[(size_t)k * ns + i] = vfull[r0 + i] * sfac;
         }
         bar_prod();
         for (int q0 = 0; q0 < LP * (k + 1); q0 += kProdThreads) {   // LP lanes per projection
