@@ -280,54 +280,46 @@ __device__ __forceinline__ double hat2(double x1, double x2, double dr) {
 // unknowns (x outer, y inner) and weights delta_sd^2 hat(x) hat(y); a point on a sub-domain
 // point takes it with weight 1 alone.  A point outside the cloud sets IB_ERR_DOMAIN (the
 // reference stops) and takes the nearest cell.
-__global__ void k_sd_interp(InterpArgs a) {
+// Four lanes an unknown, each with one of its four hat functions and one of its four entries: three
+// divisions after one another instead of ten (a thread an unknown took 7.7 us).
+__global__ void __launch_bounds__(128) k_sd_interp(InterpArgs a) {
   IB_GRID_DEP_WAIT();
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= a.nf) return;
+  const unsigned full = 0xffffffffu;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool live = (t >> 2) < a.nf;
+  const int k = min(t >> 2, a.nf - 1), i = t & 3, quad = (threadIdx.x & 31) & ~3;
   const bool isx = a.comp[k] == 1;
   const int yoff = isx ? 0 : a.nb_sd;
   const int rp = a.rigid[k];
+  const double d = a.dsd;
+  // lanes 0, 1: the cloud columns left and right of the point; 2, 3: the rows below and above
+  const bool row = i >= 2;
+  const double z = row ? a.yb[k] : a.xb[k], s0 = row ? a.sdyi : a.sdxi;
+  const double fz = __dadd_rn(__ddiv_rn(__dsub_rn(z, s0), d), 1.0);
+  int c = (int)fz;   // Fortran INT (toward zero)
+  const int n = row ? a.ny : a.nx;
+  if (c < 1 || c + 1 > n) {
+    if (live && rp < 0) atomicExch(a.err, IB_ERR_DOMAIN);
+    c = min(max(c, 1), n - 1);
+  }
+  const double sz = __dadd_rn(s0, __dmul_rn((double)(c + (i & 1) - 1), d));
+  const double hz = hat2(sz, z, d), dz = __dsub_rn(z, sz);
+  // entry i = 2 l + p: column l, row p
+  const int l = i >> 1, p = i & 1;
+  const int l0 = __shfl_sync(full, c, quad), p0 = __shfl_sync(full, c, quad + 2);
+  const double hx = __shfl_sync(full, hz, quad + l), hy = __shfl_sync(full, hz, quad + 2 + p);
+  const double dx = __shfl_sync(full, dz, quad + l), dy = __shfl_sync(full, dz, quad + 2 + p);
+  const bool exact = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)) == 0.0;
+  const bool any = (__ballot_sync(full, exact) >> quad) & 0xfu;
+  if (!live) return;
   if (rp >= 0) {   // the body point is sub-domain point rp (the others are weightless dummies)
-    const int dummy = min(rp + 1, a.nb_sd - 1);
-    a.pidx[4 * k] = rp + yoff;
-    a.pw[4 * k] = 1.0;
-    for (int i = 1; i < 4; ++i) {
-      a.pidx[4 * k + i] = dummy + yoff;
-      a.pw[4 * k + i] = 0.0;
-    }
+    a.pidx[4 * k + i] = (i == 0 ? rp : min(rp + 1, a.nb_sd - 1)) + yoff;
+    a.pw[4 * k + i] = i == 0 ? 1.0 : 0.0;
     return;
   }
-  const double xb = a.xb[k], yb = a.yb[k], d = a.dsd;
-  const double fx = __dadd_rn(__ddiv_rn(__dsub_rn(xb, a.sdxi), d), 1.0);
-  const double fy = __dadd_rn(__ddiv_rn(__dsub_rn(yb, a.sdyi), d), 1.0);
-  int l0 = (int)fx, p0 = (int)fy;   // Fortran INT (toward zero)
-  if (l0 < 1 || l0 + 1 > a.nx || p0 < 1 || p0 + 1 > a.ny) {
-    atomicExch(a.err, IB_ERR_DOMAIN);
-    l0 = min(max(l0, 1), a.nx - 1);
-    p0 = min(max(p0, 1), a.ny - 1);
-  }
-  int nn[4];
-  double w[4];
-  bool exact[4];
-  bool any = false;
-  const double d2 = __dmul_rn(d, d);
-  for (int l = 0; l < 2; ++l) {
-    for (int p = 0; p < 2; ++p) {
-      const int i = 2 * l + p;
-      const int ll = l0 + l, pp = p0 + p;
-      nn[i] = a.nr_sd + (pp - 1) * a.nx + (ll - 1);
-      const double sx = __dadd_rn(a.sdxi, __dmul_rn((double)(ll - 1), d));
-      const double sy = __dadd_rn(a.sdyi, __dmul_rn((double)(pp - 1), d));
-      const double dx = __dsub_rn(xb, sx), dy = __dsub_rn(yb, sy);
-      exact[i] = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)) == 0.0;
-      any = any || exact[i];
-      w[i] = __dmul_rn(__dmul_rn(d2, hat2(sx, xb, d)), hat2(sy, yb, d));
-    }
-  }
-  for (int i = 0; i < 4; ++i) {
-    a.pidx[4 * k + i] = nn[i] + yoff;
-    a.pw[4 * k + i] = exact[i] ? 1.0 : (any ? 0.0 : w[i]);
-  }
+  const double w = __dmul_rn(__dmul_rn(__dmul_rn(d, d), hx), hy);
+  a.pidx[4 * k + i] = a.nr_sd + (p0 + p - 1) * a.nx + (l0 + l - 1) + yoff;
+  a.pw[4 * k + i] = exact ? 1.0 : (any ? 0.0 : w);
 }
 
 // B(b, a): row b of column a, zero where dropped (binary search over the column's rows)
@@ -350,7 +342,7 @@ __device__ __forceinline__ double b_at(const long long* __restrict__ colptr, con
 // takes 32 entries l of column k: its threads find the 16 B entries of each (binary searches in
 // the columns, the latency) and their products, then one warp sums each entry in the order above.
 constexpr int kLumatRows = 32;
-__global__ void __launch_bounds__(256) k_sd_lumat(int nf, const int* __restrict__ pidx, const double* __restrict__ pw,
+__global__ void __launch_bounds__(kLumatRows * 16) k_sd_lumat(int nf, const int* __restrict__ pidx, const double* __restrict__ pw,
                                                   const long long* __restrict__ colptr, const int* __restrict__ nz,
                                                   const int* __restrict__ rows, const double* __restrict__ vals,
                                                   const double* __restrict__ brv, const double* __restrict__ bco,
@@ -358,8 +350,8 @@ __global__ void __launch_bounds__(256) k_sd_lumat(int nf, const int* __restrict_
   IB_GRID_DEP_WAIT();
   __shared__ double prod[kLumatRows][17];
   const int k = blockIdx.y, l0 = blockIdx.x * kLumatRows;
-  for (int t = threadIdx.x; t < kLumatRows * 16; t += blockDim.x) {
-    const int e = t >> 4, sub = t & 15, q = sub >> 2, r = sub & 3, l = l0 + e;
+  {   // a thread per entry: the searches' dependent loads are what bounds it
+    const int t = threadIdx.x, e = t >> 4, sub = t & 15, q = sub >> 2, r = sub & 3, l = l0 + e;
     if (l < nf)
       prod[e][sub] = __dmul_rn(b_at(colptr, nz, rows, vals, pidx[4 * l + r], pidx[4 * k + q]), pw[4 * l + r]);
   }
@@ -422,7 +414,7 @@ __global__ void __launch_bounds__(128) k_sd_ptf(int nf, int nf_sd, const int* __
                                                 const double* __restrict__ pw, const double* __restrict__ f,
                                                 double* __restrict__ fsd) {
   constexpr int kChunk = 1024;
-  __shared__ int sidx[kChunk];
+  __shared__ __align__(16) int sidx[kChunk];
   __shared__ double sprod[kChunk];
   IB_GRID_DEP_WAIT();
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
@@ -430,24 +422,27 @@ __global__ void __launch_bounds__(128) k_sd_ptf(int nf, int nf_sd, const int* __
   for (int e0 = 0; e0 < 4 * nf; e0 += kChunk) {
     const int ne = min(kChunk, 4 * nf - e0);
     __syncthreads();
-    for (int e = threadIdx.x; e < ne; e += blockDim.x) {
-      sidx[e] = pidx[e0 + e];
-      sprod[e] = __dmul_rn(pw[e0 + e], f[(e0 + e) >> 2]);
+    for (int e = threadIdx.x; e < ((ne + 31) & ~31); e += blockDim.x) {
+      sidx[e] = e < ne ? pidx[e0 + e] : -1;   // no unknown's
+      sprod[e] = e < ne ? __dmul_rn(pw[e0 + e], f[(e0 + e) >> 2]) : 0.0;
     }
     __syncthreads();
-    // the entries of this unknown first (integer work), then their sum in order, so that the
-    // FP64 adds are issued for the few entries that match only
-    int hit[8];
-    int nh = 0;
-    for (int e = 0; e < ne; ++e) {
-      if (sidx[e] != a) continue;
-      if (nh == 8) {   // more than eight: add the ones held, keep collecting
-        for (int h = 0; h < 8; ++h) acc = __dadd_rn(acc, sprod[hit[h]]);
-        nh = 0;
+    // 32 entries at a time: which are this unknown's (integer work), then their sum in order, so that
+    // the FP64 adds are issued for the few entries that match only
+    for (int g0 = 0; g0 < ne; g0 += 32) {
+      unsigned m = 0;
+#pragma unroll
+      for (int u = 0; u < 32; u += 4) {
+        const int4 s4 = *reinterpret_cast<const int4*>(&sidx[g0 + u]);
+        m |= (s4.x == a ? 1u << u : 0u) | (s4.y == a ? 2u << u : 0u) | (s4.z == a ? 4u << u : 0u) |
+             (s4.w == a ? 8u << u : 0u);
       }
-      hit[nh++] = e;
+      while (m) {
+        const int e = __ffs(m) - 1;
+        m &= m - 1;
+        acc = __dadd_rn(acc, sprod[g0 + e]);
+      }
     }
-    for (int h = 0; h < nh; ++h) acc = __dadd_rn(acc, sprod[hit[h]]);
   }
   if (a < nf_sd) fsd[a] = acc;
 }
@@ -462,7 +457,7 @@ int launch_sd_interp(Ctx* c, cudaStream_t st) {
   a.xb = c->xb; a.yb = c->yb; a.comp = c->comp; a.rigid = S.rigid;
   a.pidx = S.pidx; a.pw = S.pw; a.err = c->d_err;
   count_launch();
-  k_sd_interp<<<cdiv(c->nf, 128), 128, 0, st>>>(a);
+  k_sd_interp<<<cdiv(4LL * c->nf, 128), 128, 0, st>>>(a);
   IB_CUDA_CHECK(cudaGetLastError());
   return IB_OK;
 }
@@ -836,7 +831,7 @@ int launch_sd_lumat(Ctx* c, cudaStream_t st) {
   SubDomain& S = c->sd;
   Influence& I = c->inf;
   count_launch();
-  k_sd_lumat<<<dim3(cdiv(c->nf, kLumatRows), c->nf), 256, 0, st>>>(c->nf, S.pidx, S.pw, S.colptr, S.nz, S.rows,
+  k_sd_lumat<<<dim3(cdiv(c->nf, kLumatRows), c->nf), kLumatRows * 16, 0, st>>>(c->nf, S.pidx, S.pw, S.colptr, S.nz, S.rows,
                                                                    S.vals, I.brv, I.bco, I.bod, I.St);
   IB_CUDA_CHECK(cudaGetLastError());
   return launch_beam_add_b(c, I.St, st);
