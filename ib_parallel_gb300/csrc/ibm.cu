@@ -5,9 +5,11 @@
 // (write_force2, operators_struct.F90:711-731).
 //
 // reg is a face-major gather: for every face of the stencil bounding box the
-// contributing unknowns are listed in ascending order, so each face sums its
-// contributions in the same order as the reference's sequential scatter-add.
+// contributing unknowns are listed in ascending order, and each face's list is summed in
+// one fixed way (eight lanes and a tree; the redistribution in the list's order).
+#include <algorithm>
 #include <cmath>
+#include <vector>
 
 #include "fsi_dev.cuh"
 
@@ -44,33 +46,41 @@ static long double delta_piece(int piece, long double r1) {
 // x in [-1, 1], as powers of x.  The nearest branch points (1/2 +- 1/sqrt(3) from a piece's start) lie
 // 5.95 half widths from the centre of the nearest part, so its coefficients fall as 11.8^-i: what
 // degree 16 leaves out is below 1e-17.
+// The coefficients times the spacing are the same for every context: formed once per process (the
+// first use's thread, as a function's static), 15 ms of the Arm host's software long double otherwise
+// paid by every context.
 size_t delta_table_doubles() { return kDeltaTable; }
-void delta_table(double delta, double* out) {
+static std::vector<long double> delta_unit_table() {
   const long double PI_L = 3.141592653589793238462643383279502884L;
   constexpr int n = kDeltaDeg + 1;
+  std::vector<long double> out(kDeltaTable);
+  long double cs[4 * n];   // cos(pi k / 2n): the nodes and every sum's factors
+  for (int k = 0; k < 4 * n; ++k) cs[k] = cosl(PI_L * k / (2 * n));
   for (int piece = 0; piece < 3; ++piece)
     for (int sub = 0; sub < kDeltaSub; ++sub) {
       long double f[n], c[n], mono[n] = {}, t0[n] = {}, t1[n] = {};
-      for (int i = 0; i < n; ++i) {
-        const long double x = cosl(PI_L * (i + 0.5L) / n);
-        f[i] = delta_piece(piece, piece + (sub + 0.5L + 0.5L * x) / kDeltaSub);
-      }
+      for (int i = 0; i < n; ++i)
+        f[i] = delta_piece(piece, piece + (sub + 0.5L + 0.5L * cs[2 * i + 1]) / kDeltaSub);
       for (int j = 0; j < n; ++j) {
         c[j] = 0.0L;
-        for (int i = 0; i < n; ++i) c[j] += f[i] * cosl(PI_L * j * (i + 0.5L) / n);
+        for (int i = 0; i < n; ++i) c[j] += f[i] * cs[j * (2 * i + 1) % (4 * n)];
         c[j] *= (j == 0 ? 1.0L : 2.0L) / n;
       }
       t0[0] = 1.0L;   // T_0 and T_1, then T_(j+1) = 2 x T_j - T_(j-1)
       t1[1] = 1.0L;
       for (int j = 0; j < n; ++j) {
-        for (int i = 0; i < n; ++i) mono[i] += c[j] * t0[i];
-        long double t2[n];
-        for (int i = 0; i < n; ++i) t2[i] = (i > 0 ? 2.0L * t1[i - 1] : 0.0L) - t0[i];
+        for (int i = 0; i <= j; ++i) mono[i] += c[j] * t0[i];
+        long double t2[n] = {};
+        for (int i = 0; i <= std::min(j + 2, n - 1); ++i) t2[i] = (i > 0 ? 2.0L * t1[i - 1] : 0.0L) - t0[i];
         for (int i = 0; i < n; ++i) { t0[i] = t1[i]; t1[i] = t2[i]; }
       }
-      for (int i = 0; i < n; ++i)
-        out[(piece * kDeltaSub + sub) * n + i] = (double)(mono[i] / (long double)delta);
+      for (int i = 0; i < n; ++i) out[(piece * kDeltaSub + sub) * n + i] = mono[i];
     }
+  return out;
+}
+void delta_table(double delta, double* out) {
+  static const std::vector<long double> unit = delta_unit_table();
+  for (int i = 0; i < kDeltaTable; ++i) out[i] = (double)(unit[i] / (long double)delta);
 }
 
 // Stencil origins and weights of 8 unknowns per CTA (reg_weights_cta).
