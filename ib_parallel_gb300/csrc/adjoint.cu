@@ -11,8 +11,8 @@
 // taped, and returns dJ/d(u, v, W) per step for J = sum of dforces . forces.  The reverse of a
 // step applies the exact transpose of every linear map of the forward in reverse order:
 //   * the spectral solves (ctci, ainv, the predictor's (I - cL)^-1 (I + cL)) are symmetric, and
-//     the predictor's transpose is two predictor solves, one on the adjoint as omega and one on
-//     it as the boundary right-hand side;
+//     the predictor's transpose is one solve, the right-hand sides' adjoint, from which omega's
+//     follows (k_adj_pred);
 //   * rot^T = curl with a zero ring and curl^T = rot plus the ring's edge gathers;
 //   * nonlinear is bilinear in (omega, q + q0) and linear in its ghost ring: k_adj_nl_vertex
 //     and k_adj_nl_faces gather each argument's adjoint;
@@ -35,8 +35,9 @@ namespace {
 constexpr int kT = 256;
 
 // The frame flux of every level, ((c0 B0) + (c1 B1)) + (c2 B2) rounded step by step: level
-// blockIdx.y's u-faces to ox, its v-faces to oy.  Memory traffic bounds it; one launch for all levels
-// (it was one or two a level, 4.2 us each at 600 x 300).
+// blockIdx.y's u-faces to ox, where B1 is zero, its v-faces to oy, where B0 is.  FP64 issue bounds it;
+// one launch for all levels, without the zero products (it was one or two a level, 4.2 us each at
+// 600 x 300).
 struct FrameArgs {
   const double* bases;   // [basis][level][u-faces, v-faces]
   double c0, c1, c2;
@@ -51,13 +52,15 @@ __global__ void __launch_bounds__(kT) k_adj_frame(FrameArgs a) {
   if (i >= per) return;
   const size_t all = (size_t)a.L * per;
   const double* b = a.bases + (size_t)k * per + i;
-  const double v = __dadd_rn(__dadd_rn(__dmul_rn(a.c0, b[0]), __dmul_rn(a.c1, b[all])), __dmul_rn(a.c2, b[2 * all]));
-  if (i < a.nu) a.ox[k][i] = v;
+  const bool u = i < a.nu;
+  const double v = __dadd_rn(__dmul_rn(u ? a.c0 : a.c1, b[u ? 0 : all]), __dmul_rn(a.c2, b[2 * all]));
+  if (u) a.ox[k][i] = v;
   else a.oy[k][i - a.nu] = v;
 }
 
 // Copies up to kMaxCopies arrays (blockIdx.y).  What bounds it is memory traffic: a copy each took
-// 5.5 us for 1.4 MB, all 21 of a 600 x 300 state 115 us.
+// 5.5 us for 1.4 MB, the 12 arrays of a 600 x 300 step's tape 66 us and all 21 of a state 115; the tape
+// takes 5 us so, a state 9.
 constexpr int kMaxCopies = 5 * kMaxLevels + 1;
 struct CopyArgs {
   const double* src[kMaxCopies];
@@ -226,12 +229,16 @@ __global__ void k_adj_coarsify(GridDims g, const double* __restrict__ coarse, do
   fine[idx] += v;
 }
 
-__global__ void k_adj_clear_centre(GridDims g, double* __restrict__ coarse) {
+// the centres that coarsify writes, zero on level blockIdx.y + 1
+struct CentreArgs {
+  double* lam[kMaxLevels];
+};
+__global__ void k_adj_clear_centres(GridDims g, CentreArgs a) {
   IB_GRID_DEP_WAIT();
   const int nj = g.n / 2 - 1, ni = g.m / 2 - 1;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= nj * ni) return;
-  coarse[(g.n / 4 + idx / ni) * g.nsx + (g.m / 4 + idx % ni)] = 0.0;
+  a.lam[blockIdx.y + 1][(g.n / 4 + idx / ni) * g.nsx + (g.m / 4 + idx % ni)] = 0.0;
 }
 
 // U (u averaged to vertices) and V at the ghosted vertex (r, c) of nonlinear's flux u = q + q0
@@ -333,8 +340,9 @@ struct DotArgs {
 constexpr int kDotBlocks = 2 * 152;
 
 // part[b][blk] = the block's slice of sum over levels of <lq0, B_b>: each thread's strided terms, a
-// shuffle tree per warp, the warps' sums in order.  Memory traffic bounds it (the adjoint read once
-// for the three bases).
+// shuffle tree per warp, the warps' sums in order.  Memory traffic bounds it: the adjoint read once
+// for the three bases, and of those the ones that are not zero (B0 on u-faces, B1 on v-faces, B2).
+// 18 us at 600 x 300 with four levels (33 with a pass of the adjoint a basis).
 __global__ void __launch_bounds__(kT) k_adj_dots(DotArgs a) {
   IB_GRID_DEP_WAIT();
   __shared__ double red[3][kT / 32];
@@ -347,9 +355,13 @@ __global__ void __launch_bounds__(kT) k_adj_dots(DotArgs a) {
     const double* ly = a.ly[k];
 #pragma unroll 4
     for (int i = blockIdx.x * kT + threadIdx.x; i < per; i += kDotBlocks * kT) {
-      double l = i < a.nu ? lx[i] : ly[i - a.nu];
-      if (k == 0) l += i < a.nu ? a.ax[i] : a.ay[i - a.nu];
-      for (int q = 0; q < 3; ++q) acc[q] = fma(l, b[q * all + i], acc[q]);
+      const bool u = i < a.nu;
+      double l = u ? lx[i] : ly[i - a.nu];
+      if (k == 0) l += u ? a.ax[i] : a.ay[i - a.nu];
+      const double p = b[(u ? 0 : all) + i];
+      acc[0] = fma(l, u ? p : 0.0, acc[0]);
+      acc[1] = fma(l, u ? 0.0 : p, acc[1]);
+      acc[2] = fma(l, b[2 * all + i], acc[2]);
     }
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -429,10 +441,15 @@ int apply_bc_T(const GridDims& g, const double* v, double fac, const double* lx,
 
 // the coarsify chain's transpose (fine to coarse in the forward: coarse to fine here)
 int coarsify_chain_T(Adj& a, double* const* lam) {
+  CentreArgs ca;
+  for (int k = 0; k < a.L; ++k) ca.lam[k] = lam[k];
   for (int k = a.L - 1; k >= 1; --k) {
-    count_launches(2);
+    count_launch();
     k_adj_coarsify<<<blocks(a.g.ns), kT, 0, a.st>>>(a.g, lam[k], lam[k - 1]);
-    k_adj_clear_centre<<<blocks((a.g.n / 2 - 1) * (a.g.m / 2 - 1)), kT, 0, a.st>>>(a.g, lam[k]);
+  }
+  if (a.L > 1) {   // no level's chain reads another's centre after its own step
+    count_launch();
+    k_adj_clear_centres<<<dim3(blocks((a.g.n / 2 - 1) * (a.g.m / 2 - 1)), a.L - 1), kT, 0, a.st>>>(a.g, ca);
   }
   IB_CUDA_CHECK(cudaGetLastError());
   return IB_OK;
