@@ -586,6 +586,16 @@ int ib_dst(IbCtx* h, const double* in, double* out) {
   return op_result(S.finish(ib::op_dst(c, i, o)), "dst failed");
 }
 
+int ib_pressure_transform(IbCtx* h, const double* in, double* out) {
+  CTX_OR_FAIL(h);
+  const size_t cells = (size_t)c->g.m * c->g.n;
+  Staging S(c);
+  const double* i = S.in(in, cells);
+  double* o = S.out(out, cells, false);
+  STAGE_CHECK(S);
+  return op_result(S.finish(ib::op_pressure_transform(c, i, o)), "pressure_transform failed");
+}
+
 int ib_ctci(IbCtx* h, const double* vort, double* s) {
   CTX_OR_FAIL(h);
   Staging S(c);

@@ -469,6 +469,7 @@ int launch_beam_add_b(Ctx* c, double* St, cudaStream_t st);
 int launch_beam_initial_acc(Ctx* c, const double* f, cudaStream_t st);
 int launch_beam_save(Ctx* c, cudaStream_t st);
 // pressure.cu: calculate_pressure (operators_pressure.F90:110-437) into pres.p
+int op_pressure_transform(Ctx* c, const double* in, double* out);
 int op_pressure(Ctx* c);
 void pressure_free(Ctx* c);
 int op_time_pressure_transform(Ctx* c, bool mma, int reps, double* avg_ms);

@@ -113,13 +113,14 @@ IB_FX int fx_exponent(unsigned hiword) {
   return e ? e : 1;
 }
 
-// The double with bits `b` as a multiple of 2^(emax - 1075 - (kFxFrac - 53)), cut off towards zero;
-// emax is at least its exponent, and both are finite.
+// The double with bits `b` as a multiple of 2^(emax - 1075 - (FRAC - 53)), below 2^FRAC and cut off
+// towards zero; emax is at least its exponent, and both are finite.
+template <int FRAC = kFxFrac>
 IB_FX fx fx_from_bits(long long b, int emax) {
   const unsigned h = (unsigned)((unsigned long long)b >> 32);
   const int e = (int)((h >> 20) & 0x7ffu);
   const unsigned mh = (h & 0xfffffu) | (e ? 0x100000u : 0u);
-  const unsigned long long m = (((unsigned long long)mh << 32) | (unsigned)b) << (kFxFrac - 53);
+  const unsigned long long m = (((unsigned long long)mh << 32) | (unsigned)b) << (FRAC - 53);
   const unsigned s = (unsigned)(emax - (e ? e : 1));
 #if defined(__CUDA_ARCH__)
   unsigned long long r;

@@ -119,23 +119,30 @@ static int launch_pgemm(bool mma, int R, int N, int K, const double* A, int lda,
 // ------------------------------------------------------------------ x transform on the tensor cores
 // Y_k = 2 sum_j x_j sin(pi j k / M), M = m + 1 odd.  sin(pi (M - j) k / M) = -(-1)^k sin(pi j k / M),
 // so odd k take u_j = x_j + x_(M-j) and even k take v_j = x_j - x_(M-j), j = 1..m/2: two products with
-// m/2 x m/2 matrices, half the multiply-adds.  Both factors are 53-bit integers (of the row's exponent,
-// and of 1) cut into eight balanced digits of 7 bits, which bf16 holds exactly; the products of digits
-// i and j with i + j = p <= 7 sum in one FP32 accumulator, exactly (8 products x 64^2 x 512 terms =
-// 2^24), and the eight accumulators of an output combine in 64-bit integers.  What is left out (p > 7)
-// is below a unit of the 53rd bit, so the result is nearer the exact product than the FP64 sum was.
-// 36 bf16 products take the place of one in FP64, at a rate over 300 times higher (the splitting is
+// m/2 x m/2 matrices, half the multiply-adds.  Both factors are integers below 2^55 (u and v in units of
+// 2^-54 of the row's peak exponent, the sines of 2^-55) cut into eight balanced digits of 7 bits, which
+// bf16 holds exactly; the products of digits i and j with i + j = p <= 8 sum in one FP32 accumulator,
+// exactly (at most 8 products x 64^2 x 512 terms = 2^24), and the nine accumulators of an output combine
+// in 64-bit integers.  What is left out (p > 8) has an rms of 2^-63 of the largest product a term, below
+// the operands' rounding, which is what the error is: in rms of a row's outputs 0.7e-16 for noise and
+// wakes, 2e-16 for samples over twelve decades and 5e-16 for a spike over a small background at m = 800,
+// where the FP64 product summed in order gave 10, 9 and 9e-16 (it is better only where the peak is the
+// last sample alone, whose product is its last addition).  Operands of 53 bits and the products up to
+// p = 7 gave 18, 59 and 130e-16: the p = 8 digits of a small sample are as large as a big one's.
+// 43 bf16 products take the place of one in FP64, at a rate over 300 times higher (the splitting is
 // the error-free one of Ozaki, Ogita, Oishi and Rump, 2012).
-// What bounds it: the latency of its dependent steps (tensor pipe 41% busy).  Measured at 800 x 400: 55 us
-// and 5 us for the folding, against 621 us with FP64 FMAs and 99 us with 32 x 32-bit integer
-// multiply-adds; in steps of 32 terms (82 KB a CTA, a second wave of 34 CTAs) 68 us.
-constexpr int kDigits = 8;
+// What bounds it: the latency of its dependent steps.  Measured at 800 x 400: 64 us and 5 us for the
+// folding, against 621 us with FP64 FMAs; with 36 products (p <= 7) 55 us, and those in steps of 32 terms
+// (82 KB a CTA, a second wave of 34 CTAs) 68 us or as 32 x 32-bit integer multiply-adds 99 us.
+constexpr int kDigits = 8, kGroups = 9;        // digits of a factor; sums of products of equal weight
+constexpr int kQBits = 55;                    // of a factor
+constexpr int kQFrac = 60;                    // of a sample before the folding
 // The CTA's tile (two warps of 16 x 32) and step: 338 CTAs at 800 x 400, all resident at once (49 KB each).
 constexpr int kQM = 32, kQN = 32, kQK = 16;
 constexpr int kQPitch = kQK + 8;              // bf16 a staged row: 48 bytes, no bank conflicts for ldmatrix
 constexpr int kQChunk = 512;                  // terms the accumulators hold exactly
 
-// v (|v| <= 2^53) in digits of 7 bits, the last one least
+// v (|v| <= 2^55) in digits of 7 bits, the last one least
 __host__ __device__ __forceinline__ void p_digits(fx v, int* d) {
 #pragma unroll
   for (int i = kDigits - 1; i > 0; --i) {
@@ -175,10 +182,10 @@ __global__ void __launch_bounds__(256) k_pfold(int m, int Rp, int Kp, const doub
   if (threadIdx.x == 0) ex[r] = e;
   const size_t plane = (size_t)Rp * Kp;
   for (int j = threadIdx.x; j < H; j += blockDim.x) {
-    const fx a = fx_from_bits(x[j], e), b = fx_from_bits(x[m - 1 - j], e);   // below 2^56
+    const fx a = fx_from_bits<kQFrac>(x[j], e), b = fx_from_bits<kQFrac>(x[m - 1 - j], e);
     int du[kDigits], dv[kDigits];
-    p_digits(fx_shr(a + b, kFxFrac - 52), du);
-    p_digits(fx_shr(a - b, kFxFrac - 52), dv);
+    p_digits(fx_shr(a + b, kQFrac + 1 - kQBits), du);
+    p_digits(fx_shr(a - b, kQFrac + 1 - kQBits), dv);
     unsigned short* u = fold + (size_t)r * Kp + j;
 #pragma unroll
     for (int i = 0; i < kDigits; ++i) {
@@ -229,20 +236,21 @@ __global__ void __launch_bounds__(64) k_pprod(int R, int m, int Rp, int Np, int 
     }
     asm volatile("cp.async.commit_group;\n");
   };
-  float acc[kDigits][4][4];
+  float acc[kGroups][4][4];
   fx tot[4][4];
 #pragma unroll
-  for (int p = 0; p < kDigits; ++p)
+  for (int p = 0; p < kGroups; ++p)
 #pragma unroll
     for (int n = 0; n < 4; ++n)
 #pragma unroll
       for (int q = 0; q < 4; ++q) acc[p][n][q] = 0.0f;
-  // sum_p acc_p 2^(7 (7 - p)) in units 2^3 (of the products' 2^49), which the 53 x 53-bit terms need
+  // sum_p acc_p 2^(7 (14 - p)) in units of 2^56 (modulo 2^64, which the whole sum is below)
   auto combine = [&](int n, int q) {
-    fx v = 0;
+    unsigned long long v = 0;
 #pragma unroll
-    for (int p = 0; p < kDigits - 1; ++p) v += (fx)__float2int_rn(acc[p][n][q]) << (7 * (kDigits - 1 - p) - 3);
-    return v + fx_shr((fx)__float2int_rn(acc[kDigits - 1][n][q]), 3);
+    for (int p = 0; p < 7; ++p) v += (unsigned long long)(fx)__float2int_rn(acc[p][n][q]) << (7 * (6 - p));
+    const fx low = (fx)__float2int_rn(acc[7][n][q]) * 128 + __float2int_rn(acc[8][n][q]);
+    return (fx)(v + (unsigned long long)fx_shr(low, 14));
   };
   if (LONG) {
 #pragma unroll
@@ -270,18 +278,17 @@ __global__ void __launch_bounds__(64) k_pprod(int R, int m, int Rp, int Np, int 
         p_ldmatrix(a[d], p_smem(sa + (d * kQM + (lane & 15)) * kQPitch + kk + (lane >> 4) * 8));
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        unsigned b[kDigits][4];
 #pragma unroll
-        for (int d = 0; d < kDigits; ++d)   // outputs 0-7 at kk, kk + 8, then outputs 8-15
-          p_ldmatrix(b[d], p_smem(sb + (d * kQN + h * 16 + (lane >> 4) * 8 + (lane & 7)) * kQPitch + kk +
-                                  ((lane >> 3) & 1) * 8));
+        for (int j = 0; j < kDigits; ++j) {
+          unsigned b[4];   // outputs 0-7 at kk, kk + 8, then outputs 8-15
+          p_ldmatrix(b, p_smem(sb + (j * kQN + h * 16 + (lane >> 4) * 8 + (lane & 7)) * kQPitch + kk +
+                               ((lane >> 3) & 1) * 8));
 #pragma unroll
-        for (int i = 0; i < kDigits; ++i)
-#pragma unroll
-          for (int j = 0; j < kDigits - i; ++j) {
-            p_mma(acc[i + j][2 * h], a[i], b[j]);
-            p_mma(acc[i + j][2 * h + 1], a[i], b[j] + 2);
+          for (int i = 0; i < kDigits && i + j < kGroups; ++i) {
+            p_mma(acc[i + j][2 * h], a[i], b);
+            p_mma(acc[i + j][2 * h + 1], a[i], b + 2);
           }
+        }
       }
     }
     if (LONG && ((s + 1) * kQK % kQChunk == 0 || s + 1 == steps)) {
@@ -291,7 +298,7 @@ __global__ void __launch_bounds__(64) k_pprod(int R, int m, int Rp, int Np, int 
         for (int q = 0; q < 4; ++q) {
           tot[n][q] += fx_shr(combine(n, q), shift);
 #pragma unroll
-          for (int p = 0; p < kDigits; ++p) acc[p][n][q] = 0.0f;
+          for (int p = 0; p < kGroups; ++p) acc[p][n][q] = 0.0f;
         }
     }
     __syncthreads();
@@ -302,7 +309,7 @@ __global__ void __launch_bounds__(64) k_pprod(int R, int m, int Rp, int Np, int 
     for (int q = 0; q < 4; ++q) {
       const int r = r0 + warp * 16 + (lane >> 2) + (q >> 1) * 8, c = c0 + n * 8 + 2 * (lane & 3) + (q & 1);
       if (r >= R || c >= H) continue;
-      // terms are (53-bit value) (53-bit sine) 2^(e - 1075 + (kFxFrac - 52) - (kFxFrac - 53)) 2^-53, twice
+      // twice the sum: units of 2^56, of 2^(e - 1022 - (kQBits - 1)) and of 2^-kQBits
       const fx v = LONG ? tot[n][q] : combine(n, q);
       const long long y = ex[r] < 2047 ? fx_to_bits(v, ex[r] - 1074 + shift) : 0x7ff8000000000000LL;
       reinterpret_cast<long long*>(C)[(size_t)r * m + 2 * c + blockIdx.z] = y;
@@ -525,11 +532,11 @@ static int pressure_setup(Ctx* c) {
       for (int k = 0; k < m; ++k)   // sin(pi r / M) is 2M-periodic in r
         W[(size_t)j * m + k] = tab[((long long)(j + 1) * (k + 1)) % (2 * M)];
     IB_CUDA_CHECK(cudaMemcpy(P.W, W.data(), 8 * W.size(), cudaMemcpyHostToDevice));
-    // the digits of sin(pi (j+1) k / M) 2^53 by parity (k_pprod)
+    // the digits of sin(pi (j+1) k / M) 2^kQBits by parity (k_pprod)
     const int H = m / 2, Hp = p_pad(H);
     std::vector<int> digit(2 * (size_t)M * kDigits);
     for (long long r = 0; r < 2 * M; ++r) {
-      const long double s = sinl(PI_L * (long double)r / (long double)M) * 9007199254740992.0L;
+      const long double s = sinl(PI_L * (long double)r / (long double)M) * (long double)(1LL << kQBits);
       p_digits((fx)(s < 0 ? s - 0.5L : s + 0.5L), digit.data() + r * kDigits);
     }
     std::vector<unsigned short> wd(2 * (size_t)kDigits * Hp * Hp, 0);
@@ -582,6 +589,11 @@ static int p_transform(Ctx* c, const double* in, double* out) {
     k_pprod<false><<<grid, 64, kQSmem, c->st>>>(n, m, Rp, Hp, Hp, fold, Wd, P.ex, out, shift);
   }
   return cudaGetLastError() == cudaSuccess ? IB_OK : IB_ERR_CUDA;
+}
+
+int op_pressure_transform(Ctx* c, const double* in, double* out) {
+  RC(pressure_setup(c));
+  return p_transform(c, in, out);
 }
 
 static int ddti(Ctx* c, const double* rhs, double* out) {

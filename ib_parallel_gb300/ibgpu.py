@@ -34,7 +34,8 @@ EXPORTS = [
     "ib_last_error", "ib_version", "ib_create", "ib_destroy", "ib_synchronize", "ib_advance",
     "ib_get_field", "ib_set_field", "ib_get_vector", "ib_set_vector", "ib_get_forces",
     "ib_get_body_state", "ib_get_counters", "ib_get_dims", "ib_nonlinear", "ib_rot", "ib_curl",
-    "ib_coarsify", "ib_get_bc", "ib_apply_bc", "ib_dst", "ib_ctci", "ib_ainv", "ib_fluid_predictor",
+    "ib_coarsify", "ib_get_bc", "ib_apply_bc", "ib_dst", "ib_pressure_transform", "ib_ctci", "ib_ainv",
+    "ib_fluid_predictor",
     "ib_vort2flux", "ib_reg_prep", "ib_reg", "ib_regT", "ib_redistribute", "ib_schur_apply",
     "ib_schur_apply_fluid", "ib_struct_btimes", "ib_struct_rhs", "ib_struct_dx", "ib_schur_solve",
     "ib_get_stream", "ib_profile", "ib_profile_read", "ib_get_work", "ib_measure_fp64_peak",
@@ -105,7 +106,7 @@ def load(path: Optional[os.PathLike] = None):
         "ib_nonlinear": ([P, P, P, P, P, P, P], C.c_int), "ib_rot": ([P, P, P, P], C.c_int),
         "ib_curl": ([P, P, P, P, P], C.c_int), "ib_coarsify": ([P, P, P], C.c_int),
         "ib_get_bc": ([P, P, C.c_double, P], C.c_int), "ib_apply_bc": ([P, P, P, C.c_double], C.c_int),
-        "ib_dst": ([P, P, P], C.c_int), "ib_ctci": ([P, P, P], C.c_int), "ib_ainv": ([P, P], C.c_int),
+        "ib_dst": ([P, P, P], C.c_int), "ib_pressure_transform": ([P, P, P], C.c_int), "ib_ctci": ([P, P, P], C.c_int), "ib_ainv": ([P, P], C.c_int),
         "ib_fluid_predictor": ([P, C.c_int, P, P, P, P], C.c_int),
         "ib_vort2flux": ([P, P, P, P, P], C.c_int), "ib_reg_prep": ([P, P, P], C.c_int),
         "ib_reg": ([P, P, P, P], C.c_int), "ib_regT": ([P, P, P, P], C.c_int),
@@ -562,6 +563,11 @@ class Simulation:
     def dst(self, x):
         out = self._o(self.shapes["omega"])
         _check(self.lib.ib_dst(self.h, _ptr(np.ascontiguousarray(x)), _ptr(out)), "ib_dst")
+        return out
+
+    def pressure_transform(self, x):
+        out = np.empty((self.params.n, self.params.m))
+        _check(self.lib.ib_pressure_transform(self.h, _ptr(np.ascontiguousarray(x)), _ptr(out)), "ib_pressure_transform")
         return out
 
     def ctci(self, x):

@@ -253,6 +253,8 @@ int ib_get_bc(IbCtx* ctx, const double* s, double fac, double* ring);
 int ib_apply_bc(IbCtx* ctx, double* vort, const double* ring, double fac);
 /* myfft.F90:207-216 dst: unnormalised 2-D DST-I (FFTW RODFT00 x RODFT00) */
 int ib_dst(IbCtx* ctx, const double* in, double* out);
+/* the x direction of ddti (myfft.F90:192-203): the unnormalised DST-I of each of the n rows of m cells */
+int ib_pressure_transform(IbCtx* ctx, const double* in, double* out);
 /* myfft.F90:177-188 ctci */
 int ib_ctci(IbCtx* ctx, const double* vort, double* s);
 /* The same Poisson solve for an m x n grid without a context and without allocating device
