@@ -84,7 +84,10 @@ __device__ __forceinline__ void reg_weights_cta(const GridDims& g, int nf, int k
   const int u = tid >> 4, axis = (tid >> 3) & 1, q = tid & 7, k = k0 + u;
   if (k < nf && q < 7) {
     const double z = pos[u][axis], o = axis ? oy : ox;
-    const int c = (int)((z + o) / d) + 1;   // Fortran INT truncates toward zero
+    // Fortran INT truncates toward zero.  A point far outside, or one that is not a number, keeps its
+    // origin within 16 cells of the grid (and is reported below): the boxes and offsets formed from
+    // origins then fit an int, and no list index does worse than leave its capacity, which is checked.
+    const int c = min(max((int)((z + o) / d), -16), (axis ? g.n : g.m) + 16) + 1;
     // The grid coordinate is rounded after the product and again after the sum, as the
     // reference's expression delta*(indexx-1+p)-offsetx is (grid.F90:459-528): the delta
     // function is discontinuous at 3 cells (its single-precision constants leave about 1e-8

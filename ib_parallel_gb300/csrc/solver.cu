@@ -1772,6 +1772,13 @@ int op_advance_end(Ctx* c) {
   return IB_OK;
 }
 
+// A step that ends without its finish: the domain error that positions without a number have left is not
+// the next step's.
+static int nonfinite(Ctx* c) {
+  IB_CUDA_CHECK(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->st));
+  return IB_ERR_NONFINITE;
+}
+
 static int advance_end(Ctx* c) {
   if (!c->end_pending) return IB_ERR_STATE;
   c->end_pending = false;
@@ -1815,7 +1822,7 @@ static int advance_end(Ctx* c) {
           I.patch_fresh = true;
           I.active = false;
           err = c->h_scal[0];
-          if (!std::isfinite(err)) return IB_ERR_NONFINITE;
+          if (!std::isfinite(err)) return nonfinite(c);
         }
       }
       while (err >= p.fsi_tol && fsi_count <= p.fsi_max_it) {
@@ -1912,7 +1919,7 @@ static int advance_end(Ctx* c) {
           I.patch_fresh = true;
         }
         err = c->h_scal[0];
-        if (!std::isfinite(err)) return IB_ERR_NONFINITE;
+        if (!std::isfinite(err)) return nonfinite(c);
       }
       c->fsi_iter = fsi_count;
       // the loop of timestepper.F90:318 ends at fsi_max_it + 1 iterations without reaching
