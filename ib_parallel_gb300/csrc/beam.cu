@@ -324,17 +324,17 @@ __global__ void __launch_bounds__(kBeamThreads) k_beam_dx(const BeamDev* __restr
     double em = 0.0;
     for (int k = threadIdx.x; k < nd; k += kBeamThreads) {
       const double dq = b.t1[k];
-      em = fmax(em, fabs(dq));
+      em = max_magnitude(em, dq);
       const double qn = b.q[k] + dq;
       b.q[k] = qn;
       b.qd[k] = -b.qd0[k] + fc.v * (qn - b.q0[k]);
       b.qdd[k] = -b.qdd0[k] - fc.a1 * b.qd0[k] + fc.a2 * (qn - b.q0[k]);
     }
-    for (int o = 16; o > 0; o >>= 1) em = fmax(em, __shfl_xor_sync(0xffffffffu, em, o));
+    for (int o = 16; o > 0; o >>= 1) em = max_magnitude(em, __shfl_xor_sync(0xffffffffu, em, o));
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = em;
     __syncthreads();
     if (threadIdx.x == 0)
-      for (int w = 0; w < kBeamThreads / 32; ++w) emax = fmax(emax, red[w]);
+      for (int w = 0; w < kBeamThreads / 32; ++w) emax = max_magnitude(emax, red[w]);
     // positions: x0 + (-sin g) d, y0 + cos g d, d = Phi q
     for (int j = threadIdx.x; j < b.npts; j += kBeamThreads) {
       const double d = beam_point_row(b.phi + (size_t)j * nd, nd, beam_point_dof(b, j), b.q);

@@ -107,13 +107,9 @@ __global__ void __launch_bounds__(128) k_fsi_update(FsiUpdateArgs a) {
     a.ts.sinv[t] = a.sin_next[t];
     a.ts.cosv[t] = a.cos_next[t];
   }
-  double e = 0.0;
-  if (a.nt == 1) {
-    e = a.err[1];
-  } else if (a.nt > 1) {
-    for (int t = 0; t < a.nt; ++t) e = fmax(e, a.err[1 + t]);
-  }
-  if (a.beam_err) e = fmax(e, *a.beam_err);
+  double e = 0.0;   // keeps NaN, which ends the loop
+  for (int t = 0; t < a.nt; ++t) e = max_magnitude(e, a.err[1 + t]);
+  if (a.beam_err) e = max_magnitude(e, *a.beam_err);
   a.err[0] = e;
   const int n = a.cnt[0] + 1;
   const int bf = *a.flag;

@@ -80,6 +80,12 @@ __device__ __forceinline__ double ring_value(const double* __restrict__ s, const
   return (p & 1) ? 0.5 * (S(I, J) + S(I, J + 1)) : S(I, J);
 }
 
+// The larger of two magnitudes, with NaN above every number (fmax drops it): by their bits, as integers.
+__device__ __forceinline__ double max_magnitude(double a, double b) {
+  const long long mask = 0x7fffffffffffffffLL;
+  return __longlong_as_double(max(__double_as_longlong(a) & mask, __double_as_longlong(b) & mask));
+}
+
 inline int cdiv(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 // Division of a non-negative int by a runtime divisor d >= 1 with a multiply-high and a

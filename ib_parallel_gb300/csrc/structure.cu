@@ -111,8 +111,8 @@ int launch_tors_consts(int nt, TorsBody* tb, double dt, double delta, cudaStream
 __global__ void k_max_reduce(int n, const double* __restrict__ v, double* out) {
   IB_GRID_DEP_WAIT();
   double m = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) m = fmax(m, v[i]);
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  for (int i = threadIdx.x; i < n; i += blockDim.x) m = max_magnitude(m, v[i]);
+  for (int o = 16; o > 0; o >>= 1) m = max_magnitude(m, __shfl_xor_sync(0xffffffffu, m, o));
   if (threadIdx.x == 0) out[0] = m;
 }
 
