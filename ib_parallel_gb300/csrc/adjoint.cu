@@ -510,7 +510,7 @@ int step_T(Adj& a, int slot, int it, const double* frame, const double* dforce_h
   k_adj_force<<<blocks(c->nf), kT, 0, st>>>(c->nf, c->nbody, c->comp, c->bid, 2.0 * c->delta / c->p.dt, A.dforce,
                                             A.lf, A.lf);
   if (c->p.num_stat) {
-    RC(launch_chol_solve(c->nf, c->cholZ, A.lf, c->chol_y, A.lrhsf, st));
+    RC(op_chol_solve(c, A.lf, A.lrhsf));
   } else {
     // S^T lrhsf = lf: the band's row-major S (rigid bodies: no structure block), or the
     // sub-domain's lumat transposed, as the column-major operator of the cluster solver, from a

@@ -754,6 +754,15 @@ int ib_schur_solve(IbCtx* h, const double* rhs, double* f, int* iterations) {
   return op_result(S.finish(rc), "schur_solve failed");
 }
 
+int ib_direct_solve(IbCtx* h, const double* rhs, double* f) {
+  CTX_OR_FAIL(h);
+  Staging S(c);
+  const double* b = S.in(rhs, c->nf);
+  double* x = S.out(f, c->nf, false);
+  STAGE_CHECK(S);
+  return op_result(S.finish(ib::op_chol_solve(c, b, x)), "direct_solve failed");
+}
+
 int ib_get_stream(IbCtx* h, void** stream) {
   CTX_OR_FAIL(h);
   if (!stream) return fail(IB_ERR_ARG, "null output");

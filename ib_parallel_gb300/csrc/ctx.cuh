@@ -368,9 +368,10 @@ struct Ctx {
   long long fsi_post_launches = 0;
   int* fsi_cnt = nullptr;
   FusedPlan fused_plan;
-  double* cholM = nullptr;         // nf x nf (num_stat): the Schur matrix, then its Cholesky factor
-  double* cholZ = nullptr;         // nf x nf: the factor's inverse in both triangles
-  double* chol_y = nullptr;        // nf: between the solve's two products
+  double* cholM = nullptr;         // nf x nf (num_stat): the Schur matrix, symmetric by its upper triangle
+  double* cholZ = nullptr;         // nf x nf: its Cholesky factor, then the factor's inverse in both triangles
+  double* chol_y = nullptr;        // nf: between the solve's products
+  double* chol_r = nullptr;        // nf: its residual
   bool chol_ready = false;
 
   // host-visible status
@@ -469,6 +470,7 @@ int launch_beam_add_b(Ctx* c, double* St, cudaStream_t st);
 int launch_beam_initial_acc(Ctx* c, const double* f, cudaStream_t st);
 int launch_beam_save(Ctx* c, cudaStream_t st);
 // pressure.cu: calculate_pressure (operators_pressure.F90:110-437) into pres.p
+int op_chol_solve(Ctx* c, const double* b, double* x);   // the stationary bodies' solve alone (num_stat)
 int op_pressure_transform(Ctx* c, const double* in, double* out);
 int op_pressure(Ctx* c);
 void pressure_free(Ctx* c);

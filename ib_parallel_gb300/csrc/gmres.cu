@@ -474,15 +474,25 @@ __global__ void k_cholesky(int n, double* A, int* err) {
   }
 }
 
-// Z = L^-1 for the Cholesky factor L (row-major, lower), one warp per column by forward substitution:
-// Z[r][c] = Z[c][r] = (L^-1)[r][c] for r >= c, so that both products of the solve read rows.  Run once
-// per factorisation.  L and Z are different arrays.
-__global__ void __launch_bounds__(32) k_tri_inverse(int n, const double* __restrict__ L, double* __restrict__ Z) {
+// M's lower triangle from its upper one, and F = M (the factorisation reads the upper triangle alone).
+__global__ void k_symmetrise(int n, double* M, double* __restrict__ F) {
+  IB_GRID_DEP_WAIT();
+  const int c = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y;
+  if (c >= n) return;
+  const double v = M[(size_t)min(r, c) * n + max(r, c)];
+  if (c < r) M[(size_t)r * n + c] = v;
+  F[(size_t)r * n + c] = v;
+}
+
+// Z = L^-1 for the Cholesky factor L (row-major, in F's lower triangle), one warp per column by forward
+// substitution, into F's upper triangle, Z[r][c] at F[c][r] for r > c, and its diagonal into diag: no
+// column reads what another writes.  Run once per factorisation, k_tri_mirror after it.
+__global__ void __launch_bounds__(32) k_tri_inverse(int n, double* F, double* __restrict__ diag) {
   IB_GRID_DEP_WAIT();
   extern __shared__ double col[];   // n entries of the column
   const int j = blockIdx.x, lane = threadIdx.x;
   for (int i = j; i < n; ++i) {
-    const double* row = L + (size_t)i * n;
+    const double* row = F + (size_t)i * n;
     double a0 = 0.0, a1 = 0.0;
     int k = j + lane;
     for (; k + 32 < i; k += 64) {
@@ -495,21 +505,25 @@ __global__ void __launch_bounds__(32) k_tri_inverse(int n, const double* __restr
     if (lane == 0) col[i] = ((i == j ? 1.0 : 0.0) - s) / row[i];
     __syncwarp();
   }
-  for (int i = j + lane; i < n; i += 32) {
-    Z[(size_t)j * n + i] = col[i];
-    Z[(size_t)i * n + j] = col[i];
-  }
+  if (lane == 0) diag[j] = col[j];
+  for (int i = j + 1 + lane; i < n; i += 32) F[(size_t)j * n + i] = col[i];
 }
 
-// y = L^-1 b (upper = 0) or y = L^-T b (upper = 1) from Z, a warp per row, four chains a lane.  The
-// stationary bodies' solve is the two products in turn (launch_chol_solve).  What bounds it: latency,
-// a few dependent FP64 operations of 64 cycles and the row's loads from L2.  The substitutions by
-// blocks of 32 it replaced ran on one CTA, 2 n / 32 dependent triangles: 304 us for the 314 unknowns
-// of the 157-point cylinder, against 7 us for the two products.
+// F's lower triangle from its upper one and its diagonal from diag: both products of the solve read rows.
+__global__ void k_tri_mirror(int n, double* F, const double* __restrict__ diag) {
+  IB_GRID_DEP_WAIT();
+  const int c = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y;
+  if (c < r) F[(size_t)r * n + c] = F[(size_t)c * n + r];
+  if (c == r) F[(size_t)r * n + r] = diag[r];
+}
+
+// y = L^-1 b (upper = 0) or y = L^-T b (upper = 1) from Z, added to y with `add`; a warp per row, four
+// chains a lane.  What bounds it: latency, a few dependent FP64 operations of 64 cycles and the row's loads
+// from L2.
 constexpr int kTriRows = 4;   // rows (warps) per CTA
 __global__ void __launch_bounds__(32 * kTriRows) k_tri_product(int n, const double* __restrict__ Z,
                                                                const double* __restrict__ b, double* __restrict__ y,
-                                                               int upper) {
+                                                               int upper, int add) {
   IB_GRID_DEP_WAIT();
   const int r = blockIdx.x * kTriRows + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (r >= n) return;
@@ -523,7 +537,41 @@ __global__ void __launch_bounds__(32 * kTriRows) k_tri_product(int n, const doub
   }
   double s = (a[0] + a[1]) + (a[2] + a[3]);
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) y[r] = s;
+  if (lane == 0) y[r] = add ? y[r] + s : s;
+}
+
+// A sum in two parts: s and what its roundings left out (Knuth's two-sum).
+struct Sum2 {
+  double s, c;
+  __device__ __forceinline__ void add(double v) {
+    const double t = s + v, z = t - s;
+    c += (s - (t - z)) + (v - z);
+    s = t;
+  }
+};
+
+// r = b - M x, each row a compensated product (Ogita, Rump and Oishi's Dot2) on one warp: as if formed in
+// twice the working precision.  FP64 issue bounds it, ten operations a term.
+__global__ void __launch_bounds__(32 * kTriRows) k_residual(int n, const double* __restrict__ M,
+                                                            const double* __restrict__ b, const double* __restrict__ x,
+                                                            double* __restrict__ r) {
+  IB_GRID_DEP_WAIT();
+  const int i = blockIdx.x * kTriRows + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (i >= n) return;
+  const double* row = M + (size_t)i * n;
+  Sum2 a{lane == 0 ? b[i] : 0.0, 0.0};
+#pragma unroll 4
+  for (int c = lane; c < n; c += 32) {
+    const double m = row[c], v = x[c], h = __dmul_rn(-m, v);   // no contraction into the sum
+    a.c -= fma(m, v, h);
+    a.add(h);
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    const double s = __shfl_xor_sync(0xffffffffu, a.s, o), c = __shfl_xor_sync(0xffffffffu, a.c, o);
+    a.add(s);
+    a.c += c;
+  }
+  if (lane == 0) r[i] = a.s + a.c;
 }
 
 __global__ void k_copy_col(int n, const double* __restrict__ src, double* M, int col) {
@@ -543,18 +591,36 @@ int launch_cholesky(int n, double* A, int* d_err, cudaStream_t st) {
   IB_CUDA_CHECK(cudaGetLastError());
   return IB_OK;
 }
-int launch_tri_inverse(int n, const double* L, double* Z, cudaStream_t st) {
+int launch_tri_inverse(int n, double* F, double* diag, cudaStream_t st) {
   const size_t smem = sizeof(double) * (size_t)n;
   IB_CUDA_CHECK(allow_dyn_smem(k_tri_inverse, smem));
-  count_launch();
-  k_tri_inverse<<<n, 32, smem, st>>>(n, L, Z);
+  count_launches(2);
+  k_tri_inverse<<<n, 32, smem, st>>>(n, F, diag);
+  k_tri_mirror<<<dim3(cdiv(n, 256), n), 256, 0, st>>>(n, F, diag);
   IB_CUDA_CHECK(cudaGetLastError());
   return IB_OK;
 }
-int launch_chol_solve(int n, const double* Z, const double* b, double* y, double* x, cudaStream_t st) {
-  count_launches(2);
-  k_tri_product<<<cdiv(n, kTriRows), 32 * kTriRows, 0, st>>>(n, Z, b, y, 0);
-  k_tri_product<<<cdiv(n, kTriRows), 32 * kTriRows, 0, st>>>(n, Z, y, x, 1);
+int launch_symmetrise(int n, double* M, double* F, cudaStream_t st) {
+  count_launch();
+  k_symmetrise<<<dim3(cdiv(n, 256), n), 256, 0, st>>>(n, M, F);
+  IB_CUDA_CHECK(cudaGetLastError());
+  return IB_OK;
+}
+// x = M^-1 b: the two products with the inverse factor, then one step of refinement.  The substitutions by
+// blocks of 32 that the products replaced ran on one CTA, 2 n / 32 dependent triangles: 304 us for the 314
+// unknowns of the 157-point cylinder, against 7 us for the two products and 18 us for the five launches.  Products
+// with an inverse alone are not backward stable: at 196 to 314 unknowns their residual was 2 to 10 times the
+// substitutions', their error up to 4 times.  The refinement, with the residual in two parts, leaves an
+// error of the result's last place, below the substitutions'.
+int launch_chol_solve(int n, const double* M, const double* Z, const double* b, double* y, double* r, double* x,
+                      cudaStream_t st) {
+  const int blocks = cdiv(n, kTriRows), threads = 32 * kTriRows;
+  count_launches(5);
+  k_tri_product<<<blocks, threads, 0, st>>>(n, Z, b, y, 0, 0);
+  k_tri_product<<<blocks, threads, 0, st>>>(n, Z, y, x, 1, 0);
+  k_residual<<<blocks, threads, 0, st>>>(n, M, b, x, r);
+  k_tri_product<<<blocks, threads, 0, st>>>(n, Z, r, y, 0, 0);
+  k_tri_product<<<blocks, threads, 0, st>>>(n, Z, y, x, 1, 1);
   IB_CUDA_CHECK(cudaGetLastError());
   return IB_OK;
 }

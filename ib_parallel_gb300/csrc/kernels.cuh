@@ -290,11 +290,14 @@ struct FusedPlan {
 int launch_gmres_fused(const GmresDev& G, FusedPlan* plan, const double* At, const double* b, double* x, double rtol,
                        double atol, int max_it, cudaStream_t st);
 
-// dense symmetric positive definite solve (stationary-body path): A = L L^T, Z = L^-1 (stored in both
-// triangles), then x = L^-T (y = L^-1 b)
-int launch_cholesky(int n, double* A, int* d_err, cudaStream_t st);
-int launch_tri_inverse(int n, const double* L, double* Z, cudaStream_t st);
-int launch_chol_solve(int n, const double* Z, const double* b, double* y, double* x, cudaStream_t st);
+// dense symmetric positive definite solve (stationary-body path).  M's lower triangle from its upper one and
+// F = M; F = L L^T (L in its lower triangle); F = Z = L^-1 in both triangles (diag: n doubles of scratch);
+// then x = L^-T L^-1 b and one step of refinement with M (y, r: n doubles of scratch)
+int launch_symmetrise(int n, double* M, double* F, cudaStream_t st);
+int launch_cholesky(int n, double* F, int* d_err, cudaStream_t st);
+int launch_tri_inverse(int n, double* F, double* diag, cudaStream_t st);
+int launch_chol_solve(int n, const double* M, const double* Z, const double* b, double* y, double* r, double* x,
+                      cudaStream_t st);
 int launch_copy_col(int n, const double* src, double* M, int col, cudaStream_t st);
 int launch_unit(int n, int i, double* e, cudaStream_t st);
 

@@ -225,7 +225,7 @@ int ctx_create(const IbParams* pin, const IbBody* bodies, int nbody, Ctx** out, 
   dbl += 3 * ((size_t)nt + 1) + 1;                       // fused FSI update: theta, sin, cos; ticket
   dbl += 8 * (size_t)nt + nt + 3;
   dbl += (size_t)(R + 1) * nf + (size_t)(R + 1) * R + 3 * (R + 1) + 4 + 4 * (size_t)nf + 2;
-  if (p.num_stat) dbl += 2 * (size_t)nf * nf + nf;
+  if (p.num_stat) dbl += 2 * (size_t)nf * nf + 2 * (size_t)nf;
   dbl += 8 * stage_n;
   size_t ints = 2 * (size_t)nf + 2 * (size_t)nf + 16 + 2 * (size_t)max_faces + 2 * 49 * (size_t)nf + 4 + 2 + 8;
   size_t bytes = dbl * 8 + ints * 4 + (size_t)nt * sizeof(TorsBody) + 256 * 400;
@@ -296,6 +296,7 @@ int ctx_create(const IbParams* pin, const IbBody* bodies, int nbody, Ctx** out, 
     c->cholM = P.take<double>((size_t)nf * nf);
     c->cholZ = P.take<double>((size_t)nf * nf);
     c->chol_y = P.take<double>(nf);
+    c->chol_r = P.take<double>(nf);
   }
   c->d_err = P.take<int>(1);
   c->stage_n = stage_n;
@@ -1110,12 +1111,23 @@ static int preprocess_chol(Ctx* c) {
     RC(op_schur(c, c->tmpf, c->tmpf2, false));
     RC(launch_copy_col(nf, c->tmpf2, c->cholM, i, c->st));
   }
-  RC(launch_cholesky(nf, c->cholM, c->d_err, c->st));
+  RC(launch_symmetrise(nf, c->cholM, c->cholZ, c->st));
+  RC(launch_cholesky(nf, c->cholZ, c->d_err, c->st));
   int e = check_err(c);
   if (e) return IB_ERR_ARG;
-  RC(launch_tri_inverse(nf, c->cholM, c->cholZ, c->st));
+  RC(launch_tri_inverse(nf, c->cholZ, c->chol_y, c->st));
   c->chol_ready = true;
   return IB_OK;
+}
+
+static int chol_solve(Ctx* c, const double* b, double* x) {
+  return launch_chol_solve(c->nf, c->cholM, c->cholZ, b, c->chol_y, c->chol_r, x, c->st);
+}
+
+int op_chol_solve(Ctx* c, const double* b, double* x) {
+  if (!c->p.num_stat || c->nf == 0) return IB_ERR_STATE;
+  if (!c->chol_ready) RC(preprocess_chol(c));
+  return chol_solve(c, b, x);
 }
 
 // mode 1: start (totals cleared) with the FSI iterations run from the host, phase by phase;
@@ -1539,7 +1551,7 @@ static int op_direct_solve(Ctx* c) {
   } else {
     RC(launch_regT(g, c->nf, c->qx[0], c->q0x[0], c->qy[0], c->q0y[0], c->reg, nullptr, c->rhsf, st));
   }
-  RC(launch_chol_solve(c->nf, c->cholZ, c->rhsf, c->chol_y, c->f, st));
+  RC(chol_solve(c, c->rhsf, c->f));
   return op_redistribute(c, c->f, c->f_rdst);
 }
 

@@ -37,7 +37,7 @@ EXPORTS = [
     "ib_coarsify", "ib_get_bc", "ib_apply_bc", "ib_dst", "ib_pressure_transform", "ib_ctci", "ib_ainv",
     "ib_fluid_predictor",
     "ib_vort2flux", "ib_reg_prep", "ib_reg", "ib_regT", "ib_redistribute", "ib_schur_apply",
-    "ib_schur_apply_fluid", "ib_struct_btimes", "ib_struct_rhs", "ib_struct_dx", "ib_schur_solve",
+    "ib_schur_apply_fluid", "ib_struct_btimes", "ib_struct_rhs", "ib_struct_dx", "ib_schur_solve", "ib_direct_solve",
     "ib_get_stream", "ib_profile", "ib_profile_read", "ib_get_work", "ib_measure_fp64_peak",
     "ib_launch_count", "ib_time_pass", "ib_profile_schur", "ib_ctci_static",
     "ib_schur_matrix", "ib_get_influence_stats", "ib_step_profile", "ib_get_launch_shapes",
@@ -113,7 +113,7 @@ def load(path: Optional[os.PathLike] = None):
         "ib_redistribute": ([P, P, P], C.c_int), "ib_schur_apply": ([P, P, P], C.c_int),
         "ib_schur_apply_fluid": ([P, P, P], C.c_int), "ib_struct_btimes": ([P, P, P], C.c_int),
         "ib_struct_rhs": ([P, P], C.c_int), "ib_struct_dx": ([P, P, P], C.c_int),
-        "ib_schur_solve": ([P, P, P, I], C.c_int),
+        "ib_schur_solve": ([P, P, P, I], C.c_int), "ib_direct_solve": ([P, P, P], C.c_int),
         "ib_get_stream": ([P, C.POINTER(P)], C.c_int), "ib_profile": ([P, C.c_int], C.c_int),
         "ib_profile_read": ([P, C.c_int, I, D, D], C.c_int),
         "ib_get_work": ([P, C.POINTER(C.c_longlong), C.POINTER(C.c_longlong)], C.c_int),
@@ -646,6 +646,11 @@ class Simulation:
                                        C.byref(its)), "ib_schur_solve")
         return f, its.value
 
+    def direct_solve(self, rhs):
+        f = np.empty(self.nf)
+        _check(self.lib.ib_direct_solve(self.h, _ptr(np.ascontiguousarray(rhs, dtype=np.float64)), _ptr(f)),
+               "ib_direct_solve")
+        return f
 
 
 class Batch:

@@ -299,6 +299,9 @@ int ib_struct_rhs(IbCtx* ctx, double* y);
 int ib_struct_dx(IbCtx* ctx, const double* f, double* err);
 /* GMRES on the Schur operator (timestepper.F90:363-366): f updated in place */
 int ib_schur_solve(IbCtx* ctx, const double* rhs, double* f, int* iterations);
+/* the stationary bodies' solve by the factorised Schur matrix (timestepper.F90:458-486); num_stat contexts
+ * alone, IB_ERR_STATE otherwise.  f must not be rhs. */
+int ib_direct_solve(IbCtx* ctx, const double* rhs, double* f);
 
 /* ---- instrumentation (no counterpart in the reference) ---- */
 /* the cudaStream_t every kernel of this context runs on */
