@@ -43,10 +43,9 @@ struct DevPool {
 struct PressureOp {
   bool ready = false, computed = false;
   double* mem = nullptr;
-  double* W = nullptr;          // m x m DST-I matrix of the cell grid's x direction
   TriOp tri;                    // per-mode (lx(k) + T_y)^-1 of the n cell rows
   std::vector<double*> rhs, p, oqx, oqy, nlx, nly;   // per level
-  double *y = nullptr, *tmp = nullptr, *hx = nullptr, *hy = nullptr, *fdt = nullptr;
+  double *y = nullptr, *hx = nullptr, *hy = nullptr, *fdt = nullptr;
   double *ubc = nullptr, *vbc = nullptr, *ring = nullptr;
   double *Wd = nullptr, *fold = nullptr;   // the x transform's bf16 digits of sin and of a level's rows
   int* ex = nullptr;                       // the rows' exponents
@@ -474,7 +473,7 @@ int op_chol_solve(Ctx* c, const double* b, double* x);   // the stationary bodie
 int op_pressure_transform(Ctx* c, const double* in, double* out);
 int op_pressure(Ctx* c);
 void pressure_free(Ctx* c);
-int op_time_pressure_transform(Ctx* c, bool mma, int reps, double* avg_ms);
+int op_time_pressure_transform(Ctx* c, int kind, int reps, double* avg_ms);
 int op_write_pressure(Ctx* c, const char* path, std::string* msg);
 // subdomain.cu: the sub-domain method (grid.F90:572-951, timestepper.F90:368-405, 602-770,
 // operators_struct.F90:840-905)

@@ -500,7 +500,7 @@ static int pressure_setup(Ctx* c) {
   const size_t cells = (size_t)m * n;
   const TriShape tri_t = tri_chunking(n, m);
   const size_t tri_n = tri_table_doubles(m, tri_t);
-  const size_t dbl = (size_t)m * m + tri_n + 2 * (size_t)L * cells + 2 * cells + 2 * (size_t)L * g.ns +
+  const size_t dbl = tri_n + 2 * (size_t)L * cells + cells + 2 * (size_t)L * g.ns +
                      (size_t)L * (g.nu + g.nv) + g.nu + g.nv + (size_t)std::max(c->nf, 1) + 2 * (size_t)g.nbc +
                      2 * (size_t)(m + n) + 64 + 4 * (size_t)p_pad(m / 2) * p_pad(m / 2) +
                      4 * (size_t)p_pad(n) * p_pad(m / 2) + (size_t)n + 16;
@@ -508,11 +508,9 @@ static int pressure_setup(Ctx* c) {
   IB_CUDA_CHECK(cudaMemset(P.mem, 0, 8 * dbl));
   double* q = P.mem;
   auto take = [&](size_t k) { double* r = q; q += (k + 3) & ~size_t(3); return r; };
-  P.W = take((size_t)m * m);
   double* tri_mem = take(tri_n);
   for (int k = 0; k < L; ++k) { P.rhs.push_back(take(cells)); P.p.push_back(take(cells)); }
   P.y = take(cells);
-  P.tmp = take(cells);
   for (int k = 0; k < L; ++k) { P.oqx.push_back(take(g.ns)); P.oqy.push_back(take(g.ns)); }
   for (int k = 0; k < L; ++k) { P.nlx.push_back(take(g.nu)); P.nly.push_back(take(g.nv)); }
   P.hx = take(g.nu); P.hy = take(g.nv);
@@ -522,17 +520,10 @@ static int pressure_setup(Ctx* c) {
   P.Wd = take(4 * (size_t)p_pad(m / 2) * p_pad(m / 2));   // 2 parities x 8 digits x 2 bytes
   P.fold = take(4 * (size_t)p_pad(n) * p_pad(m / 2));
   P.ex = reinterpret_cast<int*>(take(n));
-  // W[j][k] = 2 sin(pi (j+1)(k+1) / (m+1)), the DST-I matrix of length m (symmetric)
+  // the digits of sin(pi (j+1) k / M) 2^kQBits by parity (k_pprod)
   {
-    std::vector<double> W((size_t)m * m), tab(2 * (size_t)(m + 1));
     const long double PI_L = 3.141592653589793238462643383279502884L;
     const long long M = m + 1;
-    for (long long r = 0; r < 2 * M; ++r) tab[r] = (double)(2.0L * sinl(PI_L * (long double)r / (long double)M));
-    for (int j = 0; j < m; ++j)
-      for (int k = 0; k < m; ++k)   // sin(pi r / M) is 2M-periodic in r
-        W[(size_t)j * m + k] = tab[((long long)(j + 1) * (k + 1)) % (2 * M)];
-    IB_CUDA_CHECK(cudaMemcpy(P.W, W.data(), 8 * W.size(), cudaMemcpyHostToDevice));
-    // the digits of sin(pi (j+1) k / M) 2^kQBits by parity (k_pprod)
     const int H = m / 2, Hp = p_pad(H);
     std::vector<int> digit(2 * (size_t)M * kDigits);
     for (long long r = 0; r < 2 * M; ++r) {
@@ -676,23 +667,41 @@ int op_pressure(Ctx* c) {
   return IB_OK;
 }
 
-// Average device time (ms) of the pressure grid's x transform (n x m times the m x m DST-I
-// matrix) on the FP64 tensor cores (mma) or with FP64 FMAs, over reps launches on inputs
-// cycling through fields larger than L2 in total.
-int op_time_pressure_transform(Ctx* c, bool mma, int reps, double* avg_ms) {
+// W[j][k] = 2 sin(pi (j+1)(k+1) / (m+1)), the DST-I matrix of length m (symmetric), into m x m doubles of
+// device memory: what the FP64 products that op_time_pressure_transform times multiply by
+static int sine_matrix(int m, double* dev) {
+  std::vector<double> W((size_t)m * m), tab(2 * (size_t)(m + 1));
+  const long double PI_L = 3.141592653589793238462643383279502884L;
+  const long long M = m + 1;
+  for (long long r = 0; r < 2 * M; ++r) tab[r] = (double)(2.0L * sinl(PI_L * (long double)r / (long double)M));
+  for (int j = 0; j < m; ++j)
+    for (int k = 0; k < m; ++k)   // sin(pi r / M) is 2M-periodic in r
+      W[(size_t)j * m + k] = tab[((long long)(j + 1) * (k + 1)) % (2 * M)];
+  IB_CUDA_CHECK(cudaMemcpy(dev, W.data(), 8 * W.size(), cudaMemcpyHostToDevice));
+  IB_CUDA_CHECK(cudaDeviceSynchronize());   // the pageable copy has landed
+  return IB_OK;
+}
+
+// Average device time (ms) of the pressure grid's x transform, over reps launches on inputs cycling through
+// fields larger than L2 in total: as the pressure runs it (kind 6), or as the product of the n x m cells and
+// the m x m DST-I matrix on the FP64 tensor cores (2) or with FP64 FMAs (3).
+int op_time_pressure_transform(Ctx* c, int kind, int reps, double* avg_ms) {
   RC(pressure_setup(c));
   const int m = c->g.m, n = c->g.n;
-  const size_t cells = (size_t)m * n;
+  const size_t cells = (size_t)m * n, wn = kind == 6 ? 0 : (size_t)m * m;
   int dev = 0, l2 = 0;
   IB_CUDA_CHECK(cudaGetDevice(&dev));
   IB_CUDA_CHECK(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
   const int nbuf = std::max(2, (int)((2 * (size_t)l2 + 8 * cells - 1) / (8 * cells)));
   double* buf = nullptr;
-  IB_CUDA_CHECK(cudaMalloc(&buf, 2 * 8 * cells * nbuf));
+  IB_CUDA_CHECK(cudaMalloc(&buf, 8 * (2 * cells * nbuf + wn)));
+  double* W = buf + 2 * cells * nbuf;
   int rc = cudaMemsetAsync(buf, 0x3f, 2 * 8 * cells * nbuf, c->st) == cudaSuccess ? IB_OK : IB_ERR_CUDA;
+  if (rc == IB_OK && wn) rc = sine_matrix(m, W);
   auto run = [&](int i) {
     double* in = buf + (size_t)(2 * (i % nbuf)) * cells;
-    return launch_pgemm(mma, n, m, m, in, m, c->pres.W, m, in + cells, m, c->st);
+    if (kind == 6) return p_transform(c, in, in + cells);
+    return launch_pgemm(kind == 2, n, m, m, in, m, W, m, in + cells, m, c->st);
   };
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (rc == IB_OK && (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess)) rc = IB_ERR_CUDA;

@@ -315,7 +315,8 @@ int ib_get_stream(IbCtx* ctx, void** stream);
  * predictor's fused nonlinear + rot stencil of every level on the context's current fields
  * (operators_fluid.F90:553-587, 203-233), with plain loads (4) or with its tiles' rows staged by
  * bulk copies (5; IB_ERR_STATE if its output differs from kind 4's in any bit), each launch
- * after a write of twice the L2 size. */
+ * after a write of twice the L2 size.  Kind 6: the pressure grid's x transform as
+ * ib_calculate_pressure runs it, timed as kinds 2 and 3 are. */
 int ib_time_pass(IbCtx* ctx, int kind, int reps, double* avg_ms);
 /* device time (ms, summed over reps back-to-back applications) of the 8 stages of the Schur
  * operator: reg+rot, ainv, coarsify, coarse levels, finest forward, finest solve, finest

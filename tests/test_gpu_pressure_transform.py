@@ -101,3 +101,11 @@ def test_transform_exponents(m):
         assert np.isnan(w[3]).all()
         assert np.array_equal(np.delete(w, 3, 0), np.delete(y, 3, 0))
     g.close()
+
+
+def test_timing_of_the_transform_that_runs():
+    g = _sim(128, 64)
+    assert g.time_pass(6, 3) > 0.0
+    with pytest.raises(G.IbError, match="ARG"):
+        g.time_pass(7, 3)
+    g.close()
