@@ -502,8 +502,8 @@ static int pressure_setup(Ctx* c) {
   const size_t tri_n = tri_table_doubles(m, tri_t);
   const size_t dbl = tri_n + 2 * (size_t)L * cells + cells + 2 * (size_t)L * g.ns +
                      (size_t)L * (g.nu + g.nv) + g.nu + g.nv + (size_t)std::max(c->nf, 1) + 2 * (size_t)g.nbc +
-                     2 * (size_t)(m + n) + 64 + 4 * (size_t)p_pad(m / 2) * p_pad(m / 2) +
-                     4 * (size_t)p_pad(n) * p_pad(m / 2) + (size_t)n + 16;
+                     2 * (size_t)(m + n) + 4 * (size_t)p_pad(m / 2) * p_pad(m / 2) +
+                     4 * (size_t)p_pad(n) * p_pad(m / 2) + (size_t)n + 3 * (size_t)(6 * L + 11);   // 3: take's rounding
   IB_CUDA_CHECK(cudaMalloc(&P.mem, 8 * dbl));
   IB_CUDA_CHECK(cudaMemset(P.mem, 0, 8 * dbl));
   double* q = P.mem;
