@@ -767,25 +767,31 @@ int op_adjoint_forward(Ctx* c, int nsteps, int K, const double* frames, double* 
   A.frames.assign(frames, frames + 3 * (size_t)nsteps);
   A.it_ckpt.assign(nseg + 1, 0);
   A.ready = false;
-  for (int n = 0; n < nsteps; ++n) {
+  auto step = [&](int n) -> int {
     if (n % K == 0) {
       RC(save_state(c, A.ckpt + sd * (n / K)));
       A.it_ckpt[n / K] = c->itime;
     }
     RC(set_frame(c, frames + 3 * (size_t)n));
     RC(op_advance(c));
-    RC(launch_force_coeffs(c->nf, c->nbody, c->comp, c->bid, c->f, c->p.dt, c->delta, c->forces, c->st,
-                           fdev + 2 * (size_t)n * c->nbody, nullptr, 0));
+    return launch_force_coeffs(c->nf, c->nbody, c->comp, c->bid, c->f, c->p.dt, c->delta, c->forces, c->st,
+                               fdev + 2 * (size_t)n * c->nbody, nullptr, 0);
+  };
+  int rc = IB_OK, done = 0;
+  while (done < nsteps && (rc = step(done)) == IB_OK) ++done;
+  if (rc == IB_OK) {
+    rc = save_state(c, A.ckpt + sd * nseg);
+    A.it_ckpt[nseg] = c->itime;
   }
-  RC(save_state(c, A.ckpt + sd * nseg));
-  A.it_ckpt[nseg] = c->itime;
-  std::vector<double> fc(2 * (size_t)nsteps * c->nbody);
+  // the coefficients of the steps that ended well, also where a later one did not
+  std::vector<double> fc(2 * (size_t)done * c->nbody);
   IB_CUDA_CHECK(cudaMemcpyAsync(fc.data(), fdev, 8 * fc.size(), cudaMemcpyDeviceToHost, c->st));
   IB_CUDA_CHECK(cudaStreamSynchronize(c->st));
-  for (int n = 0; n < nsteps; ++n)
+  for (int n = 0; n < done; ++n)
     for (int b = 0; b < c->nbody; ++b)
       for (int q = 0; q < 2; ++q)
         forces[((size_t)n * c->nbody + b) * 2 + q] = fc[(2 * (size_t)n + q) * c->nbody + b];
+  RC(rc);
   A.ready = true;
   return IB_OK;
 }
@@ -806,7 +812,6 @@ int op_adjoint_backward(Ctx* c, const double* dforces, double* dframes, std::str
   IB_CUDA_CHECK(cudaMemsetAsync(A.lro[0], 0, 8 * (size_t)L * g.ns, c->st));
   IB_CUDA_CHECK(cudaMemsetAsync(A.lqx[0], 0, 8 * (size_t)L * g.nu, c->st));
   IB_CUDA_CHECK(cudaMemsetAsync(A.lqy[0], 0, 8 * (size_t)L * g.nv, c->st));
-  const bool graphs = c->use_whole_step;
   for (int seg = A.nseg - 1; seg >= 0; --seg) {
     const int n0 = seg * A.K, n1 = std::min(A.nsteps, n0 + A.K);
     // recompute the segment from its checkpoint, taping each step's inputs
@@ -824,7 +829,6 @@ int op_adjoint_backward(Ctx* c, const double* dforces, double* dframes, std::str
                 A.dframe + 3 * (size_t)n));
     }
   }
-  (void)graphs;
   IB_CUDA_CHECK(cudaMemcpyAsync(dframes, A.dframe, 24 * (size_t)A.nsteps, cudaMemcpyDeviceToHost, c->st));
   // the context continues from the end of the forward
   RC(load_state(c, A.ckpt + sd * A.nseg));

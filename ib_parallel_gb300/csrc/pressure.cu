@@ -620,8 +620,8 @@ int op_pressure(Ctx* c) {
     }
     const double d = c->delta * (double)(1 << k);
     count_launch();
-    k_p_corner2edge<<<cdiv(g.nu + g.nv, B), B, 0, st>>>(g, P.oqx[k], P.oqy[k], P.ubc, P.vbc, 2.0 * (d * d), 0.5 / (d * d),
-                                                        P.nlx[k], P.nly[k]);
+    k_p_corner2edge<<<cdiv(g.nu + g.nv, B), B, 0, st>>>(g, P.oqx[k], P.oqy[k], P.ubc, P.vbc, 2.0 * (d * d),
+                                                        0.5 / (d * d), P.nlx[k], P.nly[k]);
   }
   // -D E^T f / dt on the finest level, restricted onto the coarser ones, then D N(q) added
   IB_CUDA_CHECK(cudaMemsetAsync(P.rhs[0], 0, 8 * cells, st));

@@ -32,8 +32,8 @@ namespace ib {
 
 static constexpr size_t kStaticDoubles = size_t(1) << 21;  // 16 MiB: the limit callers are given
 // Room for the transform's fixed-point tables, which take 2.5 (m/2) doubles more than the doubles the
-// limit counts; grids whose lines fit a CTA's shared memory (24 m bytes) need no more.
-static constexpr size_t kTableSlack = 16384;
+// limit counts: enough for every line that fits a CTA's shared memory (16 m bytes of 227 KB: m to 14500).
+static constexpr size_t kTableSlack = 18432;
 
 static __device__ __align__(256) double g_ctci_scratch[kStaticDoubles + kTableSlack];
 
