@@ -150,7 +150,10 @@ int beam_build(Ctx* c, const IbBody* bodies, int nbody, std::string* msg) {
   c->nbeam = (int)hdev.size();
   c->beams_h = hdev;
   if (c->nbeam > 0) {
-    if (cudaMalloc(&c->beams, sizeof(BeamDev) * c->nbeam + sizeof(double)) != cudaSuccess) { *msg = "beam allocation failed"; return IB_ERR_NOMEM; }
+    if (cudaMalloc(&c->beams, sizeof(BeamDev) * c->nbeam + sizeof(double)) != cudaSuccess) {
+      *msg = "beam allocation failed";
+      return IB_ERR_NOMEM;
+    }
     c->beam_err = (double*)(c->beams + c->nbeam);
     if (cudaMemcpy(c->beams, hdev.data(), sizeof(BeamDev) * c->nbeam, cudaMemcpyHostToDevice) != cudaSuccess)
       return IB_ERR_CUDA;
@@ -202,7 +205,8 @@ __device__ __forceinline__ double beam_lane_sum(double s) {
 }
 
 // y = A x for a dense matrix, kBeamLanes lanes a row; every thread of the CTA calls it
-__device__ __forceinline__ void beam_dense(const double* __restrict__ A, int rows, int cols, const double* x, double* y) {
+__device__ __forceinline__ void beam_dense(const double* __restrict__ A, int rows, int cols, const double* x,
+                                           double* y) {
   const int l = threadIdx.x % kBeamLanes;
   for (int r0 = 0; r0 < rows; r0 += kBeamThreads / kBeamLanes) {
     const int r = r0 + threadIdx.x / kBeamLanes;

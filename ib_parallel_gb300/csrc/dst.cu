@@ -611,6 +611,8 @@ __global__ void __launch_bounds__(512, 2) k_dst_x(DstDev pl, int nrows, int ld, 
 // the first two groups alone (sd and edge null); a caller that reads sd and edge only launches the
 // second group empty (nbt 0, ring null).  What bounds it is FP64: the bottom and top vertices are a
 // quarter of its dot products at 800 x 400.
+// The solve launched next may read the modes behind its right-hand side before it waits for this kernel
+// (TriBc::early): so every thread here waits first, and none triggers dependents early.
 // 4 against 8 warps: 401 CTAs against 187 at 800 x 400, so no SM has twice its share; 7.6 against 7.9 us
 // (8.2 before the two edge sums of a mode shared one reduction, warp_sum2)
 constexpr int kReWarps = 4;
@@ -868,7 +870,8 @@ int dst_x_bc_modes(const DstPlan& px, const GridDims& g, const double* ring, con
   const int nblk = nEdge + cdiv(std::max(0, g.nsy - 2), kRowsPerCta);
   DstDev d = to_dev(px);
   count_launch();
-  k_dst_bc_modes<<<nblk, 256, smem, st>>>(d, g, ring, W, sk2, post_add, post_scale, out, nEdge, fft_edges ? 1 : 0, LineShape(1, 256));
+  k_dst_bc_modes<<<nblk, 256, smem, st>>>(d, g, ring, W, sk2, post_add, post_scale, out, nEdge, fft_edges ? 1 : 0,
+                                          LineShape(1, 256));
   IB_CUDA_CHECK(cudaGetLastError());
   return IB_OK;
 }
@@ -942,7 +945,9 @@ static int launch_cfg(K kern, size_t smem) {
 
 int dst_pass_x(const DstPlan& px, int nrows, int ld, DstPre pre, const DstXArgs& a, const GridDims& g,
                const DstLaunch& L, cudaStream_t st) {
-  if (L.B > kMaxLines || L.NT > 32 * kMaxWarps || a.nlev < 0 || a.nlev > kMaxBatch || (a.nlev && pre != PRE_COPY && pre != PRE_PRED)) return IB_ERR_ARG;
+  if (L.B > kMaxLines || L.NT > 32 * kMaxWarps || a.nlev < 0 || a.nlev > kMaxBatch ||
+      (a.nlev && pre != PRE_COPY && pre != PRE_PRED))
+    return IB_ERR_ARG;
   DstDev d = to_dev(px);
   size_t smem = dst_smem_x(px, L.B);
   dim3 grid(cdiv(a.nlines ? a.nlines : nrows, L.B), a.nlev ? a.nlev : 1);

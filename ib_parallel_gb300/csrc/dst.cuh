@@ -103,7 +103,7 @@ struct DstPlan {
   double* sn = nullptr;    // P+1: sin(j pi / M)
 };
 
-// Launch geometry of one pass (chosen by the tuner in dst.cu).
+// Launch geometry of one pass (chosen by the tuner in solver.cu).
 struct DstLaunch {
   int B = 1;       // lines per CTA
   int NT = 128;    // threads per CTA

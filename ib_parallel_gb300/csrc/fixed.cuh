@@ -44,9 +44,9 @@ inline FxW fx_factor(long double w) {
   return r;
 }
 
-// x w, |x| < 2^60, to within 0.75 of a unit: the product of the low halves is left out (at most a
-// quarter of a unit, of zero mean: both halves are balanced, so nothing adds up along the prefix
-// sums).  Three 32 x 32 + 64-bit multiply-adds.
+// x w, |x| below 2^61 (4 x and the carry of its halves fit), to within 0.75 of a unit: the product of
+// the low halves is left out (at most a quarter of a unit, of zero mean: both halves are balanced, so
+// nothing adds up along the prefix sums).  Three 32 x 32 + 64-bit multiply-adds.
 IB_FX fx fx_mul(fx x, int whi, int wlo) {
   const fx x4 = (fx)((unsigned long long)x << 2);
   const int lo = (int)(unsigned)(unsigned long long)x4;

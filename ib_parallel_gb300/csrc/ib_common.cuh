@@ -107,8 +107,12 @@ struct FastDiv {
 
 // Programmatic dependent launch: in the captured step graphs the edges between kernels are
 // programmatic (make_edges_programmatic), so a kernel's CTAs may be scheduled while its
-// predecessor finishes.  Every kernel of this library therefore waits here, first thing, for
-// its predecessor's completion and memory; launched without such an edge it returns at once.
+// predecessor finishes.  Every kernel of this library therefore waits here, on every thread and before
+// it reads what a kernel wrote or writes anything, for its predecessor's completion and memory; launched
+// without such an edge it returns at once.  None triggers its dependents early.  So when a kernel starts,
+// every thread of its predecessor has passed this wait, and what the kernels before that one wrote is
+// complete: the tridiagonal solves read constant tables, and with TriBc::early their right-hand sides,
+// ahead of the wait.
 #define IB_GRID_DEP_WAIT() asm volatile("griddepcontrol.wait;" ::: "memory")
 
 // Number of kernels this library has launched (all contexts), for the benchmark's

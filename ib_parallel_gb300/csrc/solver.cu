@@ -333,7 +333,8 @@ int ctx_create(const IbParams* pin, const IbBody* bodies, int nbody, Ctx** out, 
     int rc2 = tri_build(&c->tri_ctci, g.nsx, g.nsy, tri_t, lamx.data(), 1.0 / (2.0 * g.m), tri_mem);
     double c1 = c->cvis[0];
     for (int k = 0; k < g.nsx; ++k) shift[k] = lamx[k] + 1.0 / c1;
-    if (rc2 == IB_OK) rc2 = tri_build(&c->tri_ainv, g.nsx, g.nsy, tri_t, shift.data(), 1.0 / (2.0 * g.m * c1), tri_mem + tri_n);
+    if (rc2 == IB_OK)
+      rc2 = tri_build(&c->tri_ainv, g.nsx, g.nsy, tri_t, shift.data(), 1.0 / (2.0 * g.m * c1), tri_mem + tri_n);
     c->tri_pred.resize(L);
     for (int k = 0; k < L && rc2 == IB_OK; ++k) {
       double ck = c->cvis[k];

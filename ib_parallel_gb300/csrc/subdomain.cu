@@ -342,11 +342,11 @@ __device__ __forceinline__ double b_at(const long long* __restrict__ colptr, con
 // takes 32 entries l of column k: its threads find the 16 B entries of each (binary searches in
 // the columns, the latency) and their products, then one warp sums each entry in the order above.
 constexpr int kLumatRows = 32;
-__global__ void __launch_bounds__(kLumatRows * 16) k_sd_lumat(int nf, const int* __restrict__ pidx, const double* __restrict__ pw,
-                                                  const long long* __restrict__ colptr, const int* __restrict__ nz,
-                                                  const int* __restrict__ rows, const double* __restrict__ vals,
-                                                  const double* __restrict__ brv, const double* __restrict__ bco,
-                                                  const int* __restrict__ bod, double* __restrict__ St) {
+__global__ void __launch_bounds__(kLumatRows * 16)
+    k_sd_lumat(int nf, const int* __restrict__ pidx, const double* __restrict__ pw,
+               const long long* __restrict__ colptr, const int* __restrict__ nz, const int* __restrict__ rows,
+               const double* __restrict__ vals, const double* __restrict__ brv, const double* __restrict__ bco,
+               const int* __restrict__ bod, double* __restrict__ St) {
   IB_GRID_DEP_WAIT();
   __shared__ double prod[kLumatRows][17];
   const int k = blockIdx.y, l0 = blockIdx.x * kLumatRows;
@@ -831,8 +831,9 @@ int launch_sd_lumat(Ctx* c, cudaStream_t st) {
   SubDomain& S = c->sd;
   Influence& I = c->inf;
   count_launch();
-  k_sd_lumat<<<dim3(cdiv(c->nf, kLumatRows), c->nf), kLumatRows * 16, 0, st>>>(c->nf, S.pidx, S.pw, S.colptr, S.nz, S.rows,
-                                                                   S.vals, I.brv, I.bco, I.bod, I.St);
+  const dim3 grid(cdiv(c->nf, kLumatRows), c->nf);
+  k_sd_lumat<<<grid, kLumatRows * 16, 0, st>>>(c->nf, S.pidx, S.pw, S.colptr, S.nz, S.rows, S.vals, I.brv, I.bco,
+                                               I.bod, I.St);
   IB_CUDA_CHECK(cudaGetLastError());
   return launch_beam_add_b(c, I.St, st);
 }

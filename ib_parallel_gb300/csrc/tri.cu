@@ -55,10 +55,10 @@ TriShape tri_chunking_even(int n, int nx) {
 }
 
 // Of the lengths with a register kernel, the cheapest; a shorter last chunk counts a tenth more (its
-// rows are predicated), and 63 rows, which spill, are taken only where no shorter chunk will do.  The shared-memory kernel took 37 us for 999 modes of 539 rows in its cheapest
-// equal chunks (15 of 35) and 160 us for 800 modes of 400 rows, whose period 401 is prime (one chunk);
-// in 14 chunks of 39 the first takes 19 us, and the second in 13 of 31 12 us.  It remains for more than
-// 32 x 64 rows.
+// rows are predicated), and 63 rows, which spill, are taken only where no shorter chunk will do.  The
+// shared-memory kernel took 37 us for 999 modes of 539 rows in its cheapest equal chunks (15 of 35) and
+// 160 us for 800 modes of 400 rows, whose period 401 is prime (one chunk); in 14 chunks of 39 the first
+// takes 19 us, and the second in 13 of 31 12 us.  It remains for more than 32 x 64 rows.
 TriShape tri_chunking(int ny, int nx, size_t max_doubles) {
   TriShape best;
   double bestc = -1.0;
@@ -442,8 +442,9 @@ __global__ void __launch_bounds__(256, 2) k_tri_reg_batch(const __grid_constant_
 }
 
 static size_t tri_reg_smem(const TriOp& op, int Mb) {
-  return sizeof(double) * (size_t)Mb * ((op.r < op.s ? 4 : 3) * (size_t)op.s + 2 * (size_t)op.C + 2 * ((size_t)op.C + 1) +
-                                             (size_t)op.C * std::max(op.C - 1, 1));
+  return sizeof(double) * (size_t)Mb *
+         ((op.r < op.s ? 4 : 3) * (size_t)op.s + 2 * (size_t)op.C + 2 * ((size_t)op.C + 1) +
+          (size_t)op.C * std::max(op.C - 1, 1));
 }
 
 template <int S, bool TAIL>

@@ -106,7 +106,8 @@ def load(path: Optional[os.PathLike] = None):
         "ib_nonlinear": ([P, P, P, P, P, P, P], C.c_int), "ib_rot": ([P, P, P, P], C.c_int),
         "ib_curl": ([P, P, P, P, P], C.c_int), "ib_coarsify": ([P, P, P], C.c_int),
         "ib_get_bc": ([P, P, C.c_double, P], C.c_int), "ib_apply_bc": ([P, P, P, C.c_double], C.c_int),
-        "ib_dst": ([P, P, P], C.c_int), "ib_pressure_transform": ([P, P, P], C.c_int), "ib_ctci": ([P, P, P], C.c_int), "ib_ainv": ([P, P], C.c_int),
+        "ib_dst": ([P, P, P], C.c_int), "ib_pressure_transform": ([P, P, P], C.c_int),
+        "ib_ctci": ([P, P, P], C.c_int), "ib_ainv": ([P, P], C.c_int),
         "ib_fluid_predictor": ([P, C.c_int, P, P, P, P], C.c_int),
         "ib_vort2flux": ([P, P, P, P, P], C.c_int), "ib_reg_prep": ([P, P, P], C.c_int),
         "ib_reg": ([P, P, P, P], C.c_int), "ib_regT": ([P, P, P, P], C.c_int),
@@ -388,7 +389,8 @@ class Simulation:
         return s.value or 0
 
     def time_pass(self, kind: int, reps: int = 20) -> float:
-        """Average device ms of one full x pass (0) or tridiagonal solve (1) timed alone."""
+        """Average device ms of one full x pass (0), tridiagonal solve (1), pressure transform as it
+        runs (6) or as FP64 products (2, 3), or nonlinear stencil (4, 5), timed alone."""
         ms = C.c_double()
         _check(self.lib.ib_time_pass(self.h, kind, reps, C.byref(ms)), "ib_time_pass")
         return ms.value
@@ -567,7 +569,8 @@ class Simulation:
 
     def pressure_transform(self, x):
         out = np.empty((self.params.n, self.params.m))
-        _check(self.lib.ib_pressure_transform(self.h, _ptr(np.ascontiguousarray(x)), _ptr(out)), "ib_pressure_transform")
+        _check(self.lib.ib_pressure_transform(self.h, _ptr(np.ascontiguousarray(x)), _ptr(out)),
+               "ib_pressure_transform")
         return out
 
     def ctci(self, x):

@@ -30,7 +30,8 @@ def test_residual_and_error_beside_substitution(m, npts):
         for _ in range(4):
             exact = exact + sla.cho_solve(L, (b - Al @ exact).astype(np.float64))
         for out, x in ((here, g.direct_solve(b)), (there, sla.cho_solve(L, b))):
-            out.append([np.linalg.norm((b - Al @ x).astype(np.float64)), np.linalg.norm((x - exact).astype(np.float64))])
+            out.append([np.linalg.norm((b - Al @ x).astype(np.float64)),
+                        np.linalg.norm((x - exact).astype(np.float64))])
     g.close()
     here, there = np.array(here).sum(axis=0), np.array(there).sum(axis=0)
     assert here[0] <= there[0]   # the residual

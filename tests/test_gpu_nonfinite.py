@@ -23,7 +23,8 @@ BODIES = {
     "plates": [_at(small_plate(), -0.4), _at(small_plate(), 0.4)],
     "beam": [GEO.beam_plate(9, 1.0, 10.0, 0.5, 1e-2)],
     "beam and plate": [_at(GEO.beam_plate(9, 1.0, 10.0, 0.5, 1e-2), -0.4), _at(small_plate(), 0.4)],
-    "rigid and beam": [GEO.cylinder(6, diameter=0.3, xc=1.0, yc=0.5), _at(GEO.beam_plate(9, 1.0, 10.0, 0.5, 1e-2), -0.4)],
+    "rigid and beam": [GEO.cylinder(6, diameter=0.3, xc=1.0, yc=0.5),
+                       _at(GEO.beam_plate(9, 1.0, 10.0, 0.5, 1e-2), -0.4)],
 }
 
 

@@ -42,7 +42,8 @@ KINDS = ["noise", "smooth", "decades", "spike"]
 # tolerance: the folded samples are multiples of 2^-54 E and the sines of 2^-55, E the power of two above the
 # row's peak, and a sum is kept to 2^-52 E: with every rounding at its most 5 units of 2^-53 E for four terms,
 # and as independent errors a sixth of 2.5 sqrt(H) units for H terms; the result's own rounding comes to that
-@pytest.mark.parametrize("m,n", [(8, 12), (60, 8), (64, 36), (72, 8), (1000, 8), (1024, 8), (1080, 8), (2048, 8), (2160, 8)])
+@pytest.mark.parametrize("m,n", [(8, 12), (60, 8), (64, 36), (72, 8), (1000, 8), (1024, 8), (1080, 8), (2048, 8),
+                                 (2160, 8)])
 def test_transform_against_extended_precision(m, n):
     rng = np.random.default_rng(m)
     x = np.concatenate([_rows(k, n // 4, m, rng) for k in KINDS])

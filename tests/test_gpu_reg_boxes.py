@@ -10,8 +10,9 @@ pytestmark = pytest.mark.gpu
 
 
 # tolerance: a face sums at most a few dozen products of weights that agree to 1e-14
-@pytest.mark.parametrize("m,centres", [(64, [(1.0, 0.0)]), (64, [(0.0, 0.0), (4.0, 0.3)]), (320, [(-1.0, -1.0), (4.9, 1.1)]),
-                                       (320, [(1.0, 0.0)]), (320, [(-1.0, 0.0), (0.0, 0.2), (4.9, -0.1)])])
+@pytest.mark.parametrize("m,centres", [(64, [(1.0, 0.0)]), (64, [(0.0, 0.0), (4.0, 0.3)]), (320, [(1.0, 0.0)]),
+                                       (320, [(-1.0, -1.0), (4.9, 1.1)]),
+                                       (320, [(-1.0, 0.0), (0.0, 0.2), (4.9, -0.1)])])
 def test_spread_over_boxes(m, centres):
     o, g = pair(dict(SMALL, m=m, n=m // 2), [GEO.cylinder(17, diameter=0.6, xc=x, yc=y) for x, y in centres])
     h = np.random.default_rng(m).standard_normal(g.nf)
