@@ -718,7 +718,7 @@ static int adjoint_alloc(Ctx* c) {
     std::vector<double> h = frame_flux_host(c, b == 0, b == 1, b == 2, cx, cy);
     IB_CUDA_CHECK(cudaMemcpy(A.bases + b * per_basis, h.data(), 8 * per_basis, cudaMemcpyHostToDevice));
   }
-  return IB_OK;
+  return wait_uploads();
 }
 
 int op_adjoint_forward(Ctx* c, int nsteps, int K, const double* frames, double* forces, std::string* msg) {

@@ -157,7 +157,7 @@ int beam_build(Ctx* c, const IbBody* bodies, int nbody, std::string* msg) {
     c->beam_err = (double*)(c->beams + c->nbeam);
     if (cudaMemcpy(c->beams, hdev.data(), sizeof(BeamDev) * c->nbeam, cudaMemcpyHostToDevice) != cudaSuccess)
       return IB_ERR_CUDA;
-    if (cudaDeviceSynchronize() != cudaSuccess) return IB_ERR_CUDA;
+    RC(wait_uploads());
   }
   return IB_OK;
 }

@@ -205,8 +205,7 @@ int run_level(Ctx* c, int k, const int* items, int n) {
       k_cr_init<<<1, 32, 0, cap>>>(col, i);
       cudaGraphConditionalHandle h = 0;
       cudaGraph_t body = nullptr;
-      if (cudaGraphConditionalHandleCreate(&h, capture_graph(cap), 1, cudaGraphCondAssignDefault) != cudaSuccess)
-        rc = IB_ERR_CUDA;
+      rc = capture_handle(cap, 1, &h);
       if (rc == IB_OK) rc = add_while(cap, h, &body);
       if (rc == IB_OK &&
           cudaStreamBeginCaptureToGraph(sc.st, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) != cudaSuccess)
@@ -385,6 +384,7 @@ int cr_prepare(Ctx* c, const std::vector<unsigned char>& fine_mask) {
     all.insert(all.end(), fresh[k].begin(), fresh[k].end());
   }
   IB_CUDA_CHECK(cudaMemcpy(cr.items, all.data(), sizeof(int) * all.size(), cudaMemcpyHostToDevice));
+  RC(wait_uploads());
   // the slots above now claim responses: if the passes fail, the context stops using them (its
   // later builds run the per-column chain)
   int rc = inf_build_scratch(c);

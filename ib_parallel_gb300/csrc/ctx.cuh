@@ -522,7 +522,7 @@ int op_read_variables(Ctx* c, const char* path, int itime, std::string* msg);
 // graph helpers (solver.cu): a while node after the capture position of st (its body graph
 // returned), the graph st is capturing, and programmatic kernel-to-kernel edges
 int add_while(cudaStream_t st, cudaGraphConditionalHandle h, cudaGraph_t* body);
-cudaGraph_t capture_graph(cudaStream_t st);
+int capture_handle(cudaStream_t st, unsigned dflt, cudaGraphConditionalHandle* h);
 void make_edges_programmatic(cudaGraph_t g);
 // patches + flag for the current weights (async); cleared: the band flag and the touched-vertex
 // flags are already zero (the device FSI loop clears them as it reads them)

@@ -746,10 +746,9 @@ __global__ void k_edge_matrix(int N, int mq, const double* __restrict__ W, doubl
 
 int dst_edge_matrix(const DstPlan& px, const GridDims& g, const double* W, double* E) {
   const long long n = (long long)px.N * ((px.N + 1) / 2);
-  k_edge_matrix<<<(unsigned)cdiv(n, 256), 256>>>(px.N, g.m / 4, W, E);
+  k_edge_matrix<<<(unsigned)cdiv(n, 256), 256, 0, cudaStreamLegacy>>>(px.N, g.m / 4, W, E);
   IB_CUDA_CHECK(cudaGetLastError());
-  IB_CUDA_CHECK(cudaDeviceSynchronize());
-  return IB_OK;
+  return wait_uploads();
 }
 
 

@@ -135,6 +135,14 @@ long long launch_count();
 
 namespace ib {
 
+// Waits for what was copied from pageable memory or cleared through the legacy stream: such a call may
+// return before its DMA has reached the device, and the library's own streams do not wait for that stream.
+// (Not cudaDeviceSynchronize: it fails while any stream of the process captures, and ends that capture.)
+inline int wait_uploads() {
+  IB_CUDA_CHECK(cudaStreamSynchronize(cudaStreamLegacy));
+  return IB_OK;
+}
+
 // Lets kernel `kern` take `bytes` of dynamic shared memory.  The limit is an attribute of the
 // function, shared by every context in the process, and captured graphs launch with the sizes
 // they were captured with: so it is only ever raised, once, to the most the device allows (the

@@ -428,7 +428,7 @@ int inf_alloc(Ctx* c) {
   I.ntx = cdiv(c->g.nsx, kT);
   I.nty = cdiv(c->g.nsy, kT);
   IB_CUDA_CHECK(cudaMalloc(&I.tile_of, sizeof(int) * (size_t)I.ntx * I.nty));
-  return IB_OK;
+  return wait_uploads();
 }
 
 static void free_band(Influence& I) {
@@ -459,6 +459,7 @@ int inf_build_scratch(Ctx* c) {
   // zero outside the centres coarsify writes
   IB_CUDA_CHECK(cudaMemset(I.bmem, 0, 8 * per * S));
   IB_CUDA_CHECK(cudaMemset(I.bint, 0xff, sizeof(int) * Influence::kSetInts * S));   // prev = -1
+  if (wait_uploads() != IB_OK) return IB_ERR_CUDA;
   // ainv's response to a unit vector on row b, (1/c1 + lam_x + T_y)^-1 per x mode, decays
   // away from row b at least as fast as rho^|r-b| with rho + 1/rho = 2 + 1/c1 (the slowest
   // mode, lam_x -> 0); past trunc_rows rows it is below 1e-18 of its peak.  Only the input of
@@ -597,6 +598,7 @@ int inf_build(Ctx* c) {
   IB_CUDA_CHECK(cudaMemcpy(I.tile_of, tile_of.data(), sizeof(int) * tile_of.size(), cudaMemcpyHostToDevice));
   const int rr_out_h[3] = {bmin, bmax + 1, ROW_SKIP};
   IB_CUDA_CHECK(cudaMemcpy(I.rr_out, rr_out_h, sizeof(rr_out_h), cudaMemcpyHostToDevice));
+  if (wait_uploads() != IB_OK) return IB_ERR_CUDA;
   // columns: unit vorticity at each band vertex through the fluid part of the operator.  The
   // columns are independent, and each is a chain of small latency-bound launches: they run on
   // kBuildStreams streams at once, column col on set col % kBuildStreams (its own unit
@@ -652,8 +654,7 @@ int inf_build(Ctx* c) {
       k_inf_col_init<<<1, 32, 0, cap>>>(col, i);
       cudaGraphConditionalHandle h = 0;
       cudaGraph_t body = nullptr;
-      if (cudaGraphConditionalHandleCreate(&h, capture_graph(cap), 1, cudaGraphCondAssignDefault) != cudaSuccess)
-        rc = IB_ERR_CUDA;
+      rc = capture_handle(cap, 1, &h);
       if (rc == IB_OK) rc = add_while(cap, h, &body);
       if (rc == IB_OK &&
           cudaStreamBeginCaptureToGraph(sc.st, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) != cudaSuccess)

@@ -551,7 +551,7 @@ static int pressure_setup(Ctx* c) {
     }
     RC(tri_build(&P.tri, m, n, tri_t, lx.data(), -1.0 / (2.0 * (m + 1)), tri_mem));
   }
-  IB_CUDA_CHECK(cudaDeviceSynchronize());   // the tables' pageable copies have landed
+  RC(wait_uploads());
   P.ready = true;
   return IB_OK;
 }
@@ -678,8 +678,7 @@ static int sine_matrix(int m, double* dev) {
     for (int k = 0; k < m; ++k)   // sin(pi r / M) is 2M-periodic in r
       W[(size_t)j * m + k] = tab[((long long)(j + 1) * (k + 1)) % (2 * M)];
   IB_CUDA_CHECK(cudaMemcpy(dev, W.data(), 8 * W.size(), cudaMemcpyHostToDevice));
-  IB_CUDA_CHECK(cudaDeviceSynchronize());   // the pageable copy has landed
-  return IB_OK;
+  return wait_uploads();
 }
 
 // Average device time (ms) of the pressure grid's x transform, over reps launches on inputs cycling through

@@ -394,7 +394,8 @@ int ctx_create(const IbParams* pin, const IbBody* bodies, int nbody, Ctx** out, 
     IB_CUDA_CHECK(cudaMemcpy(c->bid, c->bid_h.data(), 4 * (size_t)nf, cudaMemcpyHostToDevice));
   }
   if (nt > 0) IB_CUDA_CHECK(cudaMemcpy(c->tb, c->tb_h.data(), sizeof(TorsBody) * nt, cudaMemcpyHostToDevice));
-  rc = launch_tors_consts(nt, c->tb, p.dt, c->delta, c->st);
+  rc = wait_uploads();
+  if (rc == IB_OK) rc = launch_tors_consts(nt, c->tb, p.dt, c->delta, c->st);
   if (rc == IB_OK) rc = launch_tors_trig(nt, c->tb, c->ts, c->st);
   if (rc != IB_OK) { *msg = "device initialisation failed"; ctx_destroy(c); return rc; }
   for (int i = 0; i < nbody; ++i) c->bodies_h.push_back(bodies[i]);
@@ -951,10 +952,11 @@ static int read_ist(Ctx* c) {
 static int add_conditional(cudaStream_t st, cudaGraphConditionalHandle h, cudaGraphConditionalNodeType type,
                            cudaGraph_t* body) {
   cudaStreamCaptureStatus stat;
-  cudaGraph_t capg;
+  cudaGraph_t capg = nullptr;
   const cudaGraphNode_t* deps = nullptr;
   size_t ndeps = 0;
   IB_CUDA_CHECK(cudaStreamGetCaptureInfo(st, &stat, nullptr, &capg, &deps, nullptr, &ndeps));
+  if (stat != cudaStreamCaptureStatusActive || !capg) return IB_ERR_CUDA;
   cudaGraphNodeParams pr = {};
   pr.type = cudaGraphNodeTypeConditional;
   pr.conditional.handle = h;
@@ -971,11 +973,15 @@ int add_while(cudaStream_t st, cudaGraphConditionalHandle h, cudaGraph_t* body) 
   return add_conditional(st, h, cudaGraphCondTypeWhile, body);
 }
 
-cudaGraph_t capture_graph(cudaStream_t st) {
+// A conditional handle of the graph `st` is capturing, `dflt` at each launch.  A capture that a
+// device-wide synchronisation of another thread has ended has no graph.
+int capture_handle(cudaStream_t st, unsigned dflt, cudaGraphConditionalHandle* h) {
   cudaStreamCaptureStatus stat;
   cudaGraph_t g = nullptr;
-  cudaStreamGetCaptureInfo(st, &stat, nullptr, &g, nullptr, nullptr, nullptr);
-  return g;
+  IB_CUDA_CHECK(cudaStreamGetCaptureInfo(st, &stat, nullptr, &g, nullptr, nullptr, nullptr));
+  if (stat != cudaStreamCaptureStatusActive || !g) return IB_ERR_CUDA;
+  IB_CUDA_CHECK(cudaGraphConditionalHandleCreate(h, g, dflt, cudaGraphCondAssignDefault));
+  return IB_OK;
 }
 
 // The Schur operator the Krylov solver applies: the assembled matrix when the influence
@@ -1001,8 +1007,7 @@ static int build_solve_graph(Ctx* c, bool dense) {
     rc = launch_gmres_init(G, st);
     cudaGraphConditionalHandle h_out = 0, h_in = 0;
     cudaGraph_t outer = nullptr, inner = nullptr;
-    if (rc == IB_OK && cudaGraphConditionalHandleCreate(&h_out, capture_graph(st), 1, cudaGraphCondAssignDefault) != cudaSuccess)
-      rc = IB_ERR_CUDA;
+    if (rc == IB_OK) rc = capture_handle(st, 1, &h_out);
     if (rc == IB_OK) rc = add_while(st, h_out, &outer);
     // restart cycle: r = b - A x, V0, then the Arnoldi loop, then x += V y
     if (rc == IB_OK && cudaStreamBeginCaptureToGraph(s1, outer, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) != cudaSuccess)
@@ -1280,8 +1285,7 @@ static int capture_fsi_loop(Ctx* c, cudaStream_t st) {
     k_fsi_loop_init<<<1, 32, 0, st>>>(c->fsi_cnt, I.flag, c->fsi_done);
     cudaGraphConditionalHandle h = 0;
     cudaGraph_t body = nullptr;
-    if (cudaGraphConditionalHandleCreate(&h, capture_graph(st), 1, cudaGraphCondAssignDefault) != cudaSuccess)
-      rc = IB_ERR_CUDA;
+    rc = capture_handle(st, 1, &h);
     if (rc == IB_OK) rc = add_while(st, h, &body);
     if (rc == IB_OK && cudaStreamBeginCaptureToGraph(s1, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) !=
                            cudaSuccess)
@@ -1617,9 +1621,7 @@ static int build_step_graph(Ctx* c, int mode) {
       I.patch_fresh = fresh;   // what the capture recorded on the host for an iteration it did not run
       I.active = active;
       loop_launches = launch_count() - b0;
-      if (rc == IB_OK &&
-          cudaGraphConditionalHandleCreate(&h, capture_graph(st), 0, cudaGraphCondAssignDefault) != cudaSuccess)
-        rc = IB_ERR_CUDA;
+      if (rc == IB_OK) rc = capture_handle(st, 0, &h);
       if (rc == IB_OK) {
         count_launch();
         k_step_gate<<<1, 1, 0, st>>>(c->fsi_cnt, c->err_fsi, p.fsi_tol, p.fsi_max_it, h);

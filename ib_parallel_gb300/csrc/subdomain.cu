@@ -725,8 +725,7 @@ int sd_precompute(Ctx* c) {
       k_sd_col_init<<<1, 32, 0, cap>>>(col, i);
       cudaGraphConditionalHandle h = 0;
       cudaGraph_t body = nullptr;
-      if (cudaGraphConditionalHandleCreate(&h, capture_graph(cap), 1, cudaGraphCondAssignDefault) != cudaSuccess)
-        rc = IB_ERR_CUDA;
+      rc = capture_handle(cap, 1, &h);
       if (rc == IB_OK) rc = add_while(cap, h, &body);
       if (rc == IB_OK &&
           cudaStreamBeginCaptureToGraph(sc.st, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) != cudaSuccess)
@@ -984,6 +983,7 @@ int sd_read(Ctx* c, const char* path, std::string* msg) {
   }
   IB_CUDA_CHECK(cudaMemcpy(S.colptr, colptr.data(), 8 * colptr.size(), cudaMemcpyHostToDevice));
   IB_CUDA_CHECK(cudaMemcpy(S.nz, nz.data(), 4 * nz.size(), cudaMemcpyHostToDevice));
+  RC(wait_uploads());
   S.kept = (long long)vals.size();
   S.ready = true;
   return IB_OK;
