@@ -167,12 +167,16 @@ def _check(rc: int, what: str = ""):
 
 
 def _ptr(a):
-    """Pointer of a float64 numpy array (host) or a CUDA tensor (device)."""
+    """Pointer of a float64 numpy array (host) or a CUDA tensor (device).  It holds the array: the copy
+    that ascontiguousarray makes of a strided or converted argument lives until the call returns."""
     if hasattr(a, "data_ptr"):
-        return C.c_void_p(a.data_ptr())
-    if not (isinstance(a, np.ndarray) and a.dtype == np.float64 and a.flags["C_CONTIGUOUS"]):
+        p = C.c_void_p(a.data_ptr())
+    elif isinstance(a, np.ndarray) and a.dtype == np.float64 and a.flags["C_CONTIGUOUS"]:
+        p = C.c_void_p(a.ctypes.data)
+    else:
         raise TypeError("arrays must be C-contiguous float64 numpy arrays or CUDA tensors")
-    return C.c_void_p(a.ctypes.data)
+    p.array = a
+    return p
 
 
 def launch_count() -> int:
