@@ -296,9 +296,9 @@ __global__ void __launch_bounds__(128) k_sd_interp(InterpArgs a) {
   const bool row = i >= 2;
   const double z = row ? a.yb[k] : a.xb[k], s0 = row ? a.sdyi : a.sdxi;
   const double fz = __dadd_rn(__ddiv_rn(__dsub_rn(z, s0), d), 1.0);
-  int c = (int)fz;   // Fortran INT (toward zero)
+  int c = (int)fz;   // Fortran INT (toward zero); a point far outside takes the largest int
   const int n = row ? a.ny : a.nx;
-  if (c < 1 || c + 1 > n) {
+  if (c < 1 || c >= n) {
     if (live && rp < 0) atomicExch(a.err, IB_ERR_DOMAIN);
     c = min(max(c, 1), n - 1);
   }
