@@ -609,9 +609,9 @@ int launch_symmetrise(int n, double* M, double* F, cudaStream_t st) {
 // x = M^-1 b: the two products with the inverse factor, then one step of refinement.  The substitutions by
 // blocks of 32 that the products replaced ran on one CTA, 2 n / 32 dependent triangles: 304 us for the 314
 // unknowns of the 157-point cylinder, against 7 us for the two products and 18 us for the five launches.  Products
-// with an inverse alone are not backward stable: at 196 to 314 unknowns their residual was 2 to 10 times the
-// substitutions', their error up to 4 times.  The refinement, with the residual in two parts, leaves an
-// error of the result's last place, below the substitutions'.
+// with an inverse alone are not backward stable: at 130 to 314 unknowns their residual was up to 10 times the
+// substitutions', their error up to 20 times, by right-hand side.  The refinement, with the residual in two
+// parts, leaves an error of the result's last place, below the substitutions'.
 int launch_chol_solve(int n, const double* M, const double* Z, const double* b, double* y, double* r, double* x,
                       cudaStream_t st) {
   const int blocks = cdiv(n, kTriRows), threads = 32 * kTriRows;
