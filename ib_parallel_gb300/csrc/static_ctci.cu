@@ -11,8 +11,7 @@
 //
 // Set-up: the first call on a device, and the first call after the grid size changes,
 // looks up the array's device address, fills the tables with host-to-device copies and waits
-// for the device to finish them (cudaDeviceSynchronize); make that call before any stream
-// capture.  Later calls with the same grid only
+// for them; make that call before any stream capture of its own thread.  Later calls with the same grid only
 // launch three kernels on the caller's stream and return without waiting for them.
 //
 // Every call on a device shares the one array, which keeps what the last call left there.
@@ -138,8 +137,8 @@ int static_ctci(int m, int n, const double* vort, double* s, cudaStream_t st) {
       if (rc != IB_OK) { set_last_error("ib_ctci_static: table upload failed"); return rc; }
       // tri_build copies from pageable host memory, and such a copy may return before its DMA
       // has reached the device; the solve kernels run on the caller's stream, which nothing
-      // orders after that copy.  Wait for it here (set-up runs outside any stream capture).
-      if (cudaDeviceSynchronize() != cudaSuccess) {
+      // orders after that copy.  Wait for it here.
+      if (wait_uploads() != IB_OK) {
         set_last_error("ib_ctci_static: table upload failed");
         return IB_ERR_CUDA;
       }

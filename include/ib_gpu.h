@@ -267,7 +267,7 @@ int ib_ctci(IbCtx* ctx, const double* vort, double* s);
  * loading the library keeps until the process exits: grids needing more ((m-1)(n-1) plus the
  * tables; 1200 x 600 fits, 1280 x 640 does not) fail with IB_ERR_ARG.  The first call on a
  * device, and the first after the grid size changes, does the set-up: it copies the tables and
- * waits for the whole device (cudaDeviceSynchronize), so make it before any stream capture.
+ * waits for them, so make it before any stream capture of its own thread.
  * All calls on a device share the array: calls whose kernels overlap on the GPU race and give
  * wrong results.  Errors are reported through ib_last_error(). */
 int ib_ctci_static(int m, int n, const double* vort, double* s, void* stream);
